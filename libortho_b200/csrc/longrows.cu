@@ -77,7 +77,7 @@ long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int st = 0; uint32_t ph = 0;
             for (int kb = kb0; kb < kb1; kb++) {
                 wait(&sm->empty[st], ph ^ 1u);
@@ -88,7 +88,7 @@ long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(TR, TT);
             const uint64_t adesc0 = umma_desc_sw128(smem_u32(as)), bdesc0 = umma_desc_sw128(smem_u32(bs));
             int st = 0; uint32_t ph = 0;

@@ -158,7 +158,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             int xi = 0, wi = 0; uint32_t xph = 0, wph = 0;
             long long pos = r_begin; Seg sg;
             while (next_seg(pos, sg)) {
@@ -178,7 +178,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(TMK, TN);
             const uint64_t adesc0 = umma_desc_sw128(smem_u32(xs));
             const uint64_t bdesc0 = umma_desc_sw128(smem_u32(bsm));

@@ -176,7 +176,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0, wsi = 0; uint32_t ph = 0, wph = 0;
             for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
                 const Unit un = unit_of(p, u);
@@ -197,7 +197,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(TH, TM);
             const uint64_t desc0 = umma_desc_sw128(smem_u32(xs));     // stage s, k step kk: + s*X_BYTES/16 + 2*kk
             int s = 0, as = 0; uint32_t ph = 0, aph = 0;

@@ -94,6 +94,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
     return false;
 }
 
+// True in exactly one lane of a converged warp.  A warp role that issues TMA or tcgen05 instructions is entered with
+// this and not with `lane == 0`: elect.sync tells the compiler that one lane is active, so the instructions' uniform
+// operands are moved once; under a lane test every tcgen05 instruction is wrapped in code that makes its operands
+// uniform again (185 cycles per tcgen05.mma in a rolled loop against 16 for a 128 x 32 x 16 one issued this way).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 // one 2-D tiled TMA load into this CTA's shared memory; x = innermost (column) coordinate
 __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *map, uint64_t *bar, int x, int y) {
     asm volatile(
