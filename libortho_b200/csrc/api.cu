@@ -5,6 +5,8 @@
 // reference dispatcher it never synchronises the device and it reports failures as status
 // codes instead of dropping them.
 #include <atomic>
+#include <chrono>
+#include <random>
 
 #include "common.cuh"
 
@@ -46,6 +48,22 @@ int device_sm_count(int dev)
         cached[dev].store(n, std::memory_order_relaxed);
     }
     return n;
+}
+
+// Counter values behind a bijective mix (the finaliser of Steele, Lea and Flood's SplitMix), from a starting point
+// that differs from process to process.
+unsigned long long next_launch_tag()
+{
+    static std::atomic<unsigned long long> counter{[]() -> unsigned long long {
+        unsigned long long v = (unsigned long long)std::chrono::steady_clock::now().time_since_epoch().count() ^ (unsigned long long)(uintptr_t)&g_launches;
+        try { v ^= (unsigned long long)std::random_device{}() << 32; } catch (...) { }
+        return v;
+    }()};
+    unsigned long long z = counter.fetch_add(1, std::memory_order_relaxed) * 0x9e3779b97f4a7c15ull;
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    z ^= z >> 31;
+    return z ? z : 1ull;
 }
 
 static int check_device()

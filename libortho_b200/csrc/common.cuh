@@ -32,6 +32,7 @@ static inline int current_device_index()
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
     return dev;
 }
+unsigned long long next_launch_tag();   // api.cu: a 64-bit value no other launch has
 int device_sm_count(int dev);          // api.cu: multiprocessor count of device `dev`, cached
 
 // ---- tuning hook state (ortho_b200_set_decode_config) ------------------------------------------------
@@ -75,6 +76,9 @@ struct Plan {
     int64_t n_long, n_pad;
     int32_t *hrow;
     __half *hdense;
+    // ordered plans only: the entries once more as lists per 32 rows x 64 k (windows.cuh), without the long rows
+    uint32_t *win_off, *win_mask_off;     // [ceil(N / 32)][ceil(K / 64) + 1], start of one allocation with
+    uint32_t *win_words, *win_masks;      // these behind them
 };
 constexpr int kLongRowMin = 64;
 constexpr int64_t kLongDenseMaxBytes = 256ll << 20;
