@@ -60,6 +60,7 @@ constexpr int KP = 128;                 // k pair: the pipeline's unit and the u
 constexpr int W_BYTES = TN * KP / 2;    // 8 KB
 constexpr int A_STAGE_COLS = KP / 2;    // tensor-memory columns of a stage's converted weights
 constexpr int ST_MAX = 7, ST_SPARSE_MAX = 4, WST_MAX = 20;
+static_assert(kWinTile == TN * KB * 2 && kWinRows == 32, "places of the window lists");
 constexpr int S_BYTES = TN * KP * 2;    // 32 KB: a stage's sparse tile, two k blocks of 128 rows x 128 B (128-byte swizzle)
 constexpr int kSmemData = 224 * 1024;   // packed-weight slots, token stages, sparse tiles
 // Converter warps form groups of four (thread = row) that take the CTA's units in turn, as many groups (Params::groups)
@@ -74,7 +75,7 @@ constexpr int EPI_WARP0 = 2 + CONV_WARPS;
 constexpr int EPI_WARPS = 4;
 constexpr int XPROD_WARP = EPI_WARP0 + EPI_WARPS;   // token tiles have a producer of their own: the packed weights run ahead of them
 constexpr int SCAT_WARP0 = XPROD_WARP + 1;
-constexpr int SCAT_WARPS = 4;           // one per 32 rows of the tile
+constexpr int SCAT_WARPS = 8;           // two sets of four that take the units in turn; a warp of a set has 32 rows of the tile
 template <bool SPARSE> constexpr int kWarps = SCAT_WARP0 + (SPARSE ? SCAT_WARPS : 0);
 constexpr int TMEM_COLS = 512;
 
@@ -91,6 +92,7 @@ struct Params {
     int nst;                    // stages: a unit's converted weights and tokens
     int wst;                    // packed-weight slots
     int groups;                 // converter groups at work
+    int sets;                   // scatter sets at work: 2 with four stages, else 1
     float *slots;               // slots[cta][nt][128]: partial sums handed to another CTA ...
     unsigned long long *flags;  // ... and flags[cta] = tag once they are there (see launch_mid)
     unsigned long long tag;
@@ -149,8 +151,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < WST_MAX; s++) { mbar_init(&sm->w_full[s], 1); mbar_init(&sm->w_empty[s], 4); }
-        // full: the four warps of a converter group, the token producer with its bytes, the scatter warps
-        for (int s = 0; s < ST_MAX; s++) { mbar_init(&sm->full[s], 5 + (SPARSE ? SCAT_WARPS : 0)); mbar_init(&sm->empty[s], 1); }
+        // full: the four warps of a converter group, the token producer with its bytes, a set of scatter warps
+        for (int s = 0; s < ST_MAX; s++) { mbar_init(&sm->full[s], 5 + (SPARSE ? 4 : 0)); mbar_init(&sm->empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&sm->d_full[s], 1); mbar_init(&sm->d_empty[s], EPI_WARPS); }
         fence_mbar_init();
         prefetch_tensormap(&xmap);
@@ -296,70 +298,72 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         }
     } else if (SPARSE && warp >= SCAT_WARP0) {
         // ================= scatter: the unit's sparse entries -> zeroed FP16 tile in shared memory (A operand) =================
-        // Entries are fetched two units ahead and their extents two units before that, so that the loads' latency is not the
-        // pace; what a warp has put into the stages is kept in registers until it takes it out again.
-        const int q = warp - SCAT_WARP0;                 // 32 rows of the tile
-        int t = t_begin, kp = kp_begin, left = units;    // unit whose extent is fetched next
-        struct Extent { uint32_t e0, e1; };
-        auto fetch_extent = [&]() -> Extent {
-            Extent x{0u, 0u};
+        // A warp's loop is a chain of dependent instructions, so the entries come with their place in the tile worked out,
+        // are fetched a turn ahead (their extent a turn before that), and stay in registers until they are taken out again.
+        // With three stages a stage would pass from set to set, so one set does it all (Params::sets).
+        const int q = (warp - SCAT_WARP0) & 3, set = (warp - SCAT_WARP0) >> 2, sets = p.sets;
+        int t = t_begin, kp = kp_begin + set, left = units - set;        // unit whose extent is fetched next
+        while (kp >= p.kpairs) { kp -= p.kpairs; t++; }
+        uint32_t x0 = 0, x1 = 0;                         // that extent
+        auto fetch_extent = [&]() {
+            x0 = x1 = 0;
             const int g = 4 * t + q;
             if (left > 0 && g < p.ngroups) {
                 const uint32_t *o = p.win_off + (size_t)g * (size_t)(p.kblocks + 1) + 2 * kp;
-                x.e0 = __ldg(o);
-                x.e1 = __ldg(o + (2 * kp + 1 < p.kblocks ? 2 : 1));
+                x0 = __ldg(o);
+                x1 = __ldg(o + (2 * kp + 1 < p.kblocks ? 2 : 1));
             }
-            left--;
-            if (++kp == p.kpairs) { kp = 0; t++; }
-            return x;
+            left -= sets;
+            kp += sets;
+            while (kp >= p.kpairs) { kp -= p.kpairs; t++; }
         };
-        struct Batch { uint32_t first, count, a, b; };   // a unit's entries: extent, this lane's first two
-        auto fetch_batch = [&](const Extent &x) -> Batch {
-            Batch r{x.e0, x.e1 - x.e0, 0u, 0u};
-            if ((uint32_t)lane < r.count) r.a = __ldg(p.win_words + x.e0 + lane);
-            if ((uint32_t)lane + 32u < r.count) r.b = __ldg(p.win_words + x.e0 + 32 + lane);
-            return r;
+        uint32_t n0 = 0, nn = 0, na = 0, nb = 0;         // the next unit: first entry, count, this lane's first two
+        auto fetch_entries = [&]() {
+            n0 = x0; nn = x1 - x0;
+            if ((uint32_t)lane < nn) na = __ldg(p.win_words + n0 + lane);
+            if ((uint32_t)lane + 32u < nn) nb = __ldg(p.win_words + n0 + 32 + lane);
         };
-        Extent x0 = fetch_extent(), x1 = fetch_extent();
-        Batch b0 = fetch_batch(x0), b1 = fetch_batch(x1);
-        x0 = fetch_extent(); x1 = fetch_extent();
-        Batch o[ST_SPARSE_MAX];                          // o[d]: what the unit d + 1 before this one put into its stage
-#pragma unroll
-        for (int d = 0; d < ST_SPARSE_MAX; d++) o[d] = Batch{0u, 0u, 0u, 0u};
-        int st = 0; uint32_t ph = 0;
-        for (int i = 0; i < units; i++) {
-            const Batch cur = b0;
-            b0 = b1;
-            b1 = fetch_batch(x0);
-            x0 = x1;
-            x1 = fetch_extent();
-            unsigned char *tile = ss + (size_t)st * S_BYTES + q * (32 * 128);
-            auto place = [&](uint32_t e) -> unsigned short * {
-                const int k = window_k(e), r = window_row(e);
-                return reinterpret_cast<unsigned short *>(tile + (k >> 6) * (S_BYTES / 2) + r * 128 + ((((k >> 3) & 7) ^ (r & 7)) << 4)) + (k & 7);
-            };
-            const Batch old = p.nst == 4 ? o[3] : p.nst == 3 ? o[2] : o[1];
+        fetch_extent();
+        fetch_entries();
+        fetch_extent();
+        // what the last three visits put into their stages; a stage comes round after nst / sets visits, 2 or 3
+        const bool three = p.nst == 3;
+        uint32_t o1n = 0, o1a = 0, o1b = 0, o2n = 0, o2a = 0, o2b = 0, o3n = 0, o3a = 0, o3b = 0;
+        const uint32_t tiles = smem_u32(ss) + (uint32_t)(q * (32 * 128));
+        auto put = [&](uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)v) : "memory"); };
+        int st = set; uint32_t ph = 0;                   // nst is 2 or more
+        for (int i = set; i < units && set < sets; i += sets) {
+            const uint32_t first = n0, count = nn, a = na, b = nb;
+            fetch_entries();
+            fetch_extent();
+            const uint32_t tile = tiles + (uint32_t)(st * S_BYTES);
+            const uint32_t on = three ? o3n : o2n, oa = three ? o3a : o2a, ob2 = three ? o3b : o2b;
             wait(&sm->empty[st], ph ^ 1u);
             __syncwarp();
-            if (old.count <= 64u) {
-                if ((uint32_t)lane < old.count) *place(old.a) = 0;
-                if ((uint32_t)lane + 32u < old.count) *place(old.b) = 0;
-            } else {
-                for (int j = lane; j < 2 * 32 * 8; j += 32)
-                    reinterpret_cast<uint4 *>(tile + (j >> 8) * (S_BYTES / 2))[j & 255] = make_uint4(0, 0, 0, 0);
+            if ((uint32_t)lane < on) put(tile + (oa & 0xFFFFu), 0u);
+            if (on > 32u) {
+                if (on <= 64u) {
+                    if ((uint32_t)lane + 32u < on) put(tile + (ob2 & 0xFFFFu), 0u);
+                } else {
+                    for (int j = lane; j < 2 * 32 * 8; j += 32)
+                        *reinterpret_cast<uint4 *>(ss + (size_t)st * S_BYTES + q * (32 * 128) + (j >> 8) * kWinTile + (j & 255) * 16) = make_uint4(0, 0, 0, 0);
+                }
             }
             __syncwarp();
-            if ((uint32_t)lane < cur.count) *place(cur.a) = (unsigned short)(cur.a >> 16);
-            if ((uint32_t)lane + 32u < cur.count) *place(cur.b) = (unsigned short)(cur.b >> 16);
-            for (uint32_t j = 64 + lane; j < cur.count; j += 32) {
-                const uint32_t e = __ldg(p.win_words + cur.first + j);
-                *place(e) = (unsigned short)(e >> 16);
+            if ((uint32_t)lane < count) put(tile + (a & 0xFFFFu), a >> 16);
+            if (count > 32u) {
+                if ((uint32_t)lane + 32u < count) put(tile + (b & 0xFFFFu), b >> 16);
+                for (uint32_t j = 64 + lane; j < count; j += 32) {
+                    const uint32_t e = __ldg(p.win_words + first + j);
+                    put(tile + (e & 0xFFFFu), e >> 16);
+                }
             }
             fence_proxy_async();                         // the tensor core reads shared memory through the async proxy
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm->full[st]);
-            o[3] = o[2]; o[2] = o[1]; o[1] = o[0]; o[0] = cur;
-            if (++st == p.nst) { st = 0; ph ^= 1u; }
+            o3n = o2n; o3a = o2a; o3b = o2b; o2n = o1n; o2a = o1a; o2b = o1b; o1n = count; o1a = a; o1b = b;
+            st += sets;
+            if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
         }
     } else {
         // ================= epilogue: TMEM -> (+ partials) -> scale, sparse term, bias -> FP16 -> global =================
@@ -681,6 +685,7 @@ int launch_mid(const FwdArgs &a)
         if (p.nst >= p.groups) break;
         if (p.groups == 2) return ORTHO_B200_ERR_SHAPE;      // not reached for up to 128 tokens
     }
+    p.sets = p.nst == 4 ? 2 : 1;
     CUtensorMap xmap, wmap;
     if (!make_tensor_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, (uint64_t)a.M, (uint64_t)a.K,
                             (uint64_t)a.K * 2, (uint32_t)p.nt, KB, CU_TENSOR_MAP_SWIZZLE_128B))
