@@ -137,7 +137,7 @@ int64_t min_workspace_bytes(int64_t M, int64_t K, int64_t N)
 extern "C" int64_t ortho_b200_workspace_bytes(int64_t M, int64_t K, int64_t N)
 {
     const int64_t other = decode_regime(M, N, K) ? 0 : prefill_workspace_bytes(M, K, N);
-    if (!mid_token_range(M)) return other;
+    if (!mid_range(M, N, K)) return other;
     const int64_t mid = mid_workspace_bytes(M, K, N);
     return mid > other ? mid : other;
 }
@@ -162,7 +162,7 @@ int forward_impl(const void *q_weight, const void *q_scales_f16,
 
 int launch_routed(const FwdArgs &a)
 {
-    switch (route_of(a.M, a.N, a.K, a.workspace, a.workspace_bytes)) {
+    switch (route_of(a)) {
         case kRouteMid: return launch_mid(a);
         case kRouteDecode: return launch_decode(a);
         default: return launch_prefill(a);
@@ -259,7 +259,7 @@ extern "C" int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers, int
                                      d.ortho_row_ptr, d.nnz, x_f16, d.y_f16, M, K, d.N, d.alpha, d.plan,
                                      workspace, workspace_bytes, stream, d.ldy, d.bias_f32);
         if (st != ORTHO_B200_OK) return st;
-        all_stream = all_stream && route_of(M, d.N, K, workspace, workspace_bytes) == kRouteDecode && stream_kernel_selected(M, K);
+        all_stream = all_stream && route_of(a[l]) == kRouteDecode && stream_kernel_selected(M, K);
     }
     if (all_stream && n_layers > 1) return launch_decode_multi(a, n_layers);
     for (int l = 0; l < n_layers; l++) {

@@ -43,9 +43,8 @@ struct Tuning {
     bool force_stream = false;          // streaming kernel with stream_s / stream_stages
     int stream_s = 0, stream_stages = 0;
     int prefill_above = 24;             // forwards with more tokens than this use the tensor-core kernels
-    // forwards with mid_lo < tokens <= mid_hi use the tokens-as-M tensor-core kernel when they bring its workspace:
-    // built in, above the streaming kernel's 16 tokens except on small layers up to 32 tokens; through the
-    // hook, first (mid_first)
+    // forwards with mid_lo < tokens <= mid_hi (and some with fewer, decode.cu) use the kernel of mid.cu when they bring its
+    // workspace; through the hook, before any other rule (mid_first)
     int mid_lo = 16, mid_hi = 128;
     bool mid_first = false;
     bool gather_per_cta = false;        // peer exchange: every CTA signals the peers itself instead of the grid's last CTA
@@ -77,8 +76,9 @@ struct Plan {
     int32_t *hrow;
     __half *hdense;
     // ordered plans only: the entries once more as lists per 32 rows x 64 k (windows.cuh), without the long rows
-    uint32_t *win_off, *win_mask_off;     // [ceil(N / 32)][ceil(K / 64) + 1], start of one allocation with
-    uint32_t *win_words, *win_masks;      // these behind them
+    uint32_t *win_off;    // [ceil(N / 32)][ceil(K / 64) + 1]
+    uint32_t *win_words;
+    void *blocks[3];      // the allocations behind entries, row_ptr, row_max and the lists
 };
 constexpr int kLongRowMin = 64;
 constexpr int64_t kLongDenseMaxBytes = 256ll << 20;
@@ -266,11 +266,12 @@ int set_decode_config(int wr, int wk, int u, int s);
 bool stream_kernel_selected(int64_t M, int64_t K);   // the forward of (M, K) will run decode_stream_kernel
 // true = decode kernels: up to Tuning::prefill_above tokens, and narrow layers of up to 64 tokens
 bool decode_regime(int64_t M, int64_t N, int64_t K);
-// which kernel family a forward takes.  The tokens-as-M kernel needs its workspace whatever alpha is; a call
-// inside its token range that brings none runs the kernels of the neighbouring regimes instead.
+// which kernel family a forward takes.  The kernel of mid.cu needs its workspace whatever alpha is; a call inside its
+// range that brings none runs the kernels of the neighbouring regimes instead.
 enum Route { kRouteDecode = 0, kRouteMid = 1, kRoutePrefill = 2 };
-bool mid_token_range(int64_t M);
-Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes);
+bool mid_range(int64_t M, int64_t N, int64_t K);
+Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool lists);
+Route route_of(const FwdArgs &a);
 int launch_mid(const FwdArgs &a);                                  // mid.cu
 int64_t mid_workspace_bytes(int64_t M, int64_t K, int64_t N);
 }  // namespace ob

@@ -288,39 +288,52 @@ static bool decode_regime_of(const Tuning &t, int64_t M, int64_t N, int64_t K)
     return (M <= 32 && N <= 4096) || N <= 1024;
 }
 bool decode_regime(int64_t M, int64_t N, int64_t K) { return decode_regime_of(tuning_snapshot(), M, N, K); }
-bool mid_token_range(int64_t M)
+// The tcgen05 kernel of mid.cu against the streaming kernel (up to 16 tokens; needs its sparse entries as window lists or
+// none at all).  Its time hardly depends on the token count, the streaming kernel's grows with it and with the
+// activation slab of a CTA (M x K halves): above 100 KB one CTA fits an SM instead of two, above 200 KB K is split over a cluster.
+// One B200, us, 0.3 % ortho, streaming / mid.cu:
+//   16 tokens: 4096->4096 9.6 / 10.3, 2048->4096 7.3 / 8.4, 8192->1024 8.4 / 10.1, but 4096->12288 19.3 / 14.8,
+//              8192->8192 32.2 / 17.7, 8192->57344 201 / 77, 28672->8192 100 / 43;   9 tokens: 8192->4096 13.8 / 13.1
+//    8 tokens: 4096->22016 18.9 / 19.8, 8192->4096 12.0 / 13.1, 28672->1024 13.3 / 16.9, but 8192->8192 18.6 / 17.6,
+//              11008->4096 16.9 / 15.0, 8192->57344 104 / 77, 28672->8192 77 / 43;   5 tokens: 14336->4096 15.0 / 17.0
+//    6 tokens: 8192->16384 26.2 / 26.8, but 8192->57344 91 / 77;
+//    4 tokens: 16384->16384 42 / 47, 8192->57344 62 / 77, but 28672->4096 29.2 / 25.6, 28672->8192 50 / 43;
+//              3 tokens: 28672->4096 21.8 / 25.6
+static bool mid_beats_stream(int64_t M, int64_t N, int64_t K)
 {
-    const Tuning t = tuning_snapshot();
-    return M > t.mid_lo && M <= t.mid_hi && M <= 128;
+    const int64_t weights = N * K, slab = 2 * M * K;
+    if (M >= 9) return weights > (int64_t)4096 * 4096;
+    if (weights < (int64_t)5 << 23) return false;
+    if (slab > (200 << 10)) return M >= 3;
+    if (M >= 6 && weights >= (int64_t)1 << 28) return true;
+    return M >= 5 && (slab >= (150 << 10) || (slab >= (128 << 10) && weights >= (int64_t)1 << 26));
 }
-// Measured on one B200 (us, 0.3 % ortho, alpha = 1, folded sparse term): 32 tokens on 8192->8192 / 8192->10240 /
-// 8192->57344 / 28672->8192 take 49 / 54 / 183 / 107 with the tokens-as-M kernel against 95 / 108 / 370 / 218 with the
-// 128 x 256-token tile of prefill.cu; at 16 tokens the streaming kernel is level on the largest layer (205) and ahead
-// on K = 4096 layers (33 against 68 on 4096->22016).  From 17 tokens on the mma.sync kernel of this file falls behind
-// quickly (20 / 24 tokens: 8192->10240 113 / 147 against 51 / 52, 8192->57344 497 / 797 against 182, 11008->4096 50 / 54
-// against 43 / 44), hence the built-in range (16, 128].
-// Narrow layers (a GPU's shard of a layer, say), tokens-as-M kernel against the mma.sync kernel of this file:
-//   32 tokens: 8192->1024 39 / 25, 8192->1280 39 / 25, 4096->2048 34 / 17, 4096->4096 35 / 33, 11008->512 41 / 25, but
-//              8192->2560 40 / 48, 8192->4096 42 / 52, 28672->1024 66 / 107, 28672->2048 64 / 86;
-//   64 tokens: 8192->1024 53 / 63, 8192->1280 53 / 166, 8192->2560 54 / 109, 4096->4096 45 / 80, 4096->2048 44 / 117,
-//              28672->1024 98 / 175 (only 4096->1024 loses: 43 / 38).
-//   17 .. 24 tokens on layers of at most 4096 x 4096 weights: the mma.sync kernel stays ahead (4096->4096 25-27 against
-//              31-33, 8192->2048 19-21 against 35-37, 4096->1024 13-14 against 31).
-// So with its workspace the tokens-as-M kernel takes everything above 16 tokens except up to 32 tokens on layers of at
-// most 4096 x 4096 weights; without the workspace the older rule between the mma.sync kernel and the prefill tile
-// (decode_regime_of) stands.
-Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes)
+static bool mid_range_of(const Tuning &t, int64_t M, int64_t N, int64_t K)
+{
+    if (M > 128) return false;
+    if (M > t.mid_lo && M <= t.mid_hi) return true;
+    return !t.mid_first && M <= 16 && t.wr == 0 && !t.force_stream && mid_beats_stream(M, N, K);
+}
+bool mid_range(int64_t M, int64_t N, int64_t K) { return mid_range_of(tuning_snapshot(), M, N, K); }
+// `lists`: the sparse term is inactive or comes as a plan's window lists.  From 17 tokens on the mma.sync kernel below is
+// behind on every layer then (32 tokens: 1024->1024 14.6 / 6.2, 4096->4096 32.4 / 12.1, 8192->2048 26.8 / 14.6,
+// 4096->22016 88 / 21).  Without lists mid.cu needs two more launches for the sparse term, which small layers do not earn
+// back (raw CSR, 0.5 %, 32 tokens: 1024->1024 14.8 / 23.8, 4096->1024 16.0 / 28.8, 4096->4096 34.8 / 30.4), and up to 16
+// tokens no layer does.  Without the workspace the rule between the mma.sync kernel and the prefill tile stands.
+Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool lists)
 {
     const Tuning t = tuning_snapshot();
-    const bool mid_ok = M > t.mid_lo && M <= t.mid_hi && M <= 128 && workspace && ((uintptr_t)workspace & 255u) == 0 &&
-                        workspace_bytes >= mid_workspace_bytes(M, K, N);
-    if (mid_ok && t.mid_first) return kRouteMid;
-    if (mid_ok) {
-        if (t.prefill_above == kPrefillAboveBuiltin && M <= 32 && N * K <= (int64_t)4096 * 4096) return kRouteDecode;
-        return kRouteMid;
+    if (mid_range_of(t, M, N, K) && workspace && ((uintptr_t)workspace & 255u) == 0 && workspace_bytes >= mid_workspace_bytes(M, K, N)) {
+        if (t.mid_first || lists) return kRouteMid;
+        if (M > 16 && !(t.prefill_above == kPrefillAboveBuiltin && M <= 32 && N * K <= (int64_t)4096 * 4096)) return kRouteMid;
     }
     if (decode_regime_of(t, M, N, K)) return kRouteDecode;
     return kRoutePrefill;
+}
+Route route_of(const FwdArgs &a)
+{
+    const bool lists = !a.has_ortho || (a.plan && a.plan->win_off && tuning_snapshot().patch_weights);
+    return route_of(a.M, a.N, a.K, a.workspace, a.workspace_bytes, lists);
 }
 
 int launch_decode_stream(const FwdArgs &a, int S, int stages);          // decode_stream.cu

@@ -53,112 +53,64 @@ __global__ void relayout_rows_kernel(const int32_t *__restrict__ row_ptr, const 
     }
 }
 
-// Window lists, step 1: ptr[(n - n0)][kb] = index of the first entry of row n at or past column 64 kb (kb = 0 ..
-// kblocks; a long row, whose entries are not listed, gets an empty extent everywhere).  One warp per row.
-__global__ void window_ptr_kernel(const uint32_t *__restrict__ entries, const int32_t *__restrict__ row_ptr, int n0, int n1,
-                                  int kblocks, int heavy, int32_t *__restrict__ ptr)
-{
-    const int lane = threadIdx.x & 31;
-    for (int n = n0 + (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); n < n1; n += gridDim.x * (blockDim.x >> 5)) {
-        int32_t *row = ptr + (size_t)(n - n0) * (size_t)(kblocks + 1);
-        const int e0 = row_ptr[n];
-        int e1 = row_ptr[n + 1];
-        if (heavy > 0 && e1 - e0 > heavy) e1 = e0;
-        for (int e = e0 + lane; e < e1; e += 32) {
-            const int kb = (int)((entries[e] & 0xFFFFu) / kWinK);
-            const int before = e > e0 ? (int)((entries[e - 1] & 0xFFFFu) / kWinK) : -1;
-            for (int j = before + 1; j <= kb; j++) row[j] = e;
-        }
-        const int last = e1 > e0 ? (int)((entries[e1 - 1] & 0xFFFFu) / kWinK) : -1;
-        for (int j = last + 1 + lane; j <= kblocks; j += 32) row[j] = e1;
-    }
-}
-
-// step 2: one CTA per group of 32 rows sizes its windows, scans the sizes and writes entries and masks.  The group's
-// entries start at the index of its first CSR entry, and so do its masks (a window has at most as many rounds as entries).
+// Window lists (windows.cuh).  One CTA per group of 32 rows, lane = row: every warp walks an eighth of the k blocks with a
+// cursor per row, once to size the windows and, after a scan over the sizes, once to write the entries, round by round.  The
+// group's entries start at the index of its first CSR entry.
+// Rows of more than `heavy` entries (0: no limit) are left out; a plan found unordered (info[1]) gets no lists.
 __global__ void __launch_bounds__(256)
-window_lists_kernel(const uint32_t *__restrict__ entries, const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ ptr,
-                    int n0, int N, int kblocks, uint32_t *__restrict__ off, uint32_t *__restrict__ words,
-                    uint32_t *__restrict__ mask_off, uint32_t *__restrict__ masks)
+window_lists_kernel(const uint32_t *__restrict__ entries, const int32_t *__restrict__ row_ptr, int N, int kblocks, int heavy,
+                    const int *__restrict__ info, uint32_t *__restrict__ off, uint32_t *__restrict__ words)
 {
-    __shared__ uint32_t size[2][65536 / kWinK + 1];      // entries, rounds
-    const int g = n0 / kWinRows + (int)blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ uint32_t size[65536 / kWinK + 1];
+    if (info[1] != 0) return;
+    const int g = (int)blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = g * kWinRows + lane;
-    const int32_t *row = ptr + (size_t)(n - n0) * (size_t)(kblocks + 1);
-    for (int kb = warp; kb < kblocks; kb += 8) {
-        const int c = n < N ? row[kb + 1] - row[kb] : 0;
-        int sum = c, most = c;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-        }
-        if (lane == 0) { size[0][kb] = (uint32_t)sum; size[1][kb] = (uint32_t)most; }
+    int e0 = 0, e1 = 0;
+    if (n < N) { e0 = row_ptr[n]; e1 = row_ptr[n + 1]; }
+    if (heavy > 0 && e1 - e0 > heavy) e1 = e0;
+    const int kb0 = kblocks * warp / 8, kb1 = kblocks * (warp + 1) / 8;
+    int start = e0;                                      // first entry at or past this warp's first column
+    for (int hi = e1; start < hi;) {
+        const int mid = (start + hi) >> 1;
+        if ((int)(entries[mid] & 0xFFFFu) < kb0 * kWinK) start = mid + 1; else hi = mid;
+    }
+    for (int kb = kb0, e = start; kb < kb1; kb++) {
+        int c = 0;
+        while (e < e1 && (int)(entries[e] & 0xFFFFu) < (kb + 1) * kWinK) { e++; c++; }
+        __syncwarp();
+        const int sum = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) size[kb] = (uint32_t)sum;
     }
     __syncthreads();
-    if (warp < 2) {                                      // exclusive scan, 32 at a time
+    if (warp == 0) {                                     // exclusive scan, 32 at a time
         uint32_t run = (uint32_t)row_ptr[g * kWinRows];
         for (int b = 0; b < kblocks; b += 32) {
-            const uint32_t v = b + lane < kblocks ? size[warp][b + lane] : 0u;
+            const uint32_t v = b + lane < kblocks ? size[b + lane] : 0u;
             uint32_t s = v;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t t = __shfl_up_sync(0xffffffffu, s, o);
                 if (lane >= o) s += t;
             }
-            if (b + lane < kblocks) size[warp][b + lane] = run + s - v;
+            if (b + lane < kblocks) size[b + lane] = run + s - v;
             run += __shfl_sync(0xffffffffu, s, 31);
         }
-        if (lane == 0) size[warp][kblocks] = run;
+        if (lane == 0) size[kblocks] = run;
     }
     __syncthreads();
-    for (int kb = threadIdx.x; kb <= kblocks; kb += 256) {
-        off[(size_t)g * (size_t)(kblocks + 1) + kb] = size[0][kb];
-        mask_off[(size_t)g * (size_t)(kblocks + 1) + kb] = size[1][kb];
-    }
-    for (int kb = warp; kb < kblocks; kb += 8) {
-        const int e = n < N ? row[kb] : 0, c = n < N ? row[kb + 1] - e : 0;
-        uint32_t at = size[0][kb], mat = size[1][kb];
-        for (int r = 0;; r++) {
-            const uint32_t mask = __ballot_sync(0xffffffffu, c > r);
+    for (int kb = threadIdx.x; kb <= kblocks; kb += 256) off[(size_t)g * (size_t)(kblocks + 1) + kb] = size[kb];
+    for (int kb = kb0, e = start; kb < kb1; kb++) {
+        uint32_t at = size[kb];
+        for (;;) {
+            uint32_t pk = 0;
+            bool has = e < e1;
+            if (has) { pk = entries[e]; has = (int)(pk & 0xFFFFu) < (kb + 1) * kWinK; }
+            const uint32_t mask = __ballot_sync(0xffffffffu, has);
             if (mask == 0u) break;
-            if (lane == 0) masks[mat + (uint32_t)r] = mask;
-            if (c > r) words[at + __popc(mask & ((1u << lane) - 1u))] = window_entry(entries[e + r], lane);
+            if (has) { words[at + __popc(mask & ((1u << lane) - 1u))] = window_entry(pk, lane); e++; }
             at += __popc(mask);
         }
     }
-}
-
-// Builds the plan's window lists on the stream.  Rows are taken in slabs so that the row x k block index of step 1
-// stays within a fixed amount of temporary memory.
-static cudaError_t build_windows(Plan *pl, cudaStream_t st)
-{
-    const int kblocks = (int)ceil_div(pl->K, kWinK);
-    const int64_t groups = ceil_div(pl->N, kWinRows);
-    int64_t slab = (16ll << 20) / ((int64_t)(kblocks + 1) * 4 * kWinRows);        // row groups per slab
-    if (slab < 1) slab = 1;
-    if (slab > groups) slab = groups;
-    int32_t *ptr = nullptr;
-    // one allocation: offsets of entries and masks, entries, masks
-    const size_t noff = (size_t)groups * (size_t)(kblocks + 1), nnz = (size_t)pl->nnz;
-    cudaError_t e = cudaMalloc(&pl->win_off, (2 * noff + 2 * nnz) * sizeof(uint32_t));
-    if (e == cudaSuccess) { pl->win_mask_off = pl->win_off + noff; pl->win_words = pl->win_mask_off + noff; pl->win_masks = pl->win_words + nnz; }
-    if (e == cudaSuccess) e = cudaMalloc(&ptr, (size_t)slab * kWinRows * (size_t)(kblocks + 1) * sizeof(int32_t));
-    for (int64_t g0 = 0; g0 < groups && e == cudaSuccess; g0 += slab) {
-        const int64_t gn = g0 + slab < groups ? slab : groups - g0;
-        const int n0 = (int)(g0 * kWinRows);
-        const int n1 = (int)((g0 + gn) * kWinRows < pl->N ? (g0 + gn) * kWinRows : pl->N);
-        const int64_t blocks = ceil_div(n1 - n0, 8);
-        window_ptr_kernel<<<(unsigned)(blocks > 148 * 16 ? 148 * 16 : blocks), 256, 0, st>>>(
-            pl->entries, pl->row_ptr, n0, n1, kblocks, pl->n_long > 0 ? pl->heavy : 0, ptr);
-        window_lists_kernel<<<(unsigned)gn, 256, 0, st>>>(pl->entries, pl->row_ptr, ptr, n0, (int)pl->N, kblocks,
-                                                          pl->win_off, pl->win_words, pl->win_mask_off, pl->win_masks);
-        count_launch(2);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (ptr) cudaFree(ptr);
-    return e;
 }
 
 // one warp per output row: the row of an entry is recovered from the plan's own row pointers
@@ -236,30 +188,60 @@ extern "C" int ortho_b200_plan_create(ortho_b200_plan **plan_out, const int32_t 
     pl->row_ptr = nullptr; pl->entries = nullptr; pl->row_max = nullptr; pl->ordered = false;
     pl->heavy = kLongRowMin; pl->n_long = 0; pl->n_pad = 0;
     pl->hrow = nullptr; pl->hdense = nullptr;
-    pl->win_off = pl->win_words = pl->win_mask_off = pl->win_masks = nullptr;
+    pl->win_off = pl->win_words = nullptr;
+    for (void *&b : pl->blocks) b = nullptr;
     cudaError_t e = cudaGetDevice(&pl->device);
     if (e != cudaSuccess) { note_cuda_error(e); delete pl; return ORTHO_B200_ERR_CUDA; }
     if (nnz > 0) {
         cudaStream_t st = (cudaStream_t)stream;
-        int *d_max = nullptr;
-        e = cudaMalloc(&pl->row_ptr, sizeof(int32_t) * (N + 1));
-        if (e == cudaSuccess) e = cudaMalloc(&pl->entries, sizeof(uint32_t) * nnz);
-        if (e == cudaSuccess) e = cudaMalloc(&pl->row_max, sizeof(float) * N);
-        if (e == cudaSuccess) e = cudaMalloc(&d_max, 2 * sizeof(int));
-        if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, 2 * sizeof(int), st);
+        // Device memory: {entries}, {row pointers, row maxima, list offsets, two result words}, {list entries}.
+        // cudaMalloc hands out pieces of up to 1 MB from blocks that it has mapped already and maps new memory for larger
+        // ones (some 400 us each, several times what all the kernels here take): three pieces for a small layer, one for a large one.
+        const int kblocks = (int)ceil_div(K, kWinK);
+        const int64_t groups = ceil_div(N, kWinRows);
+        const size_t noff = (size_t)groups * (size_t)(kblocks + 1);
+        const size_t size[3] = {(size_t)nnz, (size_t)(N + 1) + (size_t)N + noff + 2, (size_t)nnz};      // words
+        const bool pieces = nnz <= (1 << 20) / 4;
+        uint32_t *at[3] = {nullptr, nullptr, nullptr};
+        if (pieces) {
+            for (int i = 0; i < 3 && e == cudaSuccess; i++) {
+                e = cudaMalloc(&pl->blocks[i], sizeof(uint32_t) * size[i]);
+                at[i] = reinterpret_cast<uint32_t *>(pl->blocks[i]);
+            }
+        } else {
+            e = cudaMalloc(&pl->blocks[0], sizeof(uint32_t) * (size[0] + size[1] + size[2]));
+            at[0] = reinterpret_cast<uint32_t *>(pl->blocks[0]);
+            for (int i = 1; i < 3; i++) at[i] = at[i - 1] + size[i - 1];
+        }
+        int *d_info = nullptr;
+        if (e == cudaSuccess) {
+            pl->entries = at[0];
+            pl->row_ptr = reinterpret_cast<int32_t *>(at[1]);
+            pl->row_max = reinterpret_cast<float *>(at[1] + N + 1);
+            pl->win_off = at[1] + 2 * N + 1;
+            d_info = reinterpret_cast<int *>(pl->win_off + noff);
+            pl->win_words = at[2];
+            e = cudaMemsetAsync(d_info, 0, 2 * sizeof(int), st);
+        }
+        auto build_windows = [&](int heavy) -> cudaError_t {
+            window_lists_kernel<<<(unsigned)groups, 256, 0, st>>>(pl->entries, pl->row_ptr, (int)N, kblocks, heavy, d_info,
+                                                                  pl->win_off, pl->win_words);
+            count_launch();
+            return cudaGetLastError();
+        };
         if (e == cudaSuccess) {
             const int threads = 256, wpb = threads / 32;
             int64_t blocks = ceil_div(N + 1, wpb);
             if (blocks > 148 * 16) blocks = 148 * 16;
             relayout_rows_kernel<<<(unsigned)blocks, threads, 0, st>>>(
-                row_ptr, col_indices, (const __half *)values_f16, (int)N, (int)K, pl->entries, pl->row_ptr, pl->row_max, d_max);
+                row_ptr, col_indices, (const __half *)values_f16, (int)N, (int)K, pl->entries, pl->row_ptr, pl->row_max, d_info);
             count_launch();
             e = cudaGetLastError();
         }
+        if (e == cudaSuccess) e = build_windows(0);      // again below in the rarer case that there are long rows to leave out
         int h_info[2] = {0, 0};
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h_info, d_max, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h_info, d_info, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (d_max) cudaFree(d_max);
         if (e != cudaSuccess) {
             note_cuda_error(e);
             ortho_b200_plan_destroy(reinterpret_cast<ortho_b200_plan *>(pl));
@@ -307,8 +289,10 @@ extern "C" int ortho_b200_plan_create(ortho_b200_plan **plan_out, const int32_t 
                 return ORTHO_B200_ERR_CUDA;
             }
         }
-        if (pl->ordered) {
-            e = build_windows(pl, st);
+        if (!pl->ordered) pl->win_off = pl->win_words = nullptr;
+        if (pl->ordered && pl->n_long > 0) {
+            e = build_windows(pl->heavy);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) {
                 note_cuda_error(e);
                 ortho_b200_plan_destroy(reinterpret_cast<ortho_b200_plan *>(pl));
@@ -325,12 +309,10 @@ extern "C" int ortho_b200_plan_destroy(ortho_b200_plan *plan)
     Plan *pl = reinterpret_cast<Plan *>(plan);
     if (!pl) return ORTHO_B200_OK;
     if (pl->magic != kPlanMagic) return ORTHO_B200_ERR_PLAN;
-    if (pl->row_ptr) cudaFree(pl->row_ptr);
-    if (pl->entries) cudaFree(pl->entries);
-    if (pl->row_max) cudaFree(pl->row_max);
+    for (void *b : pl->blocks)
+        if (b) cudaFree(b);
     if (pl->hrow) cudaFree(pl->hrow);
     if (pl->hdense) cudaFree(pl->hdense);
-    if (pl->win_off) cudaFree(pl->win_off);
     pl->magic = 0;
     delete pl;
     return ORTHO_B200_OK;
@@ -362,7 +344,7 @@ extern "C" int64_t ortho_b200_plan_workspace_bytes(const ortho_b200_plan *plan, 
     if (pl->nnz == 0) return 0;
     const int64_t plain = ortho_b200_workspace_bytes(M, pl->K, pl->N);
     // the tensor-core kernels take the sums of the plan's long rows from a pre-pass
-    return plain + (decode_regime(M, pl->N, pl->K) && !mid_token_range(M) ? 0 : long_rows_workspace_bytes(pl, M));
+    return plain + (decode_regime(M, pl->N, pl->K) && !mid_range(M, pl->N, pl->K) ? 0 : long_rows_workspace_bytes(pl, M));
 }
 
 extern "C" int ortho_b200_plan_decode_dump(const ortho_b200_plan *plan, int32_t *rows_out, int32_t *cols_out,

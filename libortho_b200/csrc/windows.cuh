@@ -5,9 +5,8 @@
 // row group are neighbours in the list too.  An entry is {f16 value | place}, the place being the byte offset of
 // (row, k) in a 128-byte swizzled FP16 tile of 32 rows x 64 k, plus kWinTile for the odd windows: a warp that scatters
 // entries adds the low half of the word to its tile's address.  Inside a window the entries are ordered by round, then
-// row: round r holds the r-th entry of every row that has more than r, and a list of 32-bit row masks, one per
-// round, lets each lane find its own entry by a popcount.
-// win_off[group * (kblocks + 1) + kb] is the first entry of a window and the next element its end; mask_off likewise.
+// row: round r holds the r-th entry of every row that has more than r.
+// win_off[group * (kblocks + 1) + kb] is the first entry of a window and the next element its end.
 // Long rows are not listed.
 #pragma once
 
