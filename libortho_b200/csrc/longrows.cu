@@ -11,10 +11,12 @@
 //     OL = HD * X^T        (tcgen05.mma kind::f16, both operands K-major from shared memory via TMA, FP32 in TMEM)
 //
 // tile = 128 long rows x 256 tokens, K cut into `nsplit` shares so that the few tiles fill the GPU; every share
-// leaves its FP32 sums in the workspace and the main kernel adds the shares, in share order, when it picks a long
-// row's sums up (no atomics: the result does not depend on scheduling).  X is read in its own layout, the
-// transposed copy is not needed here.  The main kernel is launched as a programmatic dependent of this one: its
-// tensor-core pipeline starts while this kernel drains, only the warps that read the sums wait for it.
+// leaves its FP32 sums in the workspace and a second small kernel adds the shares, in share order (no atomics: the
+// result does not depend on scheduling).  (Left to the main kernel's epilogue, where a thread holds a row, the shares of a
+// long row are dependent loads by the thousand: 8192->8192 with Zipf rows at 512 tokens took 923 us that way.)  X is
+// read in its own layout, the transposed copy is not needed here.  Each of the three kernels is launched as a
+// programmatic dependent of the one before: the main kernel's pipeline starts while these drain, only the warps that
+// read the sums wait for them.
 // The reference walks every coordinate serially per token (src/ortho.c:384-398).
 #include <cstring>
 
@@ -137,6 +139,27 @@ long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, TT); }
 }
 
+// part[0] += part[1] + ... + part[nsplit - 1], for the n_long rows (Mp floats each); four tokens per thread
+__global__ void __launch_bounds__(256)
+long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, int nsplit)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= quads) return;
+    float4 acc = __ldcg(part + i);
+    for (int s = 1; s < nsplit; s += 4) {
+        float4 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (s + j < nsplit) t[j] = __ldcg(part + i + (s + j) * stride);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (s + j < nsplit) { acc.x += t[j].x; acc.y += t[j].y; acc.z += t[j].z; acc.w += t[j].w; }
+    }
+    part[i] = acc;
+}
+
 // ---- plan side: the dense copy of the long rows --------------------------------------------------------------
 // One CTA per long row: writes the row's entries into the (zeroed) dense row and marks every column in a
 // shared-memory bitmap; a column met twice (a CSR row that repeats a column, which the dense form cannot hold)
@@ -207,9 +230,9 @@ int64_t long_rows_workspace_bytes(const Plan *pl, int64_t M)
     return (((int64_t)long_rows_splits(pl, M) * pl->n_pad * Mp * 4 + 255) / 256) * 256;
 }
 
-// ws: long_rows_workspace_bytes() bytes, 256-byte aligned; Mp = tokens rounded up to 256.  The sums of long row h for
-// token m are  sum over s < *nsplit_out of  (*part_out)[(s * n_pad + h) * Mp + m].
-int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **part_out, int *nsplit_out)
+// ws: long_rows_workspace_bytes() bytes, 256-byte aligned; Mp = tokens rounded up to 256.  The sum of long row h for
+// token m is (*sums_out)[h * Mp + m].
+int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
 {
     using namespace lg;
     const Plan *pl = a.plan;
@@ -237,8 +260,19 @@ int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **part_out,
     long_gemm_kernel<<<g1, NWARPS * 32, kSmemBytes, a.stream>>>(amap, xmap, p);
     count_launch();
     OB_CUDA(cudaGetLastError());
-    *part_out = p.part;
-    *nsplit_out = p.nsplit;
+    if (p.nsplit > 1) {
+        const long long quads = (long long)p.n_long * Mp / 4, stride = (long long)p.n_pad * Mp / 4;
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3((unsigned)ceil_div(quads, 256)); cfg.blockDim = dim3(256); cfg.stream = a.stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        OB_CUDA(cudaLaunchKernelEx(&cfg, long_sum_kernel, reinterpret_cast<float4 *>(p.part), quads, stride, p.nsplit));
+        count_launch();
+    }
+    *sums_out = p.part;
     return ORTHO_B200_OK;
 }
 

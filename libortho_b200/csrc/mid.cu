@@ -97,9 +97,9 @@ struct Params {
     unsigned long long *flags;  // ... and flags[cta] = tag once they are there (see launch_mid)
     unsigned long long tag;
     const float *o; float alpha; int has_ortho;    // O[m][n], row pitch N
-    // sparse instantiation (a plan with ordered rows): the window lists; long rows are read from the pre-pass's shares
+    // sparse instantiation (a plan with ordered rows): the window lists; long rows are read from the pre-pass's sums
     const uint32_t *win_off, *win_words; int ngroups;
-    const int32_t *row_ptr; const float *ol; int ol_splits, ol_pad, ol_mp; const int32_t *hrow; int n_long, heavy;
+    const int32_t *row_ptr; const float *ol; int ol_mp; const int32_t *hrow; int n_long, heavy;
     int *status;
     int gather;
     GatherView gv;
@@ -109,6 +109,7 @@ struct Smem {
     uint64_t w_full[WST_MAX], w_empty[WST_MAX];
     uint64_t full[ST_MAX], empty[ST_MAX];
     uint64_t d_full[2], d_empty[2];
+    uint64_t all_done;          // the CTA's last piece is complete (one phase: the converters have not followed d_full)
     uint32_t tmem_base;
 };
 constexpr size_t kSmemBytes = 1024 + (size_t)kSmemData + sizeof(Smem);
@@ -154,6 +155,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         // full: the four warps of a converter group, the token producer with its bytes, a set of scatter warps
         for (int s = 0; s < ST_MAX; s++) { mbar_init(&sm->full[s], 5 + (SPARSE ? 4 : 0)); mbar_init(&sm->empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&sm->d_full[s], 1); mbar_init(&sm->d_empty[s], EPI_WARPS); }
+        mbar_init(&sm->all_done, 1);
         fence_mbar_init();
         prefetch_tensormap(&xmap);
         prefetch_tensormap(&wmap);
@@ -253,48 +255,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 }
                 umma_commit(&sm->d_full[a]);
             }
-        }
-    } else if (warp < EPI_WARP0) {
-        // ================= converters: packed INT4 (smem) -> FP16 -> A operand in tensor memory =================
-        const int q = warp & 3;                          // tensor-memory lane quarter this warp may touch
-        const int grp = (warp - 2) >> 2;
-        const int row = q * 32 + lane;                   // weight row inside the tile
-        const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;     // 64-byte swizzle: 16-byte chunk c sits at c ^ ((row >> 1) & 3)
-        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(p.nacc * p.acc_cols);
-        const unsigned char *wrow = ws + row * (KP / 2);
-        int wi = grp, st = grp;                          // slot and stage of the group's unit
-        uint32_t wph = 0, ph = 0;
-        for (int i = grp; i < units && grp < p.groups; i += p.groups) {
-            wait(&sm->w_full[wi], wph);
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
-                const uint4 w0 = *reinterpret_cast<const uint4 *>(wrow + (size_t)wi * W_BYTES + ((uint32_t)(32 * half) ^ swz));
-                const uint4 w1 = *reinterpret_cast<const uint4 *>(wrow + (size_t)wi * W_BYTES + ((uint32_t)(32 * half + 16) ^ swz));
-                const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-                uint32_t h[32];
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    uint32_t o[4];
-                    int4x8_to_half2x4_natural(ww[j], o);
-                    h[4 * j] = o[0]; h[4 * j + 1] = o[1]; h[4 * j + 2] = o[2]; h[4 * j + 3] = o[3];
-                }
-                if (half == 0) {
-                    wait(&sm->empty[st], ph ^ 1u);
-                    tc_fence_after();
-                }
-                __syncwarp();
-                tmem_st_32x32b_x32(ta + (uint32_t)(st * A_STAGE_COLS + half * (KB / 2)), h);
-            }
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            // The slot is given back here and not right behind the loads above: an arrive does not wait for loads in flight,
-            // and with the tensor core reading shared memory hard the next TMA box was seen to overtake them.
-            if (lane == 0) { mbar_arrive(&sm->full[st]); mbar_arrive(&sm->w_empty[wi]); }
-            wi += p.groups;
-            if (wi >= p.wst) { wi -= p.wst; wph ^= 1u; }
-            st += p.groups;
-            if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
+            umma_commit(&sm->all_done);
         }
     } else if (SPARSE && warp >= SCAT_WARP0) {
         // ================= scatter: the unit's sparse entries -> zeroed FP16 tile in shared memory (A operand) =================
@@ -366,16 +327,64 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
         }
     } else {
+        const int grp = (warp - 2) >> 2;                 // converter group; MAX_GROUPS: the epilogue warps
+        if (grp < p.groups) {
+        // ================= converters: packed INT4 (smem) -> FP16 -> A operand in tensor memory =================
+        const int q = warp & 3;                          // tensor-memory lane quarter this warp may touch
+        const int row = q * 32 + lane;                   // weight row inside the tile
+        const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;     // 64-byte swizzle: 16-byte chunk c sits at c ^ ((row >> 1) & 3)
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(p.nacc * p.acc_cols);
+        const unsigned char *wrow = ws + row * (KP / 2);
+        int wi = grp, st = grp;                          // slot and stage of the group's unit
+        uint32_t wph = 0, ph = 0;
+        for (int i = grp; i < units; i += p.groups) {
+            wait(&sm->w_full[wi], wph);
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                const uint4 w0 = *reinterpret_cast<const uint4 *>(wrow + (size_t)wi * W_BYTES + ((uint32_t)(32 * half) ^ swz));
+                const uint4 w1 = *reinterpret_cast<const uint4 *>(wrow + (size_t)wi * W_BYTES + ((uint32_t)(32 * half + 16) ^ swz));
+                const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                uint32_t h[32];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    uint32_t o[4];
+                    int4x8_to_half2x4_natural(ww[j], o);
+                    h[4 * j] = o[0]; h[4 * j + 1] = o[1]; h[4 * j + 2] = o[2]; h[4 * j + 3] = o[3];
+                }
+                if (half == 0) {
+                    wait(&sm->empty[st], ph ^ 1u);
+                    tc_fence_after();
+                }
+                __syncwarp();
+                tmem_st_32x32b_x32(ta + (uint32_t)(st * A_STAGE_COLS + half * (KB / 2)), h);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            // The slot is given back here and not right behind the loads above: an arrive does not wait for loads in flight,
+            // and with the tensor core reading shared memory hard the next TMA box was seen to overtake them.
+            if (lane == 0) { mbar_arrive(&sm->full[st]); mbar_arrive(&sm->w_empty[wi]); }
+            wi += p.groups;
+            if (wi >= p.wst) { wi -= p.wst; wph ^= 1u; }
+            st += p.groups;
+            if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
+        }
+        }
+        // The CTA's last piece is finished by the converters too, which have nothing left to do: five sets of four warps take
+        // every fifth chunk of 16 tokens.  (Collecting the other pieces of a cut tile is a chain of loads from L2 per chunk: by
+        // the four epilogue warps alone it took 15-25 us at the end of a forward.)
         // ================= epilogue: TMEM -> (+ partials) -> scale, sparse term, bias -> FP16 -> global =================
-        // these warps alone read what the long-row pre-pass wrote
         if (SPARSE && p.n_long > 0) asm volatile("griddepcontrol.wait;" ::: "memory");
         const int q = warp & 3;                          // TMEM lane quarter of this warp
-        const int et = (warp - EPI_WARP0) * 32 + lane;   // 0..127 among the epilogue threads
+        const int et = (warp - EPI_WARP0) * 32 + lane;   // 0..127 among the epilogue threads, negative in the converters
         Pieces pc(t_begin, kp_begin, units, p.kpairs);
         int pos = r_begin;                               // first unit of the current piece
         for (int it = 0; pc.next(); it++) {
             const int a = p.nacc == 2 ? it & 1 : 0, use = p.nacc == 2 ? it >> 1 : it;
-            const bool owner = pc.kp0 == 0;
+            const bool owner = pc.kp0 == 0, last = pc.left == 0;
+            if (!last && grp < MAX_GROUPS) { pos += pc.kp1 - pc.kp0; continue; }
+            const int set = last ? (grp + 1) % (MAX_GROUPS + 1) : 0, sets = last ? MAX_GROUPS + 1 : 1;
+            auto sync_sets = [&]() { if (last) named_bar_sync(2, (CONV_WARPS + EPI_WARPS) * 32); else named_bar_sync(1, EPI_WARPS * 32); };
             const int n = pc.t * TN + q * 32 + lane;     // weight row of this thread
             const bool n_ok = n < p.N;
             // contributors: the CTAs behind this one whose share starts inside the same row tile
@@ -401,7 +410,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             }
             // every row of this warp goes to one plain matrix, with nothing to add beside the accumulators
             const bool plain = !__any_sync(0xffffffffu, li >= 0) && !p.has_ortho && !p.gather;
-            wait(&sm->d_full[a], (uint32_t)(use & 1));
+            if (grp < MAX_GROUPS) wait(&sm->all_done, 0u); else wait(&sm->d_full[a], (uint32_t)(use & 1));
             __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * p.acc_cols);
@@ -423,8 +432,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             };
             if (!owner) {
                 // the first piece of a share that starts inside a tile: its FP32 sums to this CTA's slot, then the flag
-                float *dst = p.slots + (size_t)cta * p.nt * TN + q * 32 + lane;
-                for (int c = 0; c < p.nt; c += 16, dst += 16 * TN) {
+                float *dst = p.slots + ((size_t)cta * p.nt + set * 16) * TN + q * 32 + lane;
+                for (int c = set * 16; c < p.nt; c += sets * 16, dst += sets * 16 * TN) {
                     float v[16];
                     load16(c, v);
 #pragma unroll
@@ -432,9 +441,9 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&sm->d_empty[a]);
+                if (!last && lane == 0) mbar_arrive(&sm->d_empty[a]);
                 __threadfence();
-                named_bar_sync(1, EPI_WARPS * 32);
+                sync_sets();
                 if (et == 0) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p.flags + cta), "l"(p.tag) : "memory");
                 continue;
             }
@@ -452,10 +461,9 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (!ok) { dead = true; atomicExch(p.status, 1); }
                 dead = __any_sync(0xffffffffu, dead);
             }
-            const float *part = p.slots + (size_t)(cta + 1) * p.nt * TN + q * 32 + lane;
+            const float *part = p.slots + ((size_t)(cta + 1) * p.nt + set * 16) * TN + q * 32 + lane;
             const size_t part_cta = (size_t)p.nt * TN;
-            __half *yp = p.y + n;
-            for (int c = 0; c < p.nt; c += 16, part += 16 * TN) {
+            for (int c = set * 16; c < p.nt; c += sets * 16, part += sets * 16 * TN) {
                 __syncwarp();
                 float v[16];
                 load16(c, v);
@@ -468,6 +476,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     for (int j = 0; j < 16; j++) v[j] += t[j];
                 }
                 if (plain) {
+                    __half *yp = p.y + (size_t)c * (size_t)p.ldy + n;
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
                         if (n_ok && c + j < p.M) *yp = __float2half_rn(v[j]);
@@ -476,18 +485,21 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     continue;
                 }
                 if (!n_ok) continue;
+                if (li >= 0) {                           // a long row's sums from the pre-pass
+                    const float4 *o4 = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.ol_mp + c);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float4 t = __ldcg(o4 + j);
+                        v[4 * j] = fmaf(p.alpha, t.x, v[4 * j]); v[4 * j + 1] = fmaf(p.alpha, t.y, v[4 * j + 1]);
+                        v[4 * j + 2] = fmaf(p.alpha, t.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(p.alpha, t.w, v[4 * j + 3]);
+                    }
+                }
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const int m = c + j;
                     if (m >= p.M) break;
                     float o = v[j];
                     if (p.has_ortho) o = fmaf(p.alpha, p.o[(size_t)m * p.N + n], o);
-                    if (li >= 0) {                       // long row: the pre-pass's shares, in share order
-                        float acc = 0.f;
-                        const float *os = p.ol + (size_t)li * p.ol_mp + m;
-                        for (int s = 0; s < p.ol_splits; s++) acc += __ldcg(os + (size_t)s * p.ol_pad * p.ol_mp);
-                        o = fmaf(p.alpha, acc, o);
-                    }
                     const __half hv = __float2half_rn(o);
                     const size_t at = (size_t)m * (size_t)p.ldy + n;
                     if (!p.gather) p.y[at] = hv;
@@ -496,10 +508,11 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             }
             __syncwarp();
             tc_fence_before();
-            if (lane == 0) mbar_arrive(&sm->d_empty[a]);
+            if (!last && lane == 0) mbar_arrive(&sm->d_empty[a]);
             if (c_last > cta) {                          // every reader is past the flags: clear them (a replayed graph brings the same tag)
-                named_bar_sync(1, EPI_WARPS * 32);
-                for (int c = cta + 1 + et; c <= c_last; c += EPI_WARPS * 32) p.flags[c] = 0ull;
+                sync_sets();
+                if (et >= 0)
+                    for (int c = cta + 1 + et; c <= c_last; c += EPI_WARPS * 32) p.flags[c] = 0ull;
             }
         }
     }
@@ -653,7 +666,6 @@ int launch_mid(const FwdArgs &a)
         p.win_off = a.plan->win_off; p.win_words = a.plan->win_words; p.ngroups = (int)ceil_div(a.N, kWinRows);
         if (long_rows) {
             p.row_ptr = a.plan->row_ptr; p.hrow = a.plan->hrow; p.n_long = (int)a.plan->n_long; p.heavy = a.plan->heavy;
-            p.ol_pad = (int)a.plan->n_pad;
         }
     } else if (a.has_ortho) {
         const int Mp = (int)mid_mp(a.M);
@@ -729,7 +741,7 @@ int launch_mid(const FwdArgs &a)
     cfg.attrs = attr; cfg.numAttrs = 1;
     if (p.n_long > 0) {                                  // the long rows' pre-pass right in front
         p.ol_mp = (int)(ceil_div(a.M, 256) * 256);
-        const int st = launch_long_rows(a, p.ol_mp, wsb + own_bytes, &p.ol, &p.ol_splits);
+        const int st = launch_long_rows(a, p.ol_mp, wsb + own_bytes, &p.ol);
         if (st != ORTHO_B200_OK) return st;
     }
     if (sparse) OB_CUDA(cudaLaunchKernelEx(&cfg, mid_kernel<true>, xmap, wmap, p));

@@ -91,9 +91,8 @@ struct Params {
     int *status;
     // sparse term: CSR view (plan entries or raw arrays) and the transposed activations Xt[k][Mp] (zero for m >= M)
     OrthoView ov; const __half *xt; int Mp; float alpha; int has_ortho;
-    // long rows of the plan: the pre-pass of longrows.cu leaves their sums as ol_splits FP32 shares,
-    // ol[(s * ol_pad + h) * Mp + m] for share s, long row h, token m
-    const float *ol; int ol_splits, ol_pad; const int32_t *hrow; int n_long, heavy;
+    // long rows of the plan: the pre-pass of longrows.cu leaves their FP32 sums, ol[h * Mp + m] for long row h, token m
+    const float *ol; const int32_t *hrow; int n_long, heavy;
     // patch != 0 (a plan whose rows list their columns in ascending order): the converters add the sparse entries
     // to the weight tile itself (see the kernel's header); row_max[n] = largest |value| of row n, x = the
     // activations in their own layout for the rows that cannot be patched
@@ -479,25 +478,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
                             }
                         }
                         if (li >= 0) {
-                            const float *src = p.ol + (size_t)li * p.Mp + (size_t)mt * TM + lane * 8;
-                            const size_t sstride = (size_t)p.ol_pad * p.Mp;
-                            for (int s2 = 0; s2 < p.ol_splits; s2 += 4) {             // four shares in flight, added in share order
-                                float4 a0[4], a1[4];
-#pragma unroll
-                                for (int i2 = 0; i2 < 4; i2++) {
-                                    if (s2 + i2 < p.ol_splits) {
-                                        const float4 *sp = reinterpret_cast<const float4 *>(src + (size_t)(s2 + i2) * sstride);
-                                        a0[i2] = __ldcg(sp); a1[i2] = __ldcg(sp + 1);
-                                    }
-                                }
-#pragma unroll
-                                for (int i2 = 0; i2 < 4; i2++) {
-                                    if (s2 + i2 < p.ol_splits) {
-                                        acc[0] += a0[i2].x; acc[1] += a0[i2].y; acc[2] += a0[i2].z; acc[3] += a0[i2].w;
-                                        acc[4] += a1[i2].x; acc[5] += a1[i2].y; acc[6] += a1[i2].z; acc[7] += a1[i2].w;
-                                    }
-                                }
-                            }
+                            const float4 *sp = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.Mp + (size_t)mt * TM + lane * 8);
+                            const float4 a0 = __ldcg(sp), a1 = __ldcg(sp + 1);
+                            acc[0] = a0.x; acc[1] = a0.y; acc[2] = a0.z; acc[3] = a0.w;
+                            acc[4] = a1.x; acc[5] = a1.y; acc[6] = a1.z; acc[7] = a1.w;
                         } else {
                             for (int eb = e0; eb < e1; eb += 32) {
                                 int cl = 0; float vl = 0.f;
@@ -689,15 +673,29 @@ static int64_t prefill_xt_bytes(int64_t M, int64_t K) { return ((K * prefill_mp(
 int64_t prefill_min_workspace_bytes(int64_t M, int64_t K, int64_t N) { (void)N; return prefill_xt_bytes(M, K); }
 // ... and what ortho_b200_workspace_bytes() reports: room behind it for the split-K partial tiles, which the
 // forward uses when it is there (also for base-only calls) and does without otherwise
+int64_t wide_split_bytes();                              // wide.cu
+int launch_wide(const FwdArgs &a, int64_t long_off);
 int64_t prefill_workspace_bytes(int64_t M, int64_t K, int64_t N)
 {
     (void)N;
-    return prefill_xt_bytes(M, K) + (int64_t)pf::kSplitBytes;
+    const int64_t split = (int64_t)pf::kSplitBytes;
+    return prefill_xt_bytes(M, K) + (wide_split_bytes() > split ? wide_split_bytes() : split);
 }
 
 int launch_prefill(const FwdArgs &a)
 {
     using namespace pf;
+    // base-only calls and plans with window lists run the kernel of wide.cu (measured there); the rest, the sparse term as
+    // gathers and the peer exchange, stays here
+    const bool lists = a.has_ortho && a.plan && a.plan->win_off && tuning_snapshot().patch_weights;
+    if (!(a.gv && a.gv->world > 1) && (!a.has_ortho || lists)) {
+        if (lists && a.plan->n_long > 0) {
+            if (!a.workspace || a.workspace_bytes < prefill_xt_bytes(a.M, a.K) + long_rows_workspace_bytes(a.plan, a.M))
+                return ORTHO_B200_ERR_WORKSPACE;
+            if (((uintptr_t)a.workspace & 255u) != 0) return ORTHO_B200_ERR_ALIGN;
+        }
+        return launch_wide(a, prefill_xt_bytes(a.M, a.K));
+    }
     Params p;
     memset(&p, 0, sizeof(p));
     p.alpha = a.alpha; p.has_ortho = 0; p.K = (int)a.K;
@@ -723,7 +721,7 @@ int launch_prefill(const FwdArgs &a)
             const int64_t lr = long_rows_workspace_bytes(a.plan, a.M);
             if (!a.workspace || a.workspace_bytes < prefill_xt_bytes(a.M, a.K) + lr) return ORTHO_B200_ERR_WORKSPACE;
             if (((uintptr_t)a.workspace & 255u) != 0) return ORTHO_B200_ERR_ALIGN;
-            p.hrow = a.plan->hrow; p.n_long = (int)a.plan->n_long; p.heavy = a.plan->heavy; p.ol_pad = (int)a.plan->n_pad;
+            p.hrow = a.plan->hrow; p.n_long = (int)a.plan->n_long; p.heavy = a.plan->heavy;
         }
     }
     CUtensorMap xmap, wmap;
@@ -775,7 +773,7 @@ int launch_prefill(const FwdArgs &a)
         // The pre-pass goes right in front of the main kernel, which is launched as its programmatic dependent: the
         // main kernel's CTAs move in as the pre-pass's CTAs leave, and only its epilogue warps wait for the sums.
         const int st2 = launch_long_rows(a, p.Mp, reinterpret_cast<unsigned char *>(a.workspace) + prefill_xt_bytes(a.M, a.K),
-                                         &p.ol, &p.ol_splits);
+                                         &p.ol);
         if (st2 != ORTHO_B200_OK) return st2;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
