@@ -259,6 +259,8 @@ int launch_decode_multi(const FwdArgs *layers, int nl);   // decode.cu: one stre
 int launch_prefill(const FwdArgs &a);
 int64_t long_rows_workspace_bytes(const Plan *pl, int64_t M);            // longrows.cu
 int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out);
+float *long_rows_rest(const FwdArgs &a, int Mp, void *ws);
+int launch_long_finish(const FwdArgs &a, int Mp, void *ws);
 int plan_build_long_rows(Plan *pl, cudaStream_t st, bool *dup_out);      // longrows.cu; returns a cudaError_t
 int64_t prefill_workspace_bytes(int64_t M, int64_t K, int64_t N);
 int64_t min_workspace_bytes(int64_t M, int64_t K, int64_t N);

@@ -11,12 +11,13 @@
 //     OL = HD * X^T        (tcgen05.mma kind::f16, both operands K-major from shared memory via TMA, FP32 in TMEM)
 //
 // tile = 128 long rows x 256 tokens, K cut into `nsplit` shares so that the few tiles fill the GPU; every share
-// leaves its FP32 sums in the workspace and a second small kernel adds the shares, in share order (no atomics: the
-// result does not depend on scheduling).  (Left to the main kernel's epilogue, where a thread holds a row, the shares of a
-// long row are dependent loads by the thousand: 8192->8192 with Zipf rows at 512 tokens took 923 us that way.)  X is
-// read in its own layout, the transposed copy is not needed here.  Each of the three kernels is launched as a
-// programmatic dependent of the one before: the main kernel's pipeline starts while these drain, only the warps that
-// read the sums wait for them.
+// leaves its FP32 sums in the workspace and a small kernel adds the shares, in share order (no atomics: the result does
+// not depend on scheduling).  X is read in its own layout, the transposed copy is not needed here.
+// Where the sums meet the rest of the row depends on the main kernel.  mid.cu and prefill.cu add them in their epilogues
+// (long_sum_kernel runs before them; they are launched as programmatic dependents, so their pipelines start while these
+// kernels drain and only the warps that read the sums wait).  wide.cu, whose epilogue is exposed and holds a row per
+// thread, leaves the FP32 values of the long rows in the workspace instead of loading sums, and long_finish_kernel adds the
+// shares and rounds once: 8192->8192 with Zipf rows at 2048 tokens 313 us with the loads in the epilogue, FINISH_US so.
 // The reference walks every coordinate serially per token (src/ortho.c:384-398).
 #include <cstring>
 
@@ -160,6 +161,27 @@ long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, in
     part[i] = acc;
 }
 
+// y[m, hrow[h]] = FP16(rest[h, m] + alpha * (part[0] + ... + part[nsplit - 1])[h, m]); one token per thread
+__global__ void __launch_bounds__(256)
+long_finish_kernel(const float *__restrict__ part, long long stride, int nsplit, const float *__restrict__ rest,
+                   const int32_t *__restrict__ hrow, float alpha, __half *__restrict__ y, long long ldy, int M, int Mp)
+{
+    const int m = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (m >= M) return;
+    const float *src = part + (size_t)h * Mp + m;
+    const float base = __ldcg(rest + (size_t)h * Mp + m);
+    float acc = 0.f;
+    for (int s = 0; s < nsplit; s += 8) {
+        float t[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) t[j] = s + j < nsplit ? __ldcg(src + (size_t)(s + j) * stride) : 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc += t[j];
+    }
+    y[(size_t)m * (size_t)ldy + hrow[h]] = __float2half_rn(fmaf(alpha, acc, base));
+}
+
 // ---- plan side: the dense copy of the long rows --------------------------------------------------------------
 // One CTA per long row: writes the row's entries into the (zeroed) dense row and marks every column in a
 // shared-memory bitmap; a column met twice (a CSR row that repeats a column, which the dense form cannot hold)
@@ -222,16 +244,37 @@ int plan_build_long_rows(Plan *pl, cudaStream_t st, bool *dup_out)
     return (int)e;
 }
 
-// per-share sums: nsplit * n_pad * Mp floats
+// per-share sums and one set more for what wide.cu leaves of the rows: (nsplit + 1) * n_pad * Mp floats
 int64_t long_rows_workspace_bytes(const Plan *pl, int64_t M)
 {
     if (!pl || pl->n_long == 0) return 0;
     const int64_t Mp = lr_mp(M);
-    return (((int64_t)long_rows_splits(pl, M) * pl->n_pad * Mp * 4 + 255) / 256) * 256;
+    return (((int64_t)(long_rows_splits(pl, M) + 1) * pl->n_pad * Mp * 4 + 255) / 256) * 256;
 }
 
 // ws: long_rows_workspace_bytes() bytes, 256-byte aligned; Mp = tokens rounded up to 256.  The sum of long row h for
-// token m is (*sums_out)[h * Mp + m].
+// token m is (*sums_out)[h * Mp + m].  With sums_out == nullptr the shares stay apart for launch_long_finish, and the
+// main kernel leaves its part of row h at long_rows_rest(...)[h * Mp + m].
+float *long_rows_rest(const FwdArgs &a, int Mp, void *ws)
+{
+    return reinterpret_cast<float *>(ws) + (size_t)long_rows_splits(a.plan, a.M) * (size_t)a.plan->n_pad * (size_t)Mp;
+}
+int launch_long_finish(const FwdArgs &a, int Mp, void *ws)
+{
+    const Plan *pl = a.plan;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)ceil_div(a.M, 256), (unsigned)pl->n_long); cfg.blockDim = dim3(256); cfg.stream = a.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    const float *part = reinterpret_cast<const float *>(ws), *rest = long_rows_rest(a, Mp, ws);
+    OB_CUDA(cudaLaunchKernelEx(&cfg, long_finish_kernel, part, (long long)pl->n_pad * Mp, long_rows_splits(pl, a.M), rest,
+                               (const int32_t *)pl->hrow, a.alpha, a.y, (long long)a.pitch_y(), (int)a.M, Mp));
+    count_launch();
+    return ORTHO_B200_OK;
+}
 int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
 {
     using namespace lg;
@@ -260,6 +303,7 @@ int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
     long_gemm_kernel<<<g1, NWARPS * 32, kSmemBytes, a.stream>>>(amap, xmap, p);
     count_launch();
     OB_CUDA(cudaGetLastError());
+    if (!sums_out) return ORTHO_B200_OK;
     if (p.nsplit > 1) {
         const long long quads = (long long)p.n_long * Mp / 4, stride = (long long)p.n_pad * Mp / 4;
         cudaLaunchConfig_t cfg;

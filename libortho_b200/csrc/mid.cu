@@ -408,8 +408,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     li = lo;
                 }
             }
-            // every row of this warp goes to one plain matrix, with nothing to add beside the accumulators
-            const bool plain = !__any_sync(0xffffffffu, li >= 0) && !p.has_ortho && !p.gather;
+            // every row of this warp goes to one plain matrix; some row of it is a long one
+            const bool plain = !p.has_ortho && !p.gather, longs = SPARSE && __any_sync(0xffffffffu, li >= 0);
             if (grp < MAX_GROUPS) wait(&sm->all_done, 0u); else wait(&sm->d_full[a], (uint32_t)(use & 1));
             __syncwarp();
             tc_fence_after();
@@ -475,6 +475,15 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
 #pragma unroll
                     for (int j = 0; j < 16; j++) v[j] += t[j];
                 }
+                if (longs && li >= 0) {                           // a long row's sums from the pre-pass
+                    const float4 *o4 = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.ol_mp + c);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const float4 t = __ldcg(o4 + j);
+                        v[4 * j] = fmaf(p.alpha, t.x, v[4 * j]); v[4 * j + 1] = fmaf(p.alpha, t.y, v[4 * j + 1]);
+                        v[4 * j + 2] = fmaf(p.alpha, t.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(p.alpha, t.w, v[4 * j + 3]);
+                    }
+                }
                 if (plain) {
                     __half *yp = p.y + (size_t)c * (size_t)p.ldy + n;
 #pragma unroll
@@ -485,15 +494,6 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     continue;
                 }
                 if (!n_ok) continue;
-                if (li >= 0) {                           // a long row's sums from the pre-pass
-                    const float4 *o4 = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.ol_mp + c);
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float4 t = __ldcg(o4 + j);
-                        v[4 * j] = fmaf(p.alpha, t.x, v[4 * j]); v[4 * j + 1] = fmaf(p.alpha, t.y, v[4 * j + 1]);
-                        v[4 * j + 2] = fmaf(p.alpha, t.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(p.alpha, t.w, v[4 * j + 3]);
-                    }
-                }
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const int m = c + j;

@@ -75,7 +75,7 @@ struct Params {
     float alpha;
     const uint32_t *win_off, *win_words; int ngroups;
     OrthoView ov; const float *row_max; const __half *x;                  // rows that FP16 cannot hold are gathered from x
-    const float *ol; int ol_mp; const int32_t *hrow; int n_long, heavy;
+    float *rest; int rest_mp; const int32_t *hrow; int n_long, heavy;     // long rows: their FP32 values go to `rest` (longrows.cu)
     int *status;
 };
 
@@ -410,8 +410,8 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
                     }
                 }
             }
-            const bool special = li >= 0 || e1 > e0;
-            const bool plain = !SPARSE || !__any_sync(0xffffffffu, special);
+            const bool gathers = SPARSE && __any_sync(0xffffffffu, e1 > e0), longs = SPARSE && __any_sync(0xffffffffu, li >= 0);
+            const bool n_st = n_ok && li < 0;            // this row goes to y from here
             if (grp < GROUPS) wait(&sm->all_done, 0u); else wait(&sm->d_full[a], (uint32_t)(use & 1));
             __syncwarp();
             tc_fence_after();
@@ -464,44 +464,32 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
 #pragma unroll
                     for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + t[j]);
                 }
-                if (plain) {
-                    __half *yp = p.y + (size_t)(m0 + c) * (size_t)p.ldy + n;
-#pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        if (n_ok && m0 + c + j < p.M) *yp = __float2half_rn(fmaf(__uint_as_float(r[j]), sc, bs));
-                        yp += p.ldy;
-                    }
-                    continue;
-                }
-                if (!n_ok) continue;
 #pragma unroll
                 for (int j = 0; j < 16; j++) r[j] = __float_as_uint(fmaf(__uint_as_float(r[j]), sc, bs));
-                if (li >= 0) {                           // a long row's sums from the pre-pass (its rows are 256 tokens a time)
-                    const float4 *o4 = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.ol_mp + m0 + c);
+                if (longs && li >= 0) {                  // a long row: its other sums are added by long_finish_kernel
+                    float4 *dst = reinterpret_cast<float4 *>(p.rest + (size_t)li * p.rest_mp + m0 + c);      // (rows of 256 tokens a time)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if (m0 + c + 4 * j >= p.M) break;
-                        const float4 t = __ldcg(o4 + j);
-                        const float tt[4] = {t.x, t.y, t.z, t.w};
+                    for (int j = 0; j < 4; j++)
+                        dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                                             __uint_as_float(r[4 * j + 3]));
+                }
+                if (gathers && e1 > e0) {                // outside the FP16 range of the weight tile: straight from x
+#pragma unroll 1
+                    for (int e = e0; e < e1; e++) {
+                        int k; float ev;
+                        ortho_entry(p.ov, e, p.K, k, ev);
+                        ev *= p.alpha;
 #pragma unroll
-                        for (int i = 0; i < 4; i++) r[4 * j + i] = __float_as_uint(fmaf(p.alpha, tt[i], __uint_as_float(r[4 * j + i])));
+                        for (int j = 0; j < 16; j++)
+                            if (m0 + c + j < p.M)
+                                r[j] = __float_as_uint(fmaf(ev, __half2float(p.x[(size_t)(m0 + c + j) * p.K + k]), __uint_as_float(r[j])));
                     }
                 }
+                __half *yp = p.y + (size_t)(m0 + c) * (size_t)p.ldy + n;
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
-                    const int m = m0 + c + j;
-                    if (m >= p.M) break;
-                    float v = __uint_as_float(r[j]);
-                    if (e1 > e0) {                  // outside the FP16 range of the weight tile: straight from x
-                        float acc = 0.f;
-                        for (int e = e0; e < e1; e++) {
-                            int k; float ev;
-                            ortho_entry(p.ov, e, p.K, k, ev);
-                            acc = fmaf(ev, __half2float(p.x[(size_t)m * p.K + k]), acc);
-                        }
-                        v = fmaf(p.alpha, acc, v);
-                    }
-                    p.y[(size_t)m * (size_t)p.ldy + n] = __float2half_rn(v);
+                    if (n_st && m0 + c + j < p.M) *yp = __float2half_rn(__uint_as_float(r[j]));
+                    yp += p.ldy;
                 }
             }
             __syncwarp();
@@ -602,8 +590,10 @@ int launch_wide(const FwdArgs &a, int64_t long_off)
         attr_set[dev] = true;
     }
     if (p.n_long > 0) {
-        p.ol_mp = (int)(ceil_div(a.M, 256) * 256);
-        const int st = launch_long_rows(a, p.ol_mp, reinterpret_cast<unsigned char *>(a.workspace) + long_off, &p.ol);
+        void *lw = reinterpret_cast<unsigned char *>(a.workspace) + long_off;
+        p.rest_mp = (int)(ceil_div(a.M, 256) * 256);
+        p.rest = long_rows_rest(a, p.rest_mp, lw);
+        const int st = launch_long_rows(a, p.rest_mp, lw, nullptr);
         if (st != ORTHO_B200_OK) return st;
     }
     cudaLaunchConfig_t cfg;
@@ -616,6 +606,7 @@ int launch_wide(const FwdArgs &a, int64_t long_off)
     if (sparse) OB_CUDA(cudaLaunchKernelEx(&cfg, wide_kernel<true>, xmap, wmap, p));
     else OB_CUDA(cudaLaunchKernelEx(&cfg, wide_kernel<false>, xmap, wmap, p));
     count_launch();
+    if (p.n_long > 0) return launch_long_finish(a, p.rest_mp, reinterpret_cast<unsigned char *>(a.workspace) + long_off);
     return ORTHO_B200_OK;
 }
 
