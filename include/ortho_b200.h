@@ -108,19 +108,20 @@ ORTHO_B200_API int ortho_b200_dequant_dump(const void *q_weight, const void *q_s
  * torch_bind/ortho_linear.py:142-151); same argument order and meaning, plus explicit sizes,
  * the optional plan, a caller-owned workspace and the stream.
  *
- *   M <= 16   : memory-bound streaming kernels; also M <= 32 on layers of at most 4096 x 4096 weights, and, for
- *               calls without a workspace, M <= 24, M <= 32 with N <= 4096 and M <= 64 with N <= 1024 while
- *               N * K <= 4096 * 8192 (ORTHO_B200_DECODE_MAX_M is the most these kernels accept).  No global scratch.
- *   17 .. 128 : tcgen05 kernel with the token block as the MMA's M operand (256 weight rows per instruction),
- *               taken when the call brings ortho_b200_workspace_bytes(M, K, N) bytes of workspace, whatever alpha
- *               is; without it the call runs the kernel of the neighbouring regime.  With a plan whose rows are in
- *               column order and that lists no long rows, the sparse entries are folded into its weight tile.
- *   larger M  : tcgen05 / TMEM prefill kernel (weight tile as the M operand).  With an active ortho term
- *               (alpha > 0 and nnz > 0) and a plan whose rows are in column order the entries are folded into the
- *               weight tile, and the workspace is needed only when the plan lists long rows (their tensor-core
- *               pre-pass sums; same size and layout as below); without such a plan the kernel gathers the term and
- *               needs the workspace for the transposed activations.  Missing workspace that is needed:
- *               ERR_WORKSPACE.  Otherwise the workspace is optional (split-K of the last wave).
+ *   M <= 16   : memory-bound streaming kernels, except where the next kernel is faster (9 .. 16 tokens on layers of more
+ *               than 4096 x 4096 weights, fewer with large activations; it then needs its workspace); the mma.sync
+ *               kernel also serves M <= 32 on layers of at most 4096 x 4096 weights when the sparse term is active
+ *               without an ordered plan, and, for calls without a workspace, M <= 24, M <= 32 with N <= 4096 and
+ *               M <= 64 with N <= 1024 while N * K <= 4096 * 8192 (ORTHO_B200_DECODE_MAX_M is the most it accepts).
+ *               No global scratch.
+ *   17 .. 128 : tcgen05 / TMEM kernel for small token blocks, taken when the call brings
+ *               ortho_b200_workspace_bytes(M, K, N) bytes of workspace, whatever alpha is; without it the call runs the
+ *               kernel of the neighbouring regime.  With a plan whose rows are in column order (ordered plan) the sparse
+ *               entries are contracted on the tensor cores as well.
+ *   larger M  : tcgen05 / TMEM kernels.  Base-only calls and ordered plans: the workspace is needed only when the plan
+ *               lists long rows (their tensor-core pre-pass sums; same size and layout as below), otherwise it is
+ *               optional (tiles of the last wave cut along K).  Without an ordered plan the kernel gathers the term and
+ *               needs the workspace for the transposed activations.  Missing workspace that is needed: ERR_WORKSPACE.
  * Size the workspace with ortho_b200_workspace_bytes / ortho_b200_plan_workspace_bytes and pass it, 256-byte
  * aligned, whenever that is not 0.  The first forward of a kernel variant on a device sets function attributes:
  * issue it outside any stream capture.
@@ -315,7 +316,7 @@ ORTHO_B200_API int ortho_b200_query_kernel_status(void);
  *                    ring slots per warp (either may be 0 for the built-in choice);
  *   row_groups == -3: forwards with more than k_split tokens (0..ORTHO_B200_DECODE_MAX_M) use the
  *                    tensor-core kernels (built-in: 24);
- *   row_groups == -4: forwards with unroll < tokens <= k_split (<= 128) use the tokens-as-M tensor-core kernel
+ *   row_groups == -4: forwards with unroll < tokens <= k_split (<= 128) use the tensor-core kernel for small token blocks
  *                    before any other rule (unroll == k_split: never); 0, 0 restores the built-in rule;
  *   row_groups == -5: plans created after the call treat rows of more than max(k_split, 4 x the mean row)
  *                    entries as long rows (8..65536; 0 restores the built-in 64);

@@ -214,6 +214,25 @@ __device__ __forceinline__ float butterfly_reduce(float (&v)[V], int lane)
     return r;
 }
 
+// ---- quantisation as the reference rounds it --------------------------------------------------------------
+// The library is built with fast-math; the packer and the sieve need the IEEE operations spelled out.
+__device__ __forceinline__ float div_ieee(float a, float b) { float r; asm("div.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float rint_even(float a) { float r; asm("cvt.rni.f32.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
+__device__ __forceinline__ float rcp_approx(float a) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
+// Reciprocal of a row scale for quant_clamped, or 0 where the shortcut below does not hold.
+__device__ __forceinline__ float quant_rscale(float scale) { return scale >= 1e-30f && scale <= 1e30f ? rcp_approx(scale) : 0.f; }
+// clamp(round_half_even(w / scale), -8, 7) with the IEEE division, NaN where that is NaN.  The division itself (some 15
+// instructions) is only done near a tie: w * rscale is within 2^-21 of the quotient relatively, so for a quotient below 16 the
+// two round alike unless the product is within 1e-4 of a half-integer, and from 16 on the clamp decides.
+__device__ __forceinline__ float quant_clamped(float w, float scale, float rscale)
+{
+    const float t = w * rscale;
+    float q = rint_even(t);
+    const bool sure = rscale != 0.f && (fabsf(t) >= 16.f || fabsf(t - q) < 0.4999f);       // NaN: not sure
+    if (!sure) q = rint_even(div_ieee(w, scale));
+    return q != q ? q : fminf(fmaxf(q, -8.f), 7.f);
+}
+
 // streaming 128-bit load of read-once weight bytes: bypass L1 allocation
 __device__ __forceinline__ uint4 ldg_stream(const void *p) {
     uint4 v;

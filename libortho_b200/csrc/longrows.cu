@@ -17,7 +17,7 @@
 // (long_sum_kernel runs before them; they are launched as programmatic dependents, so their pipelines start while these
 // kernels drain and only the warps that read the sums wait).  wide.cu, whose epilogue is exposed and holds a row per
 // thread, leaves the FP32 values of the long rows in the workspace instead of loading sums, and long_finish_kernel adds the
-// shares and rounds once: 8192->8192 with Zipf rows at 2048 tokens 313 us with the loads in the epilogue, FINISH_US so.
+// shares and rounds once: 8192->8192 with Zipf rows at 2048 tokens 313 us with the loads in the epilogue, 222 so.
 // The reference walks every coordinate serially per token (src/ortho.c:384-398).
 #include <cstring>
 

@@ -11,7 +11,9 @@
 // a shared-memory B tile of 256 rows) spent 512 cycles of tensor pipe per 256 x 64 weights whatever the token count
 // and 4 bytes of shared-memory traffic per weight.  What bounds it now is the conversion: 12 instructions per eight
 // weights, two thirds of them on the integer pipe (about 130 of those 180 cycles), plus the sparse entries.
-// MEASURED
+// One B200, us, base-only / 0.3 % entries, against the form before: 8192->10240 at 32 tokens 17 / 22 (45 / 54), at 128
+// 24 / 33 (83 / 90); 8192->57344 at 32 tokens 59 / 84 (169 / 185), at 128 99 / 170 (198 / 224); 28672->8192 at 100 tokens
+// 48 / 72 (129 / 135).
 // Replaces, for this token range, the reference's one-thread-per-output kernel (src/dual_gemm.cu:176-225) and its WMMA
 // variant (src/dual_gemm_tensor_core.cu:215-337).
 //
@@ -36,7 +38,7 @@
 // of those MMAs comes from that tile (40 to 64 cycles per K = 16, whatever the density).  Adding the entries to the
 // converted weights in registers, a round of predicated additions per entry and row, doubled the work of the
 // converters, whose integer and FP16 pipes are the bound: 8192->57344 at 32 tokens and 0.3 % took 122 us that way against
-// 64 base-only and SCATTER_US now.  The plan's long rows come from the tensor-core pre-pass of longrows.cu.
+// 64 base-only, 84 with the scattered tiles.  The plan's long rows come from the tensor-core pre-pass of longrows.cu.
 // Without such a plan the term is computed ahead into O[m][n] (token-major FP32, in the workspace) by
 // ortho_tokens_kernel from the once-transposed activations (a warp per 8 weight rows, lanes = tokens) and added in
 // the FP32 epilogue.
@@ -728,7 +730,7 @@ int launch_mid(const FwdArgs &a)
     if (grid < 1) grid = 1;
     p.share = (int)(total / grid); p.extra = (int)(total % grid);
     // A contributor's flag is "this launch's tag is in my word".  The workspace comes as it is (clearing the words on the
-    // stream first cost TAG_COST per forward), so a tag is a 64-bit value that no other launch of any process has and that
+    // stream first would be one more node per forward, and no programmatic launch past it), so a tag is a 64-bit value that no other launch of any process has and that
     // a stale word holds with probability 2^-64; the collecting CTA clears the words it has seen, so that a replay of
     // a captured graph, which brings the same tag again, finds them cleared.
     p.tag = next_launch_tag();

@@ -1,4 +1,5 @@
-// Prefill-regime (large M) OrthoLinear forward for sm_100a on the 5th-generation tensor cores.
+// Prefill-regime (large M) OrthoLinear forward for sm_100a on the 5th-generation tensor cores, for the calls that wide.cu
+// does not take: a sparse term that has to be gathered (raw CSR, unordered plan) and the peer exchange of a sharded layer.
 //
 // Replaces the reference's WMMA kernels (src/dual_gemm_tensor_core.cu:70-174, 215-337), which
 // quantise activations to int8 and scan the whole coordinate list per output element.  Here the
@@ -276,17 +277,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
             }
             for (int kb4 = un.kb0; kb4 < un.kb1; kb4 += WKB) {
                 // one packed-weight stage = four k blocks (kb0 is a multiple of four): this thread's four 16-byte slices
-                // go to registers at once and the stage is handed back right away, so that its next load has the
-                // time of three more k blocks to arrive
+                // go to registers at once
                 wait(&sm->w_full[wsi], wph);
                 const unsigned char *wrow = ws + (size_t)wsi * W_BYTES + row * 128;
                 uint4 wq[WKB];
 #pragma unroll
                 for (int sub = 0; sub < WKB; sub++)
                     wq[sub] = *reinterpret_cast<const uint4 *>(wrow + ((((uint32_t)(2 * sub + half)) ^ swz) << 4));
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sm->w_empty[wsi]);
-                if (++wsi == WSTAGES) { wsi = 0; wph ^= 1u; }
 #pragma unroll
                 for (int sub = 0; sub < WKB; sub++) {
                 const int kb = kb4 + sub;
@@ -347,6 +344,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__
                 pend_as = as;
                 if (++as == ASTAGES) { as = 0; aph ^= 1u; }
                 }
+                // the stage is given back behind the stores that use all of its slices: an arrive does not wait for the
+                // loads above, and the next TMA box can overtake loads in flight (seen in mid.cu)
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm->w_empty[wsi]);
+                if (++wsi == WSTAGES) { wsi = 0; wph ^= 1u; }
             }
         }
         if (pend_as >= 0) {

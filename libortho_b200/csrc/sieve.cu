@@ -9,28 +9,35 @@
 //   score     = residual^2 / (diag(H_inv) + 1e-6)
 //   ortho     = residual * (score > threshold)
 // The threshold is a given constant (curvature threshold) or the k-th largest score ("keep the top
-// fraction", tools/sieve.py:61-66); the k-th largest is found with a four-pass byte-wise radix select over
-// the scores' bit patterns, recomputing the scores from W in every pass instead of storing them.
-// Everything is element-wise, HBM-bound work: W is read once per pass with 16-byte loads.
+// fraction", tools/sieve.py:61-66), found by a radix select over the scores' order-preserving keys: the first pass over W
+// takes the row scales and counts the keys' top 12 bits; the second counts the next 10 bits of the keys in the
+// selected bin and lists those keys (in the residual's output buffer, which is written later); the last 10 bits are
+// counted from that short list.  The last CTA of each pass selects the bin.
+// Everything is element-wise work; with the IEEE divisions (two of some 15 instructions per weight and pass) spelled out
+// each pass was bound by instructions, so they are only done where an approximate quotient cannot decide:
+// near a rounding tie (quant_clamped), near the edge of a bin or near the threshold.
+// 4096->11008, keep the top 1 %: 344 us for the call (rows 115, bin 126, list 8, split 94); six passes with the divisions
+// spelled out took about 700.
+#include <cstring>
+
 #include "common.cuh"
 
 namespace ob {
 
-__device__ __forceinline__ float sv_div(float a, float b) { float r; asm("div.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ float sv_rint(float a) { float r; asm("cvt.rni.f32.f32 %0, %1;" : "=f"(r) : "f"(a)); return r; }
 __device__ __forceinline__ bool sv_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
-// base value and residual of one weight; returns the score
-__device__ __forceinline__ float sieve_one(float w, float scale, float hs, float &base, float &res)
+// base value and residual of one weight; returns residual^2
+__device__ __forceinline__ float sieve_one(float w, float scale, float rscale, float &base, float &res)
 {
-    float q = sv_rint(sv_div(w, scale));
-    const bool q_nan = (q != q);
-    q = fminf(fmaxf(q, -8.f), 7.f);
+    const float q = quant_clamped(w, scale, rscale);
     base = __fmul_rn(q, scale);
-    if (q_nan || !sv_finite(base)) base = 0.f;
+    if (q != q || !sv_finite(base)) base = 0.f;
     res = __fsub_rn(w, base);
-    return sv_div(__fmul_rn(res, res), hs);
+    return __fmul_rn(res, res);
 }
+// The score is r2 / hs in IEEE arithmetic.  r2 * rcp(hs) is within 2^-21 of it relatively while everything is in the normal
+// range with room: the callers use it only then.
+__device__ __forceinline__ bool approx_ok(float r2, float hs) { return r2 >= 1e-30f && r2 <= 1e30f && hs >= 1e-30f && hs <= 1e4f; }
 // order-preserving map of a float to an unsigned key (larger float <-> larger key)
 __device__ __forceinline__ uint32_t score_key(float s)
 {
@@ -42,87 +49,177 @@ __device__ __forceinline__ float key_score(uint32_t k)
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// one CTA per row: scale[n] = max(rowmax|W|, 1e-8) / 7
+constexpr int kBins0 = 4096, kBins = 1024;       // 12 + 10 + 10 bits
+// radix-select state in device memory, cleared before the first pass
+struct SelectState {
+    unsigned int hist0[kBins0], hist1[kBins], hist2[kBins];
+    unsigned int done[3];                        // CTAs of a pass that have added their counts
+    unsigned int prefix[3];                      // selected bin of each pass
+    unsigned int listed;                         // keys in the list
+    unsigned long long krem[3];                  // rank inside the selected bin
+    float threshold;
+};
+
+// Adds the CTA's counts h[BINS] to the global ones; the last CTA then finds the bin that holds the k-th largest key
+// (k counted from the top bin downwards).  Called by all 256 threads.
+template <int BINS>
+__device__ __forceinline__ void add_and_select(const unsigned int *h, unsigned int *hist, SelectState *st, int pass, unsigned long long k)
+{
+    __shared__ unsigned int is_last;
+    __shared__ unsigned long long warp_sum[8];
+    __syncthreads();
+    for (int i = threadIdx.x; i < BINS; i += 256)
+        if (h[i]) atomicAdd(&hist[i], h[i]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(&st->done[pass], 1u) == gridDim.x - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    // thread t owns bins [t * PER, (t + 1) * PER); keys in the bins above its own: a suffix sum over the threads
+    constexpr int PER = BINS / 256;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    unsigned long long mine = 0;
+    for (int i = 0; i < PER; i++) mine += __ldcg(&hist[t * PER + i]);
+    unsigned long long suf = mine;               // inclusive over lanes >= lane
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_down_sync(0xffffffffu, suf, o);
+        if (lane + o < 32) suf += u;
+    }
+    if (lane == 0) warp_sum[warp] = suf;
+    __syncthreads();
+    unsigned long long above = suf - mine;
+    for (int w2 = warp + 1; w2 < 8; w2++) above += warp_sum[w2];
+    for (int i = PER - 1; i >= 0; i--) {
+        const unsigned long long cnt = __ldcg(&hist[t * PER + i]);
+        if (above < k && k <= above + cnt) { st->prefix[pass] = (unsigned)(t * PER + i); st->krem[pass] = k - above; }
+        above += cnt;
+    }
+    if (pass == 2) {
+        __syncthreads();
+        if (t == 0) st->threshold = key_score((st->prefix[0] << 20) | (st->prefix[1] << 10) | st->prefix[2]);
+    }
+}
+
+// First pass, one CTA per row at a time: scale[n] = max(rowmax|W|, 1e-8) / 7, and with k > 0 the counts of the keys' top
+// 12 bits (the row's second reading hits L1)
 __global__ void __launch_bounds__(256)
-sieve_row_scale_kernel(const float *__restrict__ w, int64_t N, int K, float *__restrict__ scales)
+sieve_rows_kernel(const float *__restrict__ w, const float *__restrict__ hinv, int64_t N, int K, float *__restrict__ scales,
+                  SelectState *__restrict__ st, unsigned long long k)
 {
     __shared__ float wmax[8];
+    __shared__ unsigned int h[kBins0];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (k)
+        for (int i = tid; i < kBins0; i += 256) h[i] = 0;
     for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
         const float4 *row = reinterpret_cast<const float4 *>(w + (size_t)n * K);
         float m = 0.f;
-        for (int i = tid; i < K / 4; i += 256) {
-            const float4 v = row[i];
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        for (int i = tid; i < K / 4; i += 1024) {
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = i + 256 * j < K / 4 ? row[i + 256 * j] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 4; j++) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
         }
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         if (lane == 0) wmax[warp] = m;
         __syncthreads();
-        if (tid == 0) {
-            float mm = wmax[0];
-            for (int i = 1; i < 8; i++) mm = fmaxf(mm, wmax[i]);
-            scales[n] = sv_div(fmaxf(mm, 1e-8f), 7.0f);
-        }
-        __syncthreads();
-    }
-}
-
-// radix-select state in device memory: hist[256], prefix, remaining rank, result
-struct SelectState { unsigned int hist[256]; unsigned int prefix; unsigned long long krem; float threshold; };
-
-// pass p (0 = most significant byte): histogram of byte p of the keys whose higher bytes equal the prefix
-__global__ void __launch_bounds__(256)
-sieve_hist_kernel(const float *__restrict__ w, const float *__restrict__ hinv, const float *__restrict__ scales,
-                  int64_t N, int K, int pass, SelectState *__restrict__ st)
-{
-    __shared__ unsigned int h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t prefix = st->prefix;
-    const int shift = 24 - 8 * pass;
-    const int64_t quads = N * (int64_t)(K / 4);
-    const int kq = K / 4;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < quads; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t n = i / kq;
-        const int c = (int)(i - n * kq) * 4;
-        const float4 v = reinterpret_cast<const float4 *>(w)[i];
-        const float4 hv = *reinterpret_cast<const float4 *>(hinv + c);
-        const float sc = scales[n];
-        const float ww[4] = {v.x, v.y, v.z, v.w}, hh[4] = {hv.x, hv.y, hv.z, hv.w};
+        float mm = wmax[0];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            float b, r;
-            const uint32_t key = score_key(sieve_one(ww[e], sc, __fadd_rn(hh[e], 1e-6f), b, r));
-            if (pass == 0 || (key >> (shift + 8)) == prefix) atomicAdd(&h[(key >> shift) & 255u], 1u);
+        for (int i = 1; i < 8; i++) mm = fmaxf(mm, wmax[i]);
+        const float scale = div_ieee(fmaxf(mm, 1e-8f), 7.0f), rscale = quant_rscale(scale);
+        if (tid == 0) scales[n] = scale;
+        if (k) {
+            for (int i = tid; i < K / 4; i += 256) {
+                const float4 v = row[i];
+                const float4 hv = *reinterpret_cast<const float4 *>(hinv + 4 * i);
+                const float ww[4] = {v.x, v.y, v.z, v.w}, hh[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    float b, r;
+                    const float hs = __fadd_rn(hh[e], 1e-6f), r2 = sieve_one(ww[e], scale, rscale, b, r);
+                    uint32_t bits = __float_as_uint(r2 * rcp_approx(hs));
+                    uint32_t key = bits | 0x80000000u;
+                    if (!approx_ok(r2, hs) || (((bits + 16u) ^ (bits - 16u)) >> 20) != 0u) key = score_key(div_ieee(r2, hs));
+                    atomicAdd(&h[key >> 20], 1u);
+                }
+            }
         }
+        __syncthreads();                         // wmax is reused by the next row
     }
-    __syncthreads();
-    if (h[threadIdx.x]) atomicAdd(&st->hist[threadIdx.x], h[threadIdx.x]);
+    if (k) add_and_select<kBins0>(h, st->hist0, st, 0, k);
 }
 
-// one CTA: the bin that holds the krem-th largest key of this pass; clears the histogram for the next pass
+// Second pass: the keys in the selected bin, counted by their next 10 bits and listed
 __global__ void __launch_bounds__(256)
-sieve_select_kernel(SelectState *__restrict__ st, int pass)
+sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, const float *__restrict__ scales,
+                 int64_t N, int K, SelectState *__restrict__ st, uint32_t *__restrict__ list)
 {
-    __shared__ unsigned long long above[257];
-    const int t = threadIdx.x;
-    if (t == 0) {
-        unsigned long long run = 0;
-        above[256] = 0;
-        for (int b = 255; b >= 0; b--) { above[b] = run; run += st->hist[b]; }     // keys in bins > b
-    }
+    __shared__ unsigned int h[kBins];
+    for (int i = threadIdx.x; i < kBins; i += 256) h[i] = 0;
     __syncthreads();
-    const unsigned long long k = st->krem;
-    const unsigned long long cnt = st->hist[t];
-    const bool mine = above[t] < k && k <= above[t] + cnt;
-    __syncthreads();
-    st->hist[t] = 0;
-    if (mine) {
-        st->prefix = (st->prefix << 8) | (unsigned)t;
-        st->krem = k - above[t];
-        if (pass == 3) st->threshold = key_score((st->prefix));
+    const uint32_t bin = st->prefix[0];
+    const int lane = threadIdx.x & 31;
+    for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
+        const float4 *row = reinterpret_cast<const float4 *>(w + (size_t)n * K);
+        const float sc = scales[n], rs = quant_rscale(sc);
+        for (int i0 = 0; i0 < K / 4; i0 += 1024) {
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = i0 + 256 * j + threadIdx.x < K / 4 ? row[i0 + 256 * j + threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int i = i0 + 256 * j + threadIdx.x;
+                const bool on = i < K / 4;
+                const float4 hv = on ? *reinterpret_cast<const float4 *>(hinv + 4 * i) : make_float4(1.f, 1.f, 1.f, 1.f);
+                const float ww[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, hh[4] = {hv.x, hv.y, hv.z, hv.w};
+                uint32_t key[4];
+                bool in[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    float b, r;
+                    const float hs = __fadd_rn(hh[e], 1e-6f), r2 = sieve_one(ww[e], sc, rs, b, r);
+                    const uint32_t bits = __float_as_uint(r2 * rcp_approx(hs)) | 0x80000000u;
+                    // clearly outside the bin: nothing to do; else the exact key
+                    key[e] = 0;
+                    in[e] = on && !(approx_ok(r2, hs) && (bits + 16u) >> 20 != bin && (bits - 16u) >> 20 != bin);
+                    if (in[e]) { key[e] = score_key(div_ieee(r2, hs)); in[e] = (key[e] >> 20) == bin; }
+                }
+                if (!__any_sync(0xffffffffu, in[0] || in[1] || in[2] || in[3])) continue;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const unsigned m = __ballot_sync(0xffffffffu, in[e]);
+                    if (m == 0u) continue;
+                    unsigned at = 0;
+                    if (lane == __ffs(m) - 1) at = atomicAdd(&st->listed, (unsigned)__popc(m));
+                    at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+                    if (in[e]) {
+                        list[at + __popc(m & ((1u << lane) - 1u))] = key[e];
+                        atomicAdd(&h[(key[e] >> 10) & 1023u], 1u);
+                    }
+                }
+            }
+        }
     }
+    add_and_select<kBins>(h, st->hist1, st, 1, st->krem[0]);
+}
+
+// Third pass: the last 10 bits, from the list
+__global__ void __launch_bounds__(256)
+sieve_list_kernel(SelectState *__restrict__ st, const uint32_t *__restrict__ list)
+{
+    __shared__ unsigned int h[kBins];
+    for (int i = threadIdx.x; i < kBins; i += 256) h[i] = 0;
+    __syncthreads();
+    const unsigned n = st->listed, mid = st->prefix[1];
+    for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const uint32_t key = list[i];
+        if (((key >> 10) & 1023u) == mid) atomicAdd(&h[key & 1023u], 1u);
+    }
+    add_and_select<kBins>(h, st->hist2, st, 2, st->krem[1]);
 }
 
 __global__ void __launch_bounds__(256)
@@ -131,32 +228,43 @@ sieve_split_kernel(const float *__restrict__ w, const float *__restrict__ hinv, 
                    float *__restrict__ w_base, float *__restrict__ w_ortho)
 {
     const float thr = thr_dev ? *thr_dev : thr_host;
-    const int64_t quads = N * (int64_t)(K / 4);
-    const int kq = K / 4;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < quads; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t n = i / kq;
-        const int c = (int)(i - n * kq) * 4;
-        const float4 v = reinterpret_cast<const float4 *>(w)[i];
-        const float4 hv = *reinterpret_cast<const float4 *>(hinv + c);
-        const float sc = scales[n];
-        const float ww[4] = {v.x, v.y, v.z, v.w}, hh[4] = {hv.x, hv.y, hv.z, hv.w};
-        float bo[4], oo[4];
+    const bool thr_ok = thr >= 1e-20f && thr <= 1e20f;
+    const float thr_lo = thr * 0.99999f, thr_hi = thr * 1.00001f;
+    for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
+        const size_t at = (size_t)n * (K / 4);
+        const float sc = scales[n], rs = quant_rscale(sc);
+        for (int i0 = threadIdx.x; i0 < K / 4; i0 += 1024) {
+            float4 v[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            float r;
-            const float s = sieve_one(ww[e], sc, __fadd_rn(hh[e], 1e-6f), bo[e], r);
-            oo[e] = __fmul_rn(r, (s > thr) ? 1.f : 0.f);        // residual * mask, signed zeros as torch produces them
+            for (int j = 0; j < 4; j++)
+                if (i0 + 256 * j < K / 4) v[j] = __ldcs(reinterpret_cast<const float4 *>(w) + at + i0 + 256 * j);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int i = i0 + 256 * j;
+                if (i >= K / 4) break;
+                const float4 hv = *reinterpret_cast<const float4 *>(hinv + 4 * i);
+                const float ww[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, hh[4] = {hv.x, hv.y, hv.z, hv.w};
+                float bo[4], oo[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    float r;
+                    const float hs = __fadd_rn(hh[e], 1e-6f), r2 = sieve_one(ww[e], sc, rs, bo[e], r);
+                    const float s = r2 * rcp_approx(hs);
+                    bool keep = s > thr_hi;
+                    if (!thr_ok || !approx_ok(r2, hs) || (s >= thr_lo && s <= thr_hi)) keep = div_ieee(r2, hs) > thr;
+                    oo[e] = __fmul_rn(r, keep ? 1.f : 0.f);         // residual * mask, signed zeros as torch produces them
+                }
+                reinterpret_cast<float4 *>(w_base)[at + i] = make_float4(bo[0], bo[1], bo[2], bo[3]);
+                reinterpret_cast<float4 *>(w_ortho)[at + i] = make_float4(oo[0], oo[1], oo[2], oo[3]);
+            }
         }
-        reinterpret_cast<float4 *>(w_base)[i] = make_float4(bo[0], bo[1], bo[2], bo[3]);
-        reinterpret_cast<float4 *>(w_ortho)[i] = make_float4(oo[0], oo[1], oo[2], oo[3]);
     }
 }
 
-static unsigned sieve_grid(int64_t quads)
+static unsigned sieve_grid(int64_t N)
 {
-    int64_t blocks = ceil_div(quads, 256 * 4);
     const int64_t cap = (int64_t)device_sm_count(current_device_index()) * 8;
-    return (unsigned)(blocks < 1 ? 1 : blocks > cap ? cap : blocks);
+    return (unsigned)(N > cap ? cap : N);
 }
 
 }  // namespace ob
@@ -179,29 +287,25 @@ extern "C" int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t
     cudaStream_t st = (cudaStream_t)stream;
     float *scales = reinterpret_cast<float *>(scratch);
     SelectState *sel = reinterpret_cast<SelectState *>(reinterpret_cast<unsigned char *>(scratch) + ((N * 4 + 255) / 256) * 256);
-    const int64_t quads = N * (K / 4);
-    sieve_row_scale_kernel<<<(unsigned)(N < 148 * 8 ? N : 148 * 8), 256, 0, st>>>(w, N, (int)K, scales);
-    count_launch();
-    OB_CUDA(cudaGetLastError());
+    const unsigned grid = sieve_grid(N);
     const float *thr_dev = nullptr;
     float thr_host = curvature_thresh;
-    if (keep_top_k > 0) {
-        // threshold = k-th largest score: four histogram passes over the key bytes
-        SelectState init;
-        memset(&init, 0, sizeof(init));
-        init.krem = (unsigned long long)keep_top_k;
-        OB_CUDA(cudaMemcpyAsync(sel, &init, sizeof(init), cudaMemcpyHostToDevice, st));
-        for (int pass = 0; pass < 4; pass++) {
-            sieve_hist_kernel<<<sieve_grid(quads), 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, pass, sel);
-            sieve_select_kernel<<<1, 256, 0, st>>>(sel, pass);
-            count_launch(2);
-            OB_CUDA(cudaGetLastError());
-        }
+    const unsigned long long k = keep_top_k > 0 ? (unsigned long long)keep_top_k : 0ull;
+    if (k) OB_CUDA(cudaMemsetAsync(sel, 0, sizeof(SelectState), st));
+    sieve_rows_kernel<<<grid, 256, 0, st>>>(w, h_inv_diag, N, (int)K, scales, sel, k);
+    count_launch();
+    OB_CUDA(cudaGetLastError());
+    if (k) {
+        uint32_t *list = reinterpret_cast<uint32_t *>(w_ortho_out);          // room for every key; the split writes it last
+        sieve_bin_kernel<<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, list);
+        sieve_list_kernel<<<(unsigned)device_sm_count(current_device_index()), 256, 0, st>>>(sel, list);
+        count_launch(2);
+        OB_CUDA(cudaGetLastError());
         thr_dev = &sel->threshold;
     } else if (keep_top_k == 0) {
         thr_host = __builtin_inff();          // "keep nothing" (tools/sieve.py:65-66)
     }
-    sieve_split_kernel<<<sieve_grid(quads), 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, thr_dev, thr_host, w_base_out, w_ortho_out);
+    sieve_split_kernel<<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, thr_dev, thr_host, w_base_out, w_ortho_out);
     count_launch();
     OB_CUDA(cudaGetLastError());
     return ORTHO_B200_OK;

@@ -22,7 +22,9 @@
 // with one coalesced load a turn ahead and goes through it round by round.  The contraction of scattered tiles that mid.cu
 // uses would double the MMAs, which are the bound here; a round costs about 75 instructions of a warp, and the
 // converters have about twice the time that the base needs.
-// MEASURED_WIDE
+// One B200, us, base-only / fused, against the 128 x 256 tile of prefill.cu: 8192->8192 at 2048 tokens, 0.3 % 190 / 204
+// (265 / 295; 1440 / 1350 TFLOP/s now), at 8192 tokens 783 / 900 (963 / 1174); 4096->4096 at 2048, 1 % 54 / 70 (76 / 108);
+// 8192->8192 with Zipf rows at 512 tokens 54 / 64 (71 / 81).  Bounds: the power cap (cuBLAS sustains 1380) and, fused, the converters.
 //
 // Work split: as many whole waves of tiles as there are, tile after tile with the token tiles of a row tile next to each
 // other (a wave then reads few weight rows, and the activations from L2); the tiles left over are cut along K into

@@ -39,19 +39,19 @@ _WATCHED = frozenset(("base_weight", "base_scales", "bias") + _ORTHO_BUFFERS)
 
 
 class _SharedWorkspace:
-    """One grow-on-demand scratch buffer per device, shared by every module on it (a model with hundreds of
-    layers runs them one at a time).  Forwards that use it must be issued on one stream at a time."""
-    _by_device = {}
+    """One grow-on-demand scratch buffer per device and stream, shared by every module that runs there (a model with
+    hundreds of layers runs them one at a time); forwards on different streams never meet in one."""
+    _by_stream = {}
 
     def __init__(self):
         self.tensor: Optional[torch.Tensor] = None
         self.gen = 0
 
     @classmethod
-    def get(cls, device: torch.device, nbytes: int) -> "_SharedWorkspace":
-        w = cls._by_device.get(device)
+    def get(cls, device: torch.device, nbytes: int, stream: int) -> "_SharedWorkspace":
+        w = cls._by_stream.get((device, stream))
         if w is None:
-            w = cls._by_device[device] = cls()
+            w = cls._by_stream[(device, stream)] = cls()
         if nbytes > 0 and (w.tensor is None or w.tensor.numel() < nbytes):
             w.tensor = torch.empty(nbytes, dtype=torch.uint8, device=device)
             w.gen += 1
@@ -59,7 +59,7 @@ class _SharedWorkspace:
 
 
 class _Bound:
-    """Everything about one (module, token count) forward that does not change from call to call: the C
+    """Everything about one (module, token count, stream) forward that does not change from call to call: the C
     argument record with all buffer pointers, the plan, the workspace.  Built (and validated) once."""
     __slots__ = ("descs", "ws", "ws_gen", "ws_ptr", "ws_bytes", "key", "fused_bias")
 
@@ -181,11 +181,12 @@ class OrthoLinear(nn.Module):
         return need
 
     def _get_workspace(self, M: int) -> Optional[torch.Tensor]:
-        """The device's shared scratch buffer, grown to what a forward of M tokens needs (None if nothing)."""
+        """The current stream's shared scratch buffer, grown to what a forward of M tokens needs (None if nothing)."""
         need = self._workspace_bytes(M)
         if need == 0:
             return None
-        return _SharedWorkspace.get(self.base_weight.device, need).tensor
+        dev = self.base_weight.device
+        return _SharedWorkspace.get(dev, need, _current_stream_handle(dev)).tensor
 
     def _versions(self):
         """What a cached call record depends on besides the token count: the storage of every buffer (a
@@ -195,7 +196,7 @@ class OrthoLinear(nn.Module):
         return (self.base_weight.data_ptr(), self.base_scales.data_ptr(), ov.data_ptr(), oc.data_ptr(), orp.data_ptr(),
                 ov._version, oc._version, orp._version, (b.data_ptr(), b.dtype) if b is not None else None)
 
-    def _bind(self, M: int, dev: torch.device) -> _Bound:
+    def _bind(self, M: int, dev: torch.device, stream: int) -> _Bound:
         N, K = self.out_features, self.in_features
         bw, bs = self.base_weight, self.base_scales
         if bw.dtype != torch.uint8 or bs.dtype != torch.float16:
@@ -216,7 +217,7 @@ class OrthoLinear(nn.Module):
         b = _Bound()
         plan = self._get_plan() if sparse else None
         need = self._workspace_bytes(M)
-        b.ws = _SharedWorkspace.get(dev, need)
+        b.ws = _SharedWorkspace.get(dev, need, stream)
         b.ws_gen = b.ws.gen
         b.ws_ptr = b.ws.tensor.data_ptr() if need else None
         b.ws_bytes = b.ws.tensor.numel() if need else 0
@@ -236,7 +237,7 @@ class OrthoLinear(nn.Module):
         b.key = (self.alpha > 0, self._versions())
         if len(self._bound) > 32:
             self._bound.clear()
-        self._bound[M] = b
+        self._bound[(M, stream)] = b
         return b
 
     # -- forward ---------------------------------------------------------------------------------
@@ -264,20 +265,20 @@ class OrthoLinear(nn.Module):
         fused_bias = False
         if M:
             alpha = float(self.alpha)
-            b = self._bound.get(M)
+            stream = _current_stream_handle(dev)
+            b = self._bound.get((M, stream))
             if b is None or b.key != (alpha > 0, self._versions()) or b.ws_gen != b.ws.gen:
-                b = self._bind(M, dev)
+                b = self._bind(M, dev, stream)
             d = b.descs[0]
             d.y_f16 = output.data_ptr()
             d.alpha = alpha
             fused_bias = b.fused_bias
             fwd = _lib.lib().ortho_b200_forward_multi
             if torch.cuda.current_device() == dev.index:
-                st = fwd(b.descs, 1, x_flat.data_ptr(), M, self.in_features, b.ws_ptr, b.ws_bytes, _current_stream_handle(dev))
+                st = fwd(b.descs, 1, x_flat.data_ptr(), M, self.in_features, b.ws_ptr, b.ws_bytes, stream)
             else:
                 with torch.cuda.device(dev):
-                    st = fwd(b.descs, 1, x_flat.data_ptr(), M, self.in_features, b.ws_ptr, b.ws_bytes,
-                             _current_stream_handle(dev))
+                    st = fwd(b.descs, 1, x_flat.data_ptr(), M, self.in_features, b.ws_ptr, b.ws_bytes, stream)
             if st:
                 _lib.check(st, "ortho_b200_forward_multi")
         if self.bias is not None and not fused_bias:

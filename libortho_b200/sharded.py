@@ -116,7 +116,8 @@ class ShardedOrthoLinear(nn.Module):
         loc = self.local
         dev = x2.device
         alpha = float(loc.alpha)
-        b = self._peer_bound.get(M)
+        stream = _current_stream_handle(dev)
+        b = self._peer_bound.get((M, stream))
         if b is None or b["key"] != (alpha > 0, loc._versions(), id(self._comm), self._comm_off) or b["ws_gen"] != b["ws"].gen:
             rows = self.n1 - self.n0
             nnz = int(loc.ortho_values.numel())
@@ -125,7 +126,7 @@ class ShardedOrthoLinear(nn.Module):
                 raise ValueError("the shard's base_weight / base_scales do not match its rows")
             plan = loc._get_plan() if (alpha > 0 and nnz > 0) else None
             need = _C.workspace_bytes(M, self.in_features, rows, plan) if rows else 0
-            ws = _SharedWorkspace.get(dev, need)
+            ws = _SharedWorkspace.get(dev, need, stream)
             b = {
                 "key": (alpha > 0, loc._versions(), id(self._comm), self._comm_off), "ws": ws, "ws_gen": ws.gen,
                 "head": (loc.base_weight.data_ptr() if rows else None, loc.base_scales.data_ptr() if rows else None,
@@ -139,17 +140,17 @@ class ShardedOrthoLinear(nn.Module):
             }
             if len(self._peer_bound) > 32:
                 self._peer_bound.clear()
-            self._peer_bound[M] = b
+            self._peer_bound[(M, stream)] = b
         slot = self._slot
         self._slot ^= 1
         fwd = _lib.lib().ortho_b200_forward_gather
         args = (*b["head"], x2.data_ptr(), M, self.in_features, self.n1 - self.n0, alpha, *b["tail"],
                 b["off"][slot], self.out_features, self.n0)
         if torch.cuda.current_device() == dev.index:
-            st = fwd(*args, _current_stream_handle(dev))
+            st = fwd(*args, stream)
         else:
             with torch.cuda.device(dev):
-                st = fwd(*args, _current_stream_handle(dev))
+                st = fwd(*args, stream)
         if st:
             _lib.check(st, "ortho_b200_forward_gather")
         return b["out"][slot]
