@@ -348,7 +348,7 @@ int set_decode_config(int wr, int wk, int u, int s)
         t.prefill_above = s;
         return ORTHO_B200_OK;
     }
-    if (wr == -4) {       // forwards with u < tokens <= s (s <= 128) use the tokens-as-M tensor-core kernel whatever the
+    if (wr == -4) {       // forwards with u < tokens <= s (s <= 128) use the kernel of mid.cu whatever the
                           // other rules say (u == s: never); u == s == 0 restores the built-in rule
         if (u < 0 || s < 0 || s > 128 || u > s) return ORTHO_B200_ERR_SHAPE;
         if (u == 0 && s == 0) { t.mid_lo = 16; t.mid_hi = 128; t.mid_first = false; }

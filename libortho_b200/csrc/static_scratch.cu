@@ -65,7 +65,7 @@ extern "C" int ortho_b200_forward_static_scratch(const void *q_weight, const voi
     // same bits; only the tensor-core regime with an active sparse term needs scratch
     const bool decode = decode_regime(M, N, K);
     const int64_t need = (has_ortho && !decode) ? min_workspace_bytes(M, K, N) : 0;
-    // (the tokens-as-M kernel is taken when its scratch fits the array, exactly as ortho_b200_forward takes it when
+    // (the kernel of mid.cu is taken when its scratch fits the array, exactly as ortho_b200_forward takes it when
     // the caller's workspace is large enough; it is never required)
     if (need > (int64_t)ORTHO_B200_STATIC_SCRATCH_BYTES) return ORTHO_B200_ERR_SCRATCH_LIMIT;
 
