@@ -105,6 +105,20 @@ __device__ __forceinline__ void ortho_entry(const OrthoView &ov, int e, int K, i
     }
 }
 
+// Sum of v * x over the entries e0 .. e1 of a plan's row whose column lies in [k0, k1); xr = the token's activations.
+// The tensor-core kernels that contract the entries from a zero-filled tile or matrix take it where their sum is NaN: a
+// zero times an infinite activation is NaN there, while an absent entry contributes nothing.
+__device__ __forceinline__ float entries_sum(const uint32_t *entries, int e0, int e1, int k0, int k1, const __half *xr)
+{
+    float s = 0.f;
+    for (int e = e0; e < e1; e++) {
+        const uint32_t pk = entries[e];
+        const int c = (int)(pk & 0xFFFFu);
+        if (c >= k0 && c < k1) s = fmaf(__half2float(__ushort_as_half((unsigned short)(pk >> 16))), __half2float(xr[c]), s);
+    }
+    return s;
+}
+
 // Scale of a row's weight corrections: a sparse entry v of row n enters the weight tile as v * alpha / scale[n]
 // (the epilogue multiplies the whole row by scale[n]).  Returns 0 when that cannot be represented safely in
 // FP16 next to the integer weights (tiny or zero scale, huge values, NaN): such a row keeps the gather path.

@@ -44,6 +44,8 @@ constexpr size_t kSmemBytes = 1024 + (size_t)ST * (A_BYTES + B_BYTES) + sizeof(S
 struct Params {
     float *part;                        // [nsplit][n_pad][Mp]
     int n_long, n_pad, Mp, kblocks, nsplit;
+    // the rows' entries and the activations, for sums that an infinite activation made NaN (zeros of HD)
+    const uint32_t *entries; const int32_t *row_ptr, *hrow; const __half *x; int M, K;
     int *status;
 };
 }  // namespace lg
@@ -127,12 +129,27 @@ long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 32), r);
             tmem_ld_wait();
             if (row < p.n_long && !dead) {
+                bool nan = false;
+#pragma unroll
+                for (int j = 0; j < 32; j++) nan = nan || __uint_as_float(r[j]) != __uint_as_float(r[j]);
+                uint32_t bad = 0;
+#pragma unroll
+                for (int j = 0; j < 32 && nan; j++) bad |= __uint_as_float(r[j]) != __uint_as_float(r[j]) ? 1u << j : 0u;
+                for (; bad; bad &= bad - 1) {
+                    const int j = __ffs(bad) - 1, m = tok0 + c * 32 + j;
+                    if (m >= p.M) break;
+                    const int n = p.hrow[row];
+                    const uint32_t t = __float_as_uint(entries_sum(p.entries, p.row_ptr[n], p.row_ptr[n + 1], kb0 * KB, kb1 * KB, p.x + (size_t)m * p.K));
+#pragma unroll
+                    for (int i = 0; i < 32; i++) r[i] = i == j ? t : r[i];
+                }
                 float4 *d4 = reinterpret_cast<float4 *>(dst + c * 32);
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     d4[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
                                         __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
             }
+            __syncwarp();
         }
         tc_fence_before();
     }
@@ -283,6 +300,7 @@ int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
     p.part = reinterpret_cast<float *>(ws);
     p.n_long = (int)pl->n_long; p.n_pad = (int)pl->n_pad; p.Mp = Mp;
     p.kblocks = (int)ceil_div(a.K, KB); p.nsplit = long_rows_splits(pl, a.M);
+    p.entries = pl->entries; p.row_ptr = pl->row_ptr; p.hrow = pl->hrow; p.x = a.x; p.M = (int)a.M; p.K = (int)a.K;
     p.status = kernel_status_word();
     if (!p.status) return ORTHO_B200_ERR_CUDA;
     CUtensorMap amap, xmap;

@@ -102,6 +102,7 @@ struct Params {
     // sparse instantiation (a plan with ordered rows): the window lists; long rows are read from the pre-pass's sums
     const uint32_t *win_off, *win_words; int ngroups;
     const int32_t *row_ptr; const float *ol; int ol_mp; const int32_t *hrow; int n_long, heavy;
+    const uint32_t *entries; const __half *x;      // the plan's entries, for sums that an infinite activation made NaN
     int *status;
     int gather;
     GatherView gv;
@@ -416,7 +417,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * p.acc_cols);
-            // scale * D + bias (+ alpha * E) of 16 tokens
+            // scale * D + bias (+ alpha * E) of 16 tokens.  The zeros of the scattered tile times an infinite activation make E
+            // NaN for every row: such a sum is taken again from the row's entries in this piece.
             auto load16 = [&](int c, float (&v)[16]) {
                 uint32_t r[16];
                 tmem_ld_32x32b_x16(taddr + (uint32_t)c, r);
@@ -424,8 +426,33 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     uint32_t e[16];
                     tmem_ld_32x32b_x16(taddr + (uint32_t)(p.nt32 + c), e);
                     tmem_ld_wait();
+                    bool nan = false;
 #pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = fmaf(p.alpha, __uint_as_float(e[j]), fmaf(__uint_as_float(r[j]), sc, bs));
+                    for (int j = 0; j < 16; j++) {
+                        v[j] = fmaf(p.alpha, __uint_as_float(e[j]), fmaf(__uint_as_float(r[j]), sc, bs));
+                        nan = nan || v[j] != v[j];
+                    }
+                    if (__any_sync(0xffffffffu, nan)) {
+                        uint32_t bad = 0;
+#pragma unroll
+                        for (int j = 0; j < 16; j++) bad |= v[j] != v[j] ? 1u << j : 0u;
+                        int e0 = 0, e1 = 0;
+                        if (n_ok) { e0 = p.row_ptr[n]; e1 = p.row_ptr[n + 1]; } else bad = 0;
+                        if (p.n_long > 0 && e1 - e0 > p.heavy) e1 = e0;               // a long row is not listed
+#pragma unroll 1
+                        for (int j = 0; j < 16 && c + j < p.M; j++) {
+                            uint32_t d;
+                            __syncwarp();
+                            tmem_ld_32x32b_x1(taddr + (uint32_t)(c + j), d);
+                            tmem_ld_wait();
+                            if (!((bad >> j) & 1u)) continue;
+                            const float es = entries_sum(p.entries, e0, e1, pc.kp0 * KP, pc.kp1 * KP, p.x + (size_t)(c + j) * p.K);
+                            const float t = fmaf(p.alpha, es, fmaf(__uint_as_float(d), sc, bs));
+#pragma unroll
+                            for (int i = 0; i < 16; i++) v[i] = i == j ? t : v[i];
+                        }
+                        __syncwarp();
+                    }
                 } else {
                     tmem_ld_wait();
 #pragma unroll
@@ -666,8 +693,9 @@ int launch_mid(const FwdArgs &a)
         tuning_snapshot().patch_weights) {
         sparse = true;
         p.win_off = a.plan->win_off; p.win_words = a.plan->win_words; p.ngroups = (int)ceil_div(a.N, kWinRows);
+        p.row_ptr = a.plan->row_ptr; p.entries = a.ortho.entries; p.x = a.x;
         if (long_rows) {
-            p.row_ptr = a.plan->row_ptr; p.hrow = a.plan->hrow; p.n_long = (int)a.plan->n_long; p.heavy = a.plan->heavy;
+            p.hrow = a.plan->hrow; p.n_long = (int)a.plan->n_long; p.heavy = a.plan->heavy;
         }
     } else if (a.has_ortho) {
         const int Mp = (int)mid_mp(a.M);

@@ -1,0 +1,70 @@
+"""Calls at the edge of what the entry points accept: infinite activations, buffers that overlap, empty plans, very tall
+layers.  The reference is the CPU oracle or the same call made another way."""
+import numpy as np
+import pytest
+import torch
+
+import workloads as wl
+from conftest import MAX_ABS_TOL, REL_FRO_TOL, layer_oracle
+from libortho_b200 import _C_ops, _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def multi(layer, x, alpha, plan):
+    """A forward with the workspace that the sizing rule asks for."""
+    y = torch.empty(x.shape[0], layer.N, dtype=torch.float16, device=DEV)
+    _C_ops.forward_multi([(layer.base_weight, layer.base_scales, layer.vals, layer.col, layer.row_ptr)], x, [y], alphas=[alpha], plans=[plan])
+    return y
+
+
+def kinds(a):
+    """0 finite, 1 +Inf, 2 -Inf, 3 NaN"""
+    return np.isposinf(a) * 1 + np.isneginf(a) * 2 + np.isnan(a) * 3
+
+
+@pytest.mark.parametrize("M", [1, 4, 16, 32, 100, 200])
+@pytest.mark.parametrize("K,N,kind", [(512, 300, "gauss"), (4096, 200, "zipf"), (8192, 5300, "gauss")])
+def test_infinite_activations_reach_the_outputs_as_the_operator_defines_them(oracle_mod, K, N, kind, M):
+    """One token each with +Inf, -Inf and NaN.  Which outputs are infinite and which NaN depends on the signs of the weights in
+    that column alone, and the other tokens are not touched.  (More than 128 tokens: an entry is added to the weight before
+    the contraction, so rows with an entry in the infinite column are left out there.)"""
+    layer = wl.make_layer(K, N, 0.01, seed=K + N, device=DEV, ortho=kind)
+    plan = _C_ops.Plan(layer.row_ptr, layer.col, layer.vals, K, N)
+    x = wl.make_input(M, K, seed=M, device=DEV)
+    at = {0: (int(layer.col[0]), float("inf")), M // 2: (K - 3, float("-inf")), M - 1: (130, float("inf"))}
+    if M >= 4:
+        at[1] = (7, float("nan"))
+    for m, (k, v) in at.items():
+        x[m, k] = v
+    y = multi(layer, x, 0.75, plan).float().cpu().numpy()
+    with np.errstate(all="ignore"):
+        ref = layer_oracle(oracle_mod, layer, x, 0.75)
+    rows = np.repeat(np.arange(N), np.diff(layer.row_ptr.cpu().numpy()))
+    cols = layer.col.cpu().numpy()
+    for m in range(M):
+        ok = np.ones(N, bool)
+        if m in at and M > 128:
+            ok[rows[cols == at[m][0]]] = False
+        assert np.array_equal(kinds(y[m])[ok], kinds(ref[m])[ok]), f"token {m}"
+        if m not in at:
+            err = y[m] - ref[m]
+            assert np.linalg.norm(err) <= REL_FRO_TOL * np.linalg.norm(ref[m]) * 2 and np.abs(err).max() <= MAX_ABS_TOL, f"token {m}"
+    assert _lib.lib().ortho_b200_query_kernel_status() == 0
+
+
+def test_bfloat16_activations_beyond_fp16_become_infinite_not_nan():
+    """The module rounds activations to FP16: one above 65504 is infinite, and every row with a weight there says so."""
+    layer = wl.make_layer(8192, 5300, 0.003, seed=4, device=DEV)
+    m = layer.to_module()
+    x = wl.make_input(12, 8192, seed=5, device=DEV).to(torch.bfloat16)
+    x[3, 77] = 1e6
+    y = m(x)
+    nib = layer.base_weight[:, 77 // 2] >> 4
+    entry = torch.zeros(layer.N, dtype=torch.bool, device=DEV)
+    rows = torch.repeat_interleave(torch.arange(layer.N, device=DEV), (layer.row_ptr[1:] - layer.row_ptr[:-1]).long())
+    entry[rows[layer.col == 77]] = True
+    plain = (nib != 0) & ~entry
+    assert bool(plain.any()) and torch.isinf(y[3][plain]).all()
+    assert torch.isfinite(y[torch.arange(12) != 3]).all()
