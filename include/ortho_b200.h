@@ -290,8 +290,9 @@ ORTHO_B200_API int ortho_b200_csr_fill(const float *w_ortho, int64_t N, int64_t 
  *   base  = clamp(round_half_even(W / s), -8, 7) * s with s = max(rowmax|W|, 1e-8) / 7
  *   ortho = (W - base) where (W - base)^2 / (h_inv_diag[k] + 1e-6) > threshold, else (signed) zero
  * keep_top_k < 0: threshold = curvature_thresh.  keep_top_k >= 0: threshold = the keep_top_k-th largest
- * score (the caller passes int(sparsity_target * N * K); 0 keeps nothing), found on the device by a
- * byte-wise radix select without storing the scores.  h_inv_diag is the FP32 [K] diagonal.  scratch:
+ * score (the caller passes int(sparsity_target * N * K); 0 keeps nothing), found on the device by a radix
+ * select (12 + 10 + 10 bits) without storing the scores; while it runs an output buffer holds some of their keys.
+ * An output may be W itself.  h_inv_diag is the FP32 [K] diagonal.  scratch:
  * ortho_b200_sieve_scratch_bytes(N) bytes, 256-byte aligned.  K a multiple of 4, pointers 16-byte aligned.
  * The outputs feed ortho_b200_pack_base / ortho_b200_csr_count / ortho_b200_csr_fill.
  * ------------------------------------------------------------------------------------------- */

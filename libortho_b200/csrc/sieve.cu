@@ -11,8 +11,9 @@
 // The threshold is a given constant (curvature threshold) or the k-th largest score ("keep the top
 // fraction", tools/sieve.py:61-66), found by a radix select over the scores' order-preserving keys: the first pass over W
 // takes the row scales and counts the keys' top 12 bits; the second counts the next 10 bits of the keys in the
-// selected bin and lists those keys (in the residual's output buffer, which is written later); the last 10 bits are
-// counted from that short list.  The last CTA of each pass selects the bin.
+// selected bin and lists those keys (in an output buffer, which is written later); the last 10 bits are
+// counted from that short list.  The last CTA of each pass selects the bin.  An output may be W itself (an element is read
+// before it is written): the list then goes to the other output, and without either the last 10 bits take a pass over W too.
 // Everything is element-wise work; with the IEEE divisions (two of some 15 instructions per weight and pass) spelled out
 // each pass was bound by instructions, so they are only done where an approximate quotient cannot decide:
 // near a rounding tie (quant_clamped), near the edge of a bin or near the threshold.
@@ -153,7 +154,9 @@ sieve_rows_kernel(const float *__restrict__ w, const float *__restrict__ hinv, i
     if (k) add_and_select<kBins0>(h, st->hist0, st, 0, k);
 }
 
-// Second pass: the keys in the selected bin, counted by their next 10 bits and listed
+// Second pass (PASS 1): the keys in the selected bin, counted by their next 10 bits and listed.  PASS 2, for want of
+// a list: the keys that agree in these bits too, counted by the last 10
+template <int PASS, bool LIST>
 __global__ void __launch_bounds__(256)
 sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, const float *__restrict__ scales,
                  int64_t N, int K, SelectState *__restrict__ st, uint32_t *__restrict__ list)
@@ -161,7 +164,7 @@ sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, co
     __shared__ unsigned int h[kBins];
     for (int i = threadIdx.x; i < kBins; i += 256) h[i] = 0;
     __syncthreads();
-    const uint32_t bin = st->prefix[0];
+    const uint32_t bin = st->prefix[0], mid = PASS == 2 ? st->prefix[1] : 0u;
     const int lane = threadIdx.x & 31;
     for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
         const float4 *row = reinterpret_cast<const float4 *>(w + (size_t)n * K);
@@ -186,7 +189,10 @@ sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, co
                     // clearly outside the bin: nothing to do; else the exact key
                     key[e] = 0;
                     in[e] = on && !(approx_ok(r2, hs) && (bits + 16u) >> 20 != bin && (bits - 16u) >> 20 != bin);
-                    if (in[e]) { key[e] = score_key(div_ieee(r2, hs)); in[e] = (key[e] >> 20) == bin; }
+                    if (in[e]) {
+                        key[e] = score_key(div_ieee(r2, hs));
+                        in[e] = PASS == 1 ? (key[e] >> 20) == bin : (key[e] >> 10) == (bin << 10 | mid);
+                    }
                 }
                 if (!__any_sync(0xffffffffu, in[0] || in[1] || in[2] || in[3])) continue;
 #pragma unroll
@@ -194,17 +200,19 @@ sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, co
                     const unsigned m = __ballot_sync(0xffffffffu, in[e]);
                     if (m == 0u) continue;
                     unsigned at = 0;
-                    if (lane == __ffs(m) - 1) at = atomicAdd(&st->listed, (unsigned)__popc(m));
-                    at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+                    if (LIST) {
+                        if (lane == __ffs(m) - 1) at = atomicAdd(&st->listed, (unsigned)__popc(m));
+                        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+                    }
                     if (in[e]) {
-                        list[at + __popc(m & ((1u << lane) - 1u))] = key[e];
-                        atomicAdd(&h[(key[e] >> 10) & 1023u], 1u);
+                        if (LIST) list[at + __popc(m & ((1u << lane) - 1u))] = key[e];
+                        atomicAdd(&h[(PASS == 1 ? key[e] >> 10 : key[e]) & 1023u], 1u);
                     }
                 }
             }
         }
     }
-    add_and_select<kBins>(h, st->hist1, st, 1, st->krem[0]);
+    add_and_select<kBins>(h, PASS == 1 ? st->hist1 : st->hist2, st, PASS, st->krem[PASS - 1]);
 }
 
 // Third pass: the last 10 bits, from the list
@@ -296,9 +304,19 @@ extern "C" int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t
     count_launch();
     OB_CUDA(cudaGetLastError());
     if (k) {
-        uint32_t *list = reinterpret_cast<uint32_t *>(w_ortho_out);          // room for every key; the split writes it last
-        sieve_bin_kernel<<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, list);
-        sieve_list_kernel<<<(unsigned)device_sm_count(current_device_index()), 256, 0, st>>>(sel, list);
+        // the list: room for every key in an output that is not read on the way to the split, which writes both
+        auto apart = [&](const float *out) {
+            const uintptr_t o = (uintptr_t)out, n = (uintptr_t)(N * K) * 4, a = (uintptr_t)w, b = (uintptr_t)h_inv_diag;
+            return (o + n <= a || a + n <= o) && (o + n <= b || b + (uintptr_t)K * 4 <= o);
+        };
+        uint32_t *list = reinterpret_cast<uint32_t *>(apart(w_ortho_out) ? w_ortho_out : apart(w_base_out) ? w_base_out : nullptr);
+        if (list) {
+            sieve_bin_kernel<1, true><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, list);
+            sieve_list_kernel<<<(unsigned)device_sm_count(current_device_index()), 256, 0, st>>>(sel, list);
+        } else {
+            sieve_bin_kernel<1, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr);
+            sieve_bin_kernel<2, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr);
+        }
         count_launch(2);
         OB_CUDA(cudaGetLastError());
         thr_dev = &sel->threshold;

@@ -68,3 +68,25 @@ def test_bfloat16_activations_beyond_fp16_become_infinite_not_nan():
     plain = (nib != 0) & ~entry
     assert bool(plain.any()) and torch.isinf(y[3][plain]).all()
     assert torch.isfinite(y[torch.arange(12) != 3]).all()
+
+
+@pytest.mark.parametrize("over", ["residual", "base", "both"])
+@pytest.mark.parametrize("N,K,keep", [(96, 512, 0.01), (40, 4096, 0.3), (7, 64, 1.0)])
+def test_sieve_outputs_may_overwrite_the_weights(N, K, keep, over):
+    """An output that is W itself: every element is read before it is written."""
+    g = torch.Generator().manual_seed(N + K)
+    w, h = (torch.randn(N, K, generator=g) * 0.02).to(DEV), (torch.rand(K, generator=g) * 2 + 0.01).to(DEV)
+    scratch = torch.empty(int(_lib.lib().ortho_b200_sieve_scratch_bytes(N)), dtype=torch.uint8, device=DEV)
+
+    def sieve(src, base, res):
+        st = _lib.lib().ortho_b200_sieve(src.data_ptr(), h.data_ptr(), N, K, 0.0, int(keep * N * K), base.data_ptr(), res.data_ptr(),
+                                         scratch.data_ptr(), scratch.numel(), torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+        return base, res
+
+    base, res = sieve(w, torch.empty_like(w), torch.empty_like(w))
+    own = w.clone()
+    b2, r2 = sieve(own, own if over != "residual" else torch.empty_like(w), own if over != "base" else torch.empty_like(w))
+    if over != "both":                                      # (then the residual, written last, is what stays)
+        assert torch.equal(b2.view(torch.int32), base.view(torch.int32))
+    assert torch.equal(r2.view(torch.int32), res.view(torch.int32))
