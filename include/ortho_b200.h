@@ -135,7 +135,7 @@ ORTHO_B200_API int ortho_b200_dequant_dump(const void *q_weight, const void *q_s
 
 ORTHO_B200_API int64_t ortho_b200_workspace_bytes(int64_t M, int64_t K, int64_t N);
 /* Workspace for forwards that pass this plan (the prefill regime keeps the pre-pass sums of the plan's long rows
- * there, so it may need more than the plan-less bound); 0 for the streaming kernels or for an empty plan. */
+ * there, so it may need more than the plan-less bound).  An empty plan answers like ortho_b200_workspace_bytes. */
 ORTHO_B200_API int64_t ortho_b200_plan_workspace_bytes(const ortho_b200_plan *plan, int64_t M);
 
 ORTHO_B200_API int ortho_b200_forward(const void *q_weight, const void *q_scales_f16,

@@ -341,8 +341,8 @@ extern "C" int64_t ortho_b200_plan_workspace_bytes(const ortho_b200_plan *plan, 
 {
     const Plan *pl = reinterpret_cast<const Plan *>(plan);
     if (!pl || pl->magic != kPlanMagic) return -1;
-    if (pl->nnz == 0) return 0;
-    const int64_t plain = ortho_b200_workspace_bytes(M, pl->K, pl->N);
+    const int64_t plain = ortho_b200_workspace_bytes(M, pl->K, pl->N);      // base-only calls too: partial sums of cut tiles
+    if (pl->nnz == 0) return plain;
     // the tensor-core kernels take the sums of the plan's long rows from a pre-pass
     return plain + (decode_regime(M, pl->N, pl->K) && !mid_range(M, pl->N, pl->K) ? 0 : long_rows_workspace_bytes(pl, M));
 }

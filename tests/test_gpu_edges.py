@@ -90,3 +90,19 @@ def test_sieve_outputs_may_overwrite_the_weights(N, K, keep, over):
     if over != "both":                                      # (then the residual, written last, is what stays)
         assert torch.equal(b2.view(torch.int32), base.view(torch.int32))
     assert torch.equal(r2.view(torch.int32), res.view(torch.int32))
+
+
+@pytest.mark.parametrize("M", [4, 8, 20, 64, 300])
+def test_an_empty_plan_runs_like_no_plan(M):
+    """A plan without entries asks for the workspace of a call without one and gets the same kernels and bits."""
+    K, N = 28672, 1536
+    layer = wl.make_layer(K, N, 0.0, seed=6, device=DEV)
+    plan = _C_ops.Plan(layer.row_ptr, layer.col, layer.vals, K, N)
+    x = wl.make_input(M, K, seed=M, device=DEV)
+    assert _C_ops.workspace_bytes(M, K, N, plan) == _C_ops.workspace_bytes(M, K, N)
+    ys, launches = [], []
+    for p in (None, plan):
+        before = _lib.lib().ortho_b200_launch_count()
+        ys.append(multi(layer, x, 1.0, p))
+        launches.append(_lib.lib().ortho_b200_launch_count() - before)
+    assert torch.equal(ys[0], ys[1]) and launches[0] == launches[1]
