@@ -181,9 +181,9 @@ long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, in
 // y[m, hrow[h]] = FP16(rest[h, m] + alpha * (part[0] + ... + part[nsplit - 1])[h, m]); one token per thread
 __global__ void __launch_bounds__(256)
 long_finish_kernel(const float *__restrict__ part, long long stride, int nsplit, const float *__restrict__ rest,
-                   const int32_t *__restrict__ hrow, float alpha, __half *__restrict__ y, long long ldy, int M, int Mp)
+                   const int32_t *__restrict__ hrow, int h0, float alpha, __half *__restrict__ y, long long ldy, int M, int Mp)
 {
-    const int m = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y;
+    const int m = blockIdx.x * 256 + threadIdx.x, h = h0 + blockIdx.y;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (m >= M) return;
     const float *src = part + (size_t)h * Mp + m;
@@ -281,15 +281,19 @@ int launch_long_finish(const FwdArgs &a, int Mp, void *ws)
     const Plan *pl = a.plan;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)ceil_div(a.M, 256), (unsigned)pl->n_long); cfg.blockDim = dim3(256); cfg.stream = a.stream;
+    cfg.blockDim = dim3(256); cfg.stream = a.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     const float *part = reinterpret_cast<const float *>(ws), *rest = long_rows_rest(a, Mp, ws);
-    OB_CUDA(cudaLaunchKernelEx(&cfg, long_finish_kernel, part, (long long)pl->n_pad * Mp, long_rows_splits(pl, a.M), rest,
-                               (const int32_t *)pl->hrow, a.alpha, a.y, (long long)a.pitch_y(), (int)a.M, Mp));
-    count_launch();
+    constexpr int64_t kRows = 65535;                     // a grid's extent along y (a loop over rows in the kernel cost 5 us at 512 tokens)
+    for (int64_t h0 = 0; h0 < pl->n_long; h0 += kRows) {
+        cfg.gridDim = dim3((unsigned)ceil_div(a.M, 256), (unsigned)(pl->n_long - h0 < kRows ? pl->n_long - h0 : kRows));
+        OB_CUDA(cudaLaunchKernelEx(&cfg, long_finish_kernel, part, (long long)pl->n_pad * Mp, long_rows_splits(pl, a.M), rest,
+                                   (const int32_t *)pl->hrow, (int)h0, a.alpha, a.y, (long long)a.pitch_y(), (int)a.M, Mp));
+        count_launch();
+    }
     return ORTHO_B200_OK;
 }
 int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)

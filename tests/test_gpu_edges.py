@@ -106,3 +106,36 @@ def test_an_empty_plan_runs_like_no_plan(M):
         ys.append(multi(layer, x, 1.0, p))
         launches.append(_lib.lib().ortho_b200_launch_count() - before)
     assert torch.equal(ys[0], ys[1]) and launches[0] == launches[1]
+
+
+def test_more_long_rows_than_a_grid_dimension_holds():
+    """70 000 long rows of a tall, narrow layer at more than 128 tokens."""
+    K, N, M, per = 64, 400000, 130, 32
+    g = torch.Generator().manual_seed(9)
+    layer = wl.make_layer(K, N, 0.0, seed=9, device=DEV)
+    long_rows = torch.arange(0, N, 4)[:70000]
+    counts = torch.zeros(N, dtype=torch.int64)
+    counts[long_rows] = per
+    ptr = torch.zeros(N + 1, dtype=torch.int32)
+    ptr[1:] = counts.cumsum(0).to(torch.int32)
+    col = torch.rand(long_rows.numel(), K, generator=g).argsort(1)[:, :per].sort(1).values.reshape(-1).to(torch.int32)
+    val = (torch.randn(col.numel(), generator=g) * 0.05).to(torch.float16)
+    ptr, col, val = ptr.to(DEV), col.to(DEV), val.to(DEV)
+    layer = wl.Layer(K, N, layer.base_weight, layer.base_scales, ptr, col, val, 1.0)
+    assert _lib.lib().ortho_b200_set_decode_config(-5, 0, 0, 8) == 0
+    try:
+        plan = _C_ops.Plan(ptr, col, val, K, N)            # mean row 6 entries: rows of more than 24 are long
+    finally:
+        _lib.lib().ortho_b200_set_decode_config(-5, 0, 0, 0)
+    x = wl.make_input(M, K, seed=1, device=DEV)
+    before = _lib.lib().ortho_b200_launch_count()
+    y = multi(layer, x, 1.0, plan)
+    assert _lib.lib().ortho_b200_launch_count() - before == 4      # the long rows' GEMM, the main kernel, the long rows' finish twice
+    q = layer.base_weight.to(torch.int16)
+    w = torch.stack((q & 15, q >> 4), dim=2).view(N, K)
+    w = (w - ((w & 8) << 1)).double() * layer.base_scales.double().unsqueeze(1)
+    rows = torch.repeat_interleave(torch.arange(N, device=DEV), counts.to(DEV))
+    w[rows, col.long()] += val.double()
+    ref = x.double() @ w.T
+    assert float((y.double() - ref).norm() / ref.norm()) <= REL_FRO_TOL
+    assert _lib.lib().ortho_b200_query_kernel_status() == 0
