@@ -73,7 +73,7 @@ __device__ __forceinline__ void add_and_select(const unsigned int *h, unsigned i
         if (h[i]) atomicAdd(&hist[i], h[i]);
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(&st->done[pass], 1u) == gridDim.x - 1 ? 1u : 0u;
+    if (threadIdx.x == 0) is_last = atomicAdd(&st->done[pass], 1u) == gridDim.x * gridDim.y - 1 ? 1u : 0u;
     __syncthreads();
     if (!is_last) return;
     __threadfence();
@@ -154,22 +154,32 @@ sieve_rows_kernel(const float *__restrict__ w, const float *__restrict__ hinv, i
     if (k) add_and_select<kBins0>(h, st->hist0, st, 0, k);
 }
 
+// the quads of a row that are this CTA's: a row is cut into gridDim.y pieces of whole 1024 quads
+struct Piece { int begin, end; };
+__device__ __forceinline__ Piece piece_of(int quads)
+{
+    const int rounds = (quads + 1023) / 1024, per = (rounds + (int)gridDim.y - 1) / (int)gridDim.y * 1024;
+    return Piece{(int)blockIdx.y * per, min(quads, ((int)blockIdx.y + 1) * per)};
+}
+
 // Second pass (PASS 1): the keys in the selected bin, counted by their next 10 bits and listed.  PASS 2, for want of
-// a list: the keys that agree in these bits too, counted by the last 10
+// a list: the keys that agree in these bits too, counted by the last 10.  PASS 0: the first pass's counts, where rows are cut
 template <int PASS, bool LIST>
 __global__ void __launch_bounds__(256)
 sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, const float *__restrict__ scales,
-                 int64_t N, int K, SelectState *__restrict__ st, uint32_t *__restrict__ list)
+                 int64_t N, int K, SelectState *__restrict__ st, uint32_t *__restrict__ list, unsigned long long k)
 {
-    __shared__ unsigned int h[kBins];
-    for (int i = threadIdx.x; i < kBins; i += 256) h[i] = 0;
+    constexpr int BINS = PASS == 0 ? kBins0 : kBins;
+    __shared__ unsigned int h[BINS];
+    for (int i = threadIdx.x; i < BINS; i += 256) h[i] = 0;
     __syncthreads();
-    const uint32_t bin = st->prefix[0], mid = PASS == 2 ? st->prefix[1] : 0u;
+    const Piece pc = piece_of(K / 4);
+    const uint32_t bin = PASS == 0 ? 0u : st->prefix[0], mid = PASS == 2 ? st->prefix[1] : 0u;
     const int lane = threadIdx.x & 31;
     for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
         const float4 *row = reinterpret_cast<const float4 *>(w + (size_t)n * K);
         const float sc = scales[n], rs = quant_rscale(sc);
-        for (int i0 = 0; i0 < K / 4; i0 += 1024) {
+        for (int i0 = pc.begin; i0 < pc.end; i0 += 1024) {
             float4 v[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) v[j] = i0 + 256 * j + threadIdx.x < K / 4 ? row[i0 + 256 * j + threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -186,6 +196,13 @@ sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, co
                     float b, r;
                     const float hs = __fadd_rn(hh[e], 1e-6f), r2 = sieve_one(ww[e], sc, rs, b, r);
                     const uint32_t bits = __float_as_uint(r2 * rcp_approx(hs)) | 0x80000000u;
+                    if (PASS == 0) {
+                        key[e] = bits;
+                        if (!approx_ok(r2, hs) || (((bits + 16u) ^ (bits - 16u)) >> 20) != 0u) key[e] = score_key(div_ieee(r2, hs));
+                        if (on) atomicAdd(&h[key[e] >> 20], 1u);
+                        in[e] = false;
+                        continue;
+                    }
                     // clearly outside the bin: nothing to do; else the exact key
                     key[e] = 0;
                     in[e] = on && !(approx_ok(r2, hs) && (bits + 16u) >> 20 != bin && (bits - 16u) >> 20 != bin);
@@ -212,7 +229,8 @@ sieve_bin_kernel(const float *__restrict__ w, const float *__restrict__ hinv, co
             }
         }
     }
-    add_and_select<kBins>(h, PASS == 1 ? st->hist1 : st->hist2, st, PASS, st->krem[PASS - 1]);
+    if constexpr (PASS == 0) add_and_select<kBins0>(h, st->hist0, st, 0, k);
+    else add_and_select<kBins>(h, PASS == 1 ? st->hist1 : st->hist2, st, PASS, st->krem[PASS - 1]);
 }
 
 // Third pass: the last 10 bits, from the list
@@ -238,10 +256,11 @@ sieve_split_kernel(const float *__restrict__ w, const float *__restrict__ hinv, 
     const float thr = thr_dev ? *thr_dev : thr_host;
     const bool thr_ok = thr >= 1e-20f && thr <= 1e20f;
     const float thr_lo = thr * 0.99999f, thr_hi = thr * 1.00001f;
+    const Piece pc = piece_of(K / 4);
     for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
         const size_t at = (size_t)n * (K / 4);
         const float sc = scales[n], rs = quant_rscale(sc);
-        for (int i0 = threadIdx.x; i0 < K / 4; i0 += 1024) {
+        for (int i0 = pc.begin + threadIdx.x; i0 < pc.end; i0 += 1024) {
             float4 v[4];
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -269,10 +288,15 @@ sieve_split_kernel(const float *__restrict__ w, const float *__restrict__ hinv, 
     }
 }
 
-static unsigned sieve_grid(int64_t N)
+// Eight CTAs per SM at most, a row each.  A matrix of fewer rows than two per SM has its rows cut (into pieces of 4096
+// weights or more) so that it still fills the GPU; its first pass then is two, the row scales and the counts.
+// Keep the top 1 %, whole / cut rows: 1 x 4194304 8.8 / 0.33 ms, 64 x 65536 200 / 106 us, 295 x 8192 82 / 75 us.
+static dim3 sieve_grid(int64_t N, int64_t K)
 {
-    const int64_t cap = (int64_t)device_sm_count(current_device_index()) * 8;
-    return (unsigned)(N > cap ? cap : N);
+    const int64_t sms = device_sm_count(current_device_index()), cap = sms * 8, rounds = ceil_div(K / 4, 1024);
+    if (N >= 2 * sms) return dim3((unsigned)(N > cap ? cap : N));
+    const int64_t pieces = ceil_div(cap, N);
+    return dim3((unsigned)N, (unsigned)(pieces < rounds ? pieces : rounds));
 }
 
 }  // namespace ob
@@ -295,13 +319,15 @@ extern "C" int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t
     cudaStream_t st = (cudaStream_t)stream;
     float *scales = reinterpret_cast<float *>(scratch);
     SelectState *sel = reinterpret_cast<SelectState *>(reinterpret_cast<unsigned char *>(scratch) + ((N * 4 + 255) / 256) * 256);
-    const unsigned grid = sieve_grid(N);
+    const dim3 grid = sieve_grid(N, K);
     const float *thr_dev = nullptr;
     float thr_host = curvature_thresh;
     const unsigned long long k = keep_top_k > 0 ? (unsigned long long)keep_top_k : 0ull;
     if (k) OB_CUDA(cudaMemsetAsync(sel, 0, sizeof(SelectState), st));
-    sieve_rows_kernel<<<grid, 256, 0, st>>>(w, h_inv_diag, N, (int)K, scales, sel, k);
-    count_launch();
+    const bool cut = grid.y > 1;
+    sieve_rows_kernel<<<grid.x, 256, 0, st>>>(w, h_inv_diag, N, (int)K, scales, sel, cut ? 0ull : k);
+    if (k && cut) sieve_bin_kernel<0, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr, k);
+    count_launch(k && cut ? 2 : 1);
     OB_CUDA(cudaGetLastError());
     if (k) {
         // the list: room for every key in an output that is not read on the way to the split, which writes both
@@ -311,11 +337,11 @@ extern "C" int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t
         };
         uint32_t *list = reinterpret_cast<uint32_t *>(apart(w_ortho_out) ? w_ortho_out : apart(w_base_out) ? w_base_out : nullptr);
         if (list) {
-            sieve_bin_kernel<1, true><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, list);
+            sieve_bin_kernel<1, true><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, list, k);
             sieve_list_kernel<<<(unsigned)device_sm_count(current_device_index()), 256, 0, st>>>(sel, list);
         } else {
-            sieve_bin_kernel<1, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr);
-            sieve_bin_kernel<2, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr);
+            sieve_bin_kernel<1, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr, k);
+            sieve_bin_kernel<2, false><<<grid, 256, 0, st>>>(w, h_inv_diag, scales, N, (int)K, sel, nullptr, k);
         }
         count_launch(2);
         OB_CUDA(cudaGetLastError());

@@ -139,3 +139,21 @@ def test_more_long_rows_than_a_grid_dimension_holds():
     ref = x.double() @ w.T
     assert float((y.double() - ref).norm() / ref.norm()) <= REL_FRO_TOL
     assert _lib.lib().ortho_b200_query_kernel_status() == 0
+
+
+@pytest.mark.parametrize("N,K", [(1, 4100), (3, 65536), (100, 20480), (295, 8196)])
+def test_sieve_of_few_long_rows(N, K):
+    """Rows cut into pieces (fewer rows than two per SM): bit for bit the torch chain on the CPU, with a list and without."""
+    from libortho_b200 import sieve
+    g = torch.Generator().manual_seed(N + K)
+    w, h = torch.randn(N, K, generator=g) * 0.02, torch.rand(K, generator=g) * 2 + 0.01
+    for target in (None, 0.01, 0.3, 1.0):
+        base_ref, ortho_ref = sieve.hessian_sieve(w, h, curvature_thresh=1e-5, sparsity_target=target)
+        base, ortho = sieve.hessian_sieve(w.to(DEV), h.to(DEV), curvature_thresh=1e-5, sparsity_target=target)
+        assert torch.equal(base.cpu().view(torch.int32), base_ref.view(torch.int32))
+        assert torch.equal(ortho.cpu().view(torch.int32), ortho_ref.view(torch.int32))
+        own, scratch = w.to(DEV), torch.empty(int(_lib.lib().ortho_b200_sieve_scratch_bytes(N)), dtype=torch.uint8, device=DEV)
+        st = _lib.lib().ortho_b200_sieve(own.data_ptr(), h.to(DEV).data_ptr(), N, K, 1e-5, -1 if target is None else int(target * N * K),
+                                         own.data_ptr(), own.data_ptr(), scratch.data_ptr(), scratch.numel(),
+                                         torch.cuda.current_stream().cuda_stream)
+        assert st == 0 and torch.equal(own.view(torch.int32), ortho.view(torch.int32))
