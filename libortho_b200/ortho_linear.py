@@ -16,7 +16,9 @@ Differences, all deliberate:
 """
 from __future__ import annotations
 
-from typing import Optional
+import threading
+import weakref
+from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
@@ -38,24 +40,62 @@ _ORTHO_BUFFERS = ("ortho_values", "ortho_col_indices", "ortho_row_ptr")
 _WATCHED = frozenset(("base_weight", "base_scales", "bias") + _ORTHO_BUFFERS)
 
 
+def _capturing(dev: torch.device) -> bool:
+    if torch.cuda.current_device() == dev.index:
+        return torch._C._cuda_isCurrentStreamCapturing()
+    with torch.cuda.device(dev):
+        return torch._C._cuda_isCurrentStreamCapturing()
+
+
 class _SharedWorkspace:
     """One grow-on-demand scratch buffer per device and stream, shared by every module that runs there (a model with
-    hundreds of layers runs them one at a time); forwards on different streams never meet in one."""
-    _by_stream = {}
+    hundreds of layers runs them one at a time).  The registry holds the MAX_STREAMS that were bound last, and only while
+    some module's call record uses them: torch's allocator gets the others back, in the order of their own stream.
 
-    def __init__(self):
+    A forward under graph capture gets a buffer of its own (`shared` is False), allocated like any temporary of the capture:
+    it belongs to the graph's memory pool, so a replay, on whatever stream, neither meets an eager forward's buffer or another
+    graph's nor addresses one that has grown away."""
+    MAX_STREAMS = 16
+    _by_stream = weakref.WeakValueDictionary()
+    _lock = threading.Lock()
+    _clock = 0
+    __slots__ = ("tensor", "gen", "shared", "bound_at", "__weakref__")
+
+    def __init__(self, shared: bool):
         self.tensor: Optional[torch.Tensor] = None
-        self.gen = 0
+        self.gen, self.shared, self.bound_at = 0, shared, 0
+
+    def _replace(self, tensor: Optional[torch.Tensor]):
+        self.gen += 1                          # before the tensor: a forward reads them the other way round
+        self.tensor = tensor
 
     @classmethod
-    def get(cls, device: torch.device, nbytes: int, stream: int) -> "_SharedWorkspace":
-        w = cls._by_stream.get((device, stream))
-        if w is None:
-            w = cls._by_stream[(device, stream)] = cls()
-        if nbytes > 0 and (w.tensor is None or w.tensor.numel() < nbytes):
-            w.tensor = torch.empty(nbytes, dtype=torch.uint8, device=device)
-            w.gen += 1
-        return w
+    def get(cls, device: torch.device, nbytes: int, stream: int) -> Tuple["_SharedWorkspace", int, Optional[torch.Tensor]]:
+        """(buffer, its generation, its tensor) with room for `nbytes`, for the current stream `stream`."""
+        if nbytes == 0:
+            return _NO_SCRATCH, 0, None
+        if _capturing(device):
+            own = cls(False)
+            own.tensor = torch.empty(nbytes, dtype=torch.uint8, device=device)
+            return own, 0, own.tensor
+        with cls._lock:
+            w = cls._by_stream.get((device, stream))
+            if w is None:
+                w = cls(True)
+                alive = list(cls._by_stream.items())
+                if len(alive) >= cls.MAX_STREAMS:
+                    key, oldest = min(alive, key=lambda kw: kw[1].bound_at)
+                    oldest._replace(None)      # its records see the generation and bind again
+                    del cls._by_stream[key]
+                cls._by_stream[(device, stream)] = w
+            cls._clock += 1
+            w.bound_at = cls._clock
+            if w.tensor is None or w.tensor.numel() < nbytes:
+                w._replace(torch.empty(nbytes, dtype=torch.uint8, device=device))
+            return w, w.gen, w.tensor
+
+
+_NO_SCRATCH = _SharedWorkspace(True)
 
 
 class _Bound:
@@ -180,14 +220,6 @@ class OrthoLinear(nn.Module):
             self._ws_need[key] = need
         return need
 
-    def _get_workspace(self, M: int) -> Optional[torch.Tensor]:
-        """The current stream's shared scratch buffer, grown to what a forward of M tokens needs (None if nothing)."""
-        need = self._workspace_bytes(M)
-        if need == 0:
-            return None
-        dev = self.base_weight.device
-        return _SharedWorkspace.get(dev, need, _current_stream_handle(dev)).tensor
-
     def _versions(self):
         """What a cached call record depends on besides the token count: the storage of every buffer (a
         ``.data =`` assignment swaps it without going through ``__setattr__``) and the contents of the CSR
@@ -196,7 +228,8 @@ class OrthoLinear(nn.Module):
         return (self.base_weight.data_ptr(), self.base_scales.data_ptr(), ov.data_ptr(), oc.data_ptr(), orp.data_ptr(),
                 ov._version, oc._version, orp._version, (b.data_ptr(), b.dtype) if b is not None else None)
 
-    def _bind(self, M: int, dev: torch.device, stream: int) -> _Bound:
+    def _bind(self, M: int, dev: torch.device, stream: int) -> Tuple[_Bound, Optional[torch.Tensor]]:
+        """The call record and its scratch, which the caller holds until the launch."""
         N, K = self.out_features, self.in_features
         bw, bs = self.base_weight, self.base_scales
         if bw.dtype != torch.uint8 or bs.dtype != torch.float16:
@@ -217,10 +250,9 @@ class OrthoLinear(nn.Module):
         b = _Bound()
         plan = self._get_plan() if sparse else None
         need = self._workspace_bytes(M)
-        b.ws = _SharedWorkspace.get(dev, need, stream)
-        b.ws_gen = b.ws.gen
-        b.ws_ptr = b.ws.tensor.data_ptr() if need else None
-        b.ws_bytes = b.ws.tensor.numel() if need else 0
+        b.ws, b.ws_gen, scratch = _SharedWorkspace.get(dev, need, stream)
+        b.ws_ptr = scratch.data_ptr() if need else None
+        b.ws_bytes = scratch.numel() if need else 0
         b.fused_bias = (self.bias is not None and self.bias.dtype == torch.float32 and self.bias.device == dev
                         and self.bias.is_contiguous())
         descs = (_lib.LayerDesc * 1)()
@@ -235,10 +267,11 @@ class OrthoLinear(nn.Module):
         d.N, d.ldy, d.reserved = N, 0, 0
         b.descs = descs
         b.key = (self.alpha > 0, self._versions())
-        if len(self._bound) > 32:
-            self._bound.clear()
-        self._bound[(M, stream)] = b
-        return b
+        if b.ws.shared:
+            if len(self._bound) > 32:
+                self._bound.clear()
+            self._bound[(M, stream)] = b
+        return b, scratch
 
     # -- forward ---------------------------------------------------------------------------------
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -267,8 +300,10 @@ class OrthoLinear(nn.Module):
             alpha = float(self.alpha)
             stream = _current_stream_handle(dev)
             b = self._bound.get((M, stream))
-            if b is None or b.key != (alpha > 0, self._versions()) or b.ws_gen != b.ws.gen:
-                b = self._bind(M, dev, stream)
+            scratch = b.ws.tensor if b is not None else None      # held until the launch, whatever other threads bind meanwhile
+            if (b is None or b.key != (alpha > 0, self._versions()) or b.ws_gen != b.ws.gen
+                    or (scratch is not None and _capturing(dev))):
+                b, scratch = self._bind(M, dev, stream)
             d = b.descs[0]
             d.y_f16 = output.data_ptr()
             d.alpha = alpha

@@ -103,7 +103,7 @@ class ShardedOrthoLinear(nn.Module):
         ``OrthoLinear`` does for its own forward."""
         from . import _C_ops as _C
         from . import _lib
-        from .ortho_linear import _SharedWorkspace, _current_stream_handle
+        from .ortho_linear import _SharedWorkspace, _capturing, _current_stream_handle
         M = x2.shape[0]
         if M > self._comm_max_m:
             raise ValueError(f"peer gather was sized for {self._comm_max_m} tokens, got {M}")
@@ -118,7 +118,9 @@ class ShardedOrthoLinear(nn.Module):
         alpha = float(loc.alpha)
         stream = _current_stream_handle(dev)
         b = self._peer_bound.get((M, stream))
-        if b is None or b["key"] != (alpha > 0, loc._versions(), id(self._comm), self._comm_off) or b["ws_gen"] != b["ws"].gen:
+        scratch = b["ws"].tensor if b is not None else None       # held until the launch
+        if (b is None or b["key"] != (alpha > 0, loc._versions(), id(self._comm), self._comm_off) or b["ws_gen"] != b["ws"].gen
+                or (scratch is not None and _capturing(dev))):
             rows = self.n1 - self.n0
             nnz = int(loc.ortho_values.numel())
             if rows and (loc.base_weight.dtype != torch.uint8 or loc.base_scales.dtype != torch.float16
@@ -126,21 +128,22 @@ class ShardedOrthoLinear(nn.Module):
                 raise ValueError("the shard's base_weight / base_scales do not match its rows")
             plan = loc._get_plan() if (alpha > 0 and nnz > 0) else None
             need = _C.workspace_bytes(M, self.in_features, rows, plan) if rows else 0
-            ws = _SharedWorkspace.get(dev, need, stream)
+            ws, ws_gen, scratch = _SharedWorkspace.get(dev, need, stream)
             b = {
-                "key": (alpha > 0, loc._versions(), id(self._comm), self._comm_off), "ws": ws, "ws_gen": ws.gen,
+                "key": (alpha > 0, loc._versions(), id(self._comm), self._comm_off), "ws": ws, "ws_gen": ws_gen,
                 "head": (loc.base_weight.data_ptr() if rows else None, loc.base_scales.data_ptr() if rows else None,
                          loc.ortho_values.data_ptr() if nnz else None, loc.ortho_col_indices.data_ptr() if nnz else None,
                          loc.ortho_row_ptr.data_ptr() if nnz else None, nnz),
-                "tail": (plan.handle if plan is not None else None, ws.tensor.data_ptr() if need else None,
-                         ws.tensor.numel() if need else 0, self._comm.handle),
+                "tail": (plan.handle if plan is not None else None, scratch.data_ptr() if need else None,
+                         scratch.numel() if need else 0, self._comm.handle),
                 "plan": plan,
                 "off": [self._comm_off + s * self._region for s in (0, 1)],
                 "out": [self._comm.output(self._comm_off + s * self._region, M, self.out_features) for s in (0, 1)],
             }
-            if len(self._peer_bound) > 32:
-                self._peer_bound.clear()
-            self._peer_bound[(M, stream)] = b
+            if ws.shared:
+                if len(self._peer_bound) > 32:
+                    self._peer_bound.clear()
+                self._peer_bound[(M, stream)] = b
         slot = self._slot
         self._slot ^= 1
         fwd = _lib.lib().ortho_b200_forward_gather

@@ -157,3 +157,80 @@ def test_sieve_of_few_long_rows(N, K):
                                          own.data_ptr(), own.data_ptr(), scratch.data_ptr(), scratch.numel(),
                                          torch.cuda.current_stream().cuda_stream)
         assert st == 0 and torch.equal(own.view(torch.int32), ortho.view(torch.int32))
+
+
+def test_a_captured_forward_owns_its_scratch():
+    """A graph of a small batch, then a larger eager forward on the capture's stream (its scratch grows), then tensors in the
+    memory that became free: a replay writes none of them and still gives the result."""
+    layer = wl.make_layer(8192, 5300, 0.003, seed=11, device=DEV)
+    m = layer.to_module()
+    x, big = wl.make_input(12, 8192, seed=1, device=DEV), wl.make_input(600, 8192, seed=2, device=DEV)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        m(x)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            y = m(x)
+        ref = m(x)
+        m(big)
+        fill = [torch.full((1 << 20,), 7, dtype=torch.int32, device=DEV) for _ in range(24)]
+        for i in range(3):
+            y.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, ref)
+            assert all(bool((f == 7).all()) for f in fill)
+    assert _lib.lib().ortho_b200_query_kernel_status() == 0
+
+
+def test_graphs_of_one_capture_stream_replay_side_by_side():
+    """Two graphs captured on the same stream, replayed on two streams at once, beside eager forwards on a third."""
+    K, N, M = 8192, 5300, 16
+    a, b = (wl.make_layer(K, N, 0.003, seed=s, device=DEV).to_module() for s in (1, 2))
+    xs = [wl.make_input(M, K, seed=s, device=DEV) for s in (1, 2)]
+    refs = [a(xs[0]).clone(), b(xs[1]).clone()]
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for m, x in zip((a, b), xs):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(8):
+                y = m(x)
+        graphs.append(g)
+        outs.append(y)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    for _ in range(10):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        with torch.cuda.stream(streams[2]):
+            eager = a(xs[0])
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], refs[0]) and torch.equal(outs[1], refs[1]) and torch.equal(eager, refs[0])
+    assert _lib.lib().ortho_b200_query_kernel_status() == 0
+
+
+def test_scratch_is_bounded_and_given_back():
+    from libortho_b200.ortho_linear import _SharedWorkspace
+    layer = wl.make_layer(8192, 5300, 0.003, seed=3, device=DEV)
+    m = layer.to_module()
+    x = wl.make_input(12, 8192, seed=1, device=DEV)
+    ref = m(x)
+    torch.cuda.synchronize()
+    handles = set()
+    for s in [torch.cuda.Stream() for _ in range(20)] + [torch.cuda.Stream(priority=-1) for _ in range(20)]:
+        with torch.cuda.stream(s):
+            y = m(x)
+            s.synchronize()
+            assert torch.equal(y, ref)
+            handles.add(s.cuda_stream)
+        assert len(_SharedWorkspace._by_stream) <= _SharedWorkspace.MAX_STREAMS
+    assert len(handles) > _SharedWorkspace.MAX_STREAMS
+    assert torch.equal(m(x), ref)                           # the first stream's buffer had been given back
+    held = set(map(id, _SharedWorkspace._by_stream.values()))
+    before = torch.cuda.memory_allocated()
+    del m
+    assert len(_SharedWorkspace._by_stream) == 0 or not held & set(map(id, _SharedWorkspace._by_stream.values()))
+    assert torch.cuda.memory_allocated() < before - (16 << 20)
