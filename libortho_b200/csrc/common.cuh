@@ -78,7 +78,7 @@ struct Plan {
     // ordered plans only: the entries once more as lists per 32 rows x 64 k (windows.cuh), without the long rows
     uint32_t *win_off;    // [ceil(N / 32)][ceil(K / 64) + 1]
     uint32_t *win_words;
-    void *blocks[3];      // the allocations behind entries, row_ptr, row_max and the lists
+    void *rows_block, *lists_block;      // the allocations behind entries, row_ptr and row_max, and behind the lists
 };
 constexpr int kLongRowMin = 64;
 constexpr int64_t kLongDenseMaxBytes = 256ll << 20;

@@ -243,8 +243,8 @@ int plan_build_long_rows(Plan *pl, cudaStream_t st, bool *dup_out)
     pl->n_pad = ceil_div(pl->n_long, lg::TR) * lg::TR;
     const size_t bytes = (size_t)pl->n_pad * (size_t)pl->K * 2;
     int *d_dup = nullptr;
-    cudaError_t e = cudaMalloc(&pl->hdense, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&d_dup, sizeof(int));
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&pl->hdense), bytes, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&d_dup), sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(pl->hdense, 0, bytes, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_dup, 0, sizeof(int), st);
     if (e == cudaSuccess) {
@@ -256,7 +256,7 @@ int plan_build_long_rows(Plan *pl, cudaStream_t st, bool *dup_out)
     int h_dup = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_dup, d_dup, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (d_dup) cudaFree(d_dup);
+    if (d_dup) cudaFreeAsync(d_dup, st);
     *dup_out = h_dup != 0;
     return (int)e;
 }

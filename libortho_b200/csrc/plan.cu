@@ -189,38 +189,34 @@ extern "C" int ortho_b200_plan_create(ortho_b200_plan **plan_out, const int32_t 
     pl->heavy = kLongRowMin; pl->n_long = 0; pl->n_pad = 0;
     pl->hrow = nullptr; pl->hdense = nullptr;
     pl->win_off = pl->win_words = nullptr;
-    for (void *&b : pl->blocks) b = nullptr;
+    pl->rows_block = pl->lists_block = nullptr;
+    cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e = cudaGetDevice(&pl->device);
+    if (e == cudaSuccess && nnz > 0) {
+        // the stream is synchronised below, and memory from the pool would become a node of the graph
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        e = cudaStreamIsCapturing(st, &cap);
+        if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+    }
     if (e != cudaSuccess) { note_cuda_error(e); delete pl; return ORTHO_B200_ERR_CUDA; }
     if (nnz > 0) {
-        cudaStream_t st = (cudaStream_t)stream;
-        // Device memory: {entries}, {row pointers, row maxima, list offsets, two result words}, {list entries}.
-        // cudaMalloc hands out pieces of up to 1 MB from blocks that it has mapped already and maps new memory for larger
-        // ones (some 400 us each, several times what all the kernels here take): three pieces for a small layer, one for a large one.
+        // Device memory: {entries, row pointers, row maxima, two result words} and {list offsets, list entries}, from the device's
+        // memory pool.  cudaMalloc maps memory 2 MB at a time for pieces of up to 1 MB, some 300 us each, and with the lists nearly
+        // every plan paid for one: a plan of 4096->4096 with 1 % took 376 us (median of 12) and takes 50, 8192->57344 with 0.3 %
+        // 464 and 119.  (The pool's first use in a process costs some 6 ms.)
         const int kblocks = (int)ceil_div(K, kWinK);
         const int64_t groups = ceil_div(N, kWinRows);
         const size_t noff = (size_t)groups * (size_t)(kblocks + 1);
-        const size_t size[3] = {(size_t)nnz, (size_t)(N + 1) + (size_t)N + noff + 2, (size_t)nnz};      // words
-        const bool pieces = nnz <= (1 << 20) / 4;
-        uint32_t *at[3] = {nullptr, nullptr, nullptr};
-        if (pieces) {
-            for (int i = 0; i < 3 && e == cudaSuccess; i++) {
-                e = cudaMalloc(&pl->blocks[i], sizeof(uint32_t) * size[i]);
-                at[i] = reinterpret_cast<uint32_t *>(pl->blocks[i]);
-            }
-        } else {
-            e = cudaMalloc(&pl->blocks[0], sizeof(uint32_t) * (size[0] + size[1] + size[2]));
-            at[0] = reinterpret_cast<uint32_t *>(pl->blocks[0]);
-            for (int i = 1; i < 3; i++) at[i] = at[i - 1] + size[i - 1];
-        }
+        e = cudaMallocAsync(&pl->rows_block, sizeof(uint32_t) * ((size_t)nnz + 2 * (size_t)N + 3), st);
+        if (e == cudaSuccess) e = cudaMallocAsync(&pl->lists_block, sizeof(uint32_t) * (noff + (size_t)nnz), st);
         int *d_info = nullptr;
         if (e == cudaSuccess) {
-            pl->entries = at[0];
-            pl->row_ptr = reinterpret_cast<int32_t *>(at[1]);
-            pl->row_max = reinterpret_cast<float *>(at[1] + N + 1);
-            pl->win_off = at[1] + 2 * N + 1;
-            d_info = reinterpret_cast<int *>(pl->win_off + noff);
-            pl->win_words = at[2];
+            pl->entries = reinterpret_cast<uint32_t *>(pl->rows_block);
+            pl->row_ptr = reinterpret_cast<int32_t *>(pl->entries + nnz);
+            pl->row_max = reinterpret_cast<float *>(pl->row_ptr + N + 1);
+            d_info = reinterpret_cast<int *>(pl->row_max + N);
+            pl->win_off = reinterpret_cast<uint32_t *>(pl->lists_block);
+            pl->win_words = pl->win_off + noff;
             e = cudaMemsetAsync(d_info, 0, 2 * sizeof(int), st);
         }
         auto build_windows = [&](int heavy) -> cudaError_t {
@@ -269,15 +265,16 @@ extern "C" int ortho_b200_plan_create(ortho_b200_plan **plan_out, const int32_t 
                 }
                 const size_t nl = hr.size();
                 if (nl > 0 && (int64_t)((nl + 127) / 128 * 128) * K * 2 <= kLongDenseMaxBytes) {
-                    e = cudaMalloc(&pl->hrow, sizeof(int32_t) * nl);
+                    e = cudaMallocAsync(reinterpret_cast<void **>(&pl->hrow), sizeof(int32_t) * nl, st);
+                    if (e == cudaSuccess) e = cudaStreamSynchronize(st);      // (the copy below is on another stream)
                     if (e == cudaSuccess) e = cudaMemcpy(pl->hrow, hr.data(), sizeof(int32_t) * nl, cudaMemcpyHostToDevice);
                     if (e == cudaSuccess) {
                         pl->n_long = (int64_t)nl;
                         bool dup = false;
                         e = (cudaError_t)plan_build_long_rows(pl, st, &dup);
                         if (e == cudaSuccess && dup) {         // a repeated column: every row stays with the in-kernel pass
-                            cudaFree(pl->hdense); pl->hdense = nullptr;
-                            cudaFree(pl->hrow); pl->hrow = nullptr;
+                            cudaFreeAsync(pl->hdense, st); pl->hdense = nullptr;
+                            cudaFreeAsync(pl->hrow, st); pl->hrow = nullptr;
                             pl->n_long = 0; pl->n_pad = 0;
                         }
                     }
@@ -289,7 +286,11 @@ extern "C" int ortho_b200_plan_create(ortho_b200_plan **plan_out, const int32_t 
                 return ORTHO_B200_ERR_CUDA;
             }
         }
-        if (!pl->ordered) pl->win_off = pl->win_words = nullptr;
+        if (!pl->ordered) {
+            pl->win_off = pl->win_words = nullptr;
+            cudaFreeAsync(pl->lists_block, st);
+            pl->lists_block = nullptr;
+        }
         if (pl->ordered && pl->n_long > 0) {
             e = build_windows(pl->heavy);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -309,10 +310,17 @@ extern "C" int ortho_b200_plan_destroy(ortho_b200_plan *plan)
     Plan *pl = reinterpret_cast<Plan *>(plan);
     if (!pl) return ORTHO_B200_OK;
     if (pl->magic != kPlanMagic) return ORTHO_B200_ERR_PLAN;
-    for (void *b : pl->blocks)
-        if (b) cudaFree(b);
-    if (pl->hrow) cudaFree(pl->hrow);
-    if (pl->hdense) cudaFree(pl->hdense);
+    void *const blocks[] = {pl->rows_block, pl->lists_block, pl->hrow, pl->hdense};
+    if (pl->nnz > 0) {
+        // cudaFree of pool memory does not wait for kernels that may still read it, as it does for cudaMalloc's
+        int dev = pl->device;
+        cudaGetDevice(&dev);
+        if (dev != pl->device) cudaSetDevice(pl->device);
+        cudaDeviceSynchronize();
+        for (void *b : blocks)
+            if (b) cudaFree(b);
+        if (dev != pl->device) cudaSetDevice(dev);
+    }
     pl->magic = 0;
     delete pl;
     return ORTHO_B200_OK;
