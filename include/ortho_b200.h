@@ -134,6 +134,9 @@ ORTHO_B200_API int ortho_b200_dequant_dump(const void *q_weight, const void *q_s
 #define ORTHO_B200_DECODE_MAX_M 64
 
 ORTHO_B200_API int64_t ortho_b200_workspace_bytes(int64_t M, int64_t K, int64_t N);
+/* The same for a forward whose sparse term is active and read from the CSR arrays: such a call of up to 16 tokens runs the
+ * streaming kernels whatever workspace it brings. */
+ORTHO_B200_API int64_t ortho_b200_csr_workspace_bytes(int64_t M, int64_t K, int64_t N);
 /* Workspace for forwards that pass this plan (the prefill regime keeps the pre-pass sums of the plan's long rows
  * there, so it may need more than the plan-less bound).  An empty plan answers like ortho_b200_workspace_bytes. */
 ORTHO_B200_API int64_t ortho_b200_plan_workspace_bytes(const ortho_b200_plan *plan, int64_t M);

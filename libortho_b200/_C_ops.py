@@ -131,7 +131,10 @@ def forward(q_weight: torch.Tensor, q_scales: torch.Tensor, ortho_values: torch.
         if ortho_row_ptr.numel() != N + 1 or ortho_col_indices.numel() != nnz:
             raise ValueError("CSR arrays have inconsistent sizes")
     # scratch of the tensor-core regimes (sparse pre-pass, partial sums of split tiles); 0 for the streaming kernels
-    need = workspace_bytes(M, K, N, plan)
+    if plan is None and nnz and alpha > 0:
+        need = int(_lib.lib().ortho_b200_csr_workspace_bytes(M, K, N))
+    else:
+        need = workspace_bytes(M, K, N, plan)
     ws_ptr, ws_bytes = None, 0
     if need:
         if workspace is None or workspace.numel() * workspace.element_size() < need:

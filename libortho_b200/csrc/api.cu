@@ -142,6 +142,11 @@ extern "C" int64_t ortho_b200_workspace_bytes(int64_t M, int64_t K, int64_t N)
     return mid > other ? mid : other;
 }
 
+extern "C" int64_t ortho_b200_csr_workspace_bytes(int64_t M, int64_t K, int64_t N)
+{
+    return M <= 16 && decode_regime(M, N, K) && !tuning_snapshot().mid_first ? 0 : ortho_b200_workspace_bytes(M, K, N);
+}
+
 namespace ob {
 int forward_impl(const void *q_weight, const void *q_scales_f16,
                  const void *ortho_values_f16, const int32_t *ortho_col_indices,
@@ -157,12 +162,12 @@ int forward_impl(const void *q_weight, const void *q_scales_f16,
                                  x_f16, y_f16, M, K, N, alpha, plan, workspace, workspace_bytes, stream, ldy, bias_f32);
     if (st != ORTHO_B200_OK || M == 0) return st;
     a.gv = gv; a.gather_fused = gather_fused;
-    return launch_routed(a);
+    return launch_routed(a, route_of(a));
 }
 
-int launch_routed(const FwdArgs &a)
+int launch_routed(const FwdArgs &a, Route route)
 {
-    switch (route_of(a)) {
+    switch (route) {
         case kRouteMid: return launch_mid(a);
         case kRouteDecode: return launch_decode(a);
         default: return launch_prefill(a);
@@ -252,18 +257,20 @@ extern "C" int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers, int
     if (n_layers == 0 || M == 0) return ORTHO_B200_OK;
     if (n_layers > ORTHO_B200_MULTI_MAX_LAYERS) return ORTHO_B200_ERR_SHAPE;
     FwdArgs a[ORTHO_B200_MULTI_MAX_LAYERS];
-    bool all_stream = true;
+    Route route[ORTHO_B200_MULTI_MAX_LAYERS];
+    bool all_stream = n_layers > 1 && stream_kernel_selected(M, K);
     for (int l = 0; l < n_layers; l++) {
         const ortho_b200_layer_desc &d = layers[l];
         const int st = make_fwd_args(a[l], d.q_weight, d.q_scales_f16, d.ortho_values_f16, d.ortho_col_indices,
                                      d.ortho_row_ptr, d.nnz, x_f16, d.y_f16, M, K, d.N, d.alpha, d.plan,
                                      workspace, workspace_bytes, stream, d.ldy, d.bias_f32);
         if (st != ORTHO_B200_OK) return st;
-        all_stream = all_stream && route_of(a[l]) == kRouteDecode && stream_kernel_selected(M, K);
+        route[l] = route_of(a[l]);
+        all_stream = all_stream && route[l] == kRouteDecode;
     }
-    if (all_stream && n_layers > 1) return launch_decode_multi(a, n_layers);
+    if (all_stream) return launch_decode_multi(a, n_layers);
     for (int l = 0; l < n_layers; l++) {
-        const int st = launch_routed(a[l]);
+        const int st = launch_routed(a[l], route[l]);
         if (st != ORTHO_B200_OK) return st;
     }
     return ORTHO_B200_OK;
@@ -274,7 +281,8 @@ extern "C" int64_t ortho_b200_multi_workspace_bytes(const ortho_b200_layer_desc 
     int64_t need = 0;
     for (int l = 0; l < n_layers; l++) {
         const ortho_b200_layer_desc &d = layers[l];
-        const int64_t w = d.plan ? ortho_b200_plan_workspace_bytes(d.plan, M) : ortho_b200_workspace_bytes(M, K, d.N);
+        const int64_t w = d.plan ? ortho_b200_plan_workspace_bytes(d.plan, M)
+                        : d.nnz > 0 && d.alpha > 0.f ? ortho_b200_csr_workspace_bytes(M, K, d.N) : ortho_b200_workspace_bytes(M, K, d.N);
         if (w < 0) return -1;
         need = w > need ? w : need;
     }

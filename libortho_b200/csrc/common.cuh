@@ -287,7 +287,6 @@ int make_fwd_args(FwdArgs &a, const void *q_weight, const void *q_scales_f16, co
                   const void *x_f16, void *y_f16, int64_t M, int64_t K, int64_t N, float alpha,
                   const ortho_b200_plan *plan, void *workspace, int64_t workspace_bytes, void *stream,
                   int64_t ldy, const float *bias_f32);
-int launch_routed(const FwdArgs &a);                      // api.cu: picks the kernel family and launches
 int launch_decode_multi(const FwdArgs *layers, int nl);   // decode.cu: one streaming launch for layers that share x
 int launch_prefill(const FwdArgs &a);
 int64_t long_rows_workspace_bytes(const Plan *pl, int64_t M);            // longrows.cu
@@ -307,6 +306,7 @@ enum Route { kRouteDecode = 0, kRouteMid = 1, kRoutePrefill = 2 };
 bool mid_range(int64_t M, int64_t N, int64_t K);
 Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool lists);
 Route route_of(const FwdArgs &a);
+int launch_routed(const FwdArgs &a, Route route);                   // api.cu
 int launch_mid(const FwdArgs &a);                                  // mid.cu
 int64_t mid_workspace_bytes(int64_t M, int64_t K, int64_t N);
 }  // namespace ob

@@ -18,6 +18,7 @@
 // across the cluster, so there is no global scratch and the result is deterministic.
 #include <cooperative_groups.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -267,10 +268,18 @@ struct DecodeCfg { int wr, wk, u, s; };
 // few per cent.
 static std::mutex g_tune_mu;
 static Tuning g_tune;
+static std::atomic<unsigned> g_tune_gen{1};       // counts the changes
+// A forward asks several times: the thread's own copy answers until the hook has been used.
 Tuning tuning_snapshot()
 {
-    std::lock_guard<std::mutex> lock(g_tune_mu);
-    return g_tune;
+    thread_local Tuning t;
+    thread_local unsigned gen = 0;
+    if (g_tune_gen.load(std::memory_order_acquire) != gen) {
+        std::lock_guard<std::mutex> lock(g_tune_mu);
+        t = g_tune;
+        gen = g_tune_gen.load(std::memory_order_relaxed);
+    }
+    return t;
 }
 
 // Which regime a forward runs in.  Above the token threshold the tensor-core kernel wins unless the layer (or
@@ -343,6 +352,7 @@ int set_decode_config(int wr, int wk, int u, int s)
 {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     Tuning &t = g_tune;
+    g_tune_gen.fetch_add(1, std::memory_order_release);      // (a reader that sees it waits for the lock)
     if (wr == -3) {       // forwards with more than s tokens (0 <= s <= 64) go to the tensor-core prefill kernel
         if (s < 0 || s > ORTHO_B200_DECODE_MAX_M) return ORTHO_B200_ERR_SHAPE;
         t.prefill_above = s;

@@ -94,5 +94,5 @@ extern "C" int ortho_b200_forward_static_scratch(const void *q_weight, const voi
     a.workspace = scratch;
     a.workspace_bytes = (int64_t)ORTHO_B200_STATIC_SCRATCH_BYTES;
     a.stream = (cudaStream_t)stream;
-    return launch_routed(a);
+    return launch_routed(a, route_of(a));
 }

@@ -234,3 +234,19 @@ def test_scratch_is_bounded_and_given_back():
     del m
     assert len(_SharedWorkspace._by_stream) == 0 or not held & set(map(id, _SharedWorkspace._by_stream.values()))
     assert torch.cuda.memory_allocated() < before - (16 << 20)
+
+
+def test_a_small_batch_on_raw_csr_brings_no_workspace():
+    """Up to 16 tokens the streaming kernels serve the CSR arrays: the binding allocates nothing on the way, and the size query
+    for such calls says so; the same layer with a plan or without a sparse term asks for room."""
+    lib, K, N = _lib.lib(), 8192, 5300
+    layer = wl.make_layer(K, N, 0.003, seed=3, device=DEV)
+    for M in (12, 16):
+        assert lib.ortho_b200_csr_workspace_bytes(M, K, N) == 0 < lib.ortho_b200_workspace_bytes(M, K, N)
+        x, y = wl.make_input(M, K, seed=1, device=DEV), torch.empty(M, N, dtype=torch.float16, device=DEV)
+        count = torch.cuda.memory_stats()["allocation.all.allocated"]
+        _C_ops.forward(layer.base_weight, layer.base_scales, layer.vals, layer.col, layer.row_ptr, x, y, 1.0)
+        _C_ops.forward_multi([(layer.base_weight, layer.base_scales, layer.vals, layer.col, layer.row_ptr)], x, [y])
+        assert torch.cuda.memory_stats()["allocation.all.allocated"] == count
+    for M in (17, 300):
+        assert lib.ortho_b200_csr_workspace_bytes(M, K, N) == lib.ortho_b200_workspace_bytes(M, K, N) > 0
