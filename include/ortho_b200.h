@@ -159,7 +159,8 @@ ORTHO_B200_API int ortho_b200_forward(const void *q_weight, const void *q_scales
  * (FP32 [N], may be NULL) is added in the kernels' FP32 epilogue before the single FP16 rounding.
  * Every layer has its own alpha (the reference's kill switch, per layer).  All layers read x [M, K];
  * layer l writes y_f16 [M, N] with row pitch ldy (0 = N).  For M <= 16 and K a multiple of 256 the tiles
- * of all layers are walked by one persistent kernel launch; otherwise the layers run one after the other on
+ * of all layers are walked by one persistent kernel launch, unless a launch per layer is faster (5 .. 16 tokens on
+ * large layers, some of them on the tensor cores); otherwise the layers run one after the other on
  * the stream, sharing the workspace (ortho_b200_multi_workspace_bytes = the largest any of them needs).
  * n_layers <= ORTHO_B200_MULTI_MAX_LAYERS.  n_layers == 1 is the ordinary forward plus the bias.
  * ------------------------------------------------------------------------------------------- */

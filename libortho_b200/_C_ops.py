@@ -157,7 +157,8 @@ def forward_multi(layers, input: torch.Tensor, outputs, alphas=None, biases=None
     """Several layers that read the same ``input`` [M, K] (separate Q / K / V or gate / up projections), each
     with its own alpha and an optional FP32 bias fused into the kernel: ``layers`` is a sequence of
     ``(q_weight, q_scales, ortho_values, ortho_col_indices, ortho_row_ptr)`` tuples, ``outputs`` the matching
-    FP16 ``[M, N_l]`` tensors written in place.  Up to 16 tokens (K a multiple of 256) run as ONE kernel launch."""
+    FP16 ``[M, N_l]`` tensors written in place.  Up to 16 tokens (K a multiple of 256) run as ONE kernel launch where
+    that is faster than one per layer."""
     n = len(layers)
     if n == 0:
         return

@@ -246,7 +246,8 @@ extern "C" int ortho_b200_forward(const void *q_weight, const void *q_scales_f16
 
 // Several layers that read the same activations (separate Q / K / V or gate / up projections): in the
 // decode regime their tiles are walked by ONE persistent launch, so that the fixed cost of a launch
-// (a few microseconds on layers that stream for 5-20) is paid once per group instead of once per layer;
+// (a few microseconds on layers that stream for 5-20) is paid once per group instead of once per layer (unless
+// the tensor-core kernel of mid.cu is faster for the group, decode.cu);
 // elsewhere the layers run one after the other on the stream.  The reference reaches the operator with
 // one blocking launch per layer (src/dual_gemm.cu:317-346,366; torch_bind/ortho_linear.py:139-151).
 extern "C" int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers, int n_layers,
@@ -258,7 +259,7 @@ extern "C" int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers, int
     if (n_layers > ORTHO_B200_MULTI_MAX_LAYERS) return ORTHO_B200_ERR_SHAPE;
     FwdArgs a[ORTHO_B200_MULTI_MAX_LAYERS];
     Route route[ORTHO_B200_MULTI_MAX_LAYERS];
-    bool all_stream = n_layers > 1 && stream_kernel_selected(M, K);
+    bool all_stream = n_layers > 1 && stream_kernel_selected(M, K), any_mid = false;
     for (int l = 0; l < n_layers; l++) {
         const ortho_b200_layer_desc &d = layers[l];
         const int st = make_fwd_args(a[l], d.q_weight, d.q_scales_f16, d.ortho_values_f16, d.ortho_col_indices,
@@ -266,8 +267,10 @@ extern "C" int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers, int
                                      workspace, workspace_bytes, stream, d.ldy, d.bias_f32);
         if (st != ORTHO_B200_OK) return st;
         route[l] = route_of(a[l]);
-        all_stream = all_stream && route[l] == kRouteDecode;
+        any_mid = any_mid || route[l] == kRouteMid;
+        all_stream = all_stream && route[l] != kRoutePrefill;
     }
+    if (all_stream && any_mid && (tuning_snapshot().mid_first || !group_streams(a, route, n_layers))) all_stream = false;
     if (all_stream) return launch_decode_multi(a, n_layers);
     for (int l = 0; l < n_layers; l++) {
         const int st = launch_routed(a[l], route[l]);

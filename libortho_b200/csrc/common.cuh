@@ -306,6 +306,7 @@ enum Route { kRouteDecode = 0, kRouteMid = 1, kRoutePrefill = 2 };
 bool mid_range(int64_t M, int64_t N, int64_t K);
 Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool lists);
 Route route_of(const FwdArgs &a);
+bool group_streams(const FwdArgs *a, const Route *route, int n);   // decode.cu
 int launch_routed(const FwdArgs &a, Route route);                   // api.cu
 int launch_mid(const FwdArgs &a);                                  // mid.cu
 int64_t mid_workspace_bytes(int64_t M, int64_t K, int64_t N);

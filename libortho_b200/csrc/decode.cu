@@ -345,6 +345,28 @@ Route route_of(const FwdArgs &a)
     return route_of(a.M, a.N, a.K, a.workspace, a.workspace_bytes, lists);
 }
 
+// Whether layers of up to 16 tokens that share their activations run as one streaming launch although mid.cu would take some of
+// them by themselves.  Estimates in us, from the layers above and groups of them (one B200, 0.3 % ortho, weights from HBM; W =
+// millions of weights): a launch of mid.cu 9.3 + 0.16 W, a streaming launch 5 + r W, where r depends on the activation slab
+// and the token count; without a sparse term the slopes are two thirds.  One streaming launch / a launch per layer, measured:
+//   8192->8192 + 2 x 1024:  8 tokens 24.8 / 34.7, 12: 32.4 / 36.5, 16: 44.1 / 36.8;   3 x 5120->5120:  9: 26.6 / 39.6, 16: 42.2 / 39.4
+//   3 x 8192->8192:  8: 53.8 / 58.4, 9: 63.3 / 58.3, 16: 99 / 59;   2 x 4096->11008:  9: 28.8 / 30.8, 12: 29.3 / 31.2, 16: 32.8 / 31.4
+//   2 x 8192->28672:  8: 118 / 90, 16: 221 / 90;   2 x 28672->1024:  9: 31.9 / 34.6, 16: 33.9 / 35.2
+bool group_streams(const FwdArgs *a, const Route *route, int n)
+{
+    const int64_t M = a[0].M, slab = 2 * M * a[0].K;
+    float r;
+    if (M > 8) r = slab > (200 << 10) ? 0.44f : M <= 12 ? 0.31f : slab > (150 << 10) ? 0.47f : 0.34f;
+    else r = slab > (200 << 10) ? 0.32f : slab > (100 << 10) ? 0.25f : 0.21f;
+    float one = 5.f, apart = 0.f;
+    for (int l = 0; l < n; l++) {
+        const float w = 1e-6f * (float)(a[l].N * a[l].K) * (a[l].has_ortho ? 1.f : 0.67f);
+        one += r * w;
+        apart += route[l] == kRouteMid ? 9.3f + 0.16f * w : 5.f + r * w;
+    }
+    return one <= apart;
+}
+
 int launch_decode_stream(const FwdArgs &a, int S, int stages);          // decode_stream.cu
 int launch_decode_stream_multi(const FwdArgs *layers, int nl, int S, int stages);
 

@@ -250,3 +250,19 @@ def test_a_small_batch_on_raw_csr_brings_no_workspace():
         assert torch.cuda.memory_stats()["allocation.all.allocated"] == count
     for M in (17, 300):
         assert lib.ortho_b200_csr_workspace_bytes(M, K, N) == lib.ortho_b200_workspace_bytes(M, K, N) > 0
+
+
+@pytest.mark.parametrize("M,K,Ns,launches", [(8, 8192, (8192, 1024, 1024), 1), (12, 8192, (8192, 1024, 1024), 1), (16, 8192, (8192, 1024, 1024), 3),
+                                             (9, 4096, (11008, 11008), 1), (16, 4096, (11008, 11008), 2), (3, 8192, (4096, 264), 1)])
+def test_layers_of_one_input_whose_own_routes_differ(M, K, Ns, launches):
+    """One streaming launch or a launch per layer, whichever is faster for the group; the same values either way."""
+    layers = [wl.make_layer(K, n, 0.003, seed=n, device=DEV) for n in Ns]
+    plans = [_C_ops.Plan(t.row_ptr, t.col, t.vals, K, t.N) for t in layers]
+    x = wl.make_input(M, K, seed=M, device=DEV)
+    ys = [torch.empty(M, n, dtype=torch.float16, device=DEV) for n in Ns]
+    before = _lib.lib().ortho_b200_launch_count()
+    _C_ops.forward_multi([(t.base_weight, t.base_scales, t.vals, t.col, t.row_ptr) for t in layers], x, ys, alphas=[1.0, 0.5, 0.0][:len(Ns)], plans=plans)
+    assert _lib.lib().ortho_b200_launch_count() - before == launches
+    for t, p, y, alpha in zip(layers, plans, ys, (1.0, 0.5, 0.0)):
+        ref = multi(t, x, alpha, p).double()
+        assert float((y.double() - ref).norm() / ref.norm()) <= REL_FRO_TOL
