@@ -108,7 +108,7 @@ ORTHO_B200_API int ortho_b200_dequant_dump(const void *q_weight, const void *q_s
  * torch_bind/ortho_linear.py:142-151); same argument order and meaning, plus explicit sizes,
  * the optional plan, a caller-owned workspace and the stream.
  *
- *   M <= 16   : memory-bound streaming kernels, except where the next kernel is faster (9 .. 16 tokens on layers of more
+ *   M <= 16   : memory-bound streaming kernels, except where the next kernel is faster (9 .. 16 tokens on most layers of more
  *               than 4096 x 4096 weights, fewer with large activations; it then needs its workspace); the mma.sync
  *               kernel also serves M <= 32 on layers of at most 4096 x 4096 weights when the sparse term is active
  *               without an ordered plan, and, for calls without a workspace, M <= 24, M <= 32 with N <= 4096 and

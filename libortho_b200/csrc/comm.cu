@@ -240,10 +240,10 @@ extern "C" int ortho_b200_forward_gather(const void *q_weight, const void *q_sca
     // deferred mode: the streaming decode kernel waits for the previous exchange itself; any other
     // kernel is preceded by the one-thread wait kernel
     const Plan *pl = reinterpret_cast<const Plan *>(plan);
-    const bool lists = !(alpha > 0.f && (pl && pl->magic == kPlanMagic ? pl->nnz : nnz) > 0) ||
-                       (pl && pl->magic == kPlanMagic && pl->win_off && tuning_snapshot().patch_weights);
+    const bool base = !(alpha > 0.f && (pl && pl->magic == kPlanMagic ? pl->nnz : nnz) > 0);
+    const bool lists = base || (pl && pl->magic == kPlanMagic && pl->win_off && tuning_snapshot().patch_weights);
     const bool self_waits = N_local > 0 && stream_kernel_selected(M, K) &&
-                            route_of(M, N_local, K, workspace, workspace_bytes, lists) == kRouteDecode;
+                            route_of(M, N_local, K, workspace, workspace_bytes, base, lists) == kRouteDecode;
     if (cm->deferred && cm->world > 1 && !self_waits) {
         gather_wait_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(gv, status);
         OB_CUDA(cudaGetLastError());

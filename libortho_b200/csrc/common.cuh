@@ -304,7 +304,7 @@ bool decode_regime(int64_t M, int64_t N, int64_t K);
 // range that brings none runs the kernels of the neighbouring regimes instead.
 enum Route { kRouteDecode = 0, kRouteMid = 1, kRoutePrefill = 2 };
 bool mid_range(int64_t M, int64_t N, int64_t K);
-Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool lists);
+Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool base, bool lists);
 Route route_of(const FwdArgs &a);
 bool group_streams(const FwdArgs *a, const Route *route, int n);   // decode.cu
 int launch_routed(const FwdArgs &a, Route route);                   // api.cu

@@ -298,41 +298,62 @@ static bool decode_regime_of(const Tuning &t, int64_t M, int64_t N, int64_t K)
 }
 bool decode_regime(int64_t M, int64_t N, int64_t K) { return decode_regime_of(tuning_snapshot(), M, N, K); }
 // The tcgen05 kernel of mid.cu against the streaming kernel (up to 16 tokens; needs its sparse entries as window lists or
-// none at all).  Its time hardly depends on the token count, the streaming kernel's grows with it and with the
-// activation slab of a CTA (M x K halves): above 100 KB one CTA fits an SM instead of two, above 200 KB K is split over a cluster.
-// One B200, us, 0.3 % ortho, streaming / mid.cu:
-//   16 tokens: 4096->4096 9.6 / 10.3, 2048->4096 7.3 / 8.4, 8192->1024 8.4 / 10.1, but 4096->12288 19.3 / 14.8,
-//              8192->8192 32.2 / 17.7, 8192->57344 201 / 77, 28672->8192 100 / 43;   9 tokens: 8192->4096 13.8 / 13.1
-//    8 tokens: 4096->22016 18.9 / 19.8, 8192->4096 12.0 / 13.1, 28672->1024 13.3 / 16.9, but 8192->8192 18.6 / 17.6,
-//              11008->4096 16.9 / 15.0, 8192->57344 104 / 77, 28672->8192 77 / 43;   5 tokens: 14336->4096 15.0 / 17.0
-//    6 tokens: 8192->16384 26.2 / 26.8, but 8192->57344 91 / 77;
-//    4 tokens: 16384->16384 42 / 47, 8192->57344 62 / 77, but 28672->4096 29.2 / 25.6, 28672->8192 50 / 43;
-//              3 tokens: 28672->4096 21.8 / 25.6
-static bool mid_beats_stream(int64_t M, int64_t N, int64_t K)
+// none at all).  Its time hardly depends on the token count (about 9 us + 0.15 us, base-only 0.1 us, per million weights + 0.1 us
+// per 1000 inputs), the streaming kernel's grows with it, with the rounds of row tiles (of 16 rows, two per SM at a time) and
+// with the activation slab of a CTA (M x K halves): above 100 KB one CTA fits an SM instead of two, above 200 KB K is split
+// over a cluster.  One B200, us, weights rotating over more than L2, streaming / mid.cu with 0.3 % ortho; base-only:
+//   16 tokens: 4096->4096 9.8 / 11.9; 8.1 / 10.4, 8192->2048 13.4 / 12.8; 10.9 / 11.2, 4096->6144 14.1 / 13.0; 11.2 / 11.5,
+//              11008->2048 14.4 / 14.2; 11.5 / 12.6, 8192->4096 20.5 / 14.5; 16.5 / 12.4, 4096->12288 19.9 / 16.2; 15.2 / 13.4
+//   12 tokens: 4096->8192 13.6 / 13.9; 10.4 / 12.1, 8192->4096 15.4 / 14.6; 12.1 / 12.6, 28672->1024 20.0 / 17.5; 14.2 / 15.2,
+//              5120->5120 15.3 / 13.3; 12.4 / 11.6, 11008->3072 18.9 / 15.2; 15.7 / 12.9
+//    9 tokens: 4096->6144 12.3 / 13.0; 9.4 / 11.5, 4096->8192 13.1 / 14.1; 9.9 / 12.2, 11008->2048 11.4 / 13.8; 9.3 / 12.3,
+//              5120->8192 15.3 / 15.5; 12.1 / 13.0, 2048->14336 14.3 / 12.6; 9.6 / 11.2, 11008->4096 17.4 / 16.5; 14.1 / 13.7,
+//              4096->10240 17.0 / 15.6; 12.8 / 13.0, 8192->57344 125 / 85; 96 / 59
+//    8 tokens: 4096->22016 20.3 / 21.4, 8192->4096 12.6 / 14.6, 8192->8192 19.6 / 19.6, 8192->10240 23.2 / 22.1, 11008->4096 17.7 / 16.5
+//    6 tokens: 12288->6144 20.7 / 21.3, 28672->1536 17.8 / 18.1, 20480->2048 15.5 / 17.4, 14336->4096 19.9 / 19.0,
+//              8192->57344 93 / 85
+//    5 tokens: 13824->5120 19.6 / 20.7, 28672->1536 15.2 / 18.6, 28672->4096 28.3 / 28.5, 28672->8192 52 / 47, 16384->16384 68 / 52
+//    4 tokens: 28672->4096 30.6 / 28.4, 28672->8192 52 / 47, 16384->16384 44 / 52;   3 tokens: 28672->4096 23.2 / 28.4
+static bool mid_beats_stream(int64_t M, int64_t N, int64_t K, bool base)
 {
     const int64_t weights = N * K, slab = 2 * M * K;
-    if (M >= 9) return weights > (int64_t)4096 * 4096;
+    const bool odd = K % 256 != 0;                       // the mma.sync kernel stands in for the streaming kernel
+    if (M >= 9) {
+        if (weights <= (int64_t)4096 * 4096) return false;
+        if (odd) return true;
+        if (base) {
+            if (M <= 12 && slab <= (100 << 10)) return weights >= (int64_t)1 << 26;
+            return weights >= (int64_t)5 << 23 || (N > 2048 && (slab > (192 << 10) || (K > 4096 && (M > 12 || K <= 6144)))) ||
+                   (N >= 2048 && slab >= (512 << 10));
+        }
+        if (M <= 12 && K <= 4096 && N <= 2 * 2 * 148 * 16) return false;            // two rounds of tiles
+        return slab > (200 << 10) || N > 2048;
+    }
     if (weights < (int64_t)5 << 23) return false;
-    if (slab > (200 << 10)) return M >= 3;
+    if (slab >= (200 << 10)) return M >= 3 && (odd || weights >= (int64_t)3 << 24);
     if (M >= 6 && weights >= (int64_t)1 << 28) return true;
-    return M >= 5 && (slab >= (150 << 10) || (slab >= (128 << 10) && weights >= (int64_t)1 << 26));
+    return M >= 5 && (slab >= (150 << 10) || ((odd || M >= 7) && slab >= (128 << 10) && weights >= (int64_t)1 << 26));
 }
-static bool mid_range_of(const Tuning &t, int64_t M, int64_t N, int64_t K)
+static bool mid_range_of(const Tuning &t, int64_t M, int64_t N, int64_t K, bool base)
 {
     if (M > 128) return false;
     if (M > t.mid_lo && M <= t.mid_hi) return true;
-    return !t.mid_first && M <= 16 && t.wr == 0 && !t.force_stream && mid_beats_stream(M, N, K);
+    return !t.mid_first && M <= 16 && t.wr == 0 && !t.force_stream && mid_beats_stream(M, N, K, base);
 }
-bool mid_range(int64_t M, int64_t N, int64_t K) { return mid_range_of(tuning_snapshot(), M, N, K); }
-// `lists`: the sparse term is inactive or comes as a plan's window lists.  From 17 tokens on the mma.sync kernel below is
+bool mid_range(int64_t M, int64_t N, int64_t K)
+{
+    const Tuning t = tuning_snapshot();
+    return mid_range_of(t, M, N, K, false) || mid_range_of(t, M, N, K, true);
+}
+// `base`: the sparse term is inactive; `lists`: it is, or it comes as a plan's window lists.  From 17 tokens on the mma.sync kernel below is
 // behind on every layer then (32 tokens: 1024->1024 14.6 / 6.2, 4096->4096 32.4 / 12.1, 8192->2048 26.8 / 14.6,
 // 4096->22016 88 / 21).  Without lists mid.cu needs two more launches for the sparse term, which small layers do not earn
 // back (raw CSR, 0.5 %, 32 tokens: 1024->1024 14.8 / 23.8, 4096->1024 16.0 / 28.8, 4096->4096 34.8 / 30.4), and up to 16
 // tokens no layer does.  Without the workspace the rule between the mma.sync kernel and the prefill tile stands.
-Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool lists)
+Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool base, bool lists)
 {
     const Tuning t = tuning_snapshot();
-    if (mid_range_of(t, M, N, K) && workspace && ((uintptr_t)workspace & 255u) == 0 && workspace_bytes >= mid_workspace_bytes(M, K, N)) {
+    if (mid_range_of(t, M, N, K, base) && workspace && ((uintptr_t)workspace & 255u) == 0 && workspace_bytes >= mid_workspace_bytes(M, K, N)) {
         if (t.mid_first || lists) return kRouteMid;
         if (M > 16 && !(t.prefill_above == kPrefillAboveBuiltin && M <= 32 && N * K <= (int64_t)4096 * 4096)) return kRouteMid;
     }
@@ -342,7 +363,7 @@ Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t w
 Route route_of(const FwdArgs &a)
 {
     const bool lists = !a.has_ortho || (a.plan && a.plan->win_off && tuning_snapshot().patch_weights);
-    return route_of(a.M, a.N, a.K, a.workspace, a.workspace_bytes, lists);
+    return route_of(a.M, a.N, a.K, a.workspace, a.workspace_bytes, !a.has_ortho, lists);
 }
 
 // Whether layers of up to 16 tokens that share their activations run as one streaming launch although mid.cu would take some of
