@@ -49,6 +49,7 @@ struct Tuning {
     bool mid_first = false;
     bool gather_per_cta = false;        // peer exchange: every CTA signals the peers itself instead of the grid's last CTA
     bool patch_weights = true;          // tensor-core kernels fold the sparse entries into the weight tile (plan with ordered rows)
+    bool wide = true;                   // more than 128 tokens: wide.cu where it can (false: prefill.cu for every call)
     int long_row_min = 64;              // = kLongRowMin: a plan's long-row threshold is max(this, 4 x the mean row)
 };
 constexpr int kPrefillAboveBuiltin = 24;

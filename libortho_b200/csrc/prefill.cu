@@ -689,8 +689,9 @@ int launch_prefill(const FwdArgs &a)
     using namespace pf;
     // base-only calls and plans with window lists run the kernel of wide.cu (measured there); the rest, the sparse term as
     // gathers and the peer exchange, stays here
-    const bool lists = a.has_ortho && a.plan && a.plan->win_off && tuning_snapshot().patch_weights;
-    if (!(a.gv && a.gv->world > 1) && (!a.has_ortho || lists)) {
+    const Tuning t = tuning_snapshot();
+    const bool lists = a.has_ortho && a.plan && a.plan->win_off && t.patch_weights;
+    if (t.wide && !(a.gv && a.gv->world > 1) && (!a.has_ortho || lists)) {
         if (lists && a.plan->n_long > 0) {
             if (!a.workspace || a.workspace_bytes < prefill_xt_bytes(a.M, a.K) + long_rows_workspace_bytes(a.plan, a.M))
                 return ORTHO_B200_ERR_WORKSPACE;

@@ -266,3 +266,15 @@ def test_layers_of_one_input_whose_own_routes_differ(M, K, Ns, launches):
     for t, p, y, alpha in zip(layers, plans, ys, (1.0, 0.5, 0.0)):
         ref = multi(t, x, alpha, p).double()
         assert float((y.double() - ref).norm() / ref.norm()) <= REL_FRO_TOL
+
+
+def test_a_plan_is_refused_under_capture_and_the_capture_goes_on():
+    layer = wl.make_layer(512, 96, 0.02, seed=1, device=DEV)
+    y = torch.zeros(4, device=DEV)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with pytest.raises(_lib.OrthoB200Error):
+            _C_ops.Plan(layer.row_ptr, layer.col, layer.vals, layer.K, layer.N)
+        y.add_(1)
+    graph.replay()
+    assert bool((y == 1).all())

@@ -446,10 +446,10 @@ def test_swapped_model_runs_and_the_kill_switch_works():
     (33, 512, 520, 0.01, "gauss", 0.25), (64, 2048, 96, 0.01, "gauss", 1.0), (128, 384, 272, 0.02, "gauss", 1.0),
     (100, 1184, 210, 0.02, "gauss", 0.75), (9, 8192, 2048, 0.003, "gauss", 1.0), (32, 11008, 512, 0.005, "gauss", 1.0),
     (48, 4096, 4352, 0.003, "gauss", 0.0)])
-def test_tokens_as_m_kernel_against_oracle(oracle_mod, M, K, N, d, kind, alpha):
-    """The tcgen05 kernel whose M operand is the token block (up to 128 tokens, 256 weight rows per MMA, stream-K
-    split with partial sums in the workspace) through the tuning hook: ragged M / N / K, shares that start inside
-    a row tile, long Zipf rows, bias, and the kill switch."""
+def test_small_token_block_kernel_against_oracle(oracle_mod, M, K, N, d, kind, alpha):
+    """The tcgen05 kernel for small token blocks (up to 128 tokens, 128 weight rows per MMA, stream-K split with partial
+    sums in the workspace) on raw CSR arrays through the tuning hook: ragged M / N / K, shares that start inside a row
+    tile, long Zipf rows, bias, and the kill switch."""
     layer = wl.make_layer(K, N, d, seed=400 + M, ortho=kind)
     x = wl.make_input(M, K, seed=400 + M)
     g = torch.Generator().manual_seed(M)
@@ -472,8 +472,8 @@ def test_tokens_as_m_kernel_against_oracle(oracle_mod, M, K, N, d, kind, alpha):
         _lib.lib().ortho_b200_set_decode_config(-4, 0, 0, 0)
     assert _lib.lib().ortho_b200_query_kernel_status() == 0
     ref = layer_oracle(oracle_mod, layer, x, alpha)
-    assert_close(ys[False].float().cpu().numpy(), ref, f"tokens-as-M M={M} {K}->{N}")
-    assert_close(ys[True].float().cpu().numpy(), ref + bias.numpy()[None, :], f"tokens-as-M + bias M={M} {K}->{N}")
+    assert_close(ys[False].float().cpu().numpy(), ref, f"small token block M={M} {K}->{N}")
+    assert_close(ys[True].float().cpu().numpy(), ref + bias.numpy()[None, :], f"small token block + bias M={M} {K}->{N}")
     assert launches[False] == (3 if (alpha > 0 and layer.nnz) else 1)       # transpose + sparse pre-pass + the MMA kernel
     empty = wl.Layer(K, N, ld.base_weight, ld.base_scales, torch.zeros(N + 1, dtype=torch.int32, device=DEV), ld.col[:0], ld.vals[:0], 1.0)
     try:
@@ -547,10 +547,10 @@ def test_rows_that_cannot_be_folded_keep_the_gather_path(oracle_mod):
 
 @pytest.mark.parametrize("M,K,N,d", [(32, 1024, 520, 0.01), (100, 4096, 300, 0.003), (128, 2048, 1100, 0.02), (48, 8192, 2048, 0.003),
                                      (100, 1184, 210, 0.02), (17, 96, 130, 0.05)])
-def test_tokens_as_m_kernel_folds_the_sparse_term(oracle_mod, M, K, N, d):
-    """17..128 tokens with a plan and a workspace: the tokens-as-M kernel adds the sparse entries to its weight tile
-    (one launch, shares that start inside a row), gathers the rows whose scale is zero or tiny in its epilogue, and
-    agrees with the oracle and with the gather form (transpose + sparse pre-pass + the MMA kernel)."""
+def test_small_token_block_kernel_contracts_the_sparse_term(oracle_mod, M, K, N, d):
+    """17..128 tokens with a plan and a workspace: one launch that contracts the sparse entries from scattered tiles with an
+    accumulator of their own (so a zero or tiny row scale needs no other path), shares that start inside a row tile; agrees
+    with the oracle and with the gather form (transpose + sparse pre-pass + the MMA kernel)."""
     layer = wl.make_layer(K, N, d, seed=900 + M)
     scales = layer.base_scales.clone()
     counts = layer.row_ptr[1:] - layer.row_ptr[:-1]
@@ -584,8 +584,8 @@ def test_tokens_as_m_kernel_folds_the_sparse_term(oracle_mod, M, K, N, d):
     assert _lib.lib().ortho_b200_query_kernel_status() == 0
     assert (la, lb) == (1, 3)
     assert bool(torch.isfinite(ya).all())
-    assert_close(ya.float().cpu().numpy(), ref, f"tokens-as-M folded M={M} {K}->{N}")
-    assert_close(yb.float().cpu().numpy(), ref, f"tokens-as-M gathered M={M} {K}->{N}")
+    assert_close(ya.float().cpu().numpy(), ref, f"contracted M={M} {K}->{N}")
+    assert_close(yb.float().cpu().numpy(), ref, f"gathered M={M} {K}->{N}")
 
 
 def test_forward_into_a_caller_buffer():

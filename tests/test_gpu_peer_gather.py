@@ -85,7 +85,7 @@ def test_two_ranks_exchange_through_peer_memory(tmp_path, per_cta):
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_second_device_in_the_same_process(oracle_mod):
     """Function attributes, SM counts and occupancy caches are kept per device: a process that has run every kernel
-    family on cuda:0 runs them on cuda:1 as well (streaming, generic decode, tokens-as-M, prefill)."""
+    family on cuda:0 runs them on cuda:1 as well (streaming, generic decode, small token block, prefill)."""
     for dev in ("cuda:0", "cuda:1"):
         for (M, K, N) in [(1, 4096, 512), (20, 1024, 208), (40, 1024, 4352), (300, 1024, 520)]:
             layer = wl.make_layer(K, N, 0.01, seed=500 + M)
