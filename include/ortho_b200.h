@@ -66,9 +66,11 @@ ORTHO_B200_API int ortho_b200_last_cuda_error(void);
  * Has no counterpart in the reference (its kernels read CSR directly,
  * src/dual_gemm.cu:106-130); it takes the place of the per-call orth_layer_t the binding builds
  * on its stack (torch_bind/bindings.cpp:19-36).  The plan owns only its own device copies
- * (packed {col16|f16 value} entries in row order, row pointers, the list of long rows and their dense FP16 copy);
- * it never retains the caller's pointers.  Creation allocates device memory, launches the
- * re-layout kernels on `stream` and synchronises that stream once.  A plan is immutable after
+ * (packed {col16|f16 value} entries in row order, row pointers, for rows in column order the entries once more as lists
+ * for the tensor-core kernels, the list of long rows and their dense FP16 copy);
+ * it never retains the caller's pointers.  Creation allocates device memory from the device's memory pool, launches the
+ * re-layout kernels on `stream` and synchronises that stream; under a capture of `stream` it is refused (ERR_CUDA).
+ * plan_destroy waits for the device, as kernels may still read the plan.  A plan is immutable after
  * creation and may be shared by concurrent forwards.  nnz == 0 yields a valid empty plan.
  * ------------------------------------------------------------------------------------------- */
 typedef struct ortho_b200_plan ortho_b200_plan;
@@ -83,7 +85,7 @@ ORTHO_B200_API int64_t ortho_b200_plan_nnz(const ortho_b200_plan *plan);
 ORTHO_B200_API int64_t ortho_b200_plan_max_row_nnz(const ortho_b200_plan *plan);
 /* 1 when every row lists its columns in strictly ascending order inside [0, in_features) (what
  * tools/sieve.py:131-136 produces), 0 otherwise, -1 for an invalid handle.  Only such plans let the tensor-core
- * kernels fold the sparse entries into their weight tiles; any other plan takes the gather path. */
+ * kernels contract the sparse entries or fold them into their weight tiles; any other plan takes the gather path. */
 ORTHO_B200_API int ortho_b200_plan_rows_ordered(const ortho_b200_plan *plan);
 
 /* Decodes the re-laid-out entries back to (row, col, f16 value) triplets, entry i of the plan
@@ -201,12 +203,13 @@ ORTHO_B200_API int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers,
  * Limits and rules:
  *  - the one case it refuses (ORTHO_B200_ERR_SCRATCH_LIMIT, nothing launched) is a prefill-regime call
  *    with an active ortho term whose transposed activations, K * roundup(M, 256) * 2 bytes, exceed
- *    ORTHO_B200_STATIC_SCRATCH_BYTES; alpha <= 0, nnz == 0 and the streaming regime need no scratch;
+ *    ORTHO_B200_STATIC_SCRATCH_BYTES; calls with alpha <= 0 or nnz == 0 are never refused (from 3 tokens on they may use
+ *    the array all the same);
  *  - the first call on a device looks up the array's device address (cudaGetSymbolAddress, no
  *    allocation); make that first call before any stream capture begins;
  *  - all calls share the one array and it keeps the previous call's contents.  Nothing in it needs
- *    clearing by the caller (each call writes what it later reads; the flag words of split tiles are
- *    cleared on the stream by the call itself), but calls that overlap on the GPU -- other streams,
+ *    clearing by the caller (each call writes what it later reads; the flag words of split tiles hold a
+ *    value of their own per launch and are cleared by the CTA that has read them), but calls that overlap on the GPU -- other streams,
  *    other host threads -- race on it: issue them one after another on one stream;
  *  - no cudaMalloc / cudaFree or any other allocating call is made.
  * Arguments as for ortho_b200_forward, without plan and workspace.
@@ -236,9 +239,9 @@ ORTHO_B200_API int ortho_b200_forward_static_scratch(const void *q_weight, const
  *               y_offset_bytes into EVERY rank's buffer.  When the stream reaches the end of the call
  *               all ranks' slices of this forward are present in the local buffer.  Every rank must
  *               issue the same sequence of forward_gather calls on a comm; a buffer region may be
- *               reused by the second next call at the earliest (alternate two regions).  For M <= 16
- *               and for M > 24 the peer stores and the flag exchange are part of the compute kernel
- *               itself; the shapes in between add one copy kernel.  A rank whose peers do not arrive within the timeout
+ *               reused by the second next call at the earliest (alternate two regions).  The peer stores
+ *               and the flag exchange are part of the streaming and the tensor-core kernels; calls that run the
+ *               mma.sync kernel (no workspace, raw CSR on small layers, K % 256 != 0) add one copy kernel.  A rank whose peers do not arrive within the timeout
  *               (default 2 s) records a kernel status (ortho_b200_query_kernel_status) and returns.
  *               n_offset must be a multiple of 8; y_offset_bytes a multiple of 16.
  * ------------------------------------------------------------------------------------------- */

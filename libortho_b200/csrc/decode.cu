@@ -346,8 +346,8 @@ bool mid_range(int64_t M, int64_t N, int64_t K)
     return mid_range_of(t, M, N, K, false) || mid_range_of(t, M, N, K, true);
 }
 // `base`: the sparse term is inactive; `lists`: it is, or it comes as a plan's window lists.  From 17 tokens on the mma.sync kernel below is
-// behind on every layer then (32 tokens: 1024->1024 14.6 / 6.2, 4096->4096 32.4 / 12.1, 8192->2048 26.8 / 14.6,
-// 4096->22016 88 / 21).  Without lists mid.cu needs two more launches for the sparse term, which small layers do not earn
+// behind on every layer then (32 tokens: 1024->1024 14.6 / 6.2, 4096->4096 32.4 / 12.2, 8192->2048 26.8 / 13.4,
+// 4096->22016 88 / 22).  Without lists mid.cu needs two more launches for the sparse term, which small layers do not earn
 // back (raw CSR, 0.5 %, 32 tokens: 1024->1024 14.8 / 23.8, 4096->1024 16.0 / 28.8, 4096->4096 34.8 / 30.4), and up to 16
 // tokens no layer does.  Without the workspace the rule between the mma.sync kernel and the prefill tile stands.
 Route route_of(int64_t M, int64_t N, int64_t K, const void *workspace, int64_t workspace_bytes, bool base, bool lists)

@@ -9,11 +9,14 @@
 // 64 tokens: HBM delivers the 4 KB of a k block (128 rows x 64 k) in about 180 cycles per SM.  Converted weights go
 // from registers straight to tensor memory; the form before this one (tokens as the M operand, weights converted into
 // a shared-memory B tile of 256 rows) spent 512 cycles of tensor pipe per 256 x 64 weights whatever the token count
-// and 4 bytes of shared-memory traffic per weight.  What bounds it now is the conversion: 12 instructions per eight
-// weights, two thirds of them on the integer pipe (about 130 of those 180 cycles), plus the sparse entries.
-// One B200, us, base-only / 0.3 % entries, against the form before: 8192->10240 at 32 tokens 17 / 22 (45 / 54), at 128
-// 24 / 33 (83 / 90); 8192->57344 at 32 tokens 59 / 84 (169 / 185), at 128 99 / 170 (198 / 224); 28672->8192 at 100 tokens
-// 48 / 72 (129 / 135).
+// and 4 bytes of shared-memory traffic per weight.
+// What bounds it, by the counters of one launch on 8192->10240 at 32 tokens with 0.3 % entries (base-only): no pipe is full.  Of
+// the active cycles the integer pipe is busy in 43 % (44), the issue slots in 48 % (47), the tensor pipe in 23 % (15), HBM in
+// 19 % (24) of the whole time; a unit's MMAs take some 450 cycles to go through (8 from shared memory at 40, 8 at 16), 40 % of the active cycles.
+// The rest is ramp, the waits between the warp roles and the collecting of cut tiles.
+// One B200, us, base-only / 0.3 % entries, weights rotating over more than L2, against the form before: 8192->10240 at 32
+// tokens 18 / 23 (45 / 54), at 128 23 / 33 (83 / 90); 8192->57344 at 32 tokens 59-72 / 84-103 (169 / 185), at 128 89 / 152 (198 /
+// 224); 28672->8192 at 32 tokens 41-45 / 58-62, at 100 48-52 / 76-84 (129 / 135).  (Ranges: from box to box.)
 // Replaces, for this token range, the reference's one-thread-per-output kernel (src/dual_gemm.cu:176-225) and its WMMA
 // variant (src/dual_gemm_tensor_core.cu:215-337).
 //

@@ -24,7 +24,9 @@
 // converters have about twice the time that the base needs.
 // One B200, us, base-only / fused, against the 128 x 256 tile of prefill.cu: 8192->8192 at 2048 tokens, 0.3 % 190 / 204
 // (265 / 295; 1440 / 1350 TFLOP/s now), at 8192 tokens 783 / 900 (963 / 1174); 4096->4096 at 2048, 1 % 54 / 70 (76 / 108);
-// 8192->8192 with Zipf rows at 512 tokens 54 / 64 (71 / 81).  Bounds: the power cap (cuBLAS sustains 1380) and, fused, the converters.
+// 8192->8192 with Zipf rows at 512 tokens 53 / 65 (71 / 81).  Bounds: the power cap (cuBLAS sustains 1400) at many tokens; in the
+// fused form the converters (4096->4096 at 2048 tokens, 1 %, by counters: tensor pipe busy in 55 % of the active cycles, issue
+// slots in 56 %, integer pipe in 47 %, DRAM 5 %).
 //
 // Work split: as many whole waves of tiles as there are, tile after tile with the token tiles of a row tile next to each
 // other (a wave then reads few weight rows, and the activations from L2); the tiles left over are cut along K into
