@@ -278,3 +278,25 @@ def test_a_plan_is_refused_under_capture_and_the_capture_goes_on():
         y.add_(1)
     graph.replay()
     assert bool((y == 1).all())
+
+
+@pytest.mark.parametrize("M", [129, 176, 177, 352, 353, 705])
+def test_rows_that_cannot_be_folded_at_the_edges_of_token_tiles(M):
+    """More than 128 tokens: rows with a zero or tiny scale are gathered by the epilogue, chunk by chunk of a token tile."""
+    K, N = 1184, 300
+    layer = wl.make_layer(K, N, 0.02, seed=12, device=DEV)
+    layer.base_scales[::37], layer.base_scales[5::61] = 0.0, 6e-8
+    plan = _C_ops.Plan(layer.row_ptr, layer.col, layer.vals, K, N)
+    x = wl.make_input(M, K, seed=M, device=DEV)
+    y = multi(layer, x, 0.75, plan)
+    q = layer.base_weight.to(torch.int16)
+    w = torch.stack((q & 15, q >> 4), dim=2).view(N, K)
+    w = (w - ((w & 8) << 1)).double() * layer.base_scales.double().unsqueeze(1)
+    rows = torch.repeat_interleave(torch.arange(N, device=DEV), (layer.row_ptr[1:] - layer.row_ptr[:-1]).long())
+    w[rows, layer.col.long()] += 0.75 * layer.vals.double()
+    ref = x.double() @ w.T
+    err = y.double() - ref
+    assert float(err.norm() / ref.norm()) <= REL_FRO_TOL and float(err.abs().max()) <= MAX_ABS_TOL
+    alone = ref[:, ::37]                                    # the gathered rows by themselves: one FP16 rounding, 2^-11 of a value
+    assert float((y[:, ::37].double() - alone).norm() / alone.norm()) <= 4.9e-4
+    assert _lib.lib().ortho_b200_query_kernel_status() == 0
