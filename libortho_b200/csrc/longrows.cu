@@ -44,14 +44,26 @@ constexpr size_t kSmemBytes = 1024 + (size_t)ST * (A_BYTES + B_BYTES) + sizeof(S
 struct Params {
     float *part;                        // [nsplit][n_pad][Mp]
     int n_long, n_pad, Mp, kblocks, nsplit;
-    // the rows' entries and the activations, for sums that an infinite activation made NaN (zeros of HD)
-    const uint32_t *entries; const int32_t *row_ptr, *hrow; const __half *x; int M, K;
     int *status;
 };
 }  // namespace lg
 
+// The rows' entries and the activations: the zeros of HD times an infinite activation are NaN, and such a sum is taken again
+// from the entries, by whoever has the whole of it first (this kernel when K is not cut; in the GEMM's exposed epilogue the
+// check of cut sums cost 1 of 80 us at 512 tokens).
+struct RowEntries { const uint32_t *entries; const int32_t *row_ptr, *hrow; const __half *x; int M, K; };
+// (out of line: these kernels are short and start with a cold instruction cache)
+__device__ __noinline__ float long_sum_again(const uint32_t *entries, const int32_t *row_ptr, int n, const __half *xr, int K)
+{
+    return entries_sum(entries, row_ptr[n], row_ptr[n + 1], 0, K, xr);
+}
+__device__ __forceinline__ float long_sum_again(const RowEntries &re, int h, int m)
+{
+    return long_sum_again(re.entries, re.row_ptr, re.hrow[h], re.x + (size_t)m * re.K, re.K);
+}
+
 __global__ void __launch_bounds__(lg::NWARPS * 32, 1)
-long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap xmap, const lg::Params p)
+long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap xmap, const lg::Params p, const RowEntries re)
 {
     using namespace lg;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -129,19 +141,17 @@ long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             tmem_ld_32x32b_x32(taddr + (uint32_t)(c * 32), r);
             tmem_ld_wait();
             if (row < p.n_long && !dead) {
-                bool nan = false;
+                if (p.nsplit == 1) {
+                    uint32_t bad = 0;
 #pragma unroll
-                for (int j = 0; j < 32; j++) nan = nan || __uint_as_float(r[j]) != __uint_as_float(r[j]);
-                uint32_t bad = 0;
+                    for (int j = 0; j < 32; j++) bad |= __uint_as_float(r[j]) != __uint_as_float(r[j]) ? 1u << j : 0u;
+                    for (; bad; bad &= bad - 1) {
+                        const int j = __ffs(bad) - 1, m = tok0 + c * 32 + j;
+                        if (m >= re.M) break;
+                        const uint32_t t = __float_as_uint(long_sum_again(re, row, m));
 #pragma unroll
-                for (int j = 0; j < 32 && nan; j++) bad |= __uint_as_float(r[j]) != __uint_as_float(r[j]) ? 1u << j : 0u;
-                for (; bad; bad &= bad - 1) {
-                    const int j = __ffs(bad) - 1, m = tok0 + c * 32 + j;
-                    if (m >= p.M) break;
-                    const int n = p.hrow[row];
-                    const uint32_t t = __float_as_uint(entries_sum(p.entries, p.row_ptr[n], p.row_ptr[n + 1], kb0 * KB, kb1 * KB, p.x + (size_t)m * p.K));
-#pragma unroll
-                    for (int i = 0; i < 32; i++) r[i] = i == j ? t : r[i];
+                        for (int i = 0; i < 32; i++) r[i] = i == j ? t : r[i];
+                    }
                 }
                 float4 *d4 = reinterpret_cast<float4 *>(dst + c * 32);
 #pragma unroll
@@ -159,7 +169,7 @@ long_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
 
 // part[0] += part[1] + ... + part[nsplit - 1], for the n_long rows (Mp floats each); four tokens per thread
 __global__ void __launch_bounds__(256)
-long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, int nsplit)
+long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, int nsplit, int Mp, const RowEntries re)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -175,17 +185,29 @@ long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, in
         for (int j = 0; j < 4; j++)
             if (s + j < nsplit) { acc.x += t[j].x; acc.y += t[j].y; acc.z += t[j].z; acc.w += t[j].w; }
     }
+    if (acc.x != acc.x || acc.y != acc.y || acc.z != acc.z || acc.w != acc.w) {
+        const int h = (int)(4 * i / Mp), m = (int)(4 * i - (long long)h * Mp);
+        float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll 1
+        for (int j = 0; j < 4 && m + j < re.M; j++) {
+            const float cur = j == 0 ? v[0] : j == 1 ? v[1] : j == 2 ? v[2] : v[3];
+            const float now = cur != cur ? long_sum_again(re, h, m + j) : cur;
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[e] = e == j ? now : v[e];
+        }
+        acc = make_float4(v[0], v[1], v[2], v[3]);
+    }
     part[i] = acc;
 }
 
 // y[m, hrow[h]] = FP16(rest[h, m] + alpha * (part[0] + ... + part[nsplit - 1])[h, m]); one token per thread
 __global__ void __launch_bounds__(256)
 long_finish_kernel(const float *__restrict__ part, long long stride, int nsplit, const float *__restrict__ rest,
-                   const int32_t *__restrict__ hrow, int h0, float alpha, __half *__restrict__ y, long long ldy, int M, int Mp)
+                   int h0, float alpha, __half *__restrict__ y, long long ldy, int Mp, const RowEntries re)
 {
     const int m = blockIdx.x * 256 + threadIdx.x, h = h0 + blockIdx.y;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (m >= M) return;
+    if (m >= re.M) return;
     const float *src = part + (size_t)h * Mp + m;
     const float base = __ldcg(rest + (size_t)h * Mp + m);
     float acc = 0.f;
@@ -196,7 +218,8 @@ long_finish_kernel(const float *__restrict__ part, long long stride, int nsplit,
 #pragma unroll
         for (int j = 0; j < 8; j++) acc += t[j];
     }
-    y[(size_t)m * (size_t)ldy + hrow[h]] = __float2half_rn(fmaf(alpha, acc, base));
+    if (acc != acc) acc = long_sum_again(re, h, m);
+    y[(size_t)m * (size_t)ldy + re.hrow[h]] = __float2half_rn(fmaf(alpha, acc, base));
 }
 
 // ---- plan side: the dense copy of the long rows --------------------------------------------------------------
@@ -276,6 +299,10 @@ float *long_rows_rest(const FwdArgs &a, int Mp, void *ws)
 {
     return reinterpret_cast<float *>(ws) + (size_t)long_rows_splits(a.plan, a.M) * (size_t)a.plan->n_pad * (size_t)Mp;
 }
+static RowEntries row_entries(const FwdArgs &a)
+{
+    return RowEntries{a.plan->entries, a.plan->row_ptr, a.plan->hrow, a.x, (int)a.M, (int)a.K};
+}
 int launch_long_finish(const FwdArgs &a, int Mp, void *ws)
 {
     const Plan *pl = a.plan;
@@ -291,7 +318,7 @@ int launch_long_finish(const FwdArgs &a, int Mp, void *ws)
     for (int64_t h0 = 0; h0 < pl->n_long; h0 += kRows) {
         cfg.gridDim = dim3((unsigned)ceil_div(a.M, 256), (unsigned)(pl->n_long - h0 < kRows ? pl->n_long - h0 : kRows));
         OB_CUDA(cudaLaunchKernelEx(&cfg, long_finish_kernel, part, (long long)pl->n_pad * Mp, long_rows_splits(pl, a.M), rest,
-                                   (const int32_t *)pl->hrow, (int)h0, a.alpha, a.y, (long long)a.pitch_y(), (int)a.M, Mp));
+                                   (int)h0, a.alpha, a.y, (long long)a.pitch_y(), Mp, row_entries(a)));
         count_launch();
     }
     return ORTHO_B200_OK;
@@ -304,7 +331,6 @@ int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
     p.part = reinterpret_cast<float *>(ws);
     p.n_long = (int)pl->n_long; p.n_pad = (int)pl->n_pad; p.Mp = Mp;
     p.kblocks = (int)ceil_div(a.K, KB); p.nsplit = long_rows_splits(pl, a.M);
-    p.entries = pl->entries; p.row_ptr = pl->row_ptr; p.hrow = pl->hrow; p.x = a.x; p.M = (int)a.M; p.K = (int)a.K;
     p.status = kernel_status_word();
     if (!p.status) return ORTHO_B200_ERR_CUDA;
     CUtensorMap amap, xmap;
@@ -322,7 +348,7 @@ int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
         attr_set[dev] = true;
     }
     dim3 g1((unsigned)p.nsplit, (unsigned)(Mp / TT), (unsigned)(pl->n_pad / TR));
-    long_gemm_kernel<<<g1, NWARPS * 32, kSmemBytes, a.stream>>>(amap, xmap, p);
+    long_gemm_kernel<<<g1, NWARPS * 32, kSmemBytes, a.stream>>>(amap, xmap, p, row_entries(a));
     count_launch();
     OB_CUDA(cudaGetLastError());
     if (!sums_out) return ORTHO_B200_OK;
@@ -335,7 +361,7 @@ int launch_long_rows(const FwdArgs &a, int Mp, void *ws, const float **sums_out)
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
-        OB_CUDA(cudaLaunchKernelEx(&cfg, long_sum_kernel, reinterpret_cast<float4 *>(p.part), quads, stride, p.nsplit));
+        OB_CUDA(cudaLaunchKernelEx(&cfg, long_sum_kernel, reinterpret_cast<float4 *>(p.part), quads, stride, p.nsplit, Mp, row_entries(a)));
         count_launch();
     }
     *sums_out = p.part;
