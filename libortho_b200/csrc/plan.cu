@@ -316,9 +316,10 @@ extern "C" int ortho_b200_plan_destroy(ortho_b200_plan *plan)
         int dev = pl->device;
         cudaGetDevice(&dev);
         if (dev != pl->device) cudaSetDevice(pl->device);
-        cudaDeviceSynchronize();
-        for (void *b : blocks)
-            if (b) cudaFree(b);
+        if (cudaDeviceSynchronize() == cudaSuccess) {    // (refused while a stream is captured: the blocks then stay allocated)
+            for (void *b : blocks)
+                if (b) cudaFree(b);
+        }
         if (dev != pl->device) cudaSetDevice(dev);
     }
     pl->magic = 0;

@@ -300,3 +300,22 @@ def test_rows_that_cannot_be_folded_at_the_edges_of_token_tiles(M):
     alone = ref[:, ::37]                                    # the gathered rows by themselves: one FP16 rounding, 2^-11 of a value
     assert float((y[:, ::37].double() - alone).norm() / alone.norm()) <= 4.9e-4
     assert _lib.lib().ortho_b200_query_kernel_status() == 0
+
+
+def test_a_plan_may_go_while_its_forward_runs():
+    """Destroying a plan waits for the kernels that read it: plans made at once in the same memory do not disturb them."""
+    K, N, M = 8192, 4096, 64
+    layer = wl.make_layer(K, N, 0.01, seed=2, device=DEV)
+    other = wl.Layer(K, N, layer.base_weight, layer.base_scales, layer.row_ptr, layer.col, -layer.vals, 1.0)
+    x = wl.make_input(M, K, seed=2, device=DEV)
+    args = (layer.base_weight, layer.base_scales, layer.vals, layer.col, layer.row_ptr)
+    ref = multi(layer, x, 1.0, _C_ops.Plan(layer.row_ptr, layer.col, layer.vals, K, N))
+    ys = [torch.empty(M, N, dtype=torch.float16, device=DEV) for _ in range(8)]
+    ws = torch.empty(_C_ops.workspace_bytes(M, K, N), dtype=torch.uint8, device=DEV)
+    for y in ys:
+        plan = _C_ops.Plan(layer.row_ptr, layer.col, layer.vals, K, N)
+        for _ in range(20):
+            _C_ops.forward(*args, x, y, 1.0, plan=plan, workspace=ws)
+        plan.close()
+        _C_ops.Plan(other.row_ptr, other.col, other.vals, K, N)
+    assert all(torch.equal(y, ref) for y in ys)
