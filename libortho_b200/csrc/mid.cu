@@ -14,9 +14,10 @@
 // the active cycles the integer pipe is busy in 43 % (44), the issue slots in 48 % (47), the tensor pipe in 23 % (15), HBM in
 // 19 % (24) of the whole time; a unit's MMAs take some 450 cycles to go through (8 from shared memory at 40, 8 at 16), 40 % of the active cycles.
 // The rest is ramp, the waits between the warp roles and the collecting of cut tiles.
-// One B200, us, base-only / 0.3 % entries, weights rotating over more than L2, against the form before: 8192->10240 at 32
-// tokens 18 / 23 (45 / 54), at 128 23 / 33 (83 / 90); 8192->57344 at 32 tokens 59-72 / 84-103 (169 / 185), at 128 89 / 152 (198 /
-// 224); 28672->8192 at 32 tokens 41-45 / 58-62, at 100 48-52 / 76-84 (129 / 135).  (Ranges: from box to box.)
+// One B200, us, base-only / with entries, weights rotating over more than L2; in brackets with one issuer, weights loaded behind
+// the predecessor and the cut tiles collected 16 tokens and one piece at a time: 8192->10240 at 32 tokens 16.0 / 20.1 (17.9 / 22.6),
+// 4096->22016 at 16 14.4 / 19.0 (16.1 / 21.1), 4096->4096 at 24 8.4 / 10.2 (10.6 / 12.4), 8192->57344 at 32 58 / 78 (59 / 88);
+// at 100 tokens on 28672->8192 47 / 73 as before: there the tensor pipe is full with both contractions (960 cycles a unit).
 // Replaces, for this token range, the reference's one-thread-per-output kernel (src/dual_gemm.cu:176-225) and its WMMA
 // variant (src/dual_gemm_tensor_core.cu:215-337).
 //
@@ -73,7 +74,8 @@ constexpr int kSmemData = 224 * 1024;   // packed-weight slots, token stages, sp
 // back after `groups` units, so stages must be at least that many (the unit before it in its stage is one whose
 // MMAs its own last store had waited for), and weight slots at least stages + groups: having stored unit i, a group knows
 // that units up to i - stages have been multiplied, hence loaded, and waits for unit i + groups next, whose slot's previous
-// load (i + groups - slots) must be one of those -- loads may complete out of order.
+// load (i + groups - slots) must be one of those -- loads may complete out of order.  With two issuers it knows so only of
+// every other unit: numbers of slots, stages and groups are even then, and i + groups - slots is one of those.
 constexpr int MAX_GROUPS = 4;
 constexpr int CONV_WARPS = 4 * MAX_GROUPS;
 constexpr int EPI_WARP0 = 2 + CONV_WARPS;
@@ -81,8 +83,11 @@ constexpr int EPI_WARPS = 4;
 constexpr int XPROD_WARP = EPI_WARP0 + EPI_WARPS;   // token tiles have a producer of their own: the packed weights run ahead of them
 constexpr int SCAT_WARP0 = XPROD_WARP + 1;
 constexpr int SCAT_WARPS = 8;           // two sets of four that take the units in turn; a warp of a set has 32 rows of the tile
-template <bool SPARSE> constexpr int kWarps = SCAT_WARP0 + (SPARSE ? SCAT_WARPS : 0);
+template <bool SPARSE> constexpr int kIssue2Warp = SCAT_WARP0 + (SPARSE ? SCAT_WARPS : 0);    // the second MMA issuer
+template <bool SPARSE> constexpr int kWarps = kIssue2Warp<SPARSE> + 1;
 constexpr int TMEM_COLS = 512;
+constexpr int kTwoIssuers = 64, kTwoIssuersSparse = 32;      // two issuers up to this many columns of D (with more, shared
+                                        // memory does not hold four stages with their sparse tiles)
 
 struct Params {
     const __half *scales; const float *bias; __half *y;
@@ -93,11 +98,12 @@ struct Params {
     int nt;                     // token columns of an MMA: M rounded up to 16
     int nt32;                   // nt rounded up to 32: columns kept for D, and for E behind it
     int nacc, acc_cols;         // accumulators (2 where tensor memory allows) and the columns of one
+    int issuers;                // threads that issue MMAs, in turns; each has accumulators of its own
     int xtile;                  // bytes of a token tile (nt x 128); a stage holds two
     int nst;                    // stages: a unit's converted weights and tokens
     int wst;                    // packed-weight slots
     int groups;                 // converter groups at work
-    int sets;                   // scatter sets at work: 2 with four stages, else 1
+    int sets;                   // scatter sets at work: 2 with two or four stages, else 1
     float *slots;               // slots[cta][nt][128]: partial sums handed to another CTA ...
     unsigned long long *flags;  // ... and flags[cta] = tag once they are there (see launch_mid)
     unsigned long long tag;
@@ -160,24 +166,20 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         for (int s = 0; s < WST_MAX; s++) { mbar_init(&sm->w_full[s], 1); mbar_init(&sm->w_empty[s], 4); }
         // full: the four warps of a converter group, the token producer with its bytes, a set of scatter warps
         for (int s = 0; s < ST_MAX; s++) { mbar_init(&sm->full[s], 5 + (SPARSE ? 4 : 0)); mbar_init(&sm->empty[s], 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(&sm->d_full[s], 1); mbar_init(&sm->d_empty[s], EPI_WARPS); }
-        mbar_init(&sm->all_done, 1);
+        for (int s = 0; s < 2; s++) { mbar_init(&sm->d_full[s], (uint32_t)p.issuers); mbar_init(&sm->d_empty[s], EPI_WARPS); }
+        mbar_init(&sm->all_done, (uint32_t)p.issuers);
         fence_mbar_init();
         prefetch_tensormap(&xmap);
         prefetch_tensormap(&wmap);
     }
     if (warp == 1) { tmem_alloc(&sm->tmem_base, TMEM_COLS); tmem_relinquish(); }
-    if constexpr (SPARSE) {
-        for (int i = threadIdx.x; i < p.nst * S_BYTES / 16; i += kWarps<SPARSE> * 32) reinterpret_cast<uint4 *>(ss)[i] = make_uint4(0, 0, 0, 0);
-        fence_proxy_async();
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sm->tmem_base;
-    // The kernel is a programmatic dependent of whatever precedes it on the stream: up to here it ran beside that
-    // kernel's tail.  Behind the long rows' pre-pass (an ordinary launch, so all earlier work is done) only the epilogue waits.
-    if (!SPARSE || p.n_long == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The kernel is a programmatic dependent of whatever precedes it on the stream and runs beside that kernel's tail: weights
+    // and window lists, constants of the layer, are loaded and converted at once; the token producer and the epilogue wait.
+    // Behind the long rows' pre-pass (an ordinary launch, so all earlier work is done) only the epilogue does.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool dead = false;
     auto wait = [&](uint64_t *bar, uint32_t parity) {
@@ -201,6 +203,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
     } else if (warp == XPROD_WARP) {
         // ================= TMA producer: token tiles =================
         if (elect_one()) {
+            if (!SPARSE || p.n_long == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
             int st = 0; uint32_t ph = 0;
             int kp = kp_begin;
             for (int i = 0; i < units; i++) {
@@ -213,34 +216,44 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (++kp == p.kpairs) kp = 0;
             }
         }
-    } else if (warp == 1) {
-        // ================= MMA issuer =================
+    } else if (warp == 1 || warp == kIssue2Warp<SPARSE>) {
+        // ================= MMA issuers =================
         // A ready mbarrier takes this one thread 60-100 cycles to see and a commit 35-60: with a wait each for tokens
         // and weights and two commits per 64 k the loop took 490 cycles per k block whatever the token count.  Hence one
-        // barrier for both operands, two k blocks per turn, and the next stage's barrier is looked at before this
-        // stage's MMAs are issued.
-        if (elect_one()) {
+        // barrier for all operands, two k blocks per turn, a look at the next stage's barrier before this stage's MMAs are issued,
+        // and up to 64 tokens two threads that take the units in turn, each into accumulators of its own: by clocks at 32 tokens
+        // one thread took 500-530 cycles a unit base-only (750 with the sparse term) while converted units piled up, for MMAs
+        // of 130 (450).  (One thread for D and one for E: slower than one for both.  A loop that the whole warp runs, with an
+        // elected lane for the MMAs alone: 8192->57344 at 32 tokens 65 us against 60.)  The number of stages is even then, so that a
+        // stage is always the same thread's and its waits stay within one phase.
+        const int who = warp == 1 ? 0 : 1;
+        if (who < p.issuers && elect_one()) {
+            const int step = p.issuers;
             const uint32_t idesc = umma_idesc_f16(TN, p.nt);
             const uint64_t bdesc0 = umma_desc_sw128(smem_u32(xs)), sdesc0 = umma_desc_sw128(smem_u32(ss));
-            int st = 0; uint32_t ph = 0;
+            const uint32_t a_tmem = tmem + (uint32_t)(p.nacc * p.acc_cols);
+            int st = who; uint32_t ph = 0;
             bool ready = false;
             Pieces pc(t_begin, kp_begin, units, p.kpairs);
+            int skip = st;                               // units to pass over: every other one belongs to the other thread
             for (int it = 0; pc.next(); it++) {
                 const int a = p.nacc == 2 ? it & 1 : 0, use = p.nacc == 2 ? it >> 1 : it;
                 wait(&sm->d_empty[a], (uint32_t)((use & 1) ^ 1));            // the epilogue has drained this accumulator
-                const uint32_t d_tmem = tmem + (uint32_t)(a * p.acc_cols);
+                const uint32_t d_tmem = tmem + (uint32_t)(a * p.acc_cols + who * (SPARSE ? 2 : 1) * p.nt32);
                 uint32_t acc = 0u;
-                for (int kp = pc.kp0; kp < pc.kp1; kp++) {
+                int kp = pc.kp0 + skip;
+                for (; kp < pc.kp1; kp += step) {
                     if (!ready) wait(&sm->full[st], ph);
                     tc_fence_after();
-                    const uint32_t at = tmem + (uint32_t)(p.nacc * p.acc_cols + st * A_STAGE_COLS);
+                    const uint32_t at = a_tmem + (uint32_t)(st * A_STAGE_COLS);
                     const uint64_t sd = sdesc0 + (uint64_t)((st * S_BYTES) >> 4);
                     const uint64_t bd = bdesc0 + (uint64_t)((2 * st * p.xtile) >> 4);
                     const uint64_t bd2 = bd + (uint64_t)(p.xtile >> 4);
-                    const uint32_t acc_e = acc;
                     uint64_t *done = &sm->empty[st];
-                    if (++st == p.nst) { st = 0; ph ^= 1u; }
-                    ready = mbar_try_wait(&sm->full[st], ph);
+                    st += step;
+                    if (st >= p.nst) { st -= p.nst; ph ^= 1u; }
+                    ready = mbar_test_wait(&sm->full[st], ph);
+                    const uint32_t acc_e = acc;
 #pragma unroll
                     for (int kk = 0; kk < KB / 16; kk++) {
                         umma_f16_ts(d_tmem, at + (uint32_t)(kk * 8), bd + (uint64_t)(2 * kk), idesc, acc);
@@ -259,11 +272,12 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     }
                     umma_commit(done);
                 }
+                skip = kp - pc.kp1;
                 umma_commit(&sm->d_full[a]);
             }
             umma_commit(&sm->all_done);
         }
-    } else if (SPARSE && warp >= SCAT_WARP0) {
+    } else if (SPARSE && warp >= SCAT_WARP0 && warp < SCAT_WARP0 + SCAT_WARPS) {
         // ================= scatter: the unit's sparse entries -> zeroed FP16 tile in shared memory (A operand) =================
         // A warp's loop is a chain of dependent instructions, so the entries come with their place in the tile worked out,
         // are fetched a turn ahead (their extent a turn before that), and stay in registers until they are taken out again.
@@ -293,8 +307,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         fetch_extent();
         fetch_entries();
         fetch_extent();
-        // what the last three visits put into their stages; a stage comes round after nst / sets visits, 2 or 3
-        const bool three = p.nst == 3;
+        // what the last three visits put into their stages; a stage comes round after nst / sets visits, 1 to 3
+        const int back = p.nst / sets;
         uint32_t o1n = 0, o1a = 0, o1b = 0, o2n = 0, o2a = 0, o2b = 0, o3n = 0, o3a = 0, o3b = 0;
         const uint32_t tiles = smem_u32(ss) + (uint32_t)(q * (32 * 128));
         auto put = [&](uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)v) : "memory"); };
@@ -304,7 +318,13 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             fetch_entries();
             fetch_extent();
             const uint32_t tile = tiles + (uint32_t)(st * S_BYTES);
-            const uint32_t on = three ? o3n : o2n, oa = three ? o3a : o2a, ob2 = three ? o3b : o2b;
+            auto clear_all = [&]() {
+                for (int j = lane; j < 2 * 32 * 8; j += 32)
+                    *reinterpret_cast<uint4 *>(ss + (size_t)st * S_BYTES + q * (32 * 128) + (j >> 8) * kWinTile + (j & 255) * 16) = make_uint4(0, 0, 0, 0);
+            };
+            if (i < p.nst) clear_all();                  // the stage's first use
+            const uint32_t on = back == 1 ? o1n : back == 2 ? o2n : o3n, oa = back == 1 ? o1a : back == 2 ? o2a : o3a;
+            const uint32_t ob2 = back == 1 ? o1b : back == 2 ? o2b : o3b;
             wait(&sm->empty[st], ph ^ 1u);
             __syncwarp();
             if ((uint32_t)lane < on) put(tile + (oa & 0xFFFFu), 0u);
@@ -312,8 +332,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (on <= 64u) {
                     if ((uint32_t)lane + 32u < on) put(tile + (ob2 & 0xFFFFu), 0u);
                 } else {
-                    for (int j = lane; j < 2 * 32 * 8; j += 32)
-                        *reinterpret_cast<uint4 *>(ss + (size_t)st * S_BYTES + q * (32 * 128) + (j >> 8) * kWinTile + (j & 255) * 16) = make_uint4(0, 0, 0, 0);
+                    clear_all();
                 }
             }
             __syncwarp();
@@ -377,10 +396,10 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         }
         }
         // The CTA's last piece is finished by the converters too, which have nothing left to do: five sets of four warps take
-        // every fifth chunk of 16 tokens.  (Collecting the other pieces of a cut tile is a chain of loads from L2 per chunk: by
+        // every fifth chunk of 8 tokens.  (Collecting the other pieces of a cut tile is a chain of loads from L2 per chunk: by
         // the four epilogue warps alone it took 15-25 us at the end of a forward.)
         // ================= epilogue: TMEM -> (+ partials) -> scale, sparse term, bias -> FP16 -> global =================
-        if (SPARSE && p.n_long > 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         const int q = warp & 3;                          // TMEM lane quarter of this warp
         const int et = (warp - EPI_WARP0) * 32 + lane;   // 0..127 among the epilogue threads, negative in the converters
         Pieces pc(t_begin, kp_begin, units, p.kpairs);
@@ -399,6 +418,10 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 const int tile_end = pos + p.kpairs;
                 while (c_last + 1 < G && p.share * (c_last + 1) + min(c_last + 1, p.extra) < tile_end) c_last++;
             }
+            // with two issuers: the accumulators that have been written (a piece of one unit fills one thread's)
+            const uint32_t own_cols = (uint32_t)((SPARSE ? 2 : 1) * p.nt32);
+            const bool both = p.issuers == 2 && pc.kp1 - pc.kp0 > 1;
+            const uint32_t d_off = p.issuers == 2 && !both && ((pos - r_begin) & 1) ? own_cols : 0u;
             pos += pc.kp1 - pc.kp0;
             float sc = 0.f, bs = 0.f;
             int li = -1;                                 // this row's index among the plan's long rows
@@ -420,63 +443,77 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * p.acc_cols);
-            // scale * D + bias (+ alpha * E) of 16 tokens.  The zeros of the scattered tile times an infinite activation make E
+            // scale * D + bias (+ alpha * E) of 8 tokens.  The zeros of the scattered tile times an infinite activation make E
             // NaN for every row: such a sum is taken again from the row's entries in this piece.
-            auto load16 = [&](int c, float (&v)[16]) {
-                uint32_t r[16];
-                tmem_ld_32x32b_x16(taddr + (uint32_t)c, r);
-                if constexpr (SPARSE) {
-                    uint32_t e[16];
-                    tmem_ld_32x32b_x16(taddr + (uint32_t)(p.nt32 + c), e);
+            auto columns8 = [&](uint32_t col, float (&v)[8]) {            // 8 accumulator columns, of both issuers
+                uint32_t r[8];
+                tmem_ld_32x32b_x8(taddr + d_off + col, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = __uint_as_float(r[j]);
+                if (both) {
+                    tmem_ld_32x32b_x8(taddr + own_cols + col, r);
                     tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] += __uint_as_float(r[j]);
+                }
+            };
+            auto load8 = [&](int c, float (&v)[8]) {
+                columns8((uint32_t)c, v);
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = fmaf(v[j], sc, bs);
+                if constexpr (SPARSE) {
+                    float e[8];
+                    columns8((uint32_t)(p.nt32 + c), e);
                     bool nan = false;
 #pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        v[j] = fmaf(p.alpha, __uint_as_float(e[j]), fmaf(__uint_as_float(r[j]), sc, bs));
+                    for (int j = 0; j < 8; j++) {
+                        v[j] = fmaf(p.alpha, e[j], v[j]);
                         nan = nan || v[j] != v[j];
                     }
                     if (__any_sync(0xffffffffu, nan)) {
                         uint32_t bad = 0;
 #pragma unroll
-                        for (int j = 0; j < 16; j++) bad |= v[j] != v[j] ? 1u << j : 0u;
+                        for (int j = 0; j < 8; j++) bad |= v[j] != v[j] ? 1u << j : 0u;
                         int e0 = 0, e1 = 0;
                         if (n_ok) { e0 = p.row_ptr[n]; e1 = p.row_ptr[n + 1]; } else bad = 0;
                         if (p.n_long > 0 && e1 - e0 > p.heavy) e1 = e0;               // a long row is not listed
 #pragma unroll 1
-                        for (int j = 0; j < 16 && c + j < p.M; j++) {
-                            uint32_t d;
+                        for (int j = 0; j < 8 && c + j < p.M; j++) {
+                            uint32_t d, d2 = 0;
                             __syncwarp();
-                            tmem_ld_32x32b_x1(taddr + (uint32_t)(c + j), d);
+                            tmem_ld_32x32b_x1(taddr + d_off + (uint32_t)(c + j), d);
+                            if (both) tmem_ld_32x32b_x1(taddr + own_cols + (uint32_t)(c + j), d2);
                             tmem_ld_wait();
                             if (!((bad >> j) & 1u)) continue;
                             const float es = entries_sum(p.entries, e0, e1, pc.kp0 * KP, pc.kp1 * KP, p.x + (size_t)(c + j) * p.K);
-                            const float t = fmaf(p.alpha, es, fmaf(__uint_as_float(d), sc, bs));
+                            const float base = both ? __uint_as_float(d) + __uint_as_float(d2) : __uint_as_float(d);
+                            const float t = fmaf(p.alpha, es, fmaf(base, sc, bs));
 #pragma unroll
-                            for (int i = 0; i < 16; i++) v[i] = i == j ? t : v[i];
+                            for (int i = 0; i < 8; i++) v[i] = i == j ? t : v[i];
                         }
                         __syncwarp();
                     }
-                } else {
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = fmaf(__uint_as_float(r[j]), sc, bs);
                 }
             };
             if (!owner) {
-                // the first piece of a share that starts inside a tile: its FP32 sums to this CTA's slot, then the flag
-                float *dst = p.slots + ((size_t)cta * p.nt + set * 16) * TN + q * 32 + lane;
-                for (int c = set * 16; c < p.nt; c += sets * 16, dst += sets * 16 * TN) {
-                    float v[16];
-                    load16(c, v);
+                // the first piece of a share that starts inside a tile: its FP32 sums to this CTA's slot, then the flag.  One fence
+                // behind the barrier covers every thread's stores.
+                float *dst = p.slots + ((size_t)cta * p.nt + set * 8) * TN + q * 32 + lane;
+                for (int c = set * 8; c < p.nt; c += sets * 8, dst += sets * 8 * TN) {
+                    float v[8];
+                    load8(c, v);
 #pragma unroll
-                    for (int j = 0; j < 16; j++) dst[j * TN] = v[j];
+                    for (int j = 0; j < 8; j++) dst[j * TN] = v[j];
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (!last && lane == 0) mbar_arrive(&sm->d_empty[a]);
-                __threadfence();
                 sync_sets();
-                if (et == 0) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p.flags + cta), "l"(p.tag) : "memory");
+                if (et == 0) {
+                    __threadfence();
+                    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p.flags + cta), "l"(p.tag) : "memory");
+                }
                 continue;
             }
             if (c_last > cta) {                          // bounded wait for the contributors' flags, one lane per contributor
@@ -493,24 +530,33 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (!ok) { dead = true; atomicExch(p.status, 1); }
                 dead = __any_sync(0xffffffffu, dead);
             }
-            const float *part = p.slots + ((size_t)(cta + 1) * p.nt + set * 16) * TN + q * 32 + lane;
+            const float *part = p.slots + ((size_t)(cta + 1) * p.nt + set * 8) * TN + q * 32 + lane;
             const size_t part_cta = (size_t)p.nt * TN;
-            for (int c = set * 16; c < p.nt; c += sets * 16, part += sets * 16 * TN) {
+            constexpr int FLY = SPARSE ? 1 : 3;          // pieces in flight (registers)
+            for (int c = set * 8; c < p.nt; c += sets * 8, part += sets * 8 * TN) {
                 __syncwarp();
-                float v[16];
-                load16(c, v);
+                float v[8];
+                load8(c, v);
                 const float *src = part;
-                for (int cc = cta + 1; cc <= c_last; cc++, src += part_cta) {        // the other pieces of the tile, in CTA order
-                    float t[16];
+                for (int cc = cta + 1; cc <= c_last; cc += FLY, src += FLY * part_cta) {     // the other pieces of the tile, in CTA order
+                    float t[FLY][8];
 #pragma unroll
-                    for (int j = 0; j < 16; j++) t[j] = __ldcg(src + j * TN);
+                    for (int i = 0; i < FLY; i++)
+                        if (cc + i <= c_last) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] += t[j];
+                            for (int j = 0; j < 8; j++) t[i][j] = __ldcg(src + i * part_cta + j * TN);
+                        }
+#pragma unroll
+                    for (int i = 0; i < FLY; i++)
+                        if (cc + i <= c_last) {
+#pragma unroll
+                            for (int j = 0; j < 8; j++) v[j] += t[i][j];
+                        }
                 }
                 if (longs && li >= 0) {                           // a long row's sums from the pre-pass
                     const float4 *o4 = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.ol_mp + c);
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
+                    for (int j = 0; j < 2; j++) {
                         const float4 t = __ldcg(o4 + j);
                         v[4 * j] = fmaf(p.alpha, t.x, v[4 * j]); v[4 * j + 1] = fmaf(p.alpha, t.y, v[4 * j + 1]);
                         v[4 * j + 2] = fmaf(p.alpha, t.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(p.alpha, t.w, v[4 * j + 3]);
@@ -519,7 +565,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (plain) {
                     __half *yp = p.y + (size_t)c * (size_t)p.ldy + n;
 #pragma unroll
-                    for (int j = 0; j < 16; j++) {
+                    for (int j = 0; j < 8; j++) {
                         if (n_ok && c + j < p.M) *yp = __float2half_rn(v[j]);
                         yp += p.ldy;
                     }
@@ -527,7 +573,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 }
                 if (!n_ok) continue;
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
+                for (int j = 0; j < 8; j++) {
                     const int m = c + j;
                     if (m >= p.M) break;
                     float o = v[j];
@@ -716,21 +762,26 @@ int launch_mid(const FwdArgs &a)
     // tiles of the same number, the rest for packed weights (8 KB slots): 64 KB or more in flight per SM where the
     // kernel runs near HBM's pace, less only for many tokens, where the MMAs are the bound.
     p.nt32 = (p.nt + 31) / 32 * 32;
-    p.acc_cols = sparse ? 2 * p.nt32 : p.nt32;
+    p.issuers = p.nt32 <= (sparse ? kTwoIssuersSparse : kTwoIssuers) ? 2 : 1;
+    p.acc_cols = (sparse ? 2 : 1) * p.issuers * p.nt32;
     p.nacc = 2 * p.acc_cols + 4 * A_STAGE_COLS <= TMEM_COLS ? 2 : 1;
     p.nst = (TMEM_COLS - p.nacc * p.acc_cols) / A_STAGE_COLS;
     if (p.nst > (sparse ? ST_SPARSE_MAX : ST_MAX)) p.nst = sparse ? ST_SPARSE_MAX : ST_MAX;
-    const int nst_max = p.nst;
-    for (p.groups = MAX_GROUPS;; p.groups--) {               // most groups first, then most stages, by the rule above MAX_GROUPS
-        for (p.nst = nst_max; p.nst >= p.groups; p.nst--) {
+    // The issuers, and the two sets of scatter warps, take turns: even numbers of stages then, and of weight slots.  Above 64 tokens,
+    // where shared memory holds three stages, three and one set are better than two and two (28672->8192 at 100: 73 us against 77).
+    const int down = p.issuers == 2 || (sparse && p.nt <= 64) ? 2 : 1;
+    const int nst_max = p.nst - p.nst % down;
+    for (p.groups = MAX_GROUPS;; p.groups -= down) {         // most groups first, then most stages, by the rule above MAX_GROUPS
+        for (p.nst = nst_max; p.nst >= p.groups; p.nst -= down) {
             p.wst = (kSmemData - p.nst * (2 * p.xtile + (sparse ? S_BYTES : 0))) / W_BYTES;
             if (p.wst > WST_MAX) p.wst = WST_MAX;
+            p.wst -= p.wst % down;
             if (p.wst >= p.nst + p.groups) break;
         }
         if (p.nst >= p.groups) break;
-        if (p.groups == 2) return ORTHO_B200_ERR_SHAPE;      // not reached for up to 128 tokens
+        if (p.groups <= 2) return ORTHO_B200_ERR_SHAPE;      // not reached for up to 128 tokens
     }
-    p.sets = p.nst == 4 ? 2 : 1;
+    p.sets = p.nst % 2 == 0 ? 2 : 1;
     CUtensorMap xmap, wmap;
     if (!make_tensor_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, (uint64_t)a.M, (uint64_t)a.K,
                             (uint64_t)a.K * 2, (uint32_t)p.nt, KB, CU_TENSOR_MAP_SWIZZLE_128B))

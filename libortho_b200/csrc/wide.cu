@@ -280,7 +280,7 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
                     const uint32_t acc0 = acc;
                     uint64_t *done = &sm->empty[st];
                     if (++st == p.nst) { st = 0; ph ^= 1u; }
-                    ready = mbar_try_wait(&sm->full[st], ph);
+                    ready = mbar_test_wait(&sm->full[st], ph);
 #pragma unroll
                     for (int kk = 0; kk < KB / 16; kk++) {
                         umma_f16_ts(d_tmem, at + (uint32_t)(kk * 8), bd + (uint64_t)(2 * kk), idesc, acc);
