@@ -290,6 +290,14 @@ ORTHO_B200_API int ortho_b200_csr_count(const float *w_ortho, int64_t N, int64_t
 ORTHO_B200_API int ortho_b200_csr_fill(const float *w_ortho, int64_t N, int64_t K, const int32_t *row_ptr,
                        int32_t *col_out, void *val_f16_out, void *stream);
 
+/* The same in two calls that read W_ortho once: csr_count_marks also notes the non-zero positions in `marks`
+ * (ortho_b200_csr_marks_bytes(N, K) bytes, 16-byte aligned, a bit per weight), from which csr_fill_marks fetches the entries.
+ * W_ortho must not change in between.  Faster than csr_fill up to a few entries in a hundred weights. */
+ORTHO_B200_API int64_t ortho_b200_csr_marks_bytes(int64_t N, int64_t K);
+ORTHO_B200_API int ortho_b200_csr_count_marks(const float *w_ortho, int64_t N, int64_t K, int32_t *row_ptr_out, void *marks, void *stream);
+ORTHO_B200_API int ortho_b200_csr_fill_marks(const float *w_ortho, int64_t N, int64_t K, const int32_t *row_ptr, const void *marks,
+                       int32_t *col_out, void *val_f16_out, void *stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Device-side Hessian sieve: splits FP32 weights W [N, K] that are already on the GPU into the
  * INT4-representable base and the sparse residual, bit-identical to hessian_sieve / quantize_int4 of
@@ -301,9 +309,12 @@ ORTHO_B200_API int ortho_b200_csr_fill(const float *w_ortho, int64_t N, int64_t 
  * select (12 + 10 + 10 bits) without storing the scores; while it runs an output buffer holds some of their keys.
  * An output may be W itself.  h_inv_diag is the FP32 [K] diagonal.  scratch:
  * ortho_b200_sieve_scratch_bytes(N) bytes, 256-byte aligned.  K a multiple of 4, pointers 16-byte aligned.
+ * With ortho_b200_sieve_onepass_scratch_bytes(N, K) bytes of scratch the top-k rule takes one pass over W and a short list
+ * where it can (outputs apart from each other and from the inputs, keep_top_k up to 4 % of N * K); the results are the same bits.
  * The outputs feed ortho_b200_pack_base / ortho_b200_csr_count / ortho_b200_csr_fill.
  * ------------------------------------------------------------------------------------------- */
 ORTHO_B200_API int64_t ortho_b200_sieve_scratch_bytes(int64_t N);
+ORTHO_B200_API int64_t ortho_b200_sieve_onepass_scratch_bytes(int64_t N, int64_t K);
 ORTHO_B200_API int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t N, int64_t K,
                        float curvature_thresh, int64_t keep_top_k,
                        float *w_base_out, float *w_ortho_out,

@@ -366,15 +366,20 @@ def pack_ortho_csr(w_ortho: torch.Tensor):
     N, K = w.shape
     dev = w.device
     row_ptr = torch.empty(N + 1, dtype=torch.int32, device=dev)
+    marks = torch.empty(N * ((K + 127) // 128), 4, dtype=torch.int32, device=dev)
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
-        _lib.check(_lib.lib().ortho_b200_csr_count(w.data_ptr(), N, K, row_ptr.data_ptr(), stream), "ortho_b200_csr_count")
+        _lib.check(_lib.lib().ortho_b200_csr_count_marks(w.data_ptr(), N, K, row_ptr.data_ptr(), marks.data_ptr(), stream),
+                   "ortho_b200_csr_count_marks")
         nnz = int(row_ptr[N].item())
         col = torch.empty(nnz, dtype=torch.int32, device=dev)
         val = torch.empty(nnz, dtype=torch.float16, device=dev)
-        if nnz:
+        if nnz > N * K // 16:                  # many entries: whole rows at a time
             _lib.check(_lib.lib().ortho_b200_csr_fill(w.data_ptr(), N, K, row_ptr.data_ptr(), col.data_ptr(), val.data_ptr(),
                                                      stream), "ortho_b200_csr_fill")
+        elif nnz:
+            _lib.check(_lib.lib().ortho_b200_csr_fill_marks(w.data_ptr(), N, K, row_ptr.data_ptr(), marks.data_ptr(), col.data_ptr(),
+                                                           val.data_ptr(), stream), "ortho_b200_csr_fill_marks")
     return row_ptr, col, val
 
 
@@ -392,7 +397,7 @@ def hessian_sieve(weight: torch.Tensor, h_inv_diag: torch.Tensor, curvature_thre
     if h.dim() != 1 or h.numel() != K:
         raise ValueError("h_inv_diag must hold one entry per input feature")
     wb, wo = torch.empty_like(w), torch.empty_like(w)
-    need = int(_lib.lib().ortho_b200_sieve_scratch_bytes(N))
+    need = int(_lib.lib().ortho_b200_sieve_onepass_scratch_bytes(N, K) if keep_top_k > 0 else _lib.lib().ortho_b200_sieve_scratch_bytes(N))
     scratch = torch.empty(need, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
         st = _lib.lib().ortho_b200_sieve(w.data_ptr(), h.data_ptr(), N, K, float(curvature_thresh), int(keep_top_k),

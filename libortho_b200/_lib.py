@@ -86,6 +86,14 @@ def _declare(l):
     l.ortho_b200_csr_count.argtypes = [vp, i64, i64, vp, vp]
     l.ortho_b200_csr_fill.restype = c.c_int
     l.ortho_b200_csr_fill.argtypes = [vp, i64, i64, vp, vp, vp, vp]
+    l.ortho_b200_csr_marks_bytes.restype = i64
+    l.ortho_b200_csr_marks_bytes.argtypes = [i64, i64]
+    l.ortho_b200_csr_count_marks.restype = c.c_int
+    l.ortho_b200_csr_count_marks.argtypes = [vp, i64, i64, vp, vp, vp]
+    l.ortho_b200_csr_fill_marks.restype = c.c_int
+    l.ortho_b200_csr_fill_marks.argtypes = [vp, i64, i64, vp, vp, vp, vp, vp]
+    l.ortho_b200_sieve_onepass_scratch_bytes.restype = i64
+    l.ortho_b200_sieve_onepass_scratch_bytes.argtypes = [i64, i64]
     l.ortho_b200_sieve_scratch_bytes.restype = i64
     l.ortho_b200_sieve_scratch_bytes.argtypes = [i64]
     l.ortho_b200_sieve.restype = c.c_int
@@ -122,7 +130,8 @@ EXPORTS = [
     "ortho_b200_comm_set_timeout_ms", "ortho_b200_comm_destroy", "ortho_b200_forward_gather",
     "ortho_b200_comm_set_deferred", "ortho_b200_comm_wait",
     "ortho_b200_pack_base", "ortho_b200_csr_count", "ortho_b200_csr_fill",
-    "ortho_b200_sieve_scratch_bytes", "ortho_b200_sieve",
+    "ortho_b200_csr_marks_bytes", "ortho_b200_csr_count_marks", "ortho_b200_csr_fill_marks",
+    "ortho_b200_sieve_scratch_bytes", "ortho_b200_sieve_onepass_scratch_bytes", "ortho_b200_sieve",
     "ortho_b200_forward_multi", "ortho_b200_multi_workspace_bytes",
 ]
 
