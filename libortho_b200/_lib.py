@@ -150,6 +150,25 @@ def lib():
     return _lib
 
 
+_fast = None
+
+
+def fast():
+    """The native host path (``csrc/fastcall.cpp``), pointed at the loaded library."""
+    global _fast
+    if _fast is None:
+        l = lib()
+        try:
+            from . import _fastcall as f
+        except ImportError as e:
+            raise ImportError("libortho_b200/_fastcall.so is missing or does not fit the installed torch. "
+                              "Build it with `python -m libortho_b200.build`.") from e
+        f.set_library(ctypes.cast(l.ortho_b200_forward_multi, ctypes.c_void_p).value,
+                      ctypes.cast(l.ortho_b200_multi_workspace_bytes, ctypes.c_void_p).value)
+        _fast = f
+    return _fast
+
+
 def check(status: int, where: str) -> None:
     if status != OK:
         raise OrthoB200Error(status, where)

@@ -21,6 +21,9 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--use_fast_math",
     "-cudart", "static",
 ]
+# the forward's host path as a CPython extension (csrc/fastcall.cpp), compiled against the installed torch
+FAST_SOURCE = os.path.join(CSRC, "fastcall.cpp")
+FAST_PATH = os.path.join(HERE, "_fastcall.so")
 
 
 def _nvcc() -> str:
@@ -36,6 +39,25 @@ def _deps() -> list:
     return out
 
 
+def build_fast(force: bool = False) -> str:
+    deps = [FAST_SOURCE, os.path.join(INCLUDE, "ortho_b200.h")]
+    if not force and os.path.exists(FAST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(FAST_PATH) for d in deps):
+        return FAST_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include"), INCLUDE]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in inc], FAST_SOURCE, "-o", FAST_PATH, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ltorch"]
+    out = subprocess.run(cmd, capture_output=True, text=True)
+    if out.returncode != 0:
+        raise RuntimeError("g++ failed on fastcall.cpp:\n" + out.stdout + out.stderr)
+    return FAST_PATH
+
+
 def needs_build() -> bool:
     if not os.path.exists(LIB_PATH):
         return True
@@ -44,6 +66,7 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_fast(force)
     if not force and not needs_build():
         return LIB_PATH
     objdir = os.path.join(HERE, "build")

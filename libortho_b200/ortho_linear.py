@@ -16,6 +16,7 @@ Differences, all deliberate:
 """
 from __future__ import annotations
 
+import ctypes
 import threading
 import weakref
 from typing import Optional, Tuple
@@ -101,7 +102,7 @@ _NO_SCRATCH = _SharedWorkspace(True)
 class _Bound:
     """Everything about one (module, token count, stream) forward that does not change from call to call: the C
     argument record with all buffer pointers, the plan, the workspace.  Built (and validated) once."""
-    __slots__ = ("descs", "ws", "ws_gen", "ws_ptr", "ws_bytes", "key", "fused_bias")
+    __slots__ = ("descs", "ws", "ws_gen", "ws_ptr", "ws_bytes", "key", "fused_bias", "fast")
 
 
 class OrthoLinear(nn.Module):
@@ -117,9 +118,9 @@ class OrthoLinear(nn.Module):
         self.q_bits = q_bits
         self.register_buffer("base_weight", torch.zeros(out_features, in_features // 2, dtype=torch.uint8, device=device))
         self.register_buffer("base_scales", torch.zeros(out_features, dtype=torch.float16, device=device))
-        self.register_buffer("ortho_values", torch.tensor([], dtype=torch.float16, device=device))
-        self.register_buffer("ortho_col_indices", torch.tensor([], dtype=torch.int32, device=device))
-        self.register_buffer("ortho_row_ptr", torch.tensor([], dtype=torch.int32, device=device))
+        self.register_buffer("ortho_values", torch.empty(0, dtype=torch.float16, device=device))
+        self.register_buffer("ortho_col_indices", torch.empty(0, dtype=torch.int32, device=device))
+        self.register_buffer("ortho_row_ptr", torch.empty(0, dtype=torch.int32, device=device))
         self.alpha = 1.0
         if bias:
             self.register_parameter("bias", nn.Parameter(torch.zeros(out_features, dtype=dtype or torch.float32, device=device)))
@@ -267,6 +268,11 @@ class OrthoLinear(nn.Module):
         d.N, d.ldy, d.reserved = N, 0, 0
         b.descs = descs
         b.key = (self.alpha > 0, self._versions())
+        # what the native path compares and launches; not for a bias that torch has to add
+        b.fast = None
+        if self.bias is None or b.fused_bias:
+            b.fast = _lib.fast().record(ctypes.addressof(descs), self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
+                                        b.ws_bytes, dev.index)
         if b.ws.shared:
             if len(self._bound) > 32:
                 self._bound.clear()
@@ -278,6 +284,13 @@ class OrthoLinear(nn.Module):
         """`out` (optional, not in the reference's signature): a contiguous FP16 CUDA tensor of `M * out_features`
         elements that receives the result instead of a fresh allocation, e.g. a slice of a serving loop's
         staging buffer."""
+        if out is None and x.is_cuda:
+            # a call like one before: FP16, this device, no scratch under capture.  None: the code below does it
+            y = _lib.fast().module(x, self._buffers, self._parameters, self._bound, self.alpha, self.in_features, self.out_features)
+            if y is not None:
+                if type(y) is int:
+                    _lib.check(y, "ortho_b200_forward_multi")
+                return y
         if not x.is_cuda:
             raise RuntimeError("OrthoLinear (libortho_b200) runs on CUDA only; there is no CPU fallback")
         original_shape = x.shape
