@@ -188,6 +188,19 @@ ORTHO_B200_API int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers,
                        const void *x_f16, int64_t M, int64_t K,
                        void *workspace, int64_t workspace_bytes, void *stream);
 
+/* The forward of one layer with activations and outputs of another type (a model in BF16 or FP32): x_type and y_type are one of
+ * ORTHO_B200_TYPE_*, and the result has the bits of converting x to FP16, the ordinary forward and converting y.
+ * typed_scratch_bytes: -1 where the call's kernel does not take other types (convert around the ordinary forward), else the size of
+ * x_scratch (16-byte aligned; 0 = none needed) for the same layer, sizes and workspace; y_f16 of the record is not looked at.
+ * Weights and window lists may be read before the work that precedes the call on its stream has finished when that work allows it
+ * (programmatic dependent launch, as in every forward): they are constants of the layer. */
+#define ORTHO_B200_TYPE_F16 0
+#define ORTHO_B200_TYPE_BF16 1
+#define ORTHO_B200_TYPE_F32 2
+ORTHO_B200_API int64_t ortho_b200_typed_scratch_bytes(const ortho_b200_layer_desc *layer, int64_t M, int64_t K, void *workspace, int64_t workspace_bytes);
+ORTHO_B200_API int ortho_b200_forward_typed(const ortho_b200_layer_desc *layer, const void *x, int x_type, int y_type, int64_t M, int64_t K,
+                       void *x_scratch, void *workspace, int64_t workspace_bytes, void *stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Forward for callers that cannot allocate device memory.  It has no counterpart in the reference.
  *

@@ -72,6 +72,10 @@ def _declare(l):
     l.ortho_b200_forward_multi.argtypes = [c.POINTER(LayerDesc), c.c_int, vp, i64, i64, vp, i64, vp]
     l.ortho_b200_multi_workspace_bytes.restype = i64
     l.ortho_b200_multi_workspace_bytes.argtypes = [c.POINTER(LayerDesc), c.c_int, i64, i64]
+    l.ortho_b200_typed_scratch_bytes.restype = i64
+    l.ortho_b200_typed_scratch_bytes.argtypes = [c.POINTER(LayerDesc), i64, i64, vp, i64]
+    l.ortho_b200_forward_typed.restype = c.c_int
+    l.ortho_b200_forward_typed.argtypes = [c.POINTER(LayerDesc), vp, c.c_int, c.c_int, i64, i64, vp, vp, i64, vp]
     l.ortho_b200_forward_static_scratch.restype = c.c_int
     l.ortho_b200_forward_static_scratch.argtypes = [vp, vp, vp, i32p, i32p, i64, vp, vp, i64, i64, i64, c.c_float, vp]
     l.ortho_b200_set_decode_config.restype = c.c_int
@@ -132,7 +136,7 @@ EXPORTS = [
     "ortho_b200_pack_base", "ortho_b200_csr_count", "ortho_b200_csr_fill",
     "ortho_b200_csr_marks_bytes", "ortho_b200_csr_count_marks", "ortho_b200_csr_fill_marks",
     "ortho_b200_sieve_scratch_bytes", "ortho_b200_sieve_onepass_scratch_bytes", "ortho_b200_sieve",
-    "ortho_b200_forward_multi", "ortho_b200_multi_workspace_bytes",
+    "ortho_b200_forward_multi", "ortho_b200_multi_workspace_bytes", "ortho_b200_forward_typed", "ortho_b200_typed_scratch_bytes",
 ]
 
 
@@ -163,8 +167,8 @@ def fast():
         except ImportError as e:
             raise ImportError("libortho_b200/_fastcall.so is missing or does not fit the installed torch. "
                               "Build it with `python -m libortho_b200.build`.") from e
-        f.set_library(ctypes.cast(l.ortho_b200_forward_multi, ctypes.c_void_p).value,
-                      ctypes.cast(l.ortho_b200_multi_workspace_bytes, ctypes.c_void_p).value)
+        f.set_library(*(ctypes.cast(fn, ctypes.c_void_p).value for fn in
+                        (l.ortho_b200_forward_multi, l.ortho_b200_multi_workspace_bytes, l.ortho_b200_forward_typed)))
         _fast = f
     return _fast
 

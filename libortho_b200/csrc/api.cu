@@ -279,6 +279,62 @@ extern "C" int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers, int
     return ORTHO_B200_OK;
 }
 
+// Which calls take activations and outputs of another type: those whose kernel stores them itself.  The streaming kernel also reads
+// them itself; the tensor-core kernels load FP16 tiles by TMA, so the activations are converted ahead into the caller's scratch.
+static bool typed_route(const FwdArgs &a, Route route, bool &converts)
+{
+    converts = route != kRouteDecode;
+    if (a.pitch_y() != a.N) return false;
+    if (route == kRouteDecode) return stream_kernel_takes(a);
+    return route == kRouteMid ? !a.has_ortho || mid_has_lists(a) : wide_takes(a);
+}
+
+static int typed_args(FwdArgs &a, Route &route, bool &converts, const ortho_b200_layer_desc *d, const void *x, int64_t M, int64_t K,
+                      void *workspace, int64_t workspace_bytes, void *stream)
+{
+    if (!d) return ORTHO_B200_ERR_NULL;
+    if (M <= 0) return ORTHO_B200_ERR_SHAPE;
+    const int st = make_fwd_args(a, d->q_weight, d->q_scales_f16, d->ortho_values_f16, d->ortho_col_indices, d->ortho_row_ptr, d->nnz, x, d->y_f16,
+                                 M, K, d->N, d->alpha, d->plan, workspace, workspace_bytes, stream, d->ldy, d->bias_f32);
+    if (st != ORTHO_B200_OK) return st;
+    route = route_of(a);
+    return typed_route(a, route, converts) ? ORTHO_B200_OK : ORTHO_B200_ERR_SHAPE;
+}
+
+extern "C" int64_t ortho_b200_typed_scratch_bytes(const ortho_b200_layer_desc *layer, int64_t M, int64_t K, void *workspace, int64_t workspace_bytes)
+{
+    FwdArgs a;
+    Route route;
+    bool converts;
+    if (!layer) return -1;
+    ortho_b200_layer_desc d = *layer;
+    d.y_f16 = const_cast<void *>(d.q_weight);            // any aligned address: nothing is launched
+    if (typed_args(a, route, converts, &d, d.q_weight, M, K, workspace, workspace_bytes, nullptr) != ORTHO_B200_OK) return -1;
+    return converts ? M * K * 2 : 0;
+}
+
+extern "C" int ortho_b200_forward_typed(const ortho_b200_layer_desc *layer, const void *x, int x_type, int y_type, int64_t M, int64_t K,
+                                        void *x_scratch, void *workspace, int64_t workspace_bytes, void *stream)
+{
+    if (x_type < kTypeF16 || x_type > kTypeF32 || y_type < kTypeF16 || y_type > kTypeF32) return ORTHO_B200_ERR_SHAPE;
+    FwdArgs a;
+    Route route;
+    bool converts;
+    int st = typed_args(a, route, converts, layer, x, M, K, workspace, workspace_bytes, stream);
+    if (st != ORTHO_B200_OK) return st;
+    a.y_type = y_type;
+    if (!converts) {
+        a.x_type = x_type;
+    } else if (x_type != kTypeF16) {
+        if (!x_scratch) return ORTHO_B200_ERR_WORKSPACE;
+        if (((uintptr_t)x_scratch & 15u) != 0) return ORTHO_B200_ERR_ALIGN;
+        st = launch_convert_x(x, x_type, (__half *)x_scratch, M * K, a.stream);
+        if (st != ORTHO_B200_OK) return st;
+        a.x = (const __half *)x_scratch;
+    }
+    return launch_routed(a, route);
+}
+
 extern "C" int64_t ortho_b200_multi_workspace_bytes(const ortho_b200_layer_desc *layers, int n_layers, int64_t M, int64_t K)
 {
     int64_t need = 0;

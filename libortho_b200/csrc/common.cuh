@@ -1,6 +1,7 @@
 // Shared device/host helpers of the sm_100a OrthoLinear forward.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -248,6 +249,39 @@ __device__ __forceinline__ float quant_clamped(float w, float scale, float rscal
     return q != q ? q : fminf(fmaxf(q, -8.f), 7.f);
 }
 
+// ---- activations and outputs of another type than FP16 ------------------------------------------------------------------
+// The operator computes on FP16 activations and rounds its sums to FP16; other types are converted on the way in and out, with
+// the bits of x.to(float16) and y.to(type).
+enum { kTypeF16 = 0, kTypeBF16 = 1, kTypeF32 = 2 };
+__device__ __forceinline__ void store_typed(void *y, size_t at, float v, int type)
+{
+    const __half h = __float2half_rn(v);
+    if (type == kTypeF16) reinterpret_cast<__half *>(y)[at] = h;
+    else if (type == kTypeBF16) reinterpret_cast<__nv_bfloat16 *>(y)[at] = __float2bfloat16_rn(__half2float(h));
+    else reinterpret_cast<float *>(y)[at] = __half2float(h);
+}
+__device__ __forceinline__ uint32_t pack_half2(float a, float b)
+{
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// eight consecutive activations from element `at` (a multiple of 8) as FP16
+__device__ __forceinline__ uint4 load8_as_half(const void *x, size_t at, int type)
+{
+    if (type == kTypeF16) return *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(x) + at);
+    if (type == kTypeBF16) {                     // a BF16 is the upper half of an FP32
+        const uint4 v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(x) + at);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = pack_half2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u));
+        return make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    const float4 *p = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(x) + at);
+    const float4 a = p[0], b = p[1];
+    return make_uint4(pack_half2(a.x, a.y), pack_half2(a.z, a.w), pack_half2(b.x, b.y), pack_half2(b.z, b.w));
+}
+
 // streaming 128-bit load of read-once weight bytes: bypass L1 allocation
 __device__ __forceinline__ uint4 ldg_stream(const void *p) {
     uint4 v;
@@ -273,6 +307,7 @@ struct FwdArgs {
     int64_t ldy = 0;
     const struct GatherView *gv = nullptr;
     bool *gather_fused = nullptr;
+    int x_type = 0, y_type = 0;           // kTypeF16 ..: what x and y point to (typed_route says which calls take others)
     int64_t pitch_y() const { return ldy ? ldy : N; }
 };
 int launch_decode(const FwdArgs &a);
@@ -310,5 +345,9 @@ Route route_of(const FwdArgs &a);
 bool group_streams(const FwdArgs *a, const Route *route, int n);   // decode.cu
 int launch_routed(const FwdArgs &a, Route route);                   // api.cu
 int launch_mid(const FwdArgs &a);                                  // mid.cu
+bool mid_has_lists(const FwdArgs &a);                              // mid.cu: the sparse term comes from the plan's lists
+bool wide_takes(const FwdArgs &a);                                 // prefill.cu: the call runs the kernel of wide.cu
+bool stream_kernel_takes(const FwdArgs &a);                        // decode.cu
+int launch_convert_x(const void *x, int type, __half *out, int64_t n, cudaStream_t stream);       // transpose.cu
 int64_t mid_workspace_bytes(int64_t M, int64_t K, int64_t N);
 }  // namespace ob

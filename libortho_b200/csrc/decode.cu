@@ -534,6 +534,8 @@ bool stream_kernel_selected(int64_t M, int64_t K)
     return M <= t.prefill_above && stream_selected(t, M, K);
 }
 
+bool stream_kernel_takes(const FwdArgs &a) { return stream_selected(tuning_snapshot(), a.M, a.K); }
+
 int launch_decode_multi(const FwdArgs *layers, int nl)
 {
     const Tuning t = tuning_snapshot();

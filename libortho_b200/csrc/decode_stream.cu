@@ -38,7 +38,7 @@ constexpr int kWarps = 8;
 // sequence is the concatenation of the layers' 16-row tiles, layer l owning tiles [tile0, next tile0).
 constexpr int kMaxLayers = 4;
 struct StreamLayer {
-    const __half *scales; __half *y; const float *bias;   // bias: optional FP32 [N], added before the FP16 rounding
+    const __half *scales; void *y; const float *bias;   // bias: optional FP32 [N], added before the FP16 rounding
     OrthoView ov; int has_ortho; float alpha;
     int N;         // output rows of this layer
     int ldy;       // elements between token rows of y
@@ -49,7 +49,8 @@ struct StreamParams {
     StreamLayer L[kMaxLayers];
     int nl;        // layers in this launch
     int any_ortho; // some layer has an active sparse term
-    const __half *x;
+    const void *x;
+    int x_type, y_type;   // kTypeF16 ..
     int M, K;
     int nboxes;    // ceil(K / weights per box row)
     int ntiles;    // 16-row tiles of all layers together
@@ -64,6 +65,7 @@ struct StreamGather {
     GatherView gv; // the finalized values are stored into every rank's output buffer
 };
 struct StreamNoGather {};
+enum { kPlain = 0, kGather = 1, kTyped = 2 };   // what an instantiation stores (MODE)
 template <bool G> struct StreamGatherArg { using type = StreamNoGather; };
 template <> struct StreamGatherArg<true> { using type = StreamGather; };
 
@@ -78,7 +80,8 @@ __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.
 
 // MV = token slots kept per output row (M <= MV, power of two).  One CTA = 8 warps that split the
 // CTA's K range of a 16-row tile; a cluster of S CTAs splits K further.
-// GATHER: instantiation with a pitched output, peer stores and the flag exchange; the plain one
+// MODE kTyped: activations and output of another type than FP16, one layer (57 us against 56 on 8192->57344 at one token when
+// the plain form looked at the types).  kGather: instantiation with a pitched output, peer stores and the flag exchange; the plain one
 // (output pitch N, one GPU) carries none of it
 // NG = warp groups per CTA.  A group is the 8-warp unit described above, with its own rings, tile barrier
 // and reduction buffers; the groups of a CTA work on different tiles and share one activation slab, which
@@ -96,11 +99,12 @@ __device__ __forceinline__ int layer_of(const StreamParams &p, int tile)
     return l;
 }
 
-template <int MV, int KBX, bool GATHER, int NG, int NL>
+template <int MV, int KBX, int MODE, int NG, int NL>
 __global__ void __launch_bounds__(NG * kWarps * 32, NG == 2 ? 1 : 2)
 decode_stream_kernel(const __grid_constant__ StreamMaps maps, const StreamParams p,
-                     const typename StreamGatherArg<GATHER>::type gp)
+                     const typename StreamGatherArg<MODE == kGather>::type gp)
 {
+    constexpr bool GATHER = MODE == kGather, TYPED = MODE == kTyped;
     constexpr int kKbx = KBX;
     constexpr int kBoxBytes = 16 * KBX * 128;
     constexpr int kBoxK = 256 * KBX;
@@ -219,7 +223,7 @@ decode_stream_kernel(const __grid_constant__ StreamMaps maps, const StreamParams
             const int r = idx / chunks_per_row, q = idx - r * chunks_per_row;
             const int k = k_lo + q * 8;
             uint4 v = make_uint4(0, 0, 0, 0);
-            if (k < K) v = *reinterpret_cast<const uint4 *>(p.x + (size_t)r * K + k);
+            if (k < K) v = load8_as_half(p.x, (size_t)r * K + k, TYPED ? p.x_type : kTypeF16);
             uint4 o;
             o.x = prmt_b32(v.x, v.z, 0x5410);
             o.y = prmt_b32(v.x, v.z, 0x7632);
@@ -295,7 +299,7 @@ decode_stream_kernel(const __grid_constant__ StreamMaps maps, const StreamParams
                 if (Ly.has_ortho) v = fmaf(Ly.alpha, o, v);
                 v += bias_prev;                                  // 0 when the layer has no bias
                 if constexpr (!GATHER) {
-                    Ly.y[(size_t)m * Ly.ldy + n] = __float2half_rn(v);
+                    store_typed(Ly.y, (size_t)m * Ly.ldy + n, v, TYPED ? p.y_type : kTypeF16);
                 } else {
                     const __half hv = __float2half_rn(v);
                     const size_t at = (size_t)m * gp.ldy + n;
@@ -458,9 +462,10 @@ static size_t stream_smem_bytes(int MV, int kbx, int64_t M, int boxes_per_cta, i
 }
 
 // layers[0..nl): layers that share x, M, K and the stream (nl == 1 for the ordinary forward)
-template <int MV, int KBX, bool GATHER, int NG, int NL>
+template <int MV, int KBX, int MODE, int NG, int NL>
 static int launch_stream_mv(const FwdArgs *layers, int nl, const StreamMaps &maps, int S, int stages, int red_bufs)
 {
+    constexpr bool GATHER = MODE == kGather;
     constexpr int kBoxK = 256 * KBX;
     const FwdArgs &a = layers[0];
     StreamParams p;
@@ -475,7 +480,7 @@ static int launch_stream_mv(const FwdArgs *layers, int nl, const StreamMaps &map
         tiles += (int)ceil_div(f.N, 16);
         p.any_ortho |= f.has_ortho;
     }
-    p.x = a.x;
+    p.x = a.x; p.x_type = a.x_type; p.y_type = a.y_type;
     p.M = (int)a.M; p.K = (int)a.K;
     p.nboxes = (int)ceil_div(a.K, kBoxK);
     p.ntiles = tiles;
@@ -499,7 +504,7 @@ static int launch_stream_mv(const FwdArgs *layers, int nl, const StreamMaps &map
     }
     const size_t smem = stream_smem_bytes(MV, KBX, a.M, boxes_per_cta, stages, NG, red_bufs);
     if (smem > 227 * 1024) return ORTHO_B200_ERR_SHAPE;
-    auto kern = decode_stream_kernel<MV, KBX, GATHER, NG, NL>;
+    auto kern = decode_stream_kernel<MV, KBX, MODE, NG, NL>;
     static bool attr_set[kMaxDevices] = {};       // the attribute is per device
     const int dev = current_device_index();
     if (dev < 0) return ORTHO_B200_ERR_CUDA;
@@ -602,11 +607,13 @@ int launch_decode_stream_multi(const FwdArgs *layers, int nl, int cfg_s, int cfg
             return ORTHO_B200_ERR_CUDA;
     // the GATHER instantiation serves the peer gather and, for one layer, any output whose pitch is not N
     const bool gather = nl == 1 && (a.gv || a.pitch_y() != a.N);
-    if (nl > 1 && a.gv) return ORTHO_B200_ERR_SHAPE;
+    const bool typed = a.x_type != kTypeF16 || a.y_type != kTypeF16;
+    if ((nl > 1 && a.gv) || (typed && (nl > 1 || gather))) return ORTHO_B200_ERR_SHAPE;
 #define OB_STREAM(MV_, KBX_, NG_) \
-    (nl > 1 ? launch_stream_mv<MV_, KBX_, false, NG_, kMaxLayers>(layers, nl, maps, S, stages, red_bufs) \
-     : gather ? launch_stream_mv<MV_, KBX_, true, NG_, 1>(layers, nl, maps, S, stages, red_bufs) \
-              : launch_stream_mv<MV_, KBX_, false, NG_, 1>(layers, nl, maps, S, stages, red_bufs))
+    (nl > 1 ? launch_stream_mv<MV_, KBX_, kPlain, NG_, kMaxLayers>(layers, nl, maps, S, stages, red_bufs) \
+     : gather ? launch_stream_mv<MV_, KBX_, kGather, NG_, 1>(layers, nl, maps, S, stages, red_bufs) \
+     : typed ? launch_stream_mv<MV_, KBX_, kTyped, NG_, 1>(layers, nl, maps, S, stages, red_bufs) \
+             : launch_stream_mv<MV_, KBX_, kPlain, NG_, 1>(layers, nl, maps, S, stages, red_bufs))
     switch (MV) {
         case 1: return ng == 2 ? OB_STREAM(1, 2, 2) : OB_STREAM(1, 2, 1);
         case 2: return ng == 2 ? OB_STREAM(2, 2, 2) : OB_STREAM(2, 2, 1);

@@ -19,7 +19,9 @@ namespace {
 
 using multi_fn = int (*)(const ortho_b200_layer_desc *, int, const void *, int64_t, int64_t, void *, int64_t, void *);
 using multi_ws_fn = int64_t (*)(const ortho_b200_layer_desc *, int, int64_t, int64_t);
+using typed_fn = int (*)(const ortho_b200_layer_desc *, const void *, int, int, int64_t, int64_t, void *, void *, int64_t, void *);
 multi_fn forward_multi = nullptr;
+typed_fn forward_typed = nullptr;
 multi_ws_fn multi_workspace = nullptr;
 
 struct Ptr { const void *data; int64_t version; };
@@ -33,6 +35,8 @@ struct Record {
     int64_t ws_gen;
     PyObject *ws;                                // the scratch's owner: `gen` and `tensor`
     int device;
+    int type;                                    // ORTHO_B200_TYPE_* of activations and output
+    void *x_scratch;                             // for activations of another type, where the kernel needs them as FP16
 };
 const char *kBuffers[5] = {"base_weight", "base_scales", "ortho_values", "ortho_col_indices", "ortho_row_ptr"};
 PyObject *s_buffers[5], *s_bias, *s_gen, *s_tensor, *s_handle, *s_value, *s_fast;
@@ -71,10 +75,10 @@ bool same_buffers(const Record &r, PyObject *buffers, PyObject *params)
     return t.has_storage() && t.scalar_type() == at::kFloat && t.const_data_ptr() == r.bias;
 }
 
-// record(desc_address, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device) -> capsule
+// record(desc_address, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, x_scratch or None) -> capsule
 PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 9) { PyErr_SetString(PyExc_TypeError, "record takes 9 arguments"); return nullptr; }
+    if (n != 11) { PyErr_SetString(PyExc_TypeError, "record takes 11 arguments"); return nullptr; }
     HANDLE_TH_ERRORS
     auto *r = new Record();
     r->desc = *static_cast<const ortho_b200_layer_desc *>(PyLong_AsVoidPtr(a[0]));
@@ -91,6 +95,8 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
     r->ws_ptr = a[6] == Py_None ? nullptr : PyLong_AsVoidPtr(a[6]);
     r->ws_bytes = PyLong_AsLongLong(a[7]);
     r->device = (int)PyLong_AsLong(a[8]);
+    r->type = (int)PyLong_AsLong(a[9]);
+    r->x_scratch = a[10] == Py_None ? nullptr : PyLong_AsVoidPtr(a[10]);
     if (PyErr_Occurred()) { delete r; return nullptr; }
     r->ws = Py_NewRef(a[4]);
     return PyCapsule_New(r, "ortho_record", free_record);
@@ -103,7 +109,10 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (n != 7) { PyErr_SetString(PyExc_TypeError, "module takes 7 arguments"); return nullptr; }
     HANDLE_TH_ERRORS
     const at::Tensor *x = plain(a[0]);
-    if (!x || x->scalar_type() != at::kHalf || !x->is_contiguous() || x->dim() < 1) Py_RETURN_NONE;
+    if (!x || !x->is_contiguous() || x->dim() < 1) Py_RETURN_NONE;
+    const auto dtype = x->scalar_type();
+    const int type = dtype == at::kHalf ? ORTHO_B200_TYPE_F16 : dtype == at::kBFloat16 ? ORTHO_B200_TYPE_BF16 : dtype == at::kFloat ? ORTHO_B200_TYPE_F32 : -1;
+    if (type < 0) Py_RETURN_NONE;
     const int64_t K = PyLong_AsLongLong(a[5]), N = PyLong_AsLongLong(a[6]);
     const double alpha = PyFloat_AsDouble(a[4]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
@@ -114,7 +123,8 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     void *stream = (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
     PyObject *rec = nullptr;
     {
-        PyObject *key = Py_BuildValue("(LK)", (long long)M, (unsigned long long)(uintptr_t)stream);
+        PyObject *key = type == ORTHO_B200_TYPE_F16 ? Py_BuildValue("(LK)", (long long)M, (unsigned long long)(uintptr_t)stream)
+                                                    : Py_BuildValue("(LKi)", (long long)M, (unsigned long long)(uintptr_t)stream, type);
         if (!key) return nullptr;
         PyObject *b = PyDict_GetItemWithError(a[3], key);
         Py_DECREF(key);
@@ -126,10 +136,10 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (rec == Py_None) Py_RETURN_NONE;
     Record *r = static_cast<Record *>(PyCapsule_GetPointer(rec, "ortho_record"));
     if (!r) { PyErr_Clear(); Py_RETURN_NONE; }
-    if (r->device != dev || (alpha > 0) != r->active || r->desc.N != N || !same_buffers(*r, a[1], a[2])) Py_RETURN_NONE;
+    if (r->device != dev || r->type != type || (alpha > 0) != r->active || r->desc.N != N || !same_buffers(*r, a[1], a[2])) Py_RETURN_NONE;
     // the scratch of the record, held over the launch whatever other threads bind meanwhile
     PyObject *scratch = nullptr;
-    if (r->ws_bytes) {
+    if (r->ws_bytes || r->x_scratch) {
         scratch = PyObject_GetAttr(r->ws, s_tensor);
         PyObject *gen = scratch ? PyObject_GetAttr(r->ws, s_gen) : nullptr;
         const bool same = gen && PyLong_AsLongLong(gen) == r->ws_gen && scratch != Py_None;
@@ -142,18 +152,19 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     {
         c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
         shape.back() = N;
-        y = at::empty(shape, at::TensorOptions().dtype(at::kHalf).device(x->device()));
+        y = at::empty(shape, at::TensorOptions().dtype(dtype).device(x->device()));
     }
     if (!y.has_storage() || y.unsafeGetTensorImpl()->is_python_dispatch()) Py_RETURN_NONE;
     ortho_b200_layer_desc d = r->desc;
     d.y_f16 = y.mutable_data_ptr();
     d.alpha = (float)alpha;
     const void *xp = x->const_data_ptr();
-    void *ws = r->ws_ptr;
+    void *ws = r->ws_ptr, *xs = r->x_scratch;
     const int64_t ws_bytes = r->ws_bytes;
     int st;
     Py_BEGIN_ALLOW_THREADS
-    st = forward_multi(&d, 1, xp, M, K, ws, ws_bytes, stream);
+    st = type == ORTHO_B200_TYPE_F16 ? forward_multi(&d, 1, xp, M, K, ws, ws_bytes, stream)
+                                     : forward_typed(&d, xp, type, type, M, K, xs, ws, ws_bytes, stream);
     Py_END_ALLOW_THREADS
     if (st) return PyLong_FromLong(st);
     return THPVariable_Wrap(std::move(y));
@@ -243,12 +254,13 @@ PyObject *layers_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     END_HANDLE_TH_ERRORS
 }
 
-// addresses of ortho_b200_forward_multi and ortho_b200_multi_workspace_bytes in the loaded library
+// addresses of ortho_b200_forward_multi, ortho_b200_multi_workspace_bytes and ortho_b200_forward_typed in the loaded library
 PyObject *set_library(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 2) { PyErr_SetString(PyExc_TypeError, "set_library takes 2 arguments"); return nullptr; }
+    if (n != 3) { PyErr_SetString(PyExc_TypeError, "set_library takes 3 arguments"); return nullptr; }
     forward_multi = reinterpret_cast<multi_fn>(PyLong_AsVoidPtr(a[0]));
     multi_workspace = reinterpret_cast<multi_ws_fn>(PyLong_AsVoidPtr(a[1]));
+    forward_typed = reinterpret_cast<typed_fn>(PyLong_AsVoidPtr(a[2]));
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
 }

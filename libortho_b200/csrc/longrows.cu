@@ -203,7 +203,7 @@ long_sum_kernel(float4 *__restrict__ part, long long quads, long long stride, in
 // y[m, hrow[h]] = FP16(rest[h, m] + alpha * (part[0] + ... + part[nsplit - 1])[h, m]); one token per thread
 __global__ void __launch_bounds__(256)
 long_finish_kernel(const float *__restrict__ part, long long stride, int nsplit, const float *__restrict__ rest,
-                   int h0, float alpha, __half *__restrict__ y, long long ldy, int Mp, const RowEntries re)
+                   int h0, float alpha, __half *__restrict__ y, int y_type, long long ldy, int Mp, const RowEntries re)
 {
     const int m = blockIdx.x * 256 + threadIdx.x, h = h0 + blockIdx.y;
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -219,7 +219,7 @@ long_finish_kernel(const float *__restrict__ part, long long stride, int nsplit,
         for (int j = 0; j < 8; j++) acc += t[j];
     }
     if (acc != acc) acc = long_sum_again(re, h, m);
-    y[(size_t)m * (size_t)ldy + re.hrow[h]] = __float2half_rn(fmaf(alpha, acc, base));
+    store_typed(y, (size_t)m * (size_t)ldy + re.hrow[h], fmaf(alpha, acc, base), y_type);
 }
 
 // ---- plan side: the dense copy of the long rows --------------------------------------------------------------
@@ -318,7 +318,7 @@ int launch_long_finish(const FwdArgs &a, int Mp, void *ws)
     for (int64_t h0 = 0; h0 < pl->n_long; h0 += kRows) {
         cfg.gridDim = dim3((unsigned)ceil_div(a.M, 256), (unsigned)(pl->n_long - h0 < kRows ? pl->n_long - h0 : kRows));
         OB_CUDA(cudaLaunchKernelEx(&cfg, long_finish_kernel, part, (long long)pl->n_pad * Mp, long_rows_splits(pl, a.M), rest,
-                                   (int)h0, a.alpha, a.y, (long long)a.pitch_y(), Mp, row_entries(a)));
+                                   (int)h0, a.alpha, a.y, a.y_type, (long long)a.pitch_y(), Mp, row_entries(a)));
         count_launch();
     }
     return ORTHO_B200_OK;

@@ -91,6 +91,7 @@ constexpr int kTwoIssuers = 64, kTwoIssuersSparse = 32;      // two issuers up t
 
 struct Params {
     const __half *scales; const float *bias; __half *y;
+    int y_type;                 // kTypeF16 ..: what y points to
     int M, K, N;
     long long ldy;
     int tiles_n, kblocks, kpairs;
@@ -143,8 +144,9 @@ struct Pieces {
 };
 }  // namespace md
 
-// SPARSE: the entries of an ordered plan are contracted from the scattered tiles; at most 4 stages then
-template <bool SPARSE>
+// SPARSE: the entries of an ordered plan are contracted from the scattered tiles; at most 4 stages then.  TYPED: y is of another type
+// than FP16 (an instantiation of its own: the branch cost the others 1-2 %).
+template <bool SPARSE, bool TYPED>
 __global__ void __launch_bounds__(md::kWarps<SPARSE> * 32, 1)
 mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const md::Params p)
 {
@@ -562,6 +564,12 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                         v[4 * j + 2] = fmaf(p.alpha, t.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(p.alpha, t.w, v[4 * j + 3]);
                     }
                 }
+                if (TYPED && plain) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (n_ok && c + j < p.M) store_typed(p.y, (size_t)(c + j) * (size_t)p.ldy + n, v[j], p.y_type);
+                    continue;
+                }
                 if (plain) {
                     __half *yp = p.y + (size_t)c * (size_t)p.ldy + n;
 #pragma unroll
@@ -708,6 +716,13 @@ int64_t mid_workspace_bytes(int64_t M, int64_t K, int64_t N)
     return mid_xt_bytes(M, K) + mid_o_bytes(M, N) + mid_slot_bytes(M) + 2048;
 }
 
+bool mid_has_lists(const FwdArgs &a)
+{
+    const int64_t long_bytes = a.plan && a.plan->n_long > 0 ? long_rows_workspace_bytes(a.plan, a.M) : 0;
+    return a.has_ortho && a.plan && a.ortho.entries && a.plan->win_off && a.workspace_bytes >= mid_workspace_bytes(a.M, a.K, a.N) + long_bytes &&
+           tuning_snapshot().patch_weights;
+}
+
 int launch_mid(const FwdArgs &a)
 {
     using namespace md;
@@ -737,9 +752,8 @@ int launch_mid(const FwdArgs &a)
     if (!p.status) return ORTHO_B200_ERR_CUDA;
     bool sparse = false;
     const bool long_rows = a.plan && a.plan->n_long > 0;
-    const int64_t long_bytes = long_rows ? long_rows_workspace_bytes(a.plan, a.M) : 0;
-    if (a.has_ortho && a.plan && a.ortho.entries && a.plan->win_off && a.workspace_bytes >= own_bytes + long_bytes &&
-        tuning_snapshot().patch_weights) {
+    p.y_type = a.y_type;
+    if (mid_has_lists(a)) {
         sparse = true;
         p.win_off = a.plan->win_off; p.win_words = a.plan->win_words; p.ngroups = (int)ceil_div(a.N, kWinRows);
         p.row_ptr = a.plan->row_ptr; p.entries = a.ortho.entries; p.x = a.x;
@@ -797,8 +811,8 @@ int launch_mid(const FwdArgs &a)
     }
     static bool attr_set[kMaxDevices] = {};
     if (!attr_set[dev]) {
-        OB_CUDA(cudaFuncSetAttribute(mid_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-        OB_CUDA(cudaFuncSetAttribute(mid_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        for (auto k : {mid_kernel<false, false>, mid_kernel<true, false>, mid_kernel<false, true>, mid_kernel<true, true>})
+            OB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
         attr_set[dev] = true;
     }
     // every CTA gets at least kMinShare units: a narrow layer cut into shares of a few would spend its time adding
@@ -828,8 +842,9 @@ int launch_mid(const FwdArgs &a)
         const int st = launch_long_rows(a, p.ol_mp, wsb + own_bytes, &p.ol);
         if (st != ORTHO_B200_OK) return st;
     }
-    if (sparse) OB_CUDA(cudaLaunchKernelEx(&cfg, mid_kernel<true>, xmap, wmap, p));
-    else OB_CUDA(cudaLaunchKernelEx(&cfg, mid_kernel<false>, xmap, wmap, p));
+    const bool typed = p.y_type != kTypeF16;
+    OB_CUDA(cudaLaunchKernelEx(&cfg, sparse ? (typed ? mid_kernel<true, true> : mid_kernel<true, false>)
+                                            : (typed ? mid_kernel<false, true> : mid_kernel<false, false>), xmap, wmap, p));
     count_launch();
     return ORTHO_B200_OK;
 }

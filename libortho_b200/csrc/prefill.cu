@@ -684,15 +684,19 @@ int64_t prefill_workspace_bytes(int64_t M, int64_t K, int64_t N)
     return prefill_xt_bytes(M, K) + (wide_split_bytes() > split ? wide_split_bytes() : split);
 }
 
+bool wide_takes(const FwdArgs &a)
+{
+    const Tuning t = tuning_snapshot();
+    return t.wide && !(a.gv && a.gv->world > 1) && (!a.has_ortho || (a.plan && a.plan->win_off && t.patch_weights));
+}
+
 int launch_prefill(const FwdArgs &a)
 {
     using namespace pf;
     // base-only calls and plans with window lists run the kernel of wide.cu (measured there); the rest, the sparse term as
     // gathers and the peer exchange, stays here
-    const Tuning t = tuning_snapshot();
-    const bool lists = a.has_ortho && a.plan && a.plan->win_off && t.patch_weights;
-    if (t.wide && !(a.gv && a.gv->world > 1) && (!a.has_ortho || lists)) {
-        if (lists && a.plan->n_long > 0) {
+    if (wide_takes(a)) {
+        if (a.has_ortho && a.plan->n_long > 0) {
             if (!a.workspace || a.workspace_bytes < prefill_xt_bytes(a.M, a.K) + long_rows_workspace_bytes(a.plan, a.M))
                 return ORTHO_B200_ERR_WORKSPACE;
             if (((uintptr_t)a.workspace & 255u) != 0) return ORTHO_B200_ERR_ALIGN;

@@ -39,6 +39,30 @@ transpose_x_kernel(const __half *__restrict__ x, __half *__restrict__ xt, int M,
     }
 }
 
+// X of another type -> FP16, eight values a thread.  The kernel behind it is its programmatic dependent: it fetches its first weights
+// meanwhile.  11008 x 777 BF16: the separate conversions to FP16 and back, by element-wise kernels, took 20 of 95 us.
+__global__ void __launch_bounds__(256)
+convert_x_kernel(const void *__restrict__ x, int type, uint4 *__restrict__ out, int64_t n8)
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n8; i += (int64_t)gridDim.x * 256) out[i] = load8_as_half(x, (size_t)i * 8, type);
+}
+
+int launch_convert_x(const void *x, int type, __half *out, int64_t n, cudaStream_t stream)
+{
+    const int64_t n8 = n / 8, blocks = ceil_div(n8, 256), most = (int64_t)device_sm_count(current_device_index()) * 8;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(blocks < most ? blocks : most)); cfg.blockDim = dim3(256); cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    OB_CUDA(cudaLaunchKernelEx(&cfg, convert_x_kernel, x, type, reinterpret_cast<uint4 *>(out), n8));
+    count_launch();
+    return ORTHO_B200_OK;
+}
+
 int launch_transpose_x(const __half *x, __half *xt, int M, int K, int Mp, cudaStream_t stream)
 {
     dim3 tg((unsigned)ceil_div(K, 64), (unsigned)ceil_div(Mp, 64));

@@ -65,6 +65,7 @@ constexpr int kSmemData = 225 * 1024;   // packed-weight slots and token stages
 
 struct Params {
     const __half *scales; const float *bias; __half *y;
+    int y_type;                 // kTypeF16 ..: what y points to
     int M, K, N;
     long long ldy;
     int tiles_n, tiles_m, kblocks, boxes;       // boxes = ceil(K / 256)
@@ -187,7 +188,8 @@ __device__ __forceinline__ void add_entries(uint32_t (&h)[32], uint32_t mine, ui
 }
 }  // namespace wd
 
-template <bool SPARSE>
+// TYPED: as in mid.cu
+template <bool SPARSE, bool TYPED>
 __global__ void __launch_bounds__(wd::NWARPS * 32, 1)
 wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const wd::Params p)
 {
@@ -280,7 +282,7 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
                     const uint32_t acc0 = acc;
                     uint64_t *done = &sm->empty[st];
                     if (++st == p.nst) { st = 0; ph ^= 1u; }
-                    ready = mbar_test_wait(&sm->full[st], ph);
+                    ready = mbar_try_wait(&sm->full[st], ph);
 #pragma unroll
                     for (int kk = 0; kk < KB / 16; kk++) {
                         umma_f16_ts(d_tmem, at + (uint32_t)(kk * 8), bd + (uint64_t)(2 * kk), idesc, acc);
@@ -489,6 +491,13 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
                                 r[j] = __float_as_uint(fmaf(ev, __half2float(p.x[(size_t)(m0 + c + j) * p.K + k]), __uint_as_float(r[j])));
                     }
                 }
+                if (TYPED) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (n_st && m0 + c + j < p.M)
+                            store_typed(p.y, (size_t)(m0 + c + j) * (size_t)p.ldy + n, __uint_as_float(r[j]), p.y_type);
+                    continue;
+                }
                 __half *yp = p.y + (size_t)(m0 + c) * (size_t)p.ldy + n;
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
@@ -528,7 +537,7 @@ int launch_wide(const FwdArgs &a, int64_t long_off)
     if (num_sms > kWideMaxSms) num_sms = kWideMaxSms;
     Params p;
     memset(&p, 0, sizeof(p));
-    p.scales = a.scales; p.bias = a.bias; p.y = a.y; p.M = (int)a.M; p.K = (int)a.K; p.N = (int)a.N; p.ldy = a.pitch_y();
+    p.scales = a.scales; p.bias = a.bias; p.y = a.y; p.M = (int)a.M; p.K = (int)a.K; p.N = (int)a.N; p.ldy = a.pitch_y(); p.y_type = a.y_type;
     const bool sparse = a.has_ortho != 0;
     const int halves = sparse ? kHalves<true> : kHalves<false>, tmax = sparse ? kTMax<true> : kTMax<false>;
     p.tiles_m = (int)ceil_div(a.M, halves * tmax);
@@ -589,8 +598,8 @@ int launch_wide(const FwdArgs &a, int64_t long_off)
         return ORTHO_B200_ERR_CUDA;
     static bool attr_set[kMaxDevices] = {};
     if (!attr_set[dev]) {
-        OB_CUDA(cudaFuncSetAttribute(wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-        OB_CUDA(cudaFuncSetAttribute(wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        for (auto k : {wide_kernel<false, false>, wide_kernel<true, false>, wide_kernel<false, true>, wide_kernel<true, true>})
+            OB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
         attr_set[dev] = true;
     }
     if (p.n_long > 0) {
@@ -607,8 +616,9 @@ int launch_wide(const FwdArgs &a, int64_t long_off)
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    if (sparse) OB_CUDA(cudaLaunchKernelEx(&cfg, wide_kernel<true>, xmap, wmap, p));
-    else OB_CUDA(cudaLaunchKernelEx(&cfg, wide_kernel<false>, xmap, wmap, p));
+    const bool typed = p.y_type != kTypeF16;
+    OB_CUDA(cudaLaunchKernelEx(&cfg, sparse ? (typed ? wide_kernel<true, true> : wide_kernel<true, false>)
+                                            : (typed ? wide_kernel<false, true> : wide_kernel<false, false>), xmap, wmap, p));
     count_launch();
     if (p.n_long > 0) return launch_long_finish(a, p.rest_mp, reinterpret_cast<unsigned char *>(a.workspace) + long_off);
     return ORTHO_B200_OK;

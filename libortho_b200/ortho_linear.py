@@ -37,6 +37,7 @@ def _current_stream_handle(dev: torch.device) -> int:
         return _raw_stream(dev.index)
     return torch.cuda.current_stream(dev).cuda_stream
 
+_TYPES = {torch.bfloat16: 1, torch.float32: 2}           # activations that are converted by the library: ORTHO_B200_TYPE_*
 _ORTHO_BUFFERS = ("ortho_values", "ortho_col_indices", "ortho_row_ptr")
 _WATCHED = frozenset(("base_weight", "base_scales", "bias") + _ORTHO_BUFFERS)
 
@@ -229,8 +230,9 @@ class OrthoLinear(nn.Module):
         return (self.base_weight.data_ptr(), self.base_scales.data_ptr(), ov.data_ptr(), oc.data_ptr(), orp.data_ptr(),
                 ov._version, oc._version, orp._version, (b.data_ptr(), b.dtype) if b is not None else None)
 
-    def _bind(self, M: int, dev: torch.device, stream: int) -> Tuple[_Bound, Optional[torch.Tensor]]:
-        """The call record and its scratch, which the caller holds until the launch."""
+    def _bind(self, M: int, dev: torch.device, stream: int, type: int = 0) -> Tuple[_Bound, Optional[torch.Tensor]]:
+        """The call record and its scratch, which the caller holds until the launch.  `type`: of activations and output, the
+        library's number; other types than FP16 get a record whose `fast` is None where the kernel does not take them."""
         N, K = self.out_features, self.in_features
         bw, bs = self.base_weight, self.base_scales
         if bw.dtype != torch.uint8 or bs.dtype != torch.float16:
@@ -250,10 +252,6 @@ class OrthoLinear(nn.Module):
                 raise ValueError("CSR arrays have inconsistent sizes")
         b = _Bound()
         plan = self._get_plan() if sparse else None
-        need = self._workspace_bytes(M)
-        b.ws, b.ws_gen, scratch = _SharedWorkspace.get(dev, need, stream)
-        b.ws_ptr = scratch.data_ptr() if need else None
-        b.ws_bytes = scratch.numel() if need else 0
         b.fused_bias = (self.bias is not None and self.bias.dtype == torch.float32 and self.bias.device == dev
                         and self.bias.is_contiguous())
         descs = (_lib.LayerDesc * 1)()
@@ -267,17 +265,47 @@ class OrthoLinear(nn.Module):
         d.bias_f32 = self.bias.data_ptr() if b.fused_bias else None
         d.N, d.ldy, d.reserved = N, 0, 0
         b.descs = descs
+        need = self._workspace_bytes(M)
+        own, convert = (need + 255) // 256 * 256, 0          # the FP16 copy of other activations lies behind what the kernels need
+        if type:
+            d.alpha = float(self.alpha)
+            if need == 0:
+                convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, None, 0)
+            if need or convert > 0:
+                need = own + 2 * M * K
+        b.ws, b.ws_gen, scratch = _SharedWorkspace.get(dev, need, stream)
+        b.ws_ptr = scratch.data_ptr() if need else None
+        b.ws_bytes = scratch.numel() if need else 0
+        x_scratch = None
+        if type and need:
+            b.ws_bytes = own
+            convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, b.ws_ptr, own)
+            x_scratch = b.ws_ptr + own if convert > 0 else None
         b.key = (self.alpha > 0, self._versions())
         # what the native path compares and launches; not for a bias that torch has to add
         b.fast = None
-        if self.bias is None or b.fused_bias:
+        if (self.bias is None or b.fused_bias) and not (type and convert < 0):
             b.fast = _lib.fast().record(ctypes.addressof(descs), self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
-                                        b.ws_bytes, dev.index)
+                                        b.ws_bytes, dev.index, type, x_scratch)
         if b.ws.shared:
             if len(self._bound) > 32:
                 self._bound.clear()
-            self._bound[(M, stream)] = b
+            self._bound[(M, stream, type) if type else (M, stream)] = b
         return b, scratch
+
+    def _bind_typed(self, x: torch.Tensor) -> bool:
+        """A record for activations of another type; False where one that fits is there already (the call is not a plain one), where
+        the kernel does not take them, and under capture (shared scratch): the general code converts then."""
+        dev, K = x.device, self.in_features
+        if x.dim() < 1 or x.shape[-1] != K or x.numel() == 0 or not x.is_contiguous() or torch.cuda.current_device() != dev.index or _capturing(dev):
+            return False
+        M, stream = x.numel() // K, _current_stream_handle(dev)
+        b = self._bound.get((M, stream, _TYPES[x.dtype]))
+        if b is not None and b.fast is None and b.key[0] == (self.alpha > 0):
+            return False
+        if b is not None and b.key == (self.alpha > 0, self._versions()) and b.ws_gen == b.ws.gen:
+            return False
+        return self._bind(M, dev, stream, _TYPES[x.dtype])[0].fast is not None
 
     # -- forward ---------------------------------------------------------------------------------
     def forward(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -287,6 +315,8 @@ class OrthoLinear(nn.Module):
         if out is None and x.is_cuda:
             # a call like one before: FP16, this device, no scratch under capture.  None: the code below does it
             y = _lib.fast().module(x, self._buffers, self._parameters, self._bound, self.alpha, self.in_features, self.out_features)
+            if y is None and x.dtype in _TYPES and self._bind_typed(x):
+                y = _lib.fast().module(x, self._buffers, self._parameters, self._bound, self.alpha, self.in_features, self.out_features)
             if y is not None:
                 if type(y) is int:
                     _lib.check(y, "ortho_b200_forward_multi")
