@@ -260,6 +260,23 @@ __device__ __forceinline__ void store_typed(void *y, size_t at, float v, int typ
     else if (type == kTypeBF16) reinterpret_cast<__nv_bfloat16 *>(y)[at] = __float2bfloat16_rn(__half2float(h));
     else reinterpret_cast<float *>(y)[at] = __half2float(h);
 }
+// N values of one column of y, a row (token) apart, `rows` of them stored: the branch on the type and the row's
+// address stay outside (2048->16384 at 1500 tokens, base: BF16 141 -> 77 us, FP32 150 -> 84; converting around the FP16 forward 137)
+template <int N, class V>
+__device__ __forceinline__ void store_column(void *y, size_t at, long long ldy, int type, int rows, bool on, const V &v)
+{
+    if (type == kTypeBF16) {
+        __nv_bfloat16 *p = reinterpret_cast<__nv_bfloat16 *>(y) + at;
+#pragma unroll
+        for (int j = 0; j < N; j++, p += ldy)
+            if (on && j < rows) *p = __float2bfloat16_rn(__half2float(__float2half_rn(v(j))));
+    } else {
+        float *p = reinterpret_cast<float *>(y) + at;
+#pragma unroll
+        for (int j = 0; j < N; j++, p += ldy)
+            if (on && j < rows) *p = __half2float(__float2half_rn(v(j)));
+    }
+}
 __device__ __forceinline__ uint32_t pack_half2(float a, float b)
 {
     const __half2 h = __floats2half2_rn(a, b);

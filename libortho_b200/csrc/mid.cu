@@ -565,9 +565,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                     }
                 }
                 if (TYPED && plain) {
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if (n_ok && c + j < p.M) store_typed(p.y, (size_t)(c + j) * (size_t)p.ldy + n, v[j], p.y_type);
+                    store_column<8>(p.y, (size_t)c * (size_t)p.ldy + n, p.ldy, p.y_type, p.M - c, n_ok, [&](int j) { return v[j]; });
                     continue;
                 }
                 if (plain) {

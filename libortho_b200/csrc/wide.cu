@@ -492,10 +492,8 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
                     }
                 }
                 if (TYPED) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (n_st && m0 + c + j < p.M)
-                            store_typed(p.y, (size_t)(m0 + c + j) * (size_t)p.ldy + n, __uint_as_float(r[j]), p.y_type);
+                    store_column<16>(p.y, (size_t)(m0 + c) * (size_t)p.ldy + n, p.ldy, p.y_type, p.M - m0 - c, n_st,
+                                     [&](int j) { return __uint_as_float(r[j]); });
                     continue;
                 }
                 __half *yp = p.y + (size_t)(m0 + c) * (size_t)p.ldy + n;
