@@ -18,7 +18,7 @@
 // each pass was bound by instructions, so they are only done where an approximate quotient cannot decide:
 // near a rounding tie (quant_clamped), near the edge of a bin or near the threshold.
 // (4096->11008, keep the top 1 %: 344 us by these passes: rows 115, bin 126, list 8, split 94.)
-// Matrices of whole rows, of 8 million weights or more, take one pass over W where the scratch holds a list of candidates: a sample of the rows brackets the
+// Matrices of whole rows, of 10 million weights or more, take one pass over W where the scratch holds a list of candidates: a sample of the rows brackets the
 // k-th largest score, the pass splits every weight at once (a row's scale first, its second reading comes from registers or L1),
 // counts the scores above the bracket and lists those inside it, a radix select over that short list finds the threshold, and the
 // listed residuals above it are written.  When the bracket turns out not to hold the k-th score, or the list overflows, the passes
@@ -610,8 +610,9 @@ extern "C" int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t
     }
     // One pass where the list can hold what a bracket of the k-th score holds (half of k and two bins' worth) and W outlives
     // the pass
-    // (below 8 million weights its ten launches cost more than the passes: 2048 x 1024 93 us against 84)
-    const bool onepass = k && !cut && N * K >= ((int64_t)1 << 23) && outs_apart && base_apart && ortho_apart && N <= 0xffffffffLL / K && k <= (unsigned long long)(N * K / 25) &&
+    // (below 10 million weights its ten launches cost as much as the passes: 2048 x 1024 93 us against 84, whole layers of 8.6 million 209 / 202,
+    // 10.2 million 217 / 238)
+    const bool onepass = k && !cut && N * K >= 10000000 && outs_apart && base_apart && ortho_apart && N <= 0xffffffffLL / K && k <= (unsigned long long)(N * K / 25) &&
                          scratch_bytes >= ortho_b200_sieve_onepass_scratch_bytes(N, K);
     if (onepass) {
         OnePass *op = reinterpret_cast<OnePass *>(reinterpret_cast<unsigned char *>(scratch) + (ortho_b200_sieve_scratch_bytes(N) + 255) / 256 * 256);

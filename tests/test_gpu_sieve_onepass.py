@@ -32,7 +32,7 @@ def weights(kind, N, K):
 
 
 @pytest.mark.parametrize("kind", ["gauss", "rows", "ties", "zeros", "outlier"])
-@pytest.mark.parametrize("N,K,target", [(300, 1024, 0.001), (4100, 2052, 0.01), (4100, 2048, 0.04), (8300, 1024, 0.02), (1030, 8200, 0.003), (2060, 4096, 0.001)])
+@pytest.mark.parametrize("N,K,target", [(300, 1024, 0.001), (5000, 2052, 0.01), (5000, 2048, 0.04), (10000, 1024, 0.02), (1300, 8200, 0.003), (2500, 4096, 0.001)])
 def test_sieve_by_one_pass(kind, N, K, target):
     w, h = weights(kind, N, K)
     base_ref, ortho_ref = sieve.hessian_sieve(w, h, sparsity_target=target)
