@@ -298,40 +298,38 @@ static bool decode_regime_of(const Tuning &t, int64_t M, int64_t N, int64_t K)
 }
 bool decode_regime(int64_t M, int64_t N, int64_t K) { return decode_regime_of(tuning_snapshot(), M, N, K); }
 // The tcgen05 kernel of mid.cu against the streaming kernel (up to 16 tokens; needs its sparse entries as window lists or
-// none at all).  Its time hardly depends on the token count (about 9 us + 0.15 us, base-only 0.1 us, per million weights + 0.1 us
-// per 1000 inputs), the streaming kernel's grows with it, with the rounds of row tiles (of 16 rows, two per SM at a time) and
+// none at all).  Its time hardly depends on the token count (about 7 us + 0.15 us, base-only 5.7 + 0.11, per million weights),
+// the streaming kernel's grows with it, with the rounds of row tiles (of 16 rows, two per SM at a time) and
 // with the activation slab of a CTA (M x K halves): above 100 KB one CTA fits an SM instead of two, above 200 KB K is split
-// over a cluster.  One B200, us, weights rotating over more than L2, streaming / mid.cu with 0.3 % ortho; base-only:
-//   16 tokens: 4096->4096 9.8 / 11.9; 8.1 / 10.4, 8192->2048 13.4 / 12.8; 10.9 / 11.2, 4096->6144 14.1 / 13.0; 11.2 / 11.5,
-//              11008->2048 14.4 / 14.2; 11.5 / 12.6, 8192->4096 20.5 / 14.5; 16.5 / 12.4, 4096->12288 19.9 / 16.2; 15.2 / 13.4
-//   12 tokens: 4096->8192 13.6 / 13.9; 10.4 / 12.1, 8192->4096 15.4 / 14.6; 12.1 / 12.6, 28672->1024 20.0 / 17.5; 14.2 / 15.2,
-//              5120->5120 15.3 / 13.3; 12.4 / 11.6, 11008->3072 18.9 / 15.2; 15.7 / 12.9
-//    9 tokens: 4096->6144 12.3 / 13.0; 9.4 / 11.5, 4096->8192 13.1 / 14.1; 9.9 / 12.2, 11008->2048 11.4 / 13.8; 9.3 / 12.3,
-//              5120->8192 15.3 / 15.5; 12.1 / 13.0, 2048->14336 14.3 / 12.6; 9.6 / 11.2, 11008->4096 17.4 / 16.5; 14.1 / 13.7,
-//              4096->10240 17.0 / 15.6; 12.8 / 13.0, 8192->57344 125 / 85; 96 / 59
-//    8 tokens: 4096->22016 20.3 / 21.4, 8192->4096 12.6 / 14.6, 8192->8192 19.6 / 19.6, 8192->10240 23.2 / 22.1, 11008->4096 17.7 / 16.5
-//    6 tokens: 12288->6144 20.7 / 21.3, 28672->1536 17.8 / 18.1, 20480->2048 15.5 / 17.4, 14336->4096 19.9 / 19.0,
-//              8192->57344 93 / 85
-//    5 tokens: 13824->5120 19.6 / 20.7, 28672->1536 15.2 / 18.6, 28672->4096 28.3 / 28.5, 28672->8192 52 / 47, 16384->16384 68 / 52
-//    4 tokens: 28672->4096 30.6 / 28.4, 28672->8192 52 / 47, 16384->16384 44 / 52;   3 tokens: 28672->4096 23.2 / 28.4
+// over a cluster.  One B200, us, weights rotating over more than L2, streaming / mid.cu base-only; with 0.3 % ortho:
+//   16 tokens: 4096->2048 6.7 / 6.0; 8.6 / 8.5, 4096->4096 8.2 / 7.2; 9.7 / 9.2, 8192->2048 11.0 / 7.4; 13.1 / 9.2, 8192->1024 6.7 / 7.1;
+//              8.6 / 8.7, 4096->6144 11.2 / 9.4; 14.0 / 11.3, 11008->2048 11.5 / 9.4; 14.2 / 11.6, 28672->1024 14.9 / 11.6; 20.6 / 14.2
+//   12 tokens: 4096->4096 7.5 / 7.2; 8.9 / 9.2, 4096->6144 9.9 / 9.2; 12.7 / 11.1, 4096->8192 10.5 / 10.2; 13.4 / 12.9,
+//              2048->14336 10.1 / 9.3; 14.8 / 11.4, 8192->2048 8.3 / 7.5; 10.0 / 9.2
+//    9 tokens: 4096->4096 7.0 / 7.1; 8.6 / 9.0, 4096->6144 9.5 / 9.3; 12.2 / 11.2, 4096->8192 10.0 / 10.5; 13.0 / 12.7,
+//              4096->11008 12.9 / 11.3; 17.2 / 13.7, 8192->2048 7.9 / 7.5; 9.8 / 9.1, 11008->2048 9.4 / 9.5; 11.2 / 11.6,
+//              2048->14336 9.7 / 9.5; 14.2 / 11.6, 8192->4096 12.2 / 10.1; 14.3 / 12.5, 28672->1024 14.0 / 11.5; 17.5 / 14.3
+//    8 tokens: 4096->22016 15.4 / 14.9; 20.6 / 20.0, 8192->4096 10.1 / 10.2; 12.6 / 12.5, 8192->8192 16.0 / 14.0; 19.9 / 17.7,
+//              11008->4096 14.0 / 11.8; 17.9 / 14.4
+//    6 tokens: 4096->22016 15.3 / 14.9; 20.6 / 20.0, 8192->8192 13.2 / 14.0; 17.1 / 17.8, 8192->10240 15.9 / 15.8; 20.6 / 20.2,
+//              8192->28672 37.6 / 29.8; 50.3 / 40.8, 14336->4096 16.1 / 13.4; 20.0 / 16.5
+//    5 tokens: 8192->28672 31.8 / 29.8; 40.0 / 40.9, 14336->4096 13.7 / 13.4; 16.1 / 16.6, 28672->8192 41.2 / 31.7; 52.9 / 42.2
+//    3 tokens: 8192->28672 31.1 / 29.8; 37.1 / 40.9, 28672->8192 36.1 / 31.5; 42.2 / 42.2, 4096->22016 14.4 / 14.9; 18.6 / 20.0
 static bool mid_beats_stream(int64_t M, int64_t N, int64_t K, bool base)
 {
     const int64_t weights = N * K, slab = 2 * M * K;
     const bool odd = K % 256 != 0;                       // the mma.sync kernel stands in for the streaming kernel
     if (M >= 9) {
-        if (weights <= (int64_t)4096 * 4096) return false;
-        if (odd) return true;
-        if (base) {
-            if (M <= 12 && slab <= (100 << 10)) return weights >= (int64_t)1 << 26;
-            return weights >= (int64_t)5 << 23 || (N > 2048 && (slab > (192 << 10) || (K > 4096 && (M > 12 || K <= 6144)))) ||
-                   (N >= 2048 && slab >= (512 << 10));
-        }
-        if (M <= 12 && K <= 4096 && N <= 2 * 2 * 148 * 16) return false;            // two rounds of tiles
-        return slab > (200 << 10) || N > 2048;
+        if (weights < (int64_t)1 << 24) return false;
+        if (odd) return weights > (int64_t)1 << 24;
+        if (base) return slab > (100 << 10) || M >= 12 || weights >= (int64_t)5 << 23;
+        if (slab <= (100 << 10)) return weights >= (int64_t)3 << 23;
+        return slab > (200 << 10) || N > 2048 || K <= 8192;
     }
     if (weights < (int64_t)5 << 23) return false;
+    if (base && M >= 3 && K >= 8192 && weights >= (int64_t)7 << 25) return true;
     if (slab >= (200 << 10)) return M >= 3 && (odd || weights >= (int64_t)3 << 24);
-    if (M >= 6 && weights >= (int64_t)1 << 28) return true;
+    if (M >= 6 && weights >= (int64_t)5 << 24) return true;
     return M >= 5 && (slab >= (150 << 10) || ((odd || M >= 7) && slab >= (128 << 10) && weights >= (int64_t)1 << 26));
 }
 static bool mid_range_of(const Tuning &t, int64_t M, int64_t N, int64_t K, bool base)
