@@ -113,6 +113,8 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     const auto dtype = x->scalar_type();
     const int type = dtype == at::kHalf ? ORTHO_B200_TYPE_F16 : dtype == at::kBFloat16 ? ORTHO_B200_TYPE_BF16 : dtype == at::kFloat ? ORTHO_B200_TYPE_F32 : -1;
     if (type < 0) Py_RETURN_NONE;
+    // the kernels read 16 bytes at a time; the general code's conversion to FP16 is a copy that is aligned
+    if (type != ORTHO_B200_TYPE_F16 && ((uintptr_t)x->const_data_ptr() & 15u) != 0) Py_RETURN_NONE;
     const int64_t K = PyLong_AsLongLong(a[5]), N = PyLong_AsLongLong(a[6]);
     const double alpha = PyFloat_AsDouble(a[4]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }

@@ -295,9 +295,10 @@ class OrthoLinear(nn.Module):
 
     def _bind_typed(self, x: torch.Tensor) -> bool:
         """A record for activations of another type; False where one that fits is there already (the call is not a plain one), where
-        the kernel does not take them, and under capture (shared scratch): the general code converts then."""
+        the kernel does not take them (alignment, too), and under capture (shared scratch): the general code converts then."""
         dev, K = x.device, self.in_features
-        if x.dim() < 1 or x.shape[-1] != K or x.numel() == 0 or not x.is_contiguous() or torch.cuda.current_device() != dev.index or _capturing(dev):
+        if (x.dim() < 1 or x.shape[-1] != K or x.numel() == 0 or not x.is_contiguous() or x.data_ptr() % 16
+                or torch.cuda.current_device() != dev.index or _capturing(dev)):
             return False
         M, stream = x.numel() // K, _current_stream_handle(dev)
         b = self._bound.get((M, stream, _TYPES[x.dtype]))

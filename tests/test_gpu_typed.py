@@ -40,6 +40,21 @@ def test_other_types_have_the_bits_of_converting_around(K, N, d, kind, dtype, bi
     assert _lib.lib().ortho_b200_query_kernel_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M", [1, 16, 24, 200])
+def test_activations_that_are_not_16_byte_aligned(M, dtype):
+    K, N = 1024, 256
+    m = wl.make_layer(K, N, 0.01, seed=3, device=DEV).to_module()
+    x = wl.make_input(M, K, seed=M, device=DEV).to(dtype)
+    want = m(x.to(torch.float16)).to(dtype)
+    buf = torch.zeros(M * K + 8, dtype=dtype, device=DEV)
+    for call in range(2):                                     # with no record of that type yet, and with one
+        for offset in (1, 2, 3):
+            odd = buf[offset:offset + M * K].view(M, K).copy_(x)
+            assert odd.data_ptr() % 16 and torch.equal(bits(m(odd)), bits(want)), (call, offset)
+        assert torch.equal(bits(m(x)), bits(want))
+
+
 @pytest.mark.parametrize("M", [1, 24, 200])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_buffers_replaced_or_edited_between_calls(M, dtype):
