@@ -168,6 +168,9 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     st = type == ORTHO_B200_TYPE_F16 ? forward_multi(&d, 1, xp, M, K, ws, ws_bytes, stream)
                                      : forward_typed(&d, xp, type, type, M, K, xs, ws, ws_bytes, stream);
     Py_END_ALLOW_THREADS
+    // The typed call is routed anew each time: with other routing settings, or an alpha too small for FP32, it may be one that the kernels
+    // do not take or that needs the FP16 copy this record has no room for.  It says so before it launches the forward.
+    if (type != ORTHO_B200_TYPE_F16 && (st == ORTHO_B200_ERR_SHAPE || st == ORTHO_B200_ERR_ALIGN || st == ORTHO_B200_ERR_WORKSPACE)) Py_RETURN_NONE;
     if (st) return PyLong_FromLong(st);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS

@@ -55,6 +55,30 @@ def test_activations_that_are_not_16_byte_aligned(M, dtype):
         assert torch.equal(bits(m(x)), bits(want))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_route_that_changed_since_the_record_was_made(dtype):
+    K, N = 4096, 4096
+    m = wl.make_layer(K, N, 0.002, seed=4, device=DEV).to_module()
+    L = _lib.lib()
+    for M, hook, builtin in ((200, (-8, 0, 0, 0), (-8, 0, 0, 1)), (12, (-4, 0, 8, 128), (-4, 0, 0, 0))):
+        x = wl.make_input(M, K, seed=M, device=DEV).to(dtype)
+        m(x)
+        assert L.ortho_b200_set_decode_config(*hook) == 0
+        try:
+            want = m(x.to(torch.float16)).to(dtype)
+            for _ in range(2):
+                assert torch.equal(bits(m(x)), bits(want)), (M, hook)
+        finally:
+            assert L.ortho_b200_set_decode_config(*builtin) == 0
+    # alpha > 0 in Python and 0 as a float: the base alone, which from 12 tokens on another kernel computes
+    x = wl.make_input(12, K, seed=5, device=DEV).to(dtype)
+    m(x)
+    m.set_alpha(1e-60)
+    y = m(x)
+    m.set_alpha(0.0)
+    assert torch.allclose(y.float(), m(x).float(), rtol=2e-3 if dtype == torch.float32 else 1.6e-2, atol=1e-2)
+
+
 @pytest.mark.parametrize("M", [1, 24, 200])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_buffers_replaced_or_edited_between_calls(M, dtype):
