@@ -49,12 +49,12 @@ void free_record(PyObject *cap)
     delete r;
 }
 
-// a plain CUDA tensor with storage, or nullptr
+// a plain CUDA tensor whose storage holds its values (no negation pending), or nullptr
 const at::Tensor *plain(PyObject *o)
 {
     if (!o || !THPVariable_CheckExact(o)) return nullptr;
     const at::Tensor &t = THPVariable_Unpack(o);
-    if (!t.defined() || !t.is_cuda() || !t.has_storage() || t.layout() != at::kStrided || t.unsafeGetTensorImpl()->is_python_dispatch()) return nullptr;
+    if (!t.defined() || !t.is_cuda() || !t.has_storage() || t.layout() != at::kStrided || t.is_neg() || t.unsafeGetTensorImpl()->is_python_dispatch()) return nullptr;
     return &t;
 }
 

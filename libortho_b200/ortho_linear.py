@@ -297,7 +297,7 @@ class OrthoLinear(nn.Module):
         """A record for activations of another type; False where one that fits is there already (the call is not a plain one), where
         the kernel does not take them (alignment, too), and under capture (shared scratch): the general code converts then."""
         dev, K = x.device, self.in_features
-        if (x.dim() < 1 or x.shape[-1] != K or x.numel() == 0 or not x.is_contiguous() or x.data_ptr() % 16
+        if (x.dim() < 1 or x.shape[-1] != K or x.numel() == 0 or not x.is_contiguous() or x.is_neg() or x.data_ptr() % 16
                 or torch.cuda.current_device() != dev.index or _capturing(dev)):
             return False
         M, stream = x.numel() // K, _current_stream_handle(dev)
@@ -328,6 +328,8 @@ class OrthoLinear(nn.Module):
         x_flat = x.reshape(-1, self.in_features)
         if x_flat.dtype != torch.float16:
             x_flat = x_flat.to(torch.float16)
+        elif x_flat.is_neg():
+            x_flat = x_flat.resolve_neg()
         if not x_flat.is_contiguous():
             x_flat = x_flat.contiguous()
         M = x_flat.shape[0]

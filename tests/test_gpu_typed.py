@@ -55,6 +55,18 @@ def test_activations_that_are_not_16_byte_aligned(M, dtype):
         assert torch.equal(bits(m(x)), bits(want))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M", [1, 40])
+def test_activations_with_a_negation_pending(M, dtype):
+    K, N = 1024, 256
+    m = wl.make_layer(K, N, 0.01, seed=3, device=DEV).to_module()
+    x = wl.make_input(M, K, seed=M, device=DEV).to(dtype)
+    want = m(-x)
+    assert torch.equal(bits(m(torch._neg_view(x))), bits(want))
+    m(x)
+    assert torch.equal(bits(m(torch._neg_view(x))), bits(want))
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_a_route_that_changed_since_the_record_was_made(dtype):
     K, N = 4096, 4096
