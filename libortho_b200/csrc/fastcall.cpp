@@ -13,6 +13,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/torch.h>
 
+#include <memory>
+
 #include "../../include/ortho_b200.h"
 
 namespace {
@@ -80,13 +82,14 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 11) { PyErr_SetString(PyExc_TypeError, "record takes 11 arguments"); return nullptr; }
     HANDLE_TH_ERRORS
-    auto *r = new Record();
+    auto r = std::make_unique<Record>();
     r->desc = *static_cast<const ortho_b200_layer_desc *>(PyLong_AsVoidPtr(a[0]));
     for (int i = 0; i < 5; i++) {
         PyObject *o = PyDict_GetItemWithError(a[1], s_buffers[i]);
-        if (!o || !THPVariable_Check(o)) { delete r; Py_RETURN_NONE; }
+        if (!o || !THPVariable_Check(o)) Py_RETURN_NONE;
         const at::Tensor &t = THPVariable_Unpack(o);
-        r->buf[i] = Ptr{t.const_data_ptr(), (int64_t)t._version()};
+        // the base buffers' contents are read anew on each forward and may be tensors made in inference mode, which have no version
+        r->buf[i] = Ptr{t.const_data_ptr(), i >= 2 ? (int64_t)t._version() : 0};
     }
     r->has_bias = a[2] != Py_None;
     if (r->has_bias) r->bias = THPVariable_Unpack(a[2]).const_data_ptr();
@@ -97,9 +100,11 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
     r->device = (int)PyLong_AsLong(a[8]);
     r->type = (int)PyLong_AsLong(a[9]);
     r->x_scratch = a[10] == Py_None ? nullptr : PyLong_AsVoidPtr(a[10]);
-    if (PyErr_Occurred()) { delete r; return nullptr; }
-    r->ws = Py_NewRef(a[4]);
-    return PyCapsule_New(r, "ortho_record", free_record);
+    if (PyErr_Occurred()) return nullptr;
+    PyObject *cap = PyCapsule_New(r.get(), "ortho_record", free_record);
+    if (!cap) return nullptr;
+    r.release()->ws = Py_NewRef(a[4]);
+    return cap;
     END_HANDLE_TH_ERRORS
 }
 

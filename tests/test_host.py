@@ -152,6 +152,21 @@ def test_swap_linear_replaces_modules_and_keeps_bias():
     assert toy.up._bound == {}
 
 
+def test_call_record_of_base_buffers_made_in_inference_mode():
+    """They have no version counter; only the CSR buffers' versions belong to a record."""
+    m = OrthoLinear(64, 32)
+    with torch.inference_mode():
+        m.base_weight.data = torch.zeros(32, 32, dtype=torch.uint8)
+        scales = torch.ones(32, dtype=torch.float16)
+    m.base_scales = scales
+    assert m.base_weight.is_inference() and m.base_scales.is_inference()
+    desc = _lib.LayerDesc()
+    rec = _lib.fast().record(ctypes.addressof(desc), m._buffers, None, True, m, 0, None, 0, 0, 0, None)
+    assert type(rec).__name__ == "PyCapsule"
+    with pytest.raises(TypeError):                            # and a bad argument is an error, not a record
+        _lib.fast().record(ctypes.addressof(desc), m._buffers, None, True, m, "x", None, 0, 0, 0, None)
+
+
 def test_kernel_status_surfaces_as_runtime_error():
     """Host side of the failure path: a non-zero status (here: a bounded device-side wait that ran out) becomes a
     RuntimeError that names the cause; no GPU is involved."""
