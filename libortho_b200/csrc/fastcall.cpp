@@ -36,6 +36,7 @@ struct Record {
     void *ws_ptr;
     int64_t ws_gen;
     PyObject *ws;                                // the scratch's owner: `gen` and `tensor`
+    PyObject *plan;                              // owner of desc.plan, or None: held, also while a launch runs without the lock
     int device;
     int type;                                    // ORTHO_B200_TYPE_* of activations and output
     void *x_scratch;                             // for activations of another type, where the kernel needs them as FP16
@@ -48,6 +49,7 @@ void free_record(PyObject *cap)
     Record *r = static_cast<Record *>(PyCapsule_GetPointer(cap, "ortho_record"));
     if (!r) { PyErr_Clear(); return; }
     Py_XDECREF(r->ws);
+    Py_XDECREF(r->plan);
     delete r;
 }
 
@@ -77,33 +79,34 @@ bool same_buffers(const Record &r, PyObject *buffers, PyObject *params)
     return t.has_storage() && t.scalar_type() == at::kFloat && t.const_data_ptr() == r.bias;
 }
 
-// record(desc_address, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, x_scratch or None) -> capsule
+// record(desc_address, plan or None, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, x_scratch or None) -> capsule
 PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 11) { PyErr_SetString(PyExc_TypeError, "record takes 11 arguments"); return nullptr; }
+    if (n != 12) { PyErr_SetString(PyExc_TypeError, "record takes 12 arguments"); return nullptr; }
     HANDLE_TH_ERRORS
     auto r = std::make_unique<Record>();
     r->desc = *static_cast<const ortho_b200_layer_desc *>(PyLong_AsVoidPtr(a[0]));
     for (int i = 0; i < 5; i++) {
-        PyObject *o = PyDict_GetItemWithError(a[1], s_buffers[i]);
+        PyObject *o = PyDict_GetItemWithError(a[2], s_buffers[i]);
         if (!o || !THPVariable_Check(o)) Py_RETURN_NONE;
         const at::Tensor &t = THPVariable_Unpack(o);
         // the base buffers' contents are read anew on each forward and may be tensors made in inference mode, which have no version
         r->buf[i] = Ptr{t.const_data_ptr(), i >= 2 ? (int64_t)t._version() : 0};
     }
-    r->has_bias = a[2] != Py_None;
-    if (r->has_bias) r->bias = THPVariable_Unpack(a[2]).const_data_ptr();
-    r->active = PyObject_IsTrue(a[3]) == 1;
-    r->ws_gen = PyLong_AsLongLong(a[5]);
-    r->ws_ptr = a[6] == Py_None ? nullptr : PyLong_AsVoidPtr(a[6]);
-    r->ws_bytes = PyLong_AsLongLong(a[7]);
-    r->device = (int)PyLong_AsLong(a[8]);
-    r->type = (int)PyLong_AsLong(a[9]);
-    r->x_scratch = a[10] == Py_None ? nullptr : PyLong_AsVoidPtr(a[10]);
+    r->has_bias = a[3] != Py_None;
+    if (r->has_bias) r->bias = THPVariable_Unpack(a[3]).const_data_ptr();
+    r->active = PyObject_IsTrue(a[4]) == 1;
+    r->ws_gen = PyLong_AsLongLong(a[6]);
+    r->ws_ptr = a[7] == Py_None ? nullptr : PyLong_AsVoidPtr(a[7]);
+    r->ws_bytes = PyLong_AsLongLong(a[8]);
+    r->device = (int)PyLong_AsLong(a[9]);
+    r->type = (int)PyLong_AsLong(a[10]);
+    r->x_scratch = a[11] == Py_None ? nullptr : PyLong_AsVoidPtr(a[11]);
     if (PyErr_Occurred()) return nullptr;
     PyObject *cap = PyCapsule_New(r.get(), "ortho_record", free_record);
     if (!cap) return nullptr;
-    r.release()->ws = Py_NewRef(a[4]);
+    r->plan = Py_NewRef(a[1]);
+    r.release()->ws = Py_NewRef(a[5]);
     return cap;
     END_HANDLE_TH_ERRORS
 }

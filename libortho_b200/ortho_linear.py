@@ -102,8 +102,9 @@ _NO_SCRATCH = _SharedWorkspace(True)
 
 class _Bound:
     """Everything about one (module, token count, stream) forward that does not change from call to call: the C
-    argument record with all buffer pointers, the plan, the workspace.  Built (and validated) once."""
-    __slots__ = ("descs", "ws", "ws_gen", "ws_ptr", "ws_bytes", "key", "fused_bias", "fast")
+    argument record with all buffer pointers, the plan (held: the record has its address), the workspace.  Built (and
+    validated) once."""
+    __slots__ = ("descs", "plan", "ws", "ws_gen", "ws_ptr", "ws_bytes", "key", "fused_bias", "fast")
 
 
 class OrthoLinear(nn.Module):
@@ -204,6 +205,7 @@ class OrthoLinear(nn.Module):
                self.ortho_row_ptr.data_ptr(), nnz, self.ortho_values._version,
                self.ortho_col_indices._version, self.ortho_row_ptr._version)
         if self._plan is None or self._plan_key != key:
+            self._bound = {}                   # records of the former plan: its buffers may come back by a `.data =`
             self._plan = _C.Plan(self.ortho_row_ptr, self.ortho_col_indices, self.ortho_values,
                                  self.in_features, self.out_features)
             self._plan_key = key
@@ -251,7 +253,7 @@ class OrthoLinear(nn.Module):
             if self.ortho_row_ptr.numel() != N + 1 or self.ortho_col_indices.numel() != nnz:
                 raise ValueError("CSR arrays have inconsistent sizes")
         b = _Bound()
-        plan = self._get_plan() if sparse else None
+        plan = b.plan = self._get_plan() if sparse else None
         b.fused_bias = (self.bias is not None and self.bias.dtype == torch.float32 and self.bias.device == dev
                         and self.bias.is_contiguous())
         descs = (_lib.LayerDesc * 1)()
@@ -285,7 +287,7 @@ class OrthoLinear(nn.Module):
         # what the native path compares and launches; not for a bias that torch has to add
         b.fast = None
         if (self.bias is None or b.fused_bias) and not (type and convert < 0):
-            b.fast = _lib.fast().record(ctypes.addressof(descs), self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
+            b.fast = _lib.fast().record(ctypes.addressof(descs), plan, self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
                                         b.ws_bytes, dev.index, type, x_scratch)
         if b.ws.shared:
             if len(self._bound) > 32:

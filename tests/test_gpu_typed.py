@@ -120,6 +120,27 @@ def test_buffers_replaced_or_edited_between_calls(M, dtype):
     assert torch.equal(y1, y0)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_a_sparse_component_that_goes_and_comes_back(dtype):
+    """By `.data =`, which changes neither the buffers' identity nor their versions: no record of the first plan is left when
+    it returns."""
+    K, N = 1024, 256
+    a, b = (wl.make_layer(K, N, 0.01, seed=s, device=DEV) for s in (1, 2))
+    m = a.to_module()
+    xs = [wl.make_input(M, K, seed=M, device=DEV).to(dtype) for M in (1, 24, 200)]
+    want = [m(x) for x in xs]
+    own = [t.data for t in (m.ortho_values, m.ortho_col_indices, m.ortho_row_ptr)]
+
+    def put(vals, col, row_ptr):
+        m.ortho_values.data, m.ortho_col_indices.data, m.ortho_row_ptr.data = vals, col, row_ptr
+    put(b.vals, b.col, b.row_ptr)
+    changed = m(xs[0])
+    assert len(m._bound) == 1 and not torch.equal(changed, want[0])
+    put(*own)
+    for x, y in zip(xs, want):
+        assert torch.equal(m(x), y)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M", [1, 40, 300])
 def test_capture_replays_on_new_activations(M, dtype):
