@@ -39,7 +39,7 @@ struct Record {
     PyObject *plan;                              // owner of desc.plan, or None: held, also while a launch runs without the lock
     int device;
     int type;                                    // ORTHO_B200_TYPE_* of activations and output
-    void *x_scratch;                             // for activations of another type, where the kernel needs them as FP16
+    bool converts;                               // activations of another type that the kernel needs as FP16
 };
 const char *kBuffers[5] = {"base_weight", "base_scales", "ortho_values", "ortho_col_indices", "ortho_row_ptr"};
 PyObject *s_buffers[5], *s_bias, *s_gen, *s_tensor, *s_handle, *s_value, *s_fast;
@@ -79,7 +79,7 @@ bool same_buffers(const Record &r, PyObject *buffers, PyObject *params)
     return t.has_storage() && t.scalar_type() == at::kFloat && t.const_data_ptr() == r.bias;
 }
 
-// record(desc_address, plan or None, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, x_scratch or None) -> capsule
+// record(desc_address, plan or None, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, converts) -> capsule
 PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 12) { PyErr_SetString(PyExc_TypeError, "record takes 12 arguments"); return nullptr; }
@@ -101,7 +101,7 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
     r->ws_bytes = PyLong_AsLongLong(a[8]);
     r->device = (int)PyLong_AsLong(a[9]);
     r->type = (int)PyLong_AsLong(a[10]);
-    r->x_scratch = a[11] == Py_None ? nullptr : PyLong_AsVoidPtr(a[11]);
+    r->converts = PyObject_IsTrue(a[11]) == 1;
     if (PyErr_Occurred()) return nullptr;
     PyObject *cap = PyCapsule_New(r.get(), "ortho_record", free_record);
     if (!cap) return nullptr;
@@ -149,7 +149,7 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (r->device != dev || r->type != type || (alpha > 0) != r->active || r->desc.N != N || !same_buffers(*r, a[1], a[2])) Py_RETURN_NONE;
     // the scratch of the record, held over the launch whatever other threads bind meanwhile
     PyObject *scratch = nullptr;
-    if (r->ws_bytes || r->x_scratch) {
+    if (r->ws_bytes) {
         scratch = PyObject_GetAttr(r->ws, s_tensor);
         PyObject *gen = scratch ? PyObject_GetAttr(r->ws, s_gen) : nullptr;
         const bool same = gen && PyLong_AsLongLong(gen) == r->ws_gen && scratch != Py_None;
@@ -169,7 +169,12 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     d.y_f16 = y.mutable_data_ptr();
     d.alpha = (float)alpha;
     const void *xp = x->const_data_ptr();
-    void *ws = r->ws_ptr, *xs = r->x_scratch;
+    at::Tensor copy;                             // back with torch's allocator, in stream order, when the call returns
+    if (r->converts) {
+        copy = at::empty({M, K}, at::TensorOptions().dtype(at::kHalf).device(x->device()));
+        if (!copy.has_storage() || copy.unsafeGetTensorImpl()->is_python_dispatch()) Py_RETURN_NONE;
+    }
+    void *ws = r->ws_ptr, *xs = r->converts ? copy.mutable_data_ptr() : nullptr;
     const int64_t ws_bytes = r->ws_bytes;
     int st;
     Py_BEGIN_ALLOW_THREADS

@@ -268,27 +268,19 @@ class OrthoLinear(nn.Module):
         d.N, d.ldy, d.reserved = N, 0, 0
         b.descs = descs
         need = self._workspace_bytes(M)
-        own, convert = (need + 255) // 256 * 256, 0          # the FP16 copy of other activations lies behind what the kernels need
-        if type:
-            d.alpha = float(self.alpha)
-            if need == 0:
-                convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, None, 0)
-            if need or convert > 0:
-                need = own + 2 * M * K
         b.ws, b.ws_gen, scratch = _SharedWorkspace.get(dev, need, stream)
         b.ws_ptr = scratch.data_ptr() if need else None
         b.ws_bytes = scratch.numel() if need else 0
-        x_scratch = None
-        if type and need:
-            b.ws_bytes = own
-            convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, b.ws_ptr, own)
-            x_scratch = b.ws_ptr + own if convert > 0 else None
+        convert = 0                            # bytes of the FP16 copy of other activations, a temporary of each call; -1: not taken
+        if type:
+            d.alpha = float(self.alpha)
+            convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, b.ws_ptr, b.ws_bytes)
         b.key = (self.alpha > 0, self._versions())
         # what the native path compares and launches; not for a bias that torch has to add
         b.fast = None
         if (self.bias is None or b.fused_bias) and not (type and convert < 0):
             b.fast = _lib.fast().record(ctypes.addressof(descs), plan, self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
-                                        b.ws_bytes, dev.index, type, x_scratch)
+                                        b.ws_bytes, dev.index, type, convert > 0)
         if b.ws.shared:
             if len(self._bound) > 32:
                 self._bound.clear()

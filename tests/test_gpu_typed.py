@@ -5,6 +5,7 @@ import torch
 
 import workloads as wl
 from libortho_b200 import _C_ops, _lib
+from libortho_b200.ortho_linear import _SharedWorkspace
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -139,6 +140,25 @@ def test_a_sparse_component_that_goes_and_comes_back(dtype):
     put(*own)
     for x, y in zip(xs, want):
         assert torch.equal(m(x), y)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_the_converted_activations_are_a_temporary_of_the_call(dtype):
+    K, N = 4096, 256
+    m = wl.make_layer(K, N, 0.01, seed=3, device=DEV).to_module()
+    side = torch.cuda.Stream()                                # with a scratch buffer of its own
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for M in (24, 400):
+            x = wl.make_input(M, K, seed=M, device=DEV)
+            want = m(x).to(dtype)
+            held = [w.tensor.numel() for (_, stream), w in _SharedWorkspace._by_stream.items() if stream == side.cuda_stream]
+            x, before = x.to(dtype), torch.cuda.memory_allocated()
+            y = m(x)
+            assert held == [w.tensor.numel() for (_, stream), w in _SharedWorkspace._by_stream.items() if stream == side.cuda_stream]
+            assert torch.cuda.memory_allocated() - before <= (y.numel() * y.element_size() + 511) // 512 * 512
+            assert torch.equal(bits(y), bits(want)) and torch.equal(bits(m(x)), bits(want))
+    side.synchronize()
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])

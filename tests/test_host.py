@@ -161,10 +161,10 @@ def test_call_record_of_base_buffers_made_in_inference_mode():
     m.base_scales = scales
     assert m.base_weight.is_inference() and m.base_scales.is_inference()
     desc = _lib.LayerDesc()
-    rec = _lib.fast().record(ctypes.addressof(desc), None, m._buffers, None, True, m, 0, None, 0, 0, 0, None)
+    rec = _lib.fast().record(ctypes.addressof(desc), None, m._buffers, None, True, m, 0, None, 0, 0, 0, False)
     assert type(rec).__name__ == "PyCapsule"
     with pytest.raises(TypeError):                            # and a bad argument is an error, not a record
-        _lib.fast().record(ctypes.addressof(desc), None, m._buffers, None, True, m, "x", None, 0, 0, 0, None)
+        _lib.fast().record(ctypes.addressof(desc), None, m._buffers, None, True, m, "x", None, 0, 0, 0, False)
 
 
 def test_kernel_status_surfaces_as_runtime_error():
