@@ -323,7 +323,9 @@ ORTHO_B200_API int ortho_b200_csr_fill_marks(const float *w_ortho, int64_t N, in
  * An output may be W itself.  h_inv_diag is the FP32 [K] diagonal.  scratch:
  * ortho_b200_sieve_scratch_bytes(N) bytes, 256-byte aligned.  K a multiple of 4, pointers 16-byte aligned.
  * With ortho_b200_sieve_onepass_scratch_bytes(N, K) bytes of scratch the top-k rule takes one pass over W and a short list
- * where it can (outputs apart from each other and from the inputs, keep_top_k up to 4 % of N * K); the results are the same bits.
+ * where it can: 10 million weights or more in rows that are not cut (twice as many rows as SMs), outputs apart from each other and
+ * from the inputs, keep_top_k up to 4 % of N * K.  The results are the same bits.  For sizes that it does not take the query answers
+ * ortho_b200_sieve_scratch_bytes(N).
  * The outputs feed ortho_b200_pack_base / ortho_b200_csr_count / ortho_b200_csr_fill.
  * ------------------------------------------------------------------------------------------- */
 ORTHO_B200_API int64_t ortho_b200_sieve_scratch_bytes(int64_t N);

@@ -410,8 +410,16 @@ def hessian_sieve(weight: torch.Tensor, h_inv_diag: torch.Tensor, curvature_thre
     if h.dim() != 1 or h.numel() != K:
         raise ValueError("h_inv_diag must hold one entry per input feature")
     wb, wo = torch.empty_like(w), torch.empty_like(w)
-    need = int(_lib.lib().ortho_b200_sieve_onepass_scratch_bytes(N, K) if keep_top_k > 0 else _lib.lib().ortho_b200_sieve_scratch_bytes(N))
-    scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    need = small = int(_lib.lib().ortho_b200_sieve_scratch_bytes(N))
+    if 0 < keep_top_k <= N * K // 25:          # room for the candidates of the one-pass form (half a byte a weight)
+        need = int(_lib.lib().ortho_b200_sieve_onepass_scratch_bytes(N, K))
+    try:
+        scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        if need == small:
+            raise
+        need = small
+        scratch = torch.empty(need, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
         st = _lib.lib().ortho_b200_sieve(w.data_ptr(), h.data_ptr(), N, K, float(curvature_thresh), int(keep_top_k),
                                         wb.data_ptr(), wo.data_ptr(), scratch.data_ptr(), need,

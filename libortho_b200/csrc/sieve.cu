@@ -562,10 +562,14 @@ static int launch_onepass(const float *w, const float *h, int64_t N, int K, floa
 
 // one-pass form: state and the list of candidates, behind the other form's scratch
 static unsigned candidate_cap(int64_t N, int64_t K) { return (unsigned)(N * K / 16 > 65536 ? N * K / 16 : 65536); }
+// Whole rows; below 10 million weights its ten launches cost as much as the passes: 2048 x 1024 93 us against 84, whole layers of
+// 8.6 million 209 / 202, 10.2 million 217 / 238
+static bool onepass_shape(int64_t N, int64_t K) { return N <= 0xffffffffLL / K && N * K >= 10000000 && sieve_grid(N, K).y == 1; }
 extern "C" int64_t ortho_b200_sieve_scratch_bytes(int64_t N);
 extern "C" int64_t ortho_b200_sieve_onepass_scratch_bytes(int64_t N, int64_t K)
 {
-    if (N <= 0 || K <= 0 || K > 0x7fffffffLL || N > 0xffffffffLL / K) return N > 0 && K > 0 ? ortho_b200_sieve_scratch_bytes(N) : -1;
+    if (N <= 0 || K <= 0) return -1;
+    if (K > 0x7fffffffLL || !onepass_shape(N, K)) return ortho_b200_sieve_scratch_bytes(N);
     return (ortho_b200_sieve_scratch_bytes(N) + 255) / 256 * 256 + (int64_t)(sizeof(OnePass) + 255) / 256 * 256 + (int64_t)candidate_cap(N, K) * (int64_t)sizeof(Candidate);
 }
 
@@ -610,9 +614,7 @@ extern "C" int ortho_b200_sieve(const float *w, const float *h_inv_diag, int64_t
     }
     // One pass where the list can hold what a bracket of the k-th score holds (half of k and two bins' worth) and W outlives
     // the pass
-    // (below 10 million weights its ten launches cost as much as the passes: 2048 x 1024 93 us against 84, whole layers of 8.6 million 209 / 202,
-    // 10.2 million 217 / 238)
-    const bool onepass = k && !cut && N * K >= 10000000 && outs_apart && base_apart && ortho_apart && N <= 0xffffffffLL / K && k <= (unsigned long long)(N * K / 25) &&
+    const bool onepass = k && onepass_shape(N, K) && outs_apart && base_apart && ortho_apart && k <= (unsigned long long)(N * K / 25) &&
                          scratch_bytes >= ortho_b200_sieve_onepass_scratch_bytes(N, K);
     if (onepass) {
         OnePass *op = reinterpret_cast<OnePass *>(reinterpret_cast<unsigned char *>(scratch) + (ortho_b200_sieve_scratch_bytes(N) + 255) / 256 * 256);

@@ -152,6 +152,15 @@ def test_swap_linear_replaces_modules_and_keeps_bias():
     assert toy.up._bound == {}
 
 
+def test_sieve_asks_for_the_larger_scratch_only_where_it_is_used():
+    l = _lib.lib()
+    small, onepass = l.ortho_b200_sieve_scratch_bytes, l.ortho_b200_sieve_onepass_scratch_bytes
+    assert onepass(11008, 4096) - small(11008) >= 11008 * 4096 // 16 * 8      # a candidate for every 16 weights
+    for N, K in ((2048, 4096), (9999, 1000), (64, 1 << 20), (1, 1 << 24)):    # fewer than 10 million weights; rows that are cut
+        assert onepass(N, K) == small(N)
+    assert onepass(0, 4096) == -1 and onepass(16, 0) == -1
+
+
 def test_call_record_of_base_buffers_made_in_inference_mode():
     """They have no version counter; only the CSR buffers' versions belong to a record."""
     m = OrthoLinear(64, 32)
