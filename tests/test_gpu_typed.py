@@ -150,10 +150,10 @@ def test_the_converted_activations_are_a_temporary_of_the_call(dtype):
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
         for M in (24, 400):
-            x = wl.make_input(M, K, seed=M, device=DEV)
-            want = m(x).to(dtype)
+            x = wl.make_input(M, K, seed=M, device=DEV).to(dtype)
+            want = m(x.to(torch.float16)).to(dtype)
             held = [w.tensor.numel() for (_, stream), w in _SharedWorkspace._by_stream.items() if stream == side.cuda_stream]
-            x, before = x.to(dtype), torch.cuda.memory_allocated()
+            before = torch.cuda.memory_allocated()
             y = m(x)
             assert held == [w.tensor.numel() for (_, stream), w in _SharedWorkspace._by_stream.items() if stream == side.cuda_stream]
             assert torch.cuda.memory_allocated() - before <= (y.numel() * y.element_size() + 511) // 512 * 512
