@@ -132,6 +132,12 @@ ORTHO_B200_API int ortho_b200_dequant_dump(const void *q_weight, const void *q_s
  * is bit-identical to the base-only result (src/ortho.c:343 and the reference null test,
  * tests/benchmark_null_test.c:127-131).  Borrowed pointers are only used until the launched
  * kernels finish.
+ *
+ * Weights, scales, CSR arrays and plan are constants of the layer: with up to 128 tokens a forward (every entry below) may read
+ * them before the kernel in front of it on the stream has ended, where that kernel lets its successor start early (one that
+ * issues griddepcontrol.launch_dependents / cudaTriggerProgrammaticLaunchCompletion itself).  Ordinary kernels and copies that
+ * write them are waited for as always; a kernel that triggers early must not write them behind its trigger, or has to be
+ * followed by an ordinary launch.  Activations, outputs and workspace are never touched ahead.
  * ------------------------------------------------------------------------------------------- */
 #define ORTHO_B200_DECODE_MAX_M 64
 
@@ -191,9 +197,7 @@ ORTHO_B200_API int ortho_b200_forward_multi(const ortho_b200_layer_desc *layers,
 /* The forward of one layer with activations and outputs of another type (a model in BF16 or FP32): x_type and y_type are one of
  * ORTHO_B200_TYPE_*, and the result has the bits of converting x to FP16, the ordinary forward and converting y.
  * typed_scratch_bytes: -1 where the call's kernel does not take other types (convert around the ordinary forward), else the size of
- * x_scratch (16-byte aligned; 0 = none needed) for the same layer, sizes and workspace; y_f16 of the record is not looked at.
- * Weights and window lists may be read before the work that precedes the call on its stream has finished when that work allows it
- * (programmatic dependent launch, as in every forward): they are constants of the layer. */
+ * x_scratch (16-byte aligned; 0 = none needed) for the same layer, sizes and workspace; y_f16 of the record is not looked at. */
 #define ORTHO_B200_TYPE_F16 0
 #define ORTHO_B200_TYPE_BF16 1
 #define ORTHO_B200_TYPE_F32 2

@@ -183,10 +183,17 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
     // and window lists, constants of the layer, are loaded and converted at once; the token producer and the epilogue wait.
     // Behind the long rows' pre-pass (an ordinary launch, so all earlier work is done) only the epilogue does.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // The roles that run ahead come to wait for units that the predecessor's end holds up, and it may take any time: a wait that runs
+    // out starts anew behind that end (here, off the loops' path; a wait for the predecessor inside them cost 1-2 %).
     bool dead = false;
     auto wait = [&](uint64_t *bar, uint32_t parity) {
         if (mbar_try_wait(bar, parity) || dead) return;
-        if (!mbar_wait(bar, parity, 1u << 24)) { dead = true; atomicExch(p.status, 1); }
+        for (int bound = 0; bound < 2; bound++) {
+            if (mbar_wait(bar, parity, 1u << 24)) return;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        dead = true;
+        atomicExch(p.status, 1);
     };
 
     if (warp == 0) {
