@@ -365,23 +365,31 @@ Route route_of(const FwdArgs &a)
 }
 
 // Whether layers of up to 16 tokens that share their activations run as one streaming launch although mid.cu would take some of
-// them by themselves.  Estimates in us, from the layers above and groups of them (one B200, 0.3 % ortho, weights from HBM; W =
-// millions of weights): a launch of mid.cu 9.3 + 0.16 W, a streaming launch 5 + r W, where r depends on the activation slab
-// and the token count; without a sparse term the slopes are two thirds.  One streaming launch / a launch per layer, measured:
-//   8192->8192 + 2 x 1024:  8 tokens 24.8 / 34.7, 12: 32.4 / 36.5, 16: 44.1 / 36.8;   3 x 5120->5120:  9: 26.6 / 39.6, 16: 42.2 / 39.4
-//   3 x 8192->8192:  8: 53.8 / 58.4, 9: 63.3 / 58.3, 16: 99 / 59;   2 x 4096->11008:  9: 28.8 / 30.8, 12: 29.3 / 31.2, 16: 32.8 / 31.4
-//   2 x 8192->28672:  8: 118 / 90, 16: 221 / 90;   2 x 28672->1024:  9: 31.9 / 34.6, 16: 33.9 / 35.2
+// them by themselves.  Estimates in us, from the layers above and groups of them (one B200, 0.3 % ortho, weights rotating over more
+// than L2; W = millions of weights): a launch of mid.cu 7 + 0.15 W, base-only 5.7 + 0.11 W, a streaming launch 5 + r W, where r
+// depends on the activation slab and the token count, base-only two thirds of it.  Where both come out within some 5 % (2 x 4096->11008
+// at 9 and 12 tokens) the group stays one launch.  One streaming launch / a launch per layer, measured; base-only:
+//   8192->8192 + 2 x 1024:  8 tokens 24.3 / 32.3; 18.8 / 25.8,  12: 31.8 / 34.3; 24.7 / 27.0,  16: 43.5 / 35.1; 33.1 / 26.8
+//   3 x 5120->5120:   12: 27.4 / 33.6; 21.8 / 25.8,  16: 41.4 / 33.8; 32.0 / 26.7
+//   3 x 8192->8192:    8: 51.7 / 52.2; 38.7 / 39.7,   9: 61.2 / 50.9; 47.2 / 39.8,  16: 97 / 52; 75 / 40
+//   2 x 4096->11008:   9: 28.0 / 26.5; 20.3 / 21.7,  12: 28.5 / 27.2; 20.9 / 21.8,  16: 31.9 / 27.3; 23.6 / 22.9
+//   2 x 4096->8192:   12: 23.1 / 25.5; 17.2 / 19.1,  16: 26.0 / 25.8; 19.5 / 20.1
+//   3 x 4096->4096:   16: 20.8 / 27.0; 15.8 / 20.9;   4096->4096 + 2 x 1024:  16: 14.6 / 25.8; 11.7 / 20.3
+//   2 x 8192->2048:   12: 16.2 / 18.1; 12.9 / 14.7,  16: 21.4 / 18.0; 17.0 / 14.5
+//   2 x 8192->28672:   3: base-only 55.1 / 60.5,  5: 57.6 / 63.0,  6: 98 / 82,  8: 114 / 83; 83 / 63
+//   2 x 28672->1024:   9: 31.7 / 27.9; 22.9 / 22.4,  16: 33.5 / 28.1; 23.6 / 22.2
 bool group_streams(const FwdArgs *a, const Route *route, int n)
 {
     const int64_t M = a[0].M, slab = 2 * M * a[0].K;
     float r;
-    if (M > 8) r = slab > (200 << 10) ? 0.44f : M <= 12 ? 0.31f : slab > (150 << 10) ? 0.47f : 0.34f;
-    else r = slab > (200 << 10) ? 0.32f : slab > (100 << 10) ? 0.25f : 0.21f;
+    if (M > 12) r = slab > (200 << 10) ? 0.46f : slab > (150 << 10) ? 0.47f : 0.30f;
+    else if (M > 8) r = slab > (200 << 10) ? 0.46f : slab > (150 << 10) ? 0.31f : slab > (100 << 10) ? 0.27f : 0.245f;
+    else r = slab > (200 << 10) ? 0.32f : slab > (100 << 10) ? 0.225f : M > 5 ? 0.20f : 0.15f;
     float one = 5.f, apart = 0.f;
     for (int l = 0; l < n; l++) {
-        const float w = 1e-6f * (float)(a[l].N * a[l].K) * (a[l].has_ortho ? 1.f : 0.67f);
-        one += r * w;
-        apart += route[l] == kRouteMid ? 9.3f + 0.16f * w : 5.f + r * w;
+        const float w = 1e-6f * (float)(a[l].N * a[l].K), streams = r * w * (a[l].has_ortho ? 1.f : 0.66f);
+        one += streams;
+        apart += route[l] != kRouteMid ? 5.f + streams : a[l].has_ortho ? 7.f + 0.15f * w : 5.7f + 0.11f * w;
     }
     return one <= apart;
 }
