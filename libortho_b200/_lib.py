@@ -162,11 +162,14 @@ def fast():
     global _fast
     if _fast is None:
         l = lib()
+        advice = "libortho_b200/_fastcall.so is missing or does not fit the installed torch. Build it with `python -m libortho_b200.build`."
         try:
             from . import _fastcall as f
         except ImportError as e:
-            raise ImportError("libortho_b200/_fastcall.so is missing or does not fit the installed torch. "
-                              "Build it with `python -m libortho_b200.build`.") from e
+            raise ImportError(advice) from e
+        import torch
+        if getattr(f, "torch_version", None) != torch.__version__:
+            raise ImportError(advice)
         f.set_library(*(ctypes.cast(fn, ctypes.c_void_p).value for fn in
                         (l.ortho_b200_forward_multi, l.ortho_b200_multi_workspace_bytes, l.ortho_b200_forward_typed)))
         _fast = f

@@ -3,7 +3,9 @@
     python -m libortho_b200.build [--force] [--verbose]
 
 Takes the place of the reference's ``setup.py`` CUDAExtension build (``setup.py:112-130``):
-one target architecture, ``-O3 -lineinfo``, static CUDA runtime, no Python headers.
+one target architecture, ``-O3 -lineinfo``, static CUDA runtime, no Python headers.  The forward's host path
+``_fastcall.so`` is a CPython extension beside it, compiled against the installed torch and rebuilt when that
+or the interpreter changes.
 """
 from __future__ import annotations
 
@@ -24,6 +26,7 @@ NVCC_FLAGS = [
 # the forward's host path as a CPython extension (csrc/fastcall.cpp), compiled against the installed torch
 FAST_SOURCE = os.path.join(CSRC, "fastcall.cpp")
 FAST_PATH = os.path.join(HERE, "_fastcall.so")
+FAST_STAMP = os.path.join(HERE, "build", "fastcall.txt")       # what the extension was compiled against
 
 
 def _nvcc() -> str:
@@ -39,9 +42,27 @@ def _deps() -> list:
     return out
 
 
-def build_fast(force: bool = False) -> str:
+def _fast_against() -> str:
+    """What ties the extension to the installation: torch's version and place, the interpreter's ABI."""
+    import sysconfig
+
+    import torch
+    return "\n".join((torch.__version__, os.path.dirname(torch.__file__), str(sysconfig.get_config_var("SOABI"))))
+
+
+def needs_build_fast() -> bool:
     deps = [FAST_SOURCE, os.path.join(INCLUDE, "ortho_b200.h")]
-    if not force and os.path.exists(FAST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(FAST_PATH) for d in deps):
+    if not os.path.exists(FAST_PATH) or any(os.path.getmtime(d) > os.path.getmtime(FAST_PATH) for d in deps):
+        return True
+    try:
+        with open(FAST_STAMP) as f:
+            return f.read() != _fast_against()
+    except FileNotFoundError:
+        return True
+
+
+def build_fast(force: bool = False) -> str:
+    if not force and not needs_build_fast():
         return FAST_PATH
     import sysconfig
 
@@ -51,10 +72,14 @@ def build_fast(force: bool = False) -> str:
     inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include"), INCLUDE]
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DORTHO_TORCH_VERSION="{torch.__version__}"',
            *[f"-I{d}" for d in inc], FAST_SOURCE, "-o", FAST_PATH, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ltorch"]
     out = subprocess.run(cmd, capture_output=True, text=True)
     if out.returncode != 0:
         raise RuntimeError("g++ failed on fastcall.cpp:\n" + out.stdout + out.stderr)
+    os.makedirs(os.path.dirname(FAST_STAMP), exist_ok=True)
+    with open(FAST_STAMP, "w") as f:
+        f.write(_fast_against())
     return FAST_PATH
 
 

@@ -302,5 +302,8 @@ PyMODINIT_FUNC PyInit__fastcall(void)
     s_handle = PyUnicode_InternFromString("handle");
     s_value = PyUnicode_InternFromString("value");
     s_fast = PyUnicode_InternFromString("fast");
-    return PyModule_Create(&module_def);
+    PyObject *m = PyModule_Create(&module_def);
+    // the torch it was compiled against: a module built for another one is not to be used
+    if (m && PyModule_AddStringConstant(m, "torch_version", ORTHO_TORCH_VERSION) < 0) { Py_DECREF(m); return nullptr; }
+    return m;
 }

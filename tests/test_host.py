@@ -176,6 +176,19 @@ def test_call_record_of_base_buffers_made_in_inference_mode():
         _lib.fast().record(ctypes.addressof(desc), None, m._buffers, None, True, m, "x", None, 0, 0, 0, False)
 
 
+def test_host_path_built_for_another_torch_is_refused_and_built_again(monkeypatch):
+    from libortho_b200 import build
+    build.build_fast()
+    assert not build.needs_build_fast()
+    monkeypatch.setattr(_lib, "_fast", None)
+    assert _lib.fast().torch_version == torch.__version__
+    monkeypatch.setattr(_lib, "_fast", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    assert build.needs_build_fast()
+    with pytest.raises(ImportError, match="libortho_b200.build"):
+        _lib.fast()
+
+
 def test_kernel_status_surfaces_as_runtime_error():
     """Host side of the failure path: a non-zero status (here: a bounded device-side wait that ran out) becomes a
     RuntimeError that names the cause; no GPU is involved."""
