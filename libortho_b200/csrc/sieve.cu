@@ -23,6 +23,7 @@
 // counts the scores above the bracket and lists those inside it, a radix select over that short list finds the threshold, and the
 // listed residuals above it are written.  When the bracket turns out not to hold the k-th score, or the list overflows, the passes
 // above run behind it (they look at a flag), so the result never depends on the sample.
+#include <cstddef>
 #include <cstring>
 
 #include "common.cuh"
@@ -80,6 +81,7 @@ struct OnePass {
     unsigned long long above, krem;
     float threshold;
 };
+static_assert(offsetof(OnePass, ok) == 3 * kBins0 * 4 + 40, "the tests read it in the scratch, behind the other form's");
 struct Candidate { uint32_t at, key; };          // flat position, key
 
 // Adds the CTA's counts h[BINS] to the global ones; true in the last CTA to do so.  Called by all 256 threads.
