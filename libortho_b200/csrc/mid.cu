@@ -83,8 +83,8 @@ constexpr int EPI_WARPS = 4;
 constexpr int XPROD_WARP = EPI_WARP0 + EPI_WARPS;   // token tiles have a producer of their own: the packed weights run ahead of them
 constexpr int SCAT_WARP0 = XPROD_WARP + 1;
 constexpr int SCAT_WARPS = 8;           // two sets of four that take the units in turn; a warp of a set has 32 rows of the tile
-template <bool SPARSE> constexpr int kIssue2Warp = SCAT_WARP0 + (SPARSE ? SCAT_WARPS : 0);    // the second MMA issuer
-template <bool SPARSE> constexpr int kWarps = kIssue2Warp<SPARSE> + 1;
+template <bool SPARSE> constexpr int kIssue2Warp = SCAT_WARP0 + (SPARSE ? SCAT_WARPS : 0);    // the second MMA issuer, where there are two
+template <bool SPARSE, int ISSUERS> constexpr int kWarps = kIssue2Warp<SPARSE> + ISSUERS - 1;
 constexpr int TMEM_COLS = 512;
 constexpr int kTwoIssuers = 64, kTwoIssuersSparse = 32;      // two issuers up to this many columns of D (with more, shared
                                         // memory does not hold four stages with their sparse tiles)
@@ -99,7 +99,7 @@ struct Params {
     int nt;                     // token columns of an MMA: M rounded up to 16
     int nt32;                   // nt rounded up to 32: columns kept for D, and for E behind it
     int nacc, acc_cols;         // accumulators (2 where tensor memory allows) and the columns of one
-    int issuers;                // threads that issue MMAs, in turns; each has accumulators of its own
+    int issuers;                // threads that issue MMAs, in turns, each with accumulators of its own (host side: ISSUERS)
     int xtile;                  // bytes of a token tile (nt x 128); a stage holds two
     int nst;                    // stages: a unit's converted weights and tokens
     int wst;                    // packed-weight slots
@@ -145,9 +145,11 @@ struct Pieces {
 }  // namespace md
 
 // SPARSE: the entries of an ordered plan are contracted from the scattered tiles; at most 4 stages then.  TYPED: y is of another type
-// than FP16 (an instantiation of its own: the branch cost the others 1-2 %).
-template <bool SPARSE, bool TYPED>
-__global__ void __launch_bounds__(md::kWarps<SPARSE> * 32, 1)
+// than FP16 (an instantiation of its own: the branch cost the others 1-2 %).  ISSUERS: threads that issue MMAs; with the number as a
+// parameter of the launch, calls of one issuer paid for the second one's code: 4096->22016 with 0.5 % at 80 / 96 / 128 tokens 35.0 / 37.9 /
+// 45.5 us against 34.5 / 37.3 / 44.8, 4096->4096 at 64 / 128 tokens 12.5 / 16.6 against 12.2 / 16.3.
+template <bool SPARSE, bool TYPED, int ISSUERS>
+__global__ void __launch_bounds__(md::kWarps<SPARSE, ISSUERS> * 32, 1)
 mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const md::Params p)
 {
     using namespace md;
@@ -168,8 +170,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         for (int s = 0; s < WST_MAX; s++) { mbar_init(&sm->w_full[s], 1); mbar_init(&sm->w_empty[s], 4); }
         // full: the four warps of a converter group, the token producer with its bytes, a set of scatter warps
         for (int s = 0; s < ST_MAX; s++) { mbar_init(&sm->full[s], 5 + (SPARSE ? 4 : 0)); mbar_init(&sm->empty[s], 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(&sm->d_full[s], (uint32_t)p.issuers); mbar_init(&sm->d_empty[s], EPI_WARPS); }
-        mbar_init(&sm->all_done, (uint32_t)p.issuers);
+        for (int s = 0; s < 2; s++) { mbar_init(&sm->d_full[s], ISSUERS); mbar_init(&sm->d_empty[s], EPI_WARPS); }
+        mbar_init(&sm->all_done, ISSUERS);
         fence_mbar_init();
         prefetch_tensormap(&xmap);
         prefetch_tensormap(&wmap);
@@ -184,16 +186,17 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
     // Behind the long rows' pre-pass (an ordinary launch, so all earlier work is done) only the epilogue does.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // The roles that run ahead come to wait for units that the predecessor's end holds up, and it may take any time: a wait that runs
-    // out starts anew behind that end (here, off the loops' path; a wait for the predecessor inside them cost 1-2 %).
+    // out starts anew behind that end (here, off the roles' loops: a wait for the predecessor inside them cost 1-2 %).
     bool dead = false;
     auto wait = [&](uint64_t *bar, uint32_t parity) {
         if (mbar_try_wait(bar, parity) || dead) return;
-        for (int bound = 0; bound < 2; bound++) {
-            if (mbar_wait(bar, parity, 1u << 24)) return;
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll 1
+        for (uint32_t i = 0; !mbar_try_wait(bar, parity); i++) {
+            if ((i & 0xFFFFFFu) == 0xFFFFFFu) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+                if (i >> 24) { dead = true; atomicExch(p.status, 1); return; }       // the second time
+            }
         }
-        dead = true;
-        atomicExch(p.status, 1);
     };
 
     if (warp == 0) {
@@ -225,7 +228,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (++kp == p.kpairs) kp = 0;
             }
         }
-    } else if (warp == 1 || warp == kIssue2Warp<SPARSE>) {
+    } else if (warp == 1 || (ISSUERS == 2 && warp == kIssue2Warp<SPARSE>)) {
         // ================= MMA issuers =================
         // A ready mbarrier takes this one thread 60-100 cycles to see and a commit 35-60: with a wait each for tokens
         // and weights and two commits per 64 k the loop took 490 cycles per k block whatever the token count.  Hence one
@@ -235,9 +238,9 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         // of 130 (450).  (One thread for D and one for E: slower than one for both.  A loop that the whole warp runs, with an
         // elected lane for the MMAs alone: 8192->57344 at 32 tokens 65 us against 60.)  The number of stages is even then, so that a
         // stage is always the same thread's and its waits stay within one phase.
-        const int who = warp == 1 ? 0 : 1;
-        if (who < p.issuers && elect_one()) {
-            const int step = p.issuers;
+        const int who = ISSUERS == 1 || warp == 1 ? 0 : 1;
+        if (elect_one()) {
+            constexpr int step = ISSUERS;
             const uint32_t idesc = umma_idesc_f16(TN, p.nt);
             const uint64_t bdesc0 = umma_desc_sw128(smem_u32(xs)), sdesc0 = umma_desc_sw128(smem_u32(ss));
             const uint32_t a_tmem = tmem + (uint32_t)(p.nacc * p.acc_cols);
@@ -286,7 +289,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             }
             umma_commit(&sm->all_done);
         }
-    } else if (SPARSE && warp >= SCAT_WARP0 && warp < SCAT_WARP0 + SCAT_WARPS) {
+    } else if (SPARSE && warp >= SCAT_WARP0) {
         // ================= scatter: the unit's sparse entries -> zeroed FP16 tile in shared memory (A operand) =================
         // A warp's loop is a chain of dependent instructions, so the entries come with their place in the tile worked out,
         // are fetched a turn ahead (their extent a turn before that), and stay in registers until they are taken out again.
@@ -429,8 +432,8 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             }
             // with two issuers: the accumulators that have been written (a piece of one unit fills one thread's)
             const uint32_t own_cols = (uint32_t)((SPARSE ? 2 : 1) * p.nt32);
-            const bool both = p.issuers == 2 && pc.kp1 - pc.kp0 > 1;
-            const uint32_t d_off = p.issuers == 2 && !both && ((pos - r_begin) & 1) ? own_cols : 0u;
+            const bool both = ISSUERS == 2 && pc.kp1 - pc.kp0 > 1;
+            const uint32_t d_off = ISSUERS == 2 && !both && ((pos - r_begin) & 1) ? own_cols : 0u;
             pos += pc.kp1 - pc.kp0;
             float sc = 0.f, bs = 0.f;
             int li = -1;                                 // this row's index among the plan's long rows
@@ -778,8 +781,8 @@ int launch_mid(const FwdArgs &a)
         p.o = o; p.has_ortho = 1;
     }
     // Tensor memory: accumulators D (and E behind it), then the converted stages.  Shared memory: token stages and sparse
-    // tiles of the same number, the rest for packed weights (8 KB slots): 64 KB or more in flight per SM where the
-    // kernel runs near HBM's pace, less only for many tokens, where the MMAs are the bound.
+    // tiles of the same number, the rest for packed weights (8 KB slots): 64 KB or more in flight per SM, but 48 KB with entries at
+    // 33-48 tokens and 40-56 KB above 64, where a stage with its sparse tiles is worth more than a slot.
     p.nt32 = (p.nt + 31) / 32 * 32;
     p.issuers = p.nt32 <= (sparse ? kTwoIssuersSparse : kTwoIssuers) ? 2 : 1;
     p.acc_cols = (sparse ? 2 : 1) * p.issuers * p.nt32;
@@ -788,6 +791,10 @@ int launch_mid(const FwdArgs &a)
     if (p.nst > (sparse ? ST_SPARSE_MAX : ST_MAX)) p.nst = sparse ? ST_SPARSE_MAX : ST_MAX;
     // The issuers, and the two sets of scatter warps, take turns: even numbers of stages then, and of weight slots.  Above 64 tokens,
     // where shared memory holds three stages, three and one set are better than two and two (28672->8192 at 100: 73 us against 77).
+    // With entries at 33-48 tokens four stages, two converter groups and six slots against three, three and eleven (one set): 8192->10240
+    // at 33 / 48 22.8 / 23.0 us against 25.9 / 25.8, 4096->22016 at 48 25.5 / 27.5, 28672->8192 at 48 58.6 / 64.7; at 49-64 two, two and
+    // sixteen against three, three and ten: 8192->10240 at 49 / 64 25.8 / 27.9 against 26.9 / 28.8, 28672->8192 at 64 66 / 70; at
+    // 113-128, two stages, one set instead of two makes no difference (4096->22016 at 128 45.2 / 45.4).
     const int down = p.issuers == 2 || (sparse && p.nt <= 64) ? 2 : 1;
     const int nst_max = p.nst - p.nst % down;
     for (p.groups = MAX_GROUPS;; p.groups -= down) {         // most groups first, then most stages, by the rule above MAX_GROUPS
@@ -816,7 +823,8 @@ int launch_mid(const FwdArgs &a)
     }
     static bool attr_set[kMaxDevices] = {};
     if (!attr_set[dev]) {
-        for (auto k : {mid_kernel<false, false>, mid_kernel<true, false>, mid_kernel<false, true>, mid_kernel<true, true>})
+        for (auto k : {mid_kernel<false, false, 1>, mid_kernel<true, false, 1>, mid_kernel<false, true, 1>, mid_kernel<true, true, 1>,
+                       mid_kernel<false, false, 2>, mid_kernel<true, false, 2>, mid_kernel<false, true, 2>, mid_kernel<true, true, 2>})
             OB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
         attr_set[dev] = true;
     }
@@ -837,7 +845,7 @@ int launch_mid(const FwdArgs &a)
     p.tag = next_launch_tag();
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3((sparse ? kWarps<true> : kWarps<false>) * 32); cfg.dynamicSmemBytes = kSmemBytes; cfg.stream = a.stream;
+    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3((unsigned)((sparse ? kWarps<true, 1> : kWarps<false, 1>) + p.issuers - 1) * 32); cfg.dynamicSmemBytes = kSmemBytes; cfg.stream = a.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -848,8 +856,10 @@ int launch_mid(const FwdArgs &a)
         if (st != ORTHO_B200_OK) return st;
     }
     const bool typed = p.y_type != kTypeF16;
-    OB_CUDA(cudaLaunchKernelEx(&cfg, sparse ? (typed ? mid_kernel<true, true> : mid_kernel<true, false>)
-                                            : (typed ? mid_kernel<false, true> : mid_kernel<false, false>), xmap, wmap, p));
+    auto pick = [&](auto one, auto two) { return p.issuers == 2 ? two : one; };
+    auto kern = sparse ? (typed ? pick(mid_kernel<true, true, 1>, mid_kernel<true, true, 2>) : pick(mid_kernel<true, false, 1>, mid_kernel<true, false, 2>))
+                       : (typed ? pick(mid_kernel<false, true, 1>, mid_kernel<false, true, 2>) : pick(mid_kernel<false, false, 1>, mid_kernel<false, false, 2>));
+    OB_CUDA(cudaLaunchKernelEx(&cfg, kern, xmap, wmap, p));
     count_launch();
     return ORTHO_B200_OK;
 }
