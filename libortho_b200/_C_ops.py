@@ -410,12 +410,13 @@ def hessian_sieve(weight: torch.Tensor, h_inv_diag: torch.Tensor, curvature_thre
     if h.dim() != 1 or h.numel() != K:
         raise ValueError("h_inv_diag must hold one entry per input feature")
     wb, wo = torch.empty_like(w), torch.empty_like(w)
-    need = small = int(_lib.lib().ortho_b200_sieve_scratch_bytes(N))
-    if 0 < keep_top_k <= N * K // 25:          # room for the candidates of the one-pass form (half a byte a weight)
-        need = int(_lib.lib().ortho_b200_sieve_onepass_scratch_bytes(N, K))
+    L = _lib.lib()
+    # with room for the candidates of the one-pass form (half a byte a weight) where that may run
+    need = int(L.ortho_b200_sieve_onepass_scratch_bytes(N, K) if 0 < keep_top_k <= N * K // 25 else L.ortho_b200_sieve_scratch_bytes(N))
     try:
         scratch = torch.empty(need, dtype=torch.uint8, device=dev)
     except torch.OutOfMemoryError:
+        small = int(L.ortho_b200_sieve_scratch_bytes(N))
         if need == small:
             raise
         need = small
