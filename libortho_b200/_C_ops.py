@@ -379,15 +379,21 @@ def pack_ortho_csr(w_ortho: torch.Tensor):
     N, K = w.shape
     dev = w.device
     row_ptr = torch.empty(N + 1, dtype=torch.int32, device=dev)
-    marks = torch.empty(N * ((K + 127) // 128), 4, dtype=torch.int32, device=dev)
+    try:
+        marks = torch.empty(N * ((K + 127) // 128), 4, dtype=torch.int32, device=dev)
+    except torch.OutOfMemoryError:             # a bit a weight: without them W is read twice
+        marks = None
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
-        _lib.check(_lib.lib().ortho_b200_csr_count_marks(w.data_ptr(), N, K, row_ptr.data_ptr(), marks.data_ptr(), stream),
-                   "ortho_b200_csr_count_marks")
+        if marks is not None:
+            _lib.check(_lib.lib().ortho_b200_csr_count_marks(w.data_ptr(), N, K, row_ptr.data_ptr(), marks.data_ptr(), stream),
+                       "ortho_b200_csr_count_marks")
+        else:
+            _lib.check(_lib.lib().ortho_b200_csr_count(w.data_ptr(), N, K, row_ptr.data_ptr(), stream), "ortho_b200_csr_count")
         nnz = int(row_ptr[N].item())
         col = torch.empty(nnz, dtype=torch.int32, device=dev)
         val = torch.empty(nnz, dtype=torch.float16, device=dev)
-        if nnz > N * K // 16:                  # many entries: whole rows at a time
+        if nnz and (marks is None or nnz > N * K // 16):                  # many entries: whole rows at a time
             _lib.check(_lib.lib().ortho_b200_csr_fill(w.data_ptr(), N, K, row_ptr.data_ptr(), col.data_ptr(), val.data_ptr(),
                                                      stream), "ortho_b200_csr_fill")
         elif nnz:
