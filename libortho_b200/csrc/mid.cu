@@ -11,13 +11,15 @@
 // a shared-memory B tile of 256 rows) spent 512 cycles of tensor pipe per 256 x 64 weights whatever the token count
 // and 4 bytes of shared-memory traffic per weight.
 // What bounds it, by the counters of one launch on 8192->10240 at 32 tokens with 0.3 % entries (base-only): no pipe is full.  Of
-// the active cycles the integer pipe is busy in 43 % (44), the issue slots in 48 % (47), the tensor pipe in 23 % (15), HBM in
-// 19 % (24) of the whole time; a unit's MMAs take some 450 cycles to go through (8 from shared memory at 40, 8 at 16), 40 % of the active cycles.
+// the active cycles the integer pipe is busy in 49 % (48), the issue slots in 59 % (54), the tensor pipe in 26 % (16), HBM in
+// 20 % (24) of the whole time; a unit's MMAs take some 450 cycles to go through (8 from shared memory at 40, 8 at 16), 45 % of the active cycles.
 // The rest is ramp, the waits between the warp roles and the collecting of cut tiles.
 // One B200, us, base-only / with entries, weights rotating over more than L2; in brackets with one issuer, weights loaded behind
-// the predecessor and the cut tiles collected 16 tokens and one piece at a time: 8192->10240 at 32 tokens 16.0 / 20.1 (17.9 / 22.6),
-// 4096->22016 at 16 14.4 / 19.0 (16.1 / 21.1), 4096->4096 at 24 8.4 / 10.2 (10.6 / 12.4), 8192->57344 at 32 58 / 78 (59 / 88);
-// at 100 tokens on 28672->8192 47 / 73 as before: there the tensor pipe is full with both contractions (960 cycles a unit).
+// the predecessor and the cut tiles collected 16 tokens and one piece at a time: 8192->10240 at 32 tokens 16.0 / 20.3 (17.4 / 22.4),
+// 4096->22016 at 16 14.1 / 19.0 (16.1 / 20.8), 4096->4096 at 24 7.8 / 10.0 (10.6 / 12.1), 28672->8192 at 32 37 / 49 (41 / 52).
+// Above 64 tokens with entries on wide layers that form was faster by 1-3 % (4096->22016 at 96 37.3 / 36.6, 8192->28672 82 / 81).
+// Long calls run into the power cap: 28672->8192 at 100 tokens 46 / 73-78 for the first milliseconds at 1.9 GHz, 56 / 85 after that at
+// 1.43 GHz, of which the 97 units of both contractions (960 cycles each) take 47 and 65 with entries.
 // Replaces, for this token range, the reference's one-thread-per-output kernel (src/dual_gemm.cu:176-225) and its WMMA
 // variant (src/dual_gemm_tensor_core.cu:215-337).
 //

@@ -39,8 +39,9 @@ transpose_x_kernel(const __half *__restrict__ x, __half *__restrict__ xt, int M,
     }
 }
 
-// X of another type -> FP16, eight values a thread.  The kernel behind it is its programmatic dependent: it fetches its first weights
-// meanwhile.  11008 x 777 BF16: the separate conversions to FP16 and back, by element-wise kernels, took 20 of 95 us.
+// X of another type -> FP16, eight values a thread.  The kernel behind it is its programmatic dependent.  mid.cu fetches its first weights
+// meanwhile, where the conversion leaves an SM room for its threads (at most four blocks here per SM: M * K up to 1.2 million); wide.cu only
+// sets itself up and waits.  11008 x 777 BF16: the separate conversions to FP16 and back, by element-wise kernels, took 20 of 95 us.
 __global__ void __launch_bounds__(256)
 convert_x_kernel(const void *__restrict__ x, int type, uint4 *__restrict__ out, int64_t n8)
 {

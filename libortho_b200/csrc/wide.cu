@@ -218,7 +218,8 @@ wide_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sm->tmem_base;
-    // programmatic dependent launch, as in mid.cu
+    // programmatic dependent launch: barriers, tensor memory and descriptors are set up beside the predecessor's tail; nothing is loaded
+    // before its end
     if (!SPARSE || p.n_long == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool dead = false;
