@@ -40,6 +40,7 @@ struct Record {
     int device;
     int type;                                    // ORTHO_B200_TYPE_* of activations and output
     bool converts;                               // activations of another type that the kernel needs as FP16
+    bool takes;                                  // no: the kernel does not take that type, the FP16 record converts around
 };
 const char *kBuffers[5] = {"base_weight", "base_scales", "ortho_values", "ortho_col_indices", "ortho_row_ptr"};
 PyObject *s_buffers[5], *s_bias, *s_gen, *s_tensor, *s_handle, *s_value, *s_fast;
@@ -79,7 +80,8 @@ bool same_buffers(const Record &r, PyObject *buffers, PyObject *params)
     return t.has_storage() && t.scalar_type() == at::kFloat && t.const_data_ptr() == r.bias;
 }
 
-// record(desc_address, plan or None, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, converts) -> capsule
+// record(desc_address, plan or None, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, converts) -> capsule.
+// converts: bytes of the FP16 copy, negative where the kernel does not take the type
 PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
     if (n != 12) { PyErr_SetString(PyExc_TypeError, "record takes 12 arguments"); return nullptr; }
@@ -101,7 +103,9 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
     r->ws_bytes = PyLong_AsLongLong(a[8]);
     r->device = (int)PyLong_AsLong(a[9]);
     r->type = (int)PyLong_AsLong(a[10]);
-    r->converts = PyObject_IsTrue(a[11]) == 1;
+    const int64_t converts = PyLong_AsLongLong(a[11]);
+    r->converts = converts > 0;
+    r->takes = converts >= 0;
     if (PyErr_Occurred()) return nullptr;
     PyObject *cap = PyCapsule_New(r.get(), "ortho_record", free_record);
     if (!cap) return nullptr;
@@ -109,6 +113,19 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
     r.release()->ws = Py_NewRef(a[5]);
     return cap;
     END_HANDLE_TH_ERRORS
+}
+
+// the record of a call, or None / nullptr (with an error set): a new reference
+PyObject *find_record(PyObject *bound, int64_t M, void *stream, int type)
+{
+    PyObject *key = type == ORTHO_B200_TYPE_F16 ? Py_BuildValue("(LK)", (long long)M, (unsigned long long)(uintptr_t)stream)
+                                                : Py_BuildValue("(LKi)", (long long)M, (unsigned long long)(uintptr_t)stream, type);
+    if (!key) return nullptr;
+    PyObject *b = PyDict_GetItemWithError(bound, key);
+    Py_DECREF(key);
+    if (b) return PyObject_GetAttr(b, s_fast);
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
 }
 
 // module(x, buffers, parameters, bound, alpha, in_features, out_features) -> output, an int status, or None
@@ -119,7 +136,7 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     const at::Tensor *x = plain(a[0]);
     if (!x || !x->is_contiguous() || x->dim() < 1) Py_RETURN_NONE;
     const auto dtype = x->scalar_type();
-    const int type = dtype == at::kHalf ? ORTHO_B200_TYPE_F16 : dtype == at::kBFloat16 ? ORTHO_B200_TYPE_BF16 : dtype == at::kFloat ? ORTHO_B200_TYPE_F32 : -1;
+    int type = dtype == at::kHalf ? ORTHO_B200_TYPE_F16 : dtype == at::kBFloat16 ? ORTHO_B200_TYPE_BF16 : dtype == at::kFloat ? ORTHO_B200_TYPE_F32 : -1;
     if (type < 0) Py_RETURN_NONE;
     // the kernels read 16 bytes at a time; the general code's conversion to FP16 is a copy that is aligned
     if (type != ORTHO_B200_TYPE_F16 && ((uintptr_t)x->const_data_ptr() & 15u) != 0) Py_RETURN_NONE;
@@ -131,22 +148,20 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     const int dev = x->get_device();
     if (c10::cuda::current_device() != dev) Py_RETURN_NONE;
     void *stream = (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-    PyObject *rec = nullptr;
-    {
-        PyObject *key = type == ORTHO_B200_TYPE_F16 ? Py_BuildValue("(LK)", (long long)M, (unsigned long long)(uintptr_t)stream)
-                                                    : Py_BuildValue("(LKi)", (long long)M, (unsigned long long)(uintptr_t)stream, type);
-        if (!key) return nullptr;
-        PyObject *b = PyDict_GetItemWithError(a[3], key);
-        Py_DECREF(key);
-        if (!b) Py_RETURN_NONE;
-        rec = PyObject_GetAttr(b, s_fast);
-        if (!rec) return nullptr;
+    std::unique_ptr<PyObject, void (*)(PyObject *)> hold_rec(nullptr, [](PyObject *o) { Py_XDECREF(o); });
+    Record *r = nullptr;
+    at::Tensor as_half;                          // activations that are converted around the FP16 forward
+    for (;;) {
+        hold_rec.reset(find_record(a[3], M, stream, type));
+        if (!hold_rec) return nullptr;
+        if (hold_rec.get() == Py_None) Py_RETURN_NONE;
+        r = static_cast<Record *>(PyCapsule_GetPointer(hold_rec.get(), "ortho_record"));
+        if (!r) { PyErr_Clear(); Py_RETURN_NONE; }
+        if (r->device != dev || r->type != type || (alpha > 0) != r->active || r->desc.N != N) Py_RETURN_NONE;
+        if (r->takes) break;
+        type = ORTHO_B200_TYPE_F16;              // (a record of that type takes it)
     }
-    std::unique_ptr<PyObject, void (*)(PyObject *)> hold_rec(rec, [](PyObject *o) { Py_DECREF(o); });
-    if (rec == Py_None) Py_RETURN_NONE;
-    Record *r = static_cast<Record *>(PyCapsule_GetPointer(rec, "ortho_record"));
-    if (!r) { PyErr_Clear(); Py_RETURN_NONE; }
-    if (r->device != dev || r->type != type || (alpha > 0) != r->active || r->desc.N != N || !same_buffers(*r, a[1], a[2])) Py_RETURN_NONE;
+    if (!same_buffers(*r, a[1], a[2])) Py_RETURN_NONE;
     // the scratch of the record, held over the launch whatever other threads bind meanwhile
     PyObject *scratch = nullptr;
     if (r->ws_bytes) {
@@ -158,11 +173,17 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
         if (!same || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) { Py_DECREF(scratch); Py_RETURN_NONE; }
     }
     std::unique_ptr<PyObject, void (*)(PyObject *)> hold_scratch(scratch, [](PyObject *o) { Py_XDECREF(o); });
+    const bool around = type == ORTHO_B200_TYPE_F16 && dtype != at::kHalf;
+    if (around) {
+        as_half = x->to(at::kHalf);
+        if (!as_half.has_storage() || as_half.unsafeGetTensorImpl()->is_python_dispatch()) Py_RETURN_NONE;
+        x = &as_half;
+    }
     at::Tensor y;
     {
         c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
         shape.back() = N;
-        y = at::empty(shape, at::TensorOptions().dtype(dtype).device(x->device()));
+        y = at::empty(shape, at::TensorOptions().dtype(x->scalar_type()).device(x->device()));
     }
     if (!y.has_storage() || y.unsafeGetTensorImpl()->is_python_dispatch()) Py_RETURN_NONE;
     ortho_b200_layer_desc d = r->desc;
@@ -185,6 +206,7 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     // do not take or that needs the FP16 copy this record has no room for.  It says so before it launches the forward.
     if (type != ORTHO_B200_TYPE_F16 && (st == ORTHO_B200_ERR_SHAPE || st == ORTHO_B200_ERR_ALIGN || st == ORTHO_B200_ERR_WORKSPACE)) Py_RETURN_NONE;
     if (st) return PyLong_FromLong(st);
+    if (around) y = y.to(dtype);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }

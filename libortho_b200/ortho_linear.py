@@ -234,7 +234,7 @@ class OrthoLinear(nn.Module):
 
     def _bind(self, M: int, dev: torch.device, stream: int, type: int = 0) -> Tuple[_Bound, Optional[torch.Tensor]]:
         """The call record and its scratch, which the caller holds until the launch.  `type`: of activations and output, the
-        library's number; other types than FP16 get a record whose `fast` is None where the kernel does not take them."""
+        library's number."""
         N, K = self.out_features, self.in_features
         bw, bs = self.base_weight, self.base_scales
         if bw.dtype != torch.uint8 or bs.dtype != torch.float16:
@@ -271,16 +271,16 @@ class OrthoLinear(nn.Module):
         b.ws, b.ws_gen, scratch = _SharedWorkspace.get(dev, need, stream)
         b.ws_ptr = scratch.data_ptr() if need else None
         b.ws_bytes = scratch.numel() if need else 0
-        convert = 0                            # bytes of the FP16 copy of other activations, a temporary of each call; -1: not taken
+        convert = 0                            # bytes of the FP16 copy of other activations, a temporary of each call; -1: converted around
         if type:
             d.alpha = float(self.alpha)
             convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, b.ws_ptr, b.ws_bytes)
         b.key = (self.alpha > 0, self._versions())
         # what the native path compares and launches; not for a bias that torch has to add
         b.fast = None
-        if (self.bias is None or b.fused_bias) and not (type and convert < 0):
+        if self.bias is None or b.fused_bias:
             b.fast = _lib.fast().record(ctypes.addressof(descs), plan, self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
-                                        b.ws_bytes, dev.index, type, convert > 0)
+                                        b.ws_bytes, dev.index, type, convert)
         if b.ws.shared:
             if len(self._bound) > 32:
                 self._bound.clear()
@@ -288,8 +288,9 @@ class OrthoLinear(nn.Module):
         return b, scratch
 
     def _bind_typed(self, x: torch.Tensor) -> bool:
-        """A record for activations of another type; False where one that fits is there already (the call is not a plain one), where
-        the kernel does not take them (alignment, too), and under capture (shared scratch): the general code converts then."""
+        """A record for activations of another type; False where one that fits is there already (the call is not a plain one, or the
+        FP16 record that it is converted around is missing), where they are not aligned, and under capture (shared scratch): the general
+        code converts then."""
         dev, K = x.device, self.in_features
         if (x.dim() < 1 or x.shape[-1] != K or x.numel() == 0 or not x.is_contiguous() or x.is_neg() or x.data_ptr() % 16
                 or torch.cuda.current_device() != dev.index or _capturing(dev)):
