@@ -107,9 +107,9 @@ def forward(q_weight: torch.Tensor, q_scales: torch.Tensor, ortho_values: torch.
             input: torch.Tensor, output: torch.Tensor, alpha: float,
             plan: Optional[Plan] = None, workspace: Optional[torch.Tensor] = None) -> None:
     """In-place ``output[M,N] = input[M,K] @ dequant(q_weight)^T + alpha * input @ W_ortho^T``."""
-    if input.is_cuda:                          # natively, when the arguments are plain and no scratch is needed
+    if input.is_cuda:                          # natively, when the arguments are plain
         st = _lib.fast().layers(((q_weight, q_scales, ortho_values, ortho_col_indices, ortho_row_ptr),), input, (output,), (alpha,),
-                                None, (plan,))
+                                None, (plan,), workspace)
         if st is not None:
             if st:
                 _lib.check(st, "ortho_b200_forward")
@@ -167,7 +167,7 @@ def forward_multi(layers, input: torch.Tensor, outputs, alphas=None, biases=None
     FP16 ``[M, N_l]`` tensors written in place.  Up to 16 tokens (K a multiple of 256) run as ONE kernel launch where
     that is faster than one per layer."""
     if input.is_cuda:                          # natively, as above
-        st = _lib.fast().layers(layers, input, outputs, alphas, biases, plans)
+        st = _lib.fast().layers(layers, input, outputs, alphas, biases, plans, workspace)
         if st is not None:
             if st:
                 _lib.check(st, "ortho_b200_forward_multi")

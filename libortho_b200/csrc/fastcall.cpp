@@ -253,11 +253,11 @@ bool layer(ortho_b200_layer_desc &d, PyObject *qw_, PyObject *qs_, PyObject *ov_
     return true;
 }
 
-// layers(list of 5-tuples, x, outputs, alphas, biases, plans): the launch, where no scratch is needed -> int status, or None.
-// alphas, biases and plans are lists / tuples or None.
+// layers(list of 5-tuples, x, outputs, alphas, biases, plans, workspace): the launch -> int status, or None.
+// alphas, biases and plans are lists / tuples or None; a workspace that is None or too small is replaced by a temporary.
 PyObject *layers_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 6) { PyErr_SetString(PyExc_TypeError, "layers takes 6 arguments"); return nullptr; }
+    if (n != 7) { PyErr_SetString(PyExc_TypeError, "layers takes 7 arguments"); return nullptr; }
     HANDLE_TH_ERRORS
     const at::Tensor *x = plain(a[1]);
     if (!x || x->scalar_type() != at::kHalf || x->dim() != 2 || !x->is_contiguous()) Py_RETURN_NONE;
@@ -283,12 +283,27 @@ PyObject *layers_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
             if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
         }
     }
-    if (multi_workspace(d, (int)nl, M, K) != 0) Py_RETURN_NONE;
+    const int64_t need = multi_workspace(d, (int)nl, M, K);
+    if (need < 0) Py_RETURN_NONE;
+    at::Tensor own;
+    void *ws = nullptr;
+    int64_t ws_bytes = 0;
+    if (need) {
+        const at::Tensor *given = a[6] == Py_None ? nullptr : plain(a[6]);
+        if (a[6] != Py_None && (!given || given->get_device() != dev)) Py_RETURN_NONE;
+        if (!given || (int64_t)given->nbytes() < need) {
+            own = at::empty({need}, at::TensorOptions().dtype(at::kByte).device(x->device()));
+            if (!own.has_storage() || own.unsafeGetTensorImpl()->is_python_dispatch()) Py_RETURN_NONE;
+            given = &own;
+        }
+        ws = given->mutable_data_ptr();
+        ws_bytes = (int64_t)given->nbytes();
+    }
     const void *xp = x->const_data_ptr();
     void *stream = (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
     int st;
     Py_BEGIN_ALLOW_THREADS
-    st = forward_multi(d, (int)nl, xp, M, K, nullptr, 0, stream);
+    st = forward_multi(d, (int)nl, xp, M, K, ws, ws_bytes, stream);
     Py_END_ALLOW_THREADS
     return PyLong_FromLong(st);
     END_HANDLE_TH_ERRORS
