@@ -134,12 +134,13 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     if (n != 7) { PyErr_SetString(PyExc_TypeError, "module takes 7 arguments"); return nullptr; }
     HANDLE_TH_ERRORS
     const at::Tensor *x = plain(a[0]);
-    if (!x || !x->is_contiguous() || x->dim() < 1) Py_RETURN_NONE;
+    if (!x || x->dim() < 1) Py_RETURN_NONE;
     const auto dtype = x->scalar_type();
     int type = dtype == at::kHalf ? ORTHO_B200_TYPE_F16 : dtype == at::kBFloat16 ? ORTHO_B200_TYPE_BF16 : dtype == at::kFloat ? ORTHO_B200_TYPE_F32 : -1;
     if (type < 0) Py_RETURN_NONE;
-    // the kernels read 16 bytes at a time; the general code's conversion to FP16 is a copy that is aligned
-    if (type != ORTHO_B200_TYPE_F16 && ((uintptr_t)x->const_data_ptr() & 15u) != 0) Py_RETURN_NONE;
+    // the kernels read rows that follow one another, 16 bytes at a time; an FP16 copy of other activations is contiguous and aligned
+    const bool in_order = x->is_contiguous();
+    if (type != ORTHO_B200_TYPE_F16 && (!in_order || ((uintptr_t)x->const_data_ptr() & 15u) != 0)) type = ORTHO_B200_TYPE_F16;
     const int64_t K = PyLong_AsLongLong(a[5]), N = PyLong_AsLongLong(a[6]);
     const double alpha = PyFloat_AsDouble(a[4]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
@@ -150,7 +151,7 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     void *stream = (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
     std::unique_ptr<PyObject, void (*)(PyObject *)> hold_rec(nullptr, [](PyObject *o) { Py_XDECREF(o); });
     Record *r = nullptr;
-    at::Tensor as_half;                          // activations that are converted around the FP16 forward
+    at::Tensor as_half;                          // the FP16 copy of activations that are converted around the FP16 forward
     for (;;) {
         hold_rec.reset(find_record(a[3], M, stream, type));
         if (!hold_rec) return nullptr;
@@ -174,8 +175,8 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     }
     std::unique_ptr<PyObject, void (*)(PyObject *)> hold_scratch(scratch, [](PyObject *o) { Py_XDECREF(o); });
     const bool around = type == ORTHO_B200_TYPE_F16 && dtype != at::kHalf;
-    if (around) {
-        as_half = x->to(at::kHalf);
+    if (around || !in_order) {
+        as_half = x->to(at::kHalf).contiguous();
         if (!as_half.has_storage() || as_half.unsafeGetTensorImpl()->is_python_dispatch()) Py_RETURN_NONE;
         x = &as_half;
     }
