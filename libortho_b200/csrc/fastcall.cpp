@@ -31,7 +31,8 @@ struct Record {
     ortho_b200_layer_desc desc;
     Ptr buf[5];                                  // base_weight, base_scales, ortho_values, ortho_col_indices, ortho_row_ptr
     const void *bias;
-    bool has_bias, active;                       // active: alpha > 0
+    int bias_type;
+    bool has_bias, add_bias, active;             // add_bias: not one that the kernel adds; active: alpha > 0
     int64_t ws_bytes;
     void *ws_ptr;
     int64_t ws_gen;
@@ -77,7 +78,8 @@ bool same_buffers(const Record &r, PyObject *buffers, PyObject *params)
     if (b == Py_None) return !r.has_bias;
     if (!r.has_bias || !THPVariable_Check(b)) return false;
     const at::Tensor &t = THPVariable_Unpack(b);
-    return t.has_storage() && t.scalar_type() == at::kFloat && t.const_data_ptr() == r.bias;
+    if (r.add_bias && (!plain(b) || t.dim() != 1)) return false;
+    return t.has_storage() && (int)t.scalar_type() == r.bias_type && t.const_data_ptr() == r.bias;
 }
 
 // record(desc_address, plan or None, buffers, bias or None, active, ws, ws_gen, ws_ptr, ws_bytes, device, type, converts) -> capsule.
@@ -96,7 +98,13 @@ PyObject *make_record(PyObject *, PyObject *const *a, Py_ssize_t n)
         r->buf[i] = Ptr{t.const_data_ptr(), i >= 2 ? (int64_t)t._version() : 0};
     }
     r->has_bias = a[3] != Py_None;
-    if (r->has_bias) r->bias = THPVariable_Unpack(a[3]).const_data_ptr();
+    if (r->has_bias) {
+        if (!r->desc.bias_f32 && !plain(a[3])) Py_RETURN_NONE;
+        const at::Tensor &b = THPVariable_Unpack(a[3]);
+        r->bias = b.const_data_ptr();
+        r->bias_type = (int)b.scalar_type();
+        r->add_bias = !r->desc.bias_f32;
+    }
     r->active = PyObject_IsTrue(a[4]) == 1;
     r->ws_gen = PyLong_AsLongLong(a[6]);
     r->ws_ptr = a[7] == Py_None ? nullptr : PyLong_AsVoidPtr(a[7]);
@@ -163,6 +171,8 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
         type = ORTHO_B200_TYPE_F16;              // (a record of that type takes it)
     }
     if (!same_buffers(*r, a[1], a[2])) Py_RETURN_NONE;
+    at::Tensor bias;                             // in hand, whatever other threads replace during the launch
+    if (r->add_bias) bias = THPVariable_Unpack(PyDict_GetItemWithError(a[2], s_bias));
     // the scratch of the record, held over the launch whatever other threads bind meanwhile
     PyObject *scratch = nullptr;
     if (r->ws_bytes) {
@@ -207,6 +217,7 @@ PyObject *module_forward(PyObject *, PyObject *const *a, Py_ssize_t n)
     // do not take or that needs the FP16 copy this record has no room for.  It says so before it launches the forward.
     if (type != ORTHO_B200_TYPE_F16 && (st == ORTHO_B200_ERR_SHAPE || st == ORTHO_B200_ERR_ALIGN || st == ORTHO_B200_ERR_WORKSPACE)) Py_RETURN_NONE;
     if (st) return PyLong_FromLong(st);
+    if (bias.defined()) y.add_(bias);
     if (around) y = y.to(dtype);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS

@@ -272,15 +272,15 @@ class OrthoLinear(nn.Module):
         b.ws_ptr = scratch.data_ptr() if need else None
         b.ws_bytes = scratch.numel() if need else 0
         convert = 0                            # bytes of the FP16 copy of other activations, a temporary of each call; -1: converted around
-        if type:
+        if type and self.bias is not None and not b.fused_bias:          # added in FP16, before the conversion
+            convert = -1
+        elif type:
             d.alpha = float(self.alpha)
             convert = _lib.lib().ortho_b200_typed_scratch_bytes(descs, M, K, b.ws_ptr, b.ws_bytes)
         b.key = (self.alpha > 0, self._versions())
-        # what the native path compares and launches; not for a bias that torch has to add
-        b.fast = None
-        if self.bias is None or b.fused_bias:
-            b.fast = _lib.fast().record(ctypes.addressof(descs), plan, self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
-                                        b.ws_bytes, dev.index, type, convert)
+        # what the native path compares and launches
+        b.fast = _lib.fast().record(ctypes.addressof(descs), plan, self._buffers, self.bias, self.alpha > 0, b.ws, b.ws_gen, b.ws_ptr,
+                                    b.ws_bytes, dev.index, type, convert)
         if b.ws.shared:
             if len(self._bound) > 32:
                 self._bound.clear()
@@ -297,8 +297,6 @@ class OrthoLinear(nn.Module):
             return False
         M, stream = x.numel() // K, _current_stream_handle(dev)
         b = self._bound.get((M, stream, _TYPES[x.dtype]))
-        if b is not None and b.fast is None and b.key[0] == (self.alpha > 0):
-            return False
         if b is not None and b.key == (self.alpha > 0, self._versions()) and b.ws_gen == b.ws.gen:
             return False
         return self._bind(M, dev, stream, _TYPES[x.dtype])[0].fast is not None
