@@ -17,7 +17,8 @@
 // One B200, us, base-only / with entries, weights rotating over more than L2; in brackets with one issuer, weights loaded behind
 // the predecessor and the cut tiles collected 16 tokens and one piece at a time: 8192->10240 at 32 tokens 16.0 / 20.3 (17.4 / 22.4),
 // 4096->22016 at 16 14.1 / 19.0 (16.1 / 20.8), 4096->4096 at 24 7.8 / 10.0 (10.6 / 12.1), 28672->8192 at 32 37 / 49 (41 / 52).
-// Above 64 tokens with entries on wide layers that form was faster by 1-3 % (4096->22016 at 96 37.3 / 36.6, 8192->28672 82 / 81).
+// 33 tokens on with entries, as 65 on without, one issuer is enough: 4096->22016 with 0.5 % at 48 / 96 / 128 24.3 / 35 / 43 (27.5 / 36 / 43),
+// 4096->4096 at 64 / 128 11.8 / 15.7 (13.4 / 17.3).
 // Long calls run into the power cap: 28672->8192 at 100 tokens 46 / 73-78 for the first milliseconds at 1.9 GHz, 56 / 85 after that at
 // 1.43 GHz, of which the 97 units of both contractions (960 cycles each) take 47 and 65 with entries.
 // Replaces, for this token range, the reference's one-thread-per-output kernel (src/dual_gemm.cu:176-225) and its WMMA
@@ -148,8 +149,8 @@ struct Pieces {
 
 // SPARSE: the entries of an ordered plan are contracted from the scattered tiles; at most 4 stages then.  TYPED: y is of another type
 // than FP16 (an instantiation of its own: the branch cost the others 1-2 %).  ISSUERS: threads that issue MMAs; with the number as a
-// parameter of the launch, calls of one issuer paid for the second one's code: 4096->22016 with 0.5 % at 80 / 96 / 128 tokens 35.0 / 37.9 /
-// 45.5 us against 34.5 / 37.3 / 44.8, 4096->4096 at 64 / 128 tokens 12.5 / 16.6 against 12.2 / 16.3.
+// parameter of the launch, calls of one issuer paid for the second one's code (4096->22016 with 0.5 % at 96 / 128 tokens 37.9 / 45.5 us
+// against 37.3 / 44.8) and had its narrow epilogue.
 template <bool SPARSE, bool TYPED, int ISSUERS>
 __global__ void __launch_bounds__(md::kWarps<SPARSE, ISSUERS> * 32, 1)
 mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const md::Params p)
@@ -410,7 +411,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
         }
         }
         // The CTA's last piece is finished by the converters too, which have nothing left to do: five sets of four warps take
-        // every fifth chunk of 8 tokens.  (Collecting the other pieces of a cut tile is a chain of loads from L2 per chunk: by
+        // every fifth chunk of tokens.  (Collecting the other pieces of a cut tile is a chain of loads from L2 per chunk: by
         // the four epilogue warps alone it took 15-25 us at the end of a forward.)
         // ================= epilogue: TMEM -> (+ partials) -> scale, sparse term, bias -> FP16 -> global =================
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -457,43 +458,55 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * p.acc_cols);
-            // scale * D + bias (+ alpha * E) of 8 tokens.  The zeros of the scattered tile times an infinite activation make E
-            // NaN for every row: such a sum is taken again from the row's entries in this piece.
-            auto columns8 = [&](uint32_t col, float (&v)[8]) {            // 8 accumulator columns, of both issuers
-                uint32_t r[8];
-                tmem_ld_32x32b_x8(taddr + d_off + col, r);
+            // scale * D + bias (+ alpha * E) of C tokens.  The zeros of the scattered tile times an infinite activation make E NaN for every
+            // row: such a sum is taken again from the row's entries in this piece.
+            // One issuer: 16 columns, of both accumulators under one wait.  Short rows are bound by this: 512->38230 with 1 % at 67 / 100 /
+            // 128 tokens 13.6 / 16.9 / 18.7 us against 17.2 / 21.7 / 24.2 with 8 columns and a wait each, base-only 9.5 / 11.9 / 12.5 against
+            // 10.6 / 12.8 / 13.8; 4096->22016 at 96 34.9 / 37.2.  (Tiles cut eight times lose at 81-112 tokens, where 16 columns divide
+            // less evenly over the sets: 8192->2048 at 100 17.6 against 16.4.)  Two issuers' four accumulators: registers for 8.
+            constexpr int C = ISSUERS == 2 ? 8 : 16;
+            auto columns = [&](uint32_t col, uint32_t (&r)[C]) {          // C accumulator columns, once tmem_ld_wait has been called
+                if constexpr (C == 8) tmem_ld_32x32b_x8(taddr + col, r); else tmem_ld_32x32b_x16(taddr + col, r);
+            };
+            auto both_columns = [&](uint32_t col, uint32_t (&r)[C]) {     // two issuers: of both
+                columns(d_off + col, r);
                 tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = __uint_as_float(r[j]);
                 if (both) {
-                    tmem_ld_32x32b_x8(taddr + own_cols + col, r);
+                    uint32_t r2[C];
+                    columns(own_cols + col, r2);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] += __uint_as_float(r[j]);
+                    for (int j = 0; j < C; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
                 }
             };
-            auto load8 = [&](int c, float (&v)[8]) {
-                columns8((uint32_t)c, v);
+            auto load = [&](int c, float (&v)[C]) {
+                uint32_t r[C], e[SPARSE ? C : 1];
+                if constexpr (ISSUERS == 2) {
+                    both_columns((uint32_t)c, r);
+                } else {
+                    columns((uint32_t)c, r);
+                    if constexpr (SPARSE) columns((uint32_t)(p.nt32 + c), e);
+                    tmem_ld_wait();
+                }
 #pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = fmaf(v[j], sc, bs);
+                for (int j = 0; j < C; j++) v[j] = fmaf(__uint_as_float(r[j]), sc, bs);
                 if constexpr (SPARSE) {
-                    float e[8];
-                    columns8((uint32_t)(p.nt32 + c), e);
+                    if constexpr (ISSUERS == 2) both_columns((uint32_t)(p.nt32 + c), e);
                     bool nan = false;
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        v[j] = fmaf(p.alpha, e[j], v[j]);
+                    for (int j = 0; j < C; j++) {
+                        v[j] = fmaf(p.alpha, __uint_as_float(e[j]), v[j]);
                         nan = nan || v[j] != v[j];
                     }
                     if (__any_sync(0xffffffffu, nan)) {
                         uint32_t bad = 0;
 #pragma unroll
-                        for (int j = 0; j < 8; j++) bad |= v[j] != v[j] ? 1u << j : 0u;
+                        for (int j = 0; j < C; j++) bad |= v[j] != v[j] ? 1u << j : 0u;
                         int e0 = 0, e1 = 0;
                         if (n_ok) { e0 = p.row_ptr[n]; e1 = p.row_ptr[n + 1]; } else bad = 0;
                         if (p.n_long > 0 && e1 - e0 > p.heavy) e1 = e0;               // a long row is not listed
 #pragma unroll 1
-                        for (int j = 0; j < 8 && c + j < p.M; j++) {
+                        for (int j = 0; j < C && c + j < p.M; j++) {
                             uint32_t d, d2 = 0;
                             __syncwarp();
                             tmem_ld_32x32b_x1(taddr + d_off + (uint32_t)(c + j), d);
@@ -504,7 +517,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                             const float base = both ? __uint_as_float(d) + __uint_as_float(d2) : __uint_as_float(d);
                             const float t = fmaf(p.alpha, es, fmaf(base, sc, bs));
 #pragma unroll
-                            for (int i = 0; i < 8; i++) v[i] = i == j ? t : v[i];
+                            for (int i = 0; i < C; i++) v[i] = i == j ? t : v[i];
                         }
                         __syncwarp();
                     }
@@ -513,12 +526,12 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
             if (!owner) {
                 // the first piece of a share that starts inside a tile: its FP32 sums to this CTA's slot, then the flag.  One fence
                 // behind the barrier covers every thread's stores.
-                float *dst = p.slots + ((size_t)cta * p.nt + set * 8) * TN + q * 32 + lane;
-                for (int c = set * 8; c < p.nt; c += sets * 8, dst += sets * 8 * TN) {
-                    float v[8];
-                    load8(c, v);
+                float *dst = p.slots + ((size_t)cta * p.nt + set * C) * TN + q * 32 + lane;
+                for (int c = set * C; c < p.nt; c += sets * C, dst += sets * C * TN) {
+                    float v[C];
+                    load(c, v);
 #pragma unroll
-                    for (int j = 0; j < 8; j++) dst[j * TN] = v[j];
+                    for (int j = 0; j < C; j++) dst[j * TN] = v[j];
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -544,46 +557,49 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 if (!ok) { dead = true; atomicExch(p.status, 1); }
                 dead = __any_sync(0xffffffffu, dead);
             }
-            const float *part = p.slots + ((size_t)(cta + 1) * p.nt + set * 8) * TN + q * 32 + lane;
+            const float *part = p.slots + ((size_t)(cta + 1) * p.nt + set * C) * TN + q * 32 + lane;
             const size_t part_cta = (size_t)p.nt * TN;
-            constexpr int FLY = SPARSE ? 1 : 3;          // pieces in flight (registers)
-            for (int c = set * 8; c < p.nt; c += sets * 8, part += sets * 8 * TN) {
+            constexpr int H = SPARSE ? C : 8, FLY = SPARSE ? 1 : 3;     // tokens and pieces in flight (registers)
+            for (int c = set * C; c < p.nt; c += sets * C, part += sets * C * TN) {
                 __syncwarp();
-                float v[8];
-                load8(c, v);
-                const float *src = part;
-                for (int cc = cta + 1; cc <= c_last; cc += FLY, src += FLY * part_cta) {     // the other pieces of the tile, in CTA order
-                    float t[FLY][8];
+                float v[C];
+                load(c, v);
 #pragma unroll
-                    for (int i = 0; i < FLY; i++)
-                        if (cc + i <= c_last) {
+                for (int h = 0; h < C; h += H) {
+                    const float *src = part + h * TN;
+                    for (int cc = cta + 1; cc <= c_last; cc += FLY, src += FLY * part_cta) { // the other pieces of the tile, in CTA order
+                        float t[FLY][H];
 #pragma unroll
-                            for (int j = 0; j < 8; j++) t[i][j] = __ldcg(src + i * part_cta + j * TN);
-                        }
+                        for (int i = 0; i < FLY; i++)
+                            if (cc + i <= c_last) {
 #pragma unroll
-                    for (int i = 0; i < FLY; i++)
-                        if (cc + i <= c_last) {
+                                for (int j = 0; j < H; j++) t[i][j] = __ldcg(src + i * part_cta + j * TN);
+                            }
 #pragma unroll
-                            for (int j = 0; j < 8; j++) v[j] += t[i][j];
-                        }
+                        for (int i = 0; i < FLY; i++)
+                            if (cc + i <= c_last) {
+#pragma unroll
+                                for (int j = 0; j < H; j++) v[h + j] += t[i][j];
+                            }
+                    }
                 }
                 if (longs && li >= 0) {                           // a long row's sums from the pre-pass
                     const float4 *o4 = reinterpret_cast<const float4 *>(p.ol + (size_t)li * p.ol_mp + c);
 #pragma unroll
-                    for (int j = 0; j < 2; j++) {
+                    for (int j = 0; j < C / 4; j++) {
                         const float4 t = __ldcg(o4 + j);
                         v[4 * j] = fmaf(p.alpha, t.x, v[4 * j]); v[4 * j + 1] = fmaf(p.alpha, t.y, v[4 * j + 1]);
                         v[4 * j + 2] = fmaf(p.alpha, t.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(p.alpha, t.w, v[4 * j + 3]);
                     }
                 }
                 if (TYPED && plain) {
-                    store_column<8>(p.y, (size_t)c * (size_t)p.ldy + n, p.ldy, p.y_type, p.M - c, n_ok, [&](int j) { return v[j]; });
+                    store_column<C>(p.y, (size_t)c * (size_t)p.ldy + n, p.ldy, p.y_type, p.M - c, n_ok, [&](int j) { return v[j]; });
                     continue;
                 }
                 if (plain) {
                     __half *yp = p.y + (size_t)c * (size_t)p.ldy + n;
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
+                    for (int j = 0; j < C; j++) {
                         if (n_ok && c + j < p.M) *yp = __float2half_rn(v[j]);
                         yp += p.ldy;
                     }
@@ -591,7 +607,7 @@ mid_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUt
                 }
                 if (!n_ok) continue;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
+                for (int j = 0; j < C; j++) {
                     const int m = c + j;
                     if (m >= p.M) break;
                     float o = v[j];
