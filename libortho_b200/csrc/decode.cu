@@ -314,6 +314,8 @@ bool decode_regime(int64_t M, int64_t N, int64_t K) { return decode_regime_of(tu
 //    6 tokens: 4096->22016 15.3 / 14.9; 20.6 / 20.0, 8192->8192 13.2 / 14.0; 17.1 / 17.8, 8192->10240 15.9 / 15.8; 20.6 / 20.2,
 //              8192->28672 37.6 / 29.8; 50.3 / 40.8, 14336->4096 16.1 / 13.4; 20.0 / 16.5
 //    5 tokens: 8192->28672 31.8 / 29.8; 40.0 / 40.9, 14336->4096 13.7 / 13.4; 16.1 / 16.6, 28672->8192 41.2 / 31.7; 52.9 / 42.2
+//   and with 0.3 %, short rows (rounds of row tiles, each with its own sums and entries): 512->33200 at 9 / 16 21.0 / 7.7 and 22.2 / 7.8,
+//              1024->16592 13.1 / 7.1 and 14.7 / 7.1, 2048->8288 9.7 / 8.9 and 11.3 / 9.3, 3072->5520 at 16 12.7 / 10.0, 4096->4880 at 9 12.0 / 10.4
 //    3 tokens: 8192->28672 31.1 / 29.8; 37.1 / 40.9, 28672->8192 36.1 / 31.5; 42.2 / 42.2, 4096->22016 14.4 / 14.9; 18.6 / 20.0
 static bool mid_beats_stream(int64_t M, int64_t N, int64_t K, bool base)
 {
@@ -323,7 +325,7 @@ static bool mid_beats_stream(int64_t M, int64_t N, int64_t K, bool base)
         if (weights < (int64_t)1 << 24) return false;
         if (odd) return weights > (int64_t)1 << 24;
         if (base) return slab > (100 << 10) || M >= 12 || weights >= (int64_t)5 << 23;
-        if (slab <= (100 << 10)) return weights >= (int64_t)3 << 23;
+        if (slab <= (100 << 10)) return weights >= (int64_t)3 << 23 || N > 2 * 148 * 16;     // more than a round of row tiles
         return slab > (200 << 10) || N > 2048 || K <= 8192;
     }
     if (weights < (int64_t)5 << 23) return false;
