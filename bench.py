@@ -759,7 +759,7 @@ def run_report(args):
     sep = "|" + "---|" * 11
     out = ["# All configurations, one B200 (`python bench.py --report <path>`)", "", head, sep, *rows, "",
            "CPU rows (host of the same box):", "", head + " note |", sep + "---|", *cpu, "",
-           "Device-side packer (algorithmic bytes: W read once + outputs; the CSR build reads W twice; includes the host "
+           "Device-side packer (algorithmic bytes: W read once + outputs; the CSR build reads W twice where more than one weight in sixteen is non-zero; includes the host "
            "read-back of nnz and the output allocations):", "",
            "| step | input | us | GB/s | % of measured HBM |", "|---|---|---|---|---|", *pack_rows, ""]
     with open(args.report, "w") as f:
